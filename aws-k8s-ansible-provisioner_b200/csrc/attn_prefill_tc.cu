@@ -20,13 +20,13 @@
 // What bounds it: per unit and key tile the MMAs take about 1 050 cycles and the exponentials 1 024 (16 a cycle and SM).  The two units
 // take turns: while one's threads form its probabilities, the tensor cores run the other's products, and the next key tiles
 // are already landing in the other stage of K and V -- the issue order is P.V(A, t), S(A, t + 1), P.V(B, t), S(B, t + 1), P.V of a tile's
-// first half as soon as its P stands.  A pair of tiles then takes about 4 000 cycles: a unit's threads work 2 230 of them (1 350 in the exponentials) and wait
+// first half as soon as its P stands.  S(t + 1) takes the columns of P(t): it is issued once P.V(t), which reads them, has ended (only
+// MMAs on one accumulator are ordered by themselves).  A pair of tiles then takes about 4 000 cycles: a unit's threads work 2 230 of them (1 350 in the exponentials) and wait
 // for P.V and S of theirs behind the other unit's.  Measured at 12 prompts of 133 to 4096 tokens, 16 heads, per layer:
 //   one unit per CTA, two CTAs per SM, K / P and V in single buffers, every step of a key tile behind the one before     737 us
 //   two units, two passes over S in TMEM                                                                                 633 us
 //   two units, two threads per row (four softmax warps a scheduler get in one another's way: 3 060 cycles a tile)        532 us
-//   two units, S of 64 keys, two of them per unit in TMEM (MMAs of different shapes are not ordered among each other, so that
-//     the next S must wait for P.V to END before it may take P's columns; a 64-key S costs 0.75 of a 128-key one)        725 us
+//   two units, S of 64 keys, two of them per unit in TMEM (a 64-key S costs 0.75 of a 128-key one)                       725 us
 //   this form                                                                                                            516 us
 // Where a launch has no more units than SMs, one unit per CTA (96 KB, two CTAs fit an SM) ends sooner: 128 tokens, 16 heads: 8.0 -> 6.7 us.
 //
@@ -307,15 +307,13 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
               if (half == 0) tc_commit(smem_u32(&o_half[u]));
             }
             if (u == last) tc_commit(smem_u32(&v_free[n % C::VS]));
-            if (t + 1 < tiles) {   // the next S takes this P's place: MMAs of one shape run in the order of their issue
-              if (u == 0) {
-                pt_wait(k_full[(n + 1) % C::KS], ((n + 1) / C::KS) & 1);
-                tc_fence_after();
-              }
+            tc_commit(smem_u32(&o_full[u]));
+            if (t + 1 < tiles) {   // the next S takes this P's place, which P.V still reads: MMAs on different accumulators have no order by themselves
+              if (u == 0) pt_wait(k_full[(n + 1) % C::KS], ((n + 1) / C::KS) & 1);
+              pt_wait(o_full[u], n & 1);
+              tc_fence_after();
               scores(u, n + 1);
               if (u == last) tc_commit(smem_u32(&k_free[(n + 1) % C::KS]));
-            } else {
-              tc_commit(smem_u32(&o_full[u]));
             }
           }
         }
@@ -326,7 +324,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     const int u = warp >> 2, r = threadIdx.x & 127, t = r & 63;
     const int h = a.pair_mode ? 0 : r >> 6;
     const uint32_t srow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 128u * u, orow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + C::O_COL + 128u * u;
-    int n = 0, ni = 0;   // key tiles and items of this unit so far
+    int n = 0;   // key tiles of this unit so far
     for (int i = 0; i < n_items; ++i) {
       const Item it = item_of(i);
       if (u == 1 && it.u[1] < 0) continue;
@@ -445,8 +443,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       float l_row = (l_0.x + l_0.y) + (l_1.x + l_1.y);
       if (a.sink != nullptr && m_ref > -INFINITY) l_row += exp2f(a.sink[kvh * a.head_step + h] * 1.4426950408889634f - m_ref);
       const float inv = l_row > 0.f ? __fdiv_rn(1.0f, l_row) : 0.f;
-      pt_wait(o_full[u], ni & 1);
-      ++ni;
+      pt_wait(o_full[u], (n - 1) & 1);   // the last tile's P.V
       tc_fence_after();
       bf16* dst = a.out + ((size_t)(mt.q_row0 + t) * a.nq + kvh * a.head_step + h) * PT_HD;
 #pragma unroll 1

@@ -738,3 +738,30 @@ def test_attn_prefill_two_units_per_cta(lib, qscale):
         ref = p @ v64
         worst = ((got[0].cuda().double() - ref).abs() / ((2.0 ** -8 + 2.0 ** -9) * (p @ v64.abs()) + 2.0 ** -8 * ref.abs() + 1e-6)).max().item()
         assert worst <= 1.0, "seq %d: %.3g of the bound" % (i, worst)
+
+
+def prefill(lib, q, kp, vp, bt, pos0, ntok, rows, nq, nkv):
+    """b2k_attn_prefill over sequences of 128-wide heads whose tokens lie one behind another in q."""
+    I32 = lambda v: (C.c_int32 * len(v))(*v)
+    out = torch.full((sum(ntok), nq * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    chk(lib, lib.b2k_attn_prefill(ptr(q), ptr(kp), ptr(vp), ptr(bt), bt.shape[1], I32([sum(ntok[:i]) for i in range(len(ntok))]), I32(pos0), I32(ntok), I32(rows),
+                                 len(ntok), ptr(out), nq, nkv, 128, 16, cuda_stream_ptr()))
+    return out
+
+
+def test_attn_prefill_repeats_itself(lib):
+    """The next key tile's scores take the place of the weights that the tensor cores still multiply: they wait for them.  Contexts of many key tiles, one and two units to
+    a CTA: every launch gives the same bits, and so does a sequence by itself."""
+    nq, nkv = 8, 4
+    pos0, ntok = [0, 2900, 1500], [1700, 200, 1000]
+    bt, kp, vp, _, _ = build_pages([p + n for p, n in zip(pos0, ntok)], nkv, 128, 16, seed=50)
+    q, kp, vp, bt = dv(bf(sum(ntok), nq * 128, scale=3.0, seed=51)), dv(kp), dv(vp), dv(bt)
+    assert sum((n + 63) // 64 for n in ntok) * nkv > 148 >= (ntok[0] + 63) // 64 * nkv
+    out = prefill(lib, q, kp, vp, bt, pos0, ntok, [0, 1, 2], nq, nkv)
+    for _ in range(20):
+        assert torch.equal(out, prefill(lib, q, kp, vp, bt, pos0, ntok, [0, 1, 2], nq, nkv))
+    at = 0
+    for i, n in enumerate(ntok):
+        for _ in range(5):
+            assert torch.equal(out[at:at + n], prefill(lib, q[at:at + n], kp, vp, bt, [pos0[i]], [n], [i], nq, nkv))
+        at += n
