@@ -130,12 +130,6 @@ __device__ __forceinline__ void pt_ld16(uint32_t taddr, uint32_t (&r)[16]) {   /
                : "r"(taddr)
                : "memory");
 }
-// (a wait that never ends would hold the GPU: after some seconds the kernel goes on and ends with wrong numbers instead)
-__device__ __forceinline__ void pt_wait(uint64_t& bar, uint32_t parity) {
-  const uint32_t b = smem_u32(&bar);
-  for (int i = 0; i < (1 << 22) && !mbar_try_wait(b, parity); ++i) {
-  }
-}
 constexpr uint32_t PT_IDESC_QK = umma_idesc_bf16(PT_M, PT_BN);                // both operands K-major
 constexpr uint32_t PT_IDESC_PV = umma_idesc_bf16(PT_M, PT_HD) | (1u << 16);  // B (V) MN-major
 
@@ -155,6 +149,7 @@ struct PtArgs {
   const float* q_rot;      // [tokens][heads][rot_dim]
   int rot_dim;
   const float* sink;       // [heads] or null
+  B2WaitLimit wait;
 };
 
 template <int NK, int NU>
@@ -167,7 +162,10 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + (base - smem_u32(smem_raw)) + C::BAR_OFF);
   // per unit: q_full, s_full, o_half (P.V of a tile's first half has landed), o_full; per unit and half: p_full; per stage: k / v full and free
   uint64_t *q_full = bars, *s_full = bars + 2, *o_half = bars + 4, *o_full = bars + 6, *p_full = bars + 8, *k_full = bars + 12, *k_free = bars + 14, *v_full = bars + 16, *v_free = bars + 18;
-  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 20);
+  uint64_t& drained = bars[20];
+  uint32_t& tmem_slot = *reinterpret_cast<uint32_t*>(bars + 21);
+  volatile uint32_t& gave_up = *reinterpret_cast<volatile uint32_t*>(bars + 22);
+  const B2Waits wait{&gave_up, a.wait};
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int kvh = blockIdx.y;
   if (threadIdx.x == 0) {
@@ -182,6 +180,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       mbar_init(smem_u32(&v_free[i]), 1);
     }
     for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&p_full[i]), PT_M);
+    mbar_init(smem_u32(&drained), 1);
+    gave_up = 0;
     mbar_fence_init();
   }
   // All 512 columns (two units) are taken only when every CTA of the kernel in front has ended, and before the kernel behind may start its CTAs
@@ -232,7 +232,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     return it;
   };
 
-  if (warp > C::MMA_WARP) {
+  int k_sent = 0, v_sent = 0;   // (loaders: key tiles whose pages this warp has asked for)
+  auto load_tiles = [&]() {
     // ---- loaders: each takes three (the last: two) of a key tile's eight pages; a tile's K goes out one tile ahead of its V ----
     const int j = warp - C::MMA_WARP - 1, p0 = 3 * j, np = min(3, 8 - p0);
     int n = 0;   // key tiles so far
@@ -244,7 +245,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       };
       auto load = [&](bool is_v, int kn, int ids) {
         const int stages = is_v ? C::VS : C::KS, st = kn % stages;
-        if (kn >= stages) pt_wait(is_v ? v_free[st] : k_free[st], (kn / stages - 1) & 1);
+        if (kn >= stages && !wait.warp(is_v ? v_free[st] : k_free[st], (kn / stages - 1) & 1)) return false;
         const uint32_t fb = smem_u32(is_v ? &v_full[st] : &k_full[st]);
         const uint32_t dst = (is_v ? v_s + st * C::V_BYTES : k_s + st * C::K_BYTES) + (uint32_t)(p0 * 16 * 128);
         if (lane == 0 && j == 0) mbar_arrive_expect_tx(fb, is_v ? C::V_BYTES : C::K_BYTES);  // the other warps only add bytes
@@ -260,66 +261,69 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           }
         }
         __syncwarp();
+        (is_v ? v_sent : k_sent) = kn + 1;
+        return true;
       };
       int ids = page_ids(it.kt0);
-      load(false, n, ids);
+      if (!load(false, n, ids)) return;
       for (int kt = it.kt0; kt < it.n_kt; ++kt, ++n) {
         const int next = page_ids(kt + 1);
-        if (NU == 2 && kt + 1 < it.n_kt) load(false, n + 1, next);
-        load(true, n, ids);
-        if (NU == 1 && kt + 1 < it.n_kt) load(false, n + 1, next);
+        if (NU == 2 && kt + 1 < it.n_kt && !load(false, n + 1, next)) return;
+        if (!load(true, n, ids)) return;
+        if (NU == 1 && kt + 1 < it.n_kt && !load(false, n + 1, next)) return;
         ids = next;
       }
     }
-  } else if (warp == C::MMA_WARP) {
-    if (lane == 0) {
-      int n = 0;    // key tiles so far (unit 1 takes part in one item only, the first: its count is the same)
-      auto scores = [&](int u, int kn) {   // S(u) = Q(u) . K^T
-        const uint32_t ks = k_s + (uint32_t)(kn % C::KS) * C::K_BYTES, qs = base + (uint32_t)u * C::Q_BYTES;
+  };
+  auto multiply = [&]() {   // (one thread)
+    int n = 0;    // key tiles so far (unit 1 takes part in one item only, the first: its count is the same)
+    auto scores = [&](int u, int kn) {   // S(u) = Q(u) . K^T
+      const uint32_t ks = k_s + (uint32_t)(kn % C::KS) * C::K_BYTES, qs = base + (uint32_t)u * C::Q_BYTES;
 #pragma unroll
-        for (int kb = 0; kb < NK; ++kb) {
-          const uint64_t da = pt_desc_k(qs + kb * PT_BLOCK), db = pt_desc_k(ks + kb * PT_BLOCK);
+      for (int kb = 0; kb < NK; ++kb) {
+        const uint64_t da = pt_desc_k(qs + kb * PT_BLOCK), db = pt_desc_k(ks + kb * PT_BLOCK);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) tc_mma_bf16(tmem + 128u * u, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), PT_IDESC_QK, (kb | k) ? 1u : 0u);
-        }
-        tc_commit(smem_u32(&s_full[u]));
-      };
-      for (int i = 0; i < n_items; ++i) {
-        const Item it = item_of(i);
-        const int last = it.u[1] >= 0 ? 1 : 0, tiles = it.n_kt - it.kt0;
-        for (int u = 0; u <= last; ++u) pt_wait(q_full[u], i & 1);
-        pt_wait(k_full[n % C::KS], (n / C::KS) & 1);
-        tc_fence_after();
-        for (int u = 0; u <= last; ++u) scores(u, n);
-        tc_commit(smem_u32(&k_free[n % C::KS]));
-        for (int t = 0; t < tiles; ++t, ++n) {
-          const uint32_t vs = v_s + (uint32_t)(n % C::VS) * C::V_BYTES;
-          for (int u = 0; u <= last; ++u) {
-            // O (+)= P . V : 8 MMAs of 16 keys, the first half of the keys as soon as their P stands.  O stays in TMEM across key tiles; the softmax
-            // threads rescale it in place when a row's reference maximum moves.
-            for (int half = 0; half < 2; ++half) {
-              pt_wait(p_full[2 * u + half], n & 1);
-              if (u == 0 && half == 0) pt_wait(v_full[n % C::VS], (n / C::VS) & 1);
-              tc_fence_after();
+        for (int k = 0; k < 4; ++k) tc_mma_bf16(tmem + 128u * u, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), PT_IDESC_QK, (kb | k) ? 1u : 0u);
+      }
+      tc_commit(smem_u32(&s_full[u]));
+    };
+    for (int i = 0; i < n_items; ++i) {
+      const Item it = item_of(i);
+      const int last = it.u[1] >= 0 ? 1 : 0, tiles = it.n_kt - it.kt0;
+      for (int u = 0; u <= last; ++u)
+        if (!wait(q_full[u], i & 1)) return;
+      if (!wait(k_full[n % C::KS], (n / C::KS) & 1)) return;
+      tc_fence_after();
+      for (int u = 0; u <= last; ++u) scores(u, n);
+      tc_commit(smem_u32(&k_free[n % C::KS]));
+      for (int t = 0; t < tiles; ++t, ++n) {
+        const uint32_t vs = v_s + (uint32_t)(n % C::VS) * C::V_BYTES;
+        for (int u = 0; u <= last; ++u) {
+          // O (+)= P . V : 8 MMAs of 16 keys, the first half of the keys as soon as their P stands.  O stays in TMEM across key tiles; the softmax
+          // threads rescale it in place when a row's reference maximum moves.
+          for (int half = 0; half < 2; ++half) {
+            if (!wait(p_full[2 * u + half], n & 1)) return;
+            if (u == 0 && half == 0 && !wait(v_full[n % C::VS], (n / C::VS) & 1)) return;
+            tc_fence_after();
 #pragma unroll
-              for (int k = 4 * half; k < 4 * half + 4; ++k)
-                pt_mma_ts(tmem + C::O_COL + 128u * u, tmem + 128u * u + 8u * k, pt_desc_mn(vs + (uint32_t)(k * 16 * 128)), PT_IDESC_PV, (t > 0 || k) ? 1u : 0u);
-              if (half == 0) tc_commit(smem_u32(&o_half[u]));
-            }
-            if (u == last) tc_commit(smem_u32(&v_free[n % C::VS]));
-            tc_commit(smem_u32(&o_full[u]));
-            if (t + 1 < tiles) {   // the next S takes this P's place, which P.V still reads: MMAs on different accumulators have no order by themselves
-              if (u == 0) pt_wait(k_full[(n + 1) % C::KS], ((n + 1) / C::KS) & 1);
-              pt_wait(o_full[u], n & 1);
-              tc_fence_after();
-              scores(u, n + 1);
-              if (u == last) tc_commit(smem_u32(&k_free[(n + 1) % C::KS]));
-            }
+            for (int k = 4 * half; k < 4 * half + 4; ++k)
+              pt_mma_ts(tmem + C::O_COL + 128u * u, tmem + 128u * u + 8u * k, pt_desc_mn(vs + (uint32_t)(k * 16 * 128)), PT_IDESC_PV, (t > 0 || k) ? 1u : 0u);
+            if (half == 0) tc_commit(smem_u32(&o_half[u]));
+          }
+          if (u == last) tc_commit(smem_u32(&v_free[n % C::VS]));
+          tc_commit(smem_u32(&o_full[u]));
+          if (t + 1 < tiles) {   // the next S takes this P's place, which P.V still reads: MMAs on different accumulators have no order by themselves
+            if (u == 0 && !wait(k_full[(n + 1) % C::KS], ((n + 1) / C::KS) & 1)) return;
+            if (!wait(o_full[u], n & 1)) return;
+            tc_fence_after();
+            scores(u, n + 1);
+            if (u == last) tc_commit(smem_u32(&k_free[(n + 1) % C::KS]));
           }
         }
       }
     }
-  } else {
+  };
+  auto weigh = [&]() {
     // ---- softmax: unit u = warp / 4; thread r owns MMA row r = (head r >> 6, query token r & 63), in pair_mode (tile r >> 6, token r & 63) ----
     const int u = warp >> 2, r = threadIdx.x & 127, t = r & 63;
     const int h = a.pair_mode ? 0 : r >> 6;
@@ -372,7 +376,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       const int lo_all = first_seen_key(tile_b.q_pos0 + PT_TQ - 1, a.window, a.chunk);
       const pt_x2 sc2 = pt_pair(a.scale_log2, a.scale_log2);
       for (int kt = it.kt0; kt < it.n_kt; ++kt, ++n) {
-        pt_wait(s_full[u], n & 1);   // (S comes behind the tile before's P.V: O is complete up to there)
+        if (!wait.warp(s_full[u], n & 1)) return;   // (S comes behind the tile before's P.V: O is complete up to there)
         tc_fence_after();
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
@@ -402,7 +406,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           if ((half == 1 || kt > it.kt0) && __any_sync(0xffffffffu, raise)) {
             const float corr = raise ? exp2f(m_ref - mx) : 1.0f;  // m_ref == -inf: 0 (O and l of such a row are zeros so far)
             if (half == 1) {
-              pt_wait(o_half[u], n & 1);   // the first half has landed in O
+              if (!wait.warp(o_half[u], n & 1)) return;   // the first half has landed in O
               tc_fence_after();
             }
 #pragma unroll 1
@@ -443,7 +447,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       float l_row = (l_0.x + l_0.y) + (l_1.x + l_1.y);
       if (a.sink != nullptr && m_ref > -INFINITY) l_row += exp2f(a.sink[kvh * a.head_step + h] * 1.4426950408889634f - m_ref);
       const float inv = l_row > 0.f ? __fdiv_rn(1.0f, l_row) : 0.f;
-      pt_wait(o_full[u], (n - 1) & 1);   // the last tile's P.V
+      if (!wait.warp(o_full[u], (n - 1) & 1)) return;   // the last tile's P.V
       tc_fence_after();
       bf16* dst = a.out + ((size_t)(mt.q_row0 + t) * a.nq + kvh * a.head_step + h) * PT_HD;
 #pragma unroll 1
@@ -463,9 +467,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       }
       tc_fence_before();   // (the next item's P arrival releases P.V over this O)
     }
+  };
+  if (warp > C::MMA_WARP) {
+    load_tiles();
+  } else if (warp == C::MMA_WARP) {
+    if (lane == 0) multiply();
+  } else {
+    weigh();
   }
   tc_fence_before();
   __syncthreads();
+  if (gave_up != 0) {   // (the same for the whole CTA: nobody waits any more) copies and MMAs under way end before shared memory and TMEM are given back
+    if (warp > C::MMA_WARP) {
+      for (int k = max(0, k_sent - C::KS); k < k_sent; ++k) b2_drain(k_full[k % C::KS], (k / C::KS) & 1);
+      for (int k = max(0, v_sent - C::VS); k < v_sent; ++k) b2_drain(v_full[k % C::VS], (k / C::VS) & 1);
+    } else if (warp == C::MMA_WARP && lane == 0) {
+      tc_commit(smem_u32(&drained));
+      b2_drain(drained, 0);
+    }
+    __syncthreads();
+  }
   if (warp == C::MMA_WARP) {
     tc_fence_after();
     tmem_dealloc(tmem, C::TMEM_COLS);
@@ -486,7 +507,7 @@ int launch_pt(const CUtensorMap& tk, const CUtensorMap& tv, const CUtensorMap& t
 // num_pages: pages in the pool k_pages / v_pages point to (the TMA maps cover exactly the pool).
 int launch_attn_prefill_tc(const bf16* q, const bf16* k_pages, const bf16* v_pages, int64_t num_pages, const int32_t* block_table,
                            int bt_stride, const PrefillTile* tiles_dev, int ntiles, bf16* out, int nq, int nkv, int hd, int block_size,
-                           cudaStream_t s, float softmax_scale, int window, int pair_mode, int chunk, const PrefillRot* rot) {
+                           cudaStream_t s, const B2WaitLimit& wait, float softmax_scale, int window, int pair_mode, int chunk, const PrefillRot* rot) {
   if (ntiles <= 0) return 0;
   const int head_step = pair_mode && nq == nkv ? 1 : 2;
   B2_REQUIRE(hd == PT_HD && block_size == 16 && nq == head_step * nkv, "attn_prefill_tc: built for 128-wide heads in GQA groups of two, 16-token pages");
@@ -511,6 +532,7 @@ int launch_attn_prefill_tc(const bf16* q, const bf16* k_pages, const bf16* v_pag
   a.nq = nq; a.nkv = nkv; a.units = pair_mode ? ntiles / 2 : ntiles;
   a.scale_log2 = (float)(scale * 1.4426950408889634);
   a.window = window; a.pair_mode = pair_mode; a.head_step = head_step; a.chunk = chunk;
+  a.wait = wait;
   // two units to a CTA once every SM has one: below that a CTA for each ends sooner (a unit by itself waits for its own MMAs only)
   const bool two = (long)a.units * nkv > 148;
   if (rot != nullptr) {

@@ -227,8 +227,18 @@ extern "C" int b2k_attn_prefill(const void* q, const void* k_pages, const void* 
       cudaMemcpy(bth.data(), block_table_dev, bth.size() * sizeof(int32_t), cudaMemcpyDeviceToHost);
       int64_t pages = 1;
       for (int32_t v : bth) pages = std::max<int64_t>(pages, (int64_t)v + 1);
+      const char* limit = getenv("B2_PREFILL_WAIT_MS");
+      uint32_t* ran_out = nullptr;
+      B2_CUDA_OK(cudaMallocHost(&ran_out, sizeof(uint32_t)));
+      *ran_out = 0;
       rc = launch_attn_prefill_tc((const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, pages, block_table_dev, bt_stride, d,
-                                  (int)tiles.size(), (bf16*)out, nq, nkv, hd, block_size, s);
+                                  (int)tiles.size(), (bf16*)out, nq, nkv, hd, block_size, s, B2WaitLimit{ran_out, limit ? std::max(0, atoi(limit)) : 2000});
+      cudaStreamSynchronize(s);
+      if (rc == 0 && *(volatile uint32_t*)ran_out != 0) {
+        b2_set_error("b2k_attn_prefill: a wait of the kernel ran out");
+        rc = -110;
+      }
+      cudaFreeHost(ran_out);
     } else {
       rc = launch_attn_prefill((const bf16*)q, (const bf16*)k_pages, (const bf16*)v_pages, block_table_dev, bt_stride, d,
                                (int)tiles.size(), (bf16*)out, nq, nkv, hd, block_size, s);

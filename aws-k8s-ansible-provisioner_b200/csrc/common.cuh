@@ -254,6 +254,37 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
   while (!mbar_try_wait(bar, parity)) {
   }
 }
+// Waits of a CTA that end.  One that has not ended within the limit gives up, and so do all others of the CTA from then on: every role leaves its loop, what
+// is on its way is waited for (b2_drain: with a limit too), and the caller finds its word set: the output is not to be used.
+struct B2WaitLimit {
+  uint32_t* ran_out;   // a word in host memory that is then 1 once the stream is synchronised
+  int limit_ms;        // 0: every wait has run out (tests)
+};
+struct B2Waits {
+  volatile uint32_t* gave_up;   // shared memory, 0 at first
+  B2WaitLimit w;
+  __device__ __forceinline__ bool operator()(uint64_t& bar, uint32_t parity) const {
+    const uint32_t b = smem_u32(&bar);
+    if (mbar_try_wait(b, parity) && w.limit_ms != 0) return true;
+    const unsigned long long t0 = b2_globaltimer();
+    while (*gave_up == 0) {
+      if (b2_globaltimer() - t0 >= (unsigned long long)w.limit_ms * 1000000ull) {
+        *gave_up = 1;
+        *(volatile uint32_t*)w.ran_out = 1;
+        __threadfence_system();
+        break;
+      }
+      if (mbar_try_wait(b, parity)) return true;
+    }
+    return false;
+  }
+  __device__ __forceinline__ bool warp(uint64_t& bar, uint32_t parity) const { return __all_sync(0xffffffffu, (*this)(bar, parity)); }   // the same in all lanes
+};
+__device__ __forceinline__ void b2_drain(uint64_t& bar, uint32_t parity) {
+  const unsigned long long t0 = b2_globaltimer();
+  while (!mbar_try_wait(smem_u32(&bar), parity) && b2_globaltimer() - t0 < 20000000ull) {
+  }
+}
 // 1-D bulk copy global -> shared, completion signalled on an mbarrier (bytes % 16 == 0).
 __device__ __forceinline__ void bulk_g2s(uint32_t dst_smem, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst_smem),

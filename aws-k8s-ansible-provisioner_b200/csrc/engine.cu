@@ -307,6 +307,9 @@ struct b2_engine {
   int l2_weight_prefetch = 0;  // B2_WPF: resid path, see forward_layers (measured slower: off)
   int prefill_resid_fused = 0;  // B2_RESID_FUSED: prefill O / down projections add into the residual stream in their epilogue (measured slower: off)
   int qkv_rope_prefill_fused = 1;  // B2_QKV_ROPE_FUSED: prefill QKV projection finishes norm / RoPE / page write itself
+  uint32_t* h_ran_out = nullptr;     // host word that the prompt attention sets when one of its waits ran out
+  int prefill_wait_ms = 2000;        // B2_PREFILL_WAIT_MS: how long such a wait may last (0: none may, for tests)
+  B2WaitLimit wait_limit() const { return B2WaitLimit{h_ran_out, prefill_wait_ms}; }
   int prefill_pairs = 1;  // B2_PREFILL_PAIRS: see prefill_tile_pairs()
   int prefill_mc = 1;  // B2_MC: prefill projections as multicast CTA pairs (gemm_mc.cu)
   int gu_prefill_fused = 1;  // B2_GU_FUSED: prefill-sized gate/up projection with SwiGLU in its epilogue (gemm_gateup.cu)
@@ -874,7 +877,7 @@ int forward_layers(b2_engine* e, const Lane& ln, int T, int ntiles) {
       if (!k.skip()) {
         if (e->prefill_tc)
           B2_TRY(launch_attn_prefill_tc(qrot, kp, vp, e->num_blocks, block_table, e->bt_stride, e->d_tiles, ntiles, attn, e->nq, e->nkv, e->hd,
-                                        c.block_size, st, e->attn_scale, c.sliding_window, prefill_tile_pairs(e) ? 1 : 0));
+                                        c.block_size, st, e->wait_limit(), e->attn_scale, c.sliding_window, prefill_tile_pairs(e) ? 1 : 0));
         else
           B2_TRY(launch_attn_prefill(qrot, kp, vp, block_table, e->bt_stride, e->d_tiles, ntiles, attn,
                                      e->nq, e->nkv, e->hd, c.block_size, st, e->attn_scale, c.sliding_window));
@@ -1125,7 +1128,7 @@ int latent_rebuilt_attention(b2_engine* e, const ListLayer& L, const char* cache
       KL k(e, B2K_MISC);
       const PrefillRot rot{q_rot, e->lx_r, sp.rot_dim, sink};
       if (!k.skip()) B2_TRY(launch_attn_prefill_tc((const bf16*)e->l_qnope, e->lx_k, e->lx_v, gp.pages, e->d_xtable, e->bt_stride, e->d_xtiles + gp.tile0, gp.ntiles,
-                                                   (bf16*)e->l_av, sp.heads, sp.heads, 128, 16, st, sp.scale, 0, 1, 0, sp.rot_dim > 0 || sink != nullptr ? &rot : nullptr));
+                                                   (bf16*)e->l_av, sp.heads, sp.heads, 128, 16, st, e->wait_limit(), sp.scale, 0, 1, 0, sp.rot_dim > 0 || sink != nullptr ? &rot : nullptr));
     }
   }
   return 0;
@@ -1371,7 +1374,7 @@ int forward_heads_list(b2_engine* e, int T, int ntiles, int nlast) {
       if (!k.skip()) {
         if (ntiles > 0)
           B2_TRY(launch_attn_prefill_tc(e->l_qb, (const bf16*)kc, (const bf16*)vc, e->num_blocks, e->d_block_table, e->bt_stride, e->d_tiles, ntiles,
-                                        (bf16*)e->l_av, sp.heads, sp.kv_heads, 128, c.block_size, st, sp.scale, 0, 0));
+                                        (bf16*)e->l_av, sp.heads, sp.kv_heads, 128, c.block_size, st, e->wait_limit(), sp.scale, 0, 0));
         else
           B2_TRY(launch_attn_decode(e->l_qb, (const bf16*)kc, (const bf16*)vc, e->d_block_table, e->bt_stride, e->d_seq_lens, e->attn_scratch, (bf16*)e->l_av, T,
                                     sp.heads, sp.kv_heads, 128, c.block_size, st, sp.scale, 0, 0));
@@ -1522,7 +1525,7 @@ int forward_state_list(b2_engine* e, int T, int ntiles, int nlast) {
         if (!k.skip()) {
           if (ntiles > 0)
             B2_TRY(launch_attn_prefill_tc(e->l_qb, (const bf16*)kc, (const bf16*)vc, e->num_blocks, e->d_block_table, e->bt_stride, e->d_tiles, ntiles,
-                                          (bf16*)e->l_av, sp.heads, sp.kv_heads, 128, c.block_size, st, sp.scale, sp.window, 0));
+                                          (bf16*)e->l_av, sp.heads, sp.kv_heads, 128, c.block_size, st, e->wait_limit(), sp.scale, sp.window, 0));
           else
             B2_TRY(launch_attn_decode(e->l_qb, (const bf16*)kc, (const bf16*)vc, e->d_block_table, e->bt_stride, e->d_seq_lens, e->attn_scratch, (bf16*)e->l_av, T,
                                       sp.heads, sp.kv_heads, 128, c.block_size, st, sp.scale, sp.window, 0));
@@ -2181,7 +2184,7 @@ int forward_streams_list(b2_engine* e, int T, int ntiles, int nlast) {
         if (!k.skip()) {
           if (ntiles > 0)
             B2_TRY(launch_attn_prefill_tc(e->l_qb, (const bf16*)kc, (const bf16*)vc, e->num_blocks, e->d_block_table, e->bt_stride, e->d_tiles, ntiles, (bf16*)e->l_ao, sp.heads,
-                                          sp.kv_heads, 128, c.block_size, st, sp.scale, 0, 0, sp.chunk));
+                                          sp.kv_heads, 128, c.block_size, st, e->wait_limit(), sp.scale, 0, 0, sp.chunk));
           else
             B2_TRY(launch_attn_decode(e->l_qb, (const bf16*)kc, (const bf16*)vc, e->d_block_table, e->bt_stride, e->d_seq_lens, e->attn_scratch, (bf16*)e->l_ao, T, sp.heads,
                                       sp.kv_heads, 128, c.block_size, st, sp.scale, 0, 0, sp.chunk));
@@ -4825,6 +4828,7 @@ extern "C" int b2_engine_create(const b2_config* cfg, const char* safetensors_pa
   e->gu_prefill_fused = env_int("B2_GU_FUSED", 1);
   e->prefill_mc = env_int("B2_MC", 1);
   e->prefill_pairs = env_int("B2_PREFILL_PAIRS", 1);
+  e->prefill_wait_ms = std::max(0, env_int("B2_PREFILL_WAIT_MS", 2000));
   e->qkv_rope_prefill_fused = env_int("B2_QKV_ROPE_FUSED", 1);
   e->prefill_resid_fused = env_int("B2_RESID_FUSED", 0);
   e->l2_weight_prefetch = env_int("B2_WPF", 0);
@@ -5012,6 +5016,8 @@ extern "C" int b2_engine_create(const b2_config* cfg, const char* safetensors_pa
     E_CUDA(cudaMallocHost(&e->h_tiles, (size_t)e->tiles_cap * sizeof(PrefillTile)));
     E_CUDA(cudaMallocHost(&e->h_out, (size_t)e->log_cap_steps * c.max_seqs * sizeof(int32_t)));
     E_CUDA(cudaMallocHost(&e->h_tok, Bcap * sizeof(int32_t)));
+    E_CUDA(cudaMallocHost(&e->h_ran_out, sizeof(uint32_t)));
+    *e->h_ran_out = 0;
     E_CUDA(cudaEventCreateWithFlags(&e->ev_tok, cudaEventDisableTiming));
     e->seqs.resize(c.max_seqs);
     // ---- KV pool ----
@@ -5226,6 +5232,7 @@ extern "C" void b2_engine_free(b2_engine* e) {
   if (e->h_tiles) cudaFreeHost(e->h_tiles);
   if (e->h_out) cudaFreeHost(e->h_out);
   if (e->h_tok) cudaFreeHost(e->h_tok);
+  if (e->h_ran_out) cudaFreeHost(e->h_ran_out);
   if (e->ev_tok) cudaEventDestroy(e->ev_tok);
   F(e->partial2); F(e->attn_scratch2); F(e->ssq);
   if (e->l_head == e->l_embed) e->l_head = nullptr;   // (a tied head is the embedding table)
@@ -5603,6 +5610,11 @@ int prefill_impl(b2_engine* e, const int32_t* ids, const int32_t* seq_offsets, i
     B2_CUDA_OK(cudaMemcpyAsync(out_logits, e->l_logits + (size_t)nseq * e->cfg.vocab, (size_t)nrows * e->cfg.vocab * 4, cudaMemcpyDeviceToHost,
                                e->stream));
   B2_CUDA_OK(cudaStreamSynchronize(e->stream));
+  if (*(volatile uint32_t*)e->h_ran_out != 0) {   // (none of the portions counts as written, none is registered in the prefix cache: the caller frees its sequences)
+    *(volatile uint32_t*)e->h_ran_out = 0;
+    b2_set_error("b2_prefill: a wait of the prompt attention did not end within %d ms; the call's results are not valid", e->prefill_wait_ms);
+    return -110;
+  }
   for (int i = 0; i < nseq; ++i) {
     Seq& s = e->seqs[seq_ids[i]];
     const int n = seq_offsets[i + 1] - seq_offsets[i] - skip[i];

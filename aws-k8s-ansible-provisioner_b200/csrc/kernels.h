@@ -198,7 +198,8 @@ int launch_attn_prefill(const bf16* q, const bf16* k_pages, const bf16* v_pages,
 // ---- attn_prefill_tc.cu: the same pass on tcgen05 (S and P.V in TMEM, K/V pages through TMA); num_pages = size of the pool ----
 int launch_attn_prefill_tc(const bf16* q, const bf16* k_pages, const bf16* v_pages, int64_t num_pages, const int32_t* block_table,
                            int bt_stride, const PrefillTile* tiles_dev, int ntiles, bf16* out, int nq, int nkv, int hd, int block_size,
-                           cudaStream_t s, float softmax_scale = 0.f, int window = 0, int pair_mode = 0, int chunk = 0, const struct PrefillRot* rot = nullptr);
+                           cudaStream_t s, const B2WaitLimit& wait, float softmax_scale = 0.f, int window = 0, int pair_mode = 0, int chunk = 0,
+                           const struct PrefillRot* rot = nullptr);
 // Layers whose heads share a rotated key piece beside their own keys: 64 more dims in every score, and a term exp(sink[head]) in the softmax's denominator.
 struct PrefillRot {
   const float* q_rot;    // [tokens][heads][rot_dim], rounded to bf16 where they become operands

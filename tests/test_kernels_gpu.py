@@ -765,3 +765,21 @@ def test_attn_prefill_repeats_itself(lib):
         for _ in range(5):
             assert torch.equal(out[at:at + n], prefill(lib, q[at:at + n], kp, vp, bt, [pos0[i]], [n], [i], nq, nkv))
         at += n
+
+
+def test_attn_prefill_wait_that_runs_out(lib, monkeypatch):
+    """With no time to wait at all every CTA gives up at its first wait: the call ends by itself, with an error instead of results, and the next call is as good as ever."""
+    nq, nkv = 8, 4
+    pos0, ntok = [0, 300], [1400, 1200]
+    bt, kp, vp, _, _ = build_pages([p + n for p, n in zip(pos0, ntok)], nkv, 128, 16, seed=52)
+    q, kp, vp, bt = dv(bf(sum(ntok), nq * 128, seed=53)), dv(kp), dv(vp), dv(bt)
+    want = prefill(lib, q, kp, vp, bt, pos0, ntok, [0, 1], nq, nkv)
+    out = torch.empty_like(want)
+    I32 = lambda v: (C.c_int32 * len(v))(*v)
+    for first, count in ((0, 2), (0, 1)):   # two units to a CTA, one
+        monkeypatch.setenv("B2_PREFILL_WAIT_MS", "0")
+        rc = lib.b2k_attn_prefill(ptr(q), ptr(kp), ptr(vp), ptr(bt), bt.shape[1], I32([0, ntok[0]]), I32(pos0), I32(ntok), I32([0, 1]), count, ptr(out), nq, nkv, 128, 16,
+                                  cuda_stream_ptr())
+        assert rc == -110 and b"ran out" in lib.b2_last_error()
+        monkeypatch.delenv("B2_PREFILL_WAIT_MS")
+        assert torch.equal(want, prefill(lib, q, kp, vp, bt, pos0, ntok, [0, 1], nq, nkv))
