@@ -211,24 +211,26 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
   }
   const int n_items = together ? 1 : u_last - u_first + 1;
   struct Item {
-    int u[2];          // second -1: none
-    int kt0, n_kt;     // key tiles [kt0, n_kt)
+    int u[2];            // second -1: none
+    int lo[2], hi[2];    // key tiles [lo, hi) of each unit: its rows meet no others (a value that is not finite would reach them through a weight of 0).  The
+                         // second starts and ends no earlier than the first, and starts no later than that ends: keys from lo[0] to n_kt come in
+    int n_kt;
     const int32_t* bt;
+    __device__ __forceinline__ bool has(int k, int kt) const { return u[k] >= 0 && kt >= lo[k] && kt < hi[k]; }
   };
   auto item_of = [&](int i) {
     Item it;
     it.u[0] = u_first + i;
     it.u[1] = together ? u_last : -1;
-    const PrefillTile f = tile_of(it.u[0], 0);
-    int kv_len = f.q_pos0 + f.nrows;
-    for (int k = 0; k < 2; ++k)
-      if (it.u[k] >= 0) {
-        const PrefillTile l = tile_of(it.u[k], 1);
-        if (l.nrows > 0) kv_len = max(kv_len, l.q_pos0 + l.nrows);
-      }
-    it.n_kt = (kv_len + PT_BN - 1) / PT_BN;
-    it.kt0 = first_seen_key(f.q_pos0, a.window, a.chunk) / PT_BN;
-    it.bt = a.block_table + (size_t)f.bt_row * a.bt_stride;
+    for (int k = 0; k < 2; ++k) {
+      it.lo[k] = it.hi[k] = 0;
+      if (it.u[k] < 0) continue;
+      const PrefillTile f = tile_of(it.u[k], 0), l = tile_of(it.u[k], 1);
+      it.lo[k] = first_seen_key(f.q_pos0, a.window, a.chunk) / PT_BN;
+      it.hi[k] = (max(f.q_pos0 + f.nrows, l.nrows > 0 ? l.q_pos0 + l.nrows : 0) + PT_BN - 1) / PT_BN;
+      if (k == 0) it.bt = a.block_table + (size_t)f.bt_row * a.bt_stride;
+    }
+    it.n_kt = max(it.hi[0], it.hi[1]);
     return it;
   };
 
@@ -264,9 +266,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
         (is_v ? v_sent : k_sent) = kn + 1;
         return true;
       };
-      int ids = page_ids(it.kt0);
+      int ids = page_ids(it.lo[0]);
       if (!load(false, n, ids)) return;
-      for (int kt = it.kt0; kt < it.n_kt; ++kt, ++n) {
+      for (int kt = it.lo[0]; kt < it.n_kt; ++kt, ++n) {
         const int next = page_ids(kt + 1);
         if (NU == 2 && kt + 1 < it.n_kt && !load(false, n + 1, next)) return;
         if (!load(true, n, ids)) return;
@@ -276,7 +278,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     }
   };
   auto multiply = [&]() {   // (one thread)
-    int n = 0;    // key tiles so far (unit 1 takes part in one item only, the first: its count is the same)
+    int n = 0;                 // key tiles that came in so far
+    int done[2] = {0, 0};      // key tiles of each unit so far
     auto scores = [&](int u, int kn) {   // S(u) = Q(u) . K^T
       const uint32_t ks = k_s + (uint32_t)(kn % C::KS) * C::K_BYTES, qs = base + (uint32_t)u * C::Q_BYTES;
 #pragma unroll
@@ -289,36 +292,46 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     };
     for (int i = 0; i < n_items; ++i) {
       const Item it = item_of(i);
-      const int last = it.u[1] >= 0 ? 1 : 0, tiles = it.n_kt - it.kt0;
-      for (int u = 0; u <= last; ++u)
-        if (!wait(q_full[u], i & 1)) return;
+#pragma unroll
+      for (int u = 0; u < NU; ++u)
+        if (it.u[u] >= 0 && !wait(q_full[u], i & 1)) return;
       if (!wait(k_full[n % C::KS], (n / C::KS) & 1)) return;
       tc_fence_after();
-      for (int u = 0; u <= last; ++u) scores(u, n);
+#pragma unroll
+      for (int u = 0; u < NU; ++u)
+        if (it.has(u, it.lo[0])) scores(u, n);
       tc_commit(smem_u32(&k_free[n % C::KS]));
-      for (int t = 0; t < tiles; ++t, ++n) {
+      for (int kt = it.lo[0]; kt < it.n_kt; ++kt, ++n) {
         const uint32_t vs = v_s + (uint32_t)(n % C::VS) * C::V_BYTES;
-        for (int u = 0; u <= last; ++u) {
+        bool v_in = false, k_in = false;
+#pragma unroll
+        for (int u = 0; u < NU; ++u) {
+          const bool now = it.has(u, kt), next = it.has(u, kt + 1);
           // O (+)= P . V : 8 MMAs of 16 keys, the first half of the keys as soon as their P stands.  O stays in TMEM across key tiles; the softmax
           // threads rescale it in place when a row's reference maximum moves.
-          for (int half = 0; half < 2; ++half) {
-            if (!wait(p_full[2 * u + half], n & 1)) return;
-            if (u == 0 && half == 0 && !wait(v_full[n % C::VS], (n / C::VS) & 1)) return;
-            tc_fence_after();
+          if (now) {
+            for (int half = 0; half < 2; ++half) {
+              if (!wait(p_full[2 * u + half], done[u] & 1)) return;
+              if (!v_in && !wait(v_full[n % C::VS], (n / C::VS) & 1)) return;
+              v_in = true;
+              tc_fence_after();
 #pragma unroll
-            for (int k = 4 * half; k < 4 * half + 4; ++k)
-              pt_mma_ts(tmem + C::O_COL + 128u * u, tmem + 128u * u + 8u * k, pt_desc_mn(vs + (uint32_t)(k * 16 * 128)), PT_IDESC_PV, (t > 0 || k) ? 1u : 0u);
-            if (half == 0) tc_commit(smem_u32(&o_half[u]));
+              for (int k = 4 * half; k < 4 * half + 4; ++k)
+                pt_mma_ts(tmem + C::O_COL + 128u * u, tmem + 128u * u + 8u * k, pt_desc_mn(vs + (uint32_t)(k * 16 * 128)), PT_IDESC_PV, (kt > it.lo[u] || k) ? 1u : 0u);
+              if (half == 0) tc_commit(smem_u32(&o_half[u]));
+            }
+            if (u == NU - 1 || !it.has(1, kt)) tc_commit(smem_u32(&v_free[n % C::VS]));
+            tc_commit(smem_u32(&o_full[u]));
           }
-          if (u == last) tc_commit(smem_u32(&v_free[n % C::VS]));
-          tc_commit(smem_u32(&o_full[u]));
-          if (t + 1 < tiles) {   // the next S takes this P's place, which P.V still reads: MMAs on different accumulators have no order by themselves
-            if (u == 0 && !wait(k_full[(n + 1) % C::KS], ((n + 1) / C::KS) & 1)) return;
-            if (!wait(o_full[u], n & 1)) return;
+          if (next) {   // the next S takes this P's place, which P.V still reads: MMAs on different accumulators have no order by themselves
+            if (!k_in && !wait(k_full[(n + 1) % C::KS], ((n + 1) / C::KS) & 1)) return;
+            k_in = true;
+            if (now && !wait(o_full[u], done[u] & 1)) return;
             tc_fence_after();
             scores(u, n + 1);
-            if (u == last) tc_commit(smem_u32(&k_free[(n + 1) % C::KS]));
+            if (u == NU - 1 || !it.has(1, kt + 1)) tc_commit(smem_u32(&k_free[(n + 1) % C::KS]));
           }
+          if (now) ++done[u];
         }
       }
     }
@@ -331,8 +344,9 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
     int n = 0;   // key tiles of this unit so far
     for (int i = 0; i < n_items; ++i) {
       const Item it = item_of(i);
-      if (u == 1 && it.u[1] < 0) continue;
-      const PrefillTile tile_a = tile_of(it.u[u], 0), tile_b = tile_of(it.u[u], 1);
+      const int unit = u == 0 ? it.u[0] : it.u[1], lo = u == 0 ? it.lo[0] : it.lo[1], hi = u == 0 ? it.hi[0] : it.hi[1];
+      if (unit < 0) continue;
+      const PrefillTile tile_a = tile_of(unit, 0), tile_b = tile_of(unit, 1);
       const PrefillTile mt = (r >> 6) ? tile_b : tile_a;  // the tile this row belongs to
       const bool row_ok = t < mt.nrows;
       const int qpos = mt.q_pos0 + t, row_kv_len = mt.q_pos0 + mt.nrows;
@@ -375,7 +389,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
       const bool all_rows = tile_a.nrows == PT_TQ && tile_b.nrows == PT_TQ;
       const int lo_all = first_seen_key(tile_b.q_pos0 + PT_TQ - 1, a.window, a.chunk);
       const pt_x2 sc2 = pt_pair(a.scale_log2, a.scale_log2);
-      for (int kt = it.kt0; kt < it.n_kt; ++kt, ++n) {
+      for (int kt = lo; kt < hi; ++kt, ++n) {
         if (!wait.warp(s_full[u], n & 1)) return;   // (S comes behind the tile before's P.V: O is complete up to there)
         tc_fence_after();
 #pragma unroll
@@ -403,7 +417,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_
           const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale_log2;
           // raise the reference?  (the very first half: O does not exist yet, the first P.V overwrites it)
           const bool raise = mx > m_ref + PT_RESCALE || (m_ref == -INFINITY && mx > -INFINITY);
-          if ((half == 1 || kt > it.kt0) && __any_sync(0xffffffffu, raise)) {
+          if ((half == 1 || kt > lo) && __any_sync(0xffffffffu, raise)) {
             const float corr = raise ? exp2f(m_ref - mx) : 1.0f;  // m_ref == -inf: 0 (O and l of such a row are zeros so far)
             if (half == 1) {
               if (!wait.warp(o_half[u], n & 1)) return;   // the first half has landed in O

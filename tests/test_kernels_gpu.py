@@ -783,3 +783,22 @@ def test_attn_prefill_wait_that_runs_out(lib, monkeypatch):
         assert rc == -110 and b"ran out" in lib.b2_last_error()
         monkeypatch.delenv("B2_PREFILL_WAIT_MS")
         assert torch.equal(want, prefill(lib, q, kp, vp, bt, pos0, ntok, [0, 1], nq, nkv))
+
+
+@pytest.mark.parametrize("pos0", [0, 64])
+def test_attn_prefill_rows_meet_their_own_key_tiles_only(lib, pos0):
+    """A value that is not finite reaches the rows whose key tiles of 128 hold it (0 times an infinity is not 0) and no others, whatever shares their CTA: the second
+    sequence's units of 64 tokens are paired differently behind one unit and behind two."""
+    nq, nkv = 8, 4
+    n, bad = 2560, pos0 + 130      # row 66 to 130 of the second sequence: their tile ends before or with position 127, or holds `bad`
+    for lead in (40, 100):
+        bt, kp, vp, _, _ = build_pages([lead, pos0 + n], nkv, 128, 16, seed=54)
+        q, kd, btd = dv(bf(lead + n, nq * 128, seed=55)), dv(kp), dv(bt)
+        want = prefill(lib, q, kd, dv(vp), btd, [0, pos0], [lead, n], [0, 1], nq, nkv)
+        v2 = vp.clone()
+        v2[int(bt[1, bad // 16]), :, bad % 16] = float("inf")
+        got = prefill(lib, q, kd, dv(v2), btd, [0, pos0], [lead, n], [0, 1], nq, nkv)
+        first = max(0, bad // 128 * 128 - pos0)          # the first token whose tiles reach `bad`, rounded down to its unit
+        clean = lead + first // 64 * 64
+        assert torch.equal(got[:clean], want[:clean])
+        assert not torch.isfinite(got[lead + bad - pos0:].float()).any()
