@@ -6,7 +6,7 @@
 //
 // A UNIT is 128 MMA rows of one kv head: one 64-query tile x both query heads of the GQA group (row r = head (r >> 6), query
 // token (r & 63)), or, for models with one query head per kv head (pair_mode), two consecutive 64-query tiles of that head.
-// A CTA takes two consecutive units of a sequence at a time and streams the keys once for both:
+// A CTA takes one unit, and two CTAs share an SM; beside a rotated key piece (below) two consecutive units of a sequence, for which the keys come in once:
 //   S[128 x 128 keys]  = Q[128 x 128 dims] . K^T      tcgen05.mma, A and B K-major from shared memory, S in TMEM
 //   softmax            : 128 threads per unit, one per row, 64 keys at a time: tcgen05.ld, scale / mask, row maximum, probabilities; P
 //                        (bf16) goes back into TMEM over S columns that have been read
@@ -17,18 +17,17 @@
 // stored swizzled): half h of key row k lands at [h][k][128 bytes], which serves as K-major B for Q.K^T and as
 // MN-major B for P.V without any re-layout.
 //
-// What bounds it: per unit and key tile the MMAs take about 1 050 cycles and the exponentials 1 024 (16 a cycle and SM).  The two units
-// take turns: while one's threads form its probabilities, the tensor cores run the other's products, and the next key tiles
-// are already landing in the other stage of K and V -- the issue order is P.V(A, t), S(A, t + 1), P.V(B, t), S(B, t + 1), P.V of a tile's
-// first half as soon as its P stands.  S(t + 1) takes the columns of P(t): it is issued once P.V(t), which reads them, has ended (only
-// MMAs on one accumulator are ordered by themselves).  A pair of tiles then takes about 4 000 cycles: a unit's threads work 2 230 of them (1 350 in the exponentials) and wait
-// for P.V and S of theirs behind the other unit's.  Measured at 12 prompts of 133 to 4096 tokens, 16 heads, per layer:
-//   one unit per CTA, two CTAs per SM, K / P and V in single buffers, every step of a key tile behind the one before     737 us
-//   two units, two passes over S in TMEM                                                                                 633 us
-//   two units, two threads per row (four softmax warps a scheduler get in one another's way: 3 060 cycles a tile)        532 us
-//   two units, S of 64 keys, two of them per unit in TMEM (a 64-key S costs 0.75 of a 128-key one)                       725 us
-//   this form                                                                                                            516 us
-// Where a launch has no more units than SMs, one unit per CTA (96 KB, two CTAs fit an SM) ends sooner: 128 tokens, 16 heads: 8.0 -> 6.7 us.
+// What bounds it: per unit and key tile the MMAs take about 1 050 cycles and the exponentials 1 024 (16 a cycle and SM), and within a unit everything
+// waits for something: S for K and for the P.V that reads the columns it is written to (only MMAs on one accumulator are ordered by themselves), the
+// probabilities for S, P.V for a half tile of probabilities.  What fills the gaps is another unit on the same SM.  As a CTA of its own (96 KB of shared memory
+// and 256 TMEM columns each, K and V in single buffers) it does so at least as well as in turn within one CTA (192 KB, K and V in two stages, one softmax thread
+// per row in both), needs no neighbour of the same sequence, and a launch that fills the chip less than twice keeps all SMs.  us per launch, 8 kv heads of 2,
+// with one unit per CTA, with two, and with one unit whose P went through shared memory over K (two threads per row, two passes over S):
+//   12 prompts of 133 to 4096 tokens    271   284   384        40 prompts of 64 tokens              16.2   22.9   16.8
+//   one prompt of 4096                  110   113   163        40 x 64 behind 1000 cached tokens    56.8   85.4   77.5
+//   one prompt of 2048                 40.8  40.5  60.6        20 x 192 behind 1000                 61.5   76.5   86.6
+//   one prompt of 1600                 32.9  31.2  47.6        24 x 64 behind 4000                  87.6   130    130
+//   one prompt of 1216                 24.4  24.8  33.0        4 x 448 behind 2048                  53.9   77.0   76.9
 //
 // rot (layers whose heads share a rotated key piece): S gets a third block of 64 dims, Q from fp32 queries, K from a pool of
 // [page][16][64] rows that all heads read; a per-head sink joins the row sum.
@@ -45,11 +44,11 @@ constexpr int PT_SN = 64;                    // keys of half a tile: what a soft
 constexpr int PT_HD = 128;
 constexpr int PT_BLOCK = PT_BN * 128;        // 128 rows x 64 dims (128 bytes): 16 KB
 constexpr int PT_MAX_PAGES = 1024;           // longest block-table row (16 K tokens of context)
-// NK: 64-dim blocks of Q . K^T (3 with a rotated piece).  NU: units of a CTA.  Two units, 192 or 224 KB: K is two stages deep, V two (one beside three
-// blocks).  One unit: single stages, 96 or 128 KB.
+// NK: 64-dim blocks of Q . K^T (3 with a rotated piece).  NU: units of a CTA.  One unit: single stages, 96 or 128 KB.  Two units (beside three blocks):
+// K is two stages deep, 224 KB.
 template <int NK, int NU>
 struct PtCfg {
-  static constexpr int KS = NU == 2 ? 2 : 1, VS = NU == 2 && NK == 2 ? 2 : 1;
+  static constexpr int KS = NU, VS = 1;
   static constexpr int Q_BYTES = NK * PT_BLOCK, K_BYTES = NK * PT_BLOCK, V_BYTES = 2 * PT_BLOCK;
   static constexpr int K_OFF = NU * Q_BYTES, V_OFF = K_OFF + KS * K_BYTES;
   static constexpr int BAR_OFF = V_OFF + VS * V_BYTES;
@@ -547,15 +546,17 @@ int launch_attn_prefill_tc(const bf16* q, const bf16* k_pages, const bf16* v_pag
   a.scale_log2 = (float)(scale * 1.4426950408889634);
   a.window = window; a.pair_mode = pair_mode; a.head_step = head_step; a.chunk = chunk;
   a.wait = wait;
-  // two units to a CTA once every SM has one: below that a CTA for each ends sooner (a unit by itself waits for its own MMAs only)
-  const bool two = (long)a.units * nkv > 148;
   if (rot != nullptr) {
     a.q_rot = rot->q_rot;
     a.rot_dim = rot->rot_dim;
     a.sink = rot->sink;
   }
-  if (rot != nullptr && rot->rot_dim > 0) return two ? launch_pt<3, 2>(tk, tv, tr, a, s) : launch_pt<3, 1>(tk, tv, tr, a, s);
-  return two ? launch_pt<2, 2>(tk, tv, tr, a, s) : launch_pt<2, 1>(tk, tv, tr, a, s);
+  if (rot == nullptr || rot->rot_dim == 0) return launch_pt<2, 1>(tk, tv, tr, a, s);
+  // Beside a rotated piece one unit takes 128 KB and an SM to itself: a second one in turn fills its gaps once every SM has a unit.  One unit / two, us at
+  // 16 heads: 1 x 1024 tokens (128 units) 25.6 / 31.5; 1 x 1280 (160) 39.1 / 39.6; 4 x 512 (256) 35.6 / 29.2; 8 x 1024 (1024) 124.8 / 103.6; units that do not
+  // continue one another 25.0 / 27.2 (10 x 128) to 30.4 / 29.4 (16 x 128), three to a sequence 35.8 / 38.3 (8 x 384).
+  static const int sms = device_num_sms();
+  return (long)a.units * nkv > sms ? launch_pt<3, 2>(tk, tv, tr, a, s) : launch_pt<3, 1>(tk, tv, tr, a, s);
 }
 
 }  // namespace b2

@@ -708,8 +708,8 @@ def test_attn_prefill(lib, case):
 
 @pytest.mark.parametrize("qscale", [1.0, 6.0])
 def test_attn_prefill_two_units_per_cta(lib, qscale):
-    """More units (64 tokens of a kv head) than SMs: a CTA takes two.  Sequences of an odd and an even number of units, so that CTAs hold two units of one sequence and
-    of two; queries behind cached prefixes, key tiles cut anywhere; with large queries the row maxima keep growing, in either half of a tile, which rescales."""
+    """More units (64 tokens of a kv head) than SMs, two to an SM.  Sequences of an odd and an even number of units; queries behind cached prefixes, key tiles cut
+    anywhere; with large queries the row maxima keep growing, in either half of a tile, which rescales."""
     a = QWEN3_0_6B
     nq, nkv, hd, bs = a.num_q_heads, a.num_kv_heads, a.head_dim, 16
     pos0, ntok = [0, 63, 1000, 128, 5, 0], [700, 65, 130, 64, 300, 129]
@@ -750,8 +750,8 @@ def prefill(lib, q, kp, vp, bt, pos0, ntok, rows, nq, nkv):
 
 
 def test_attn_prefill_repeats_itself(lib):
-    """The next key tile's scores take the place of the weights that the tensor cores still multiply: they wait for them.  Contexts of many key tiles, one and two units to
-    a CTA: every launch gives the same bits, and so does a sequence by itself."""
+    """The next key tile's scores take the place of the weights that the tensor cores still multiply: they wait for them.  Contexts of many key tiles, SMs with one CTA
+    and with two: every launch gives the same bits, and so does a sequence by itself."""
     nq, nkv = 8, 4
     pos0, ntok = [0, 2900, 1500], [1700, 200, 1000]
     bt, kp, vp, _, _ = build_pages([p + n for p, n in zip(pos0, ntok)], nkv, 128, 16, seed=50)
@@ -776,7 +776,7 @@ def test_attn_prefill_wait_that_runs_out(lib, monkeypatch):
     want = prefill(lib, q, kp, vp, bt, pos0, ntok, [0, 1], nq, nkv)
     out = torch.empty_like(want)
     I32 = lambda v: (C.c_int32 * len(v))(*v)
-    for first, count in ((0, 2), (0, 1)):   # two units to a CTA, one
+    for count in (2, 1):
         monkeypatch.setenv("B2_PREFILL_WAIT_MS", "0")
         rc = lib.b2k_attn_prefill(ptr(q), ptr(kp), ptr(vp), ptr(bt), bt.shape[1], I32([0, ntok[0]]), I32(pos0), I32(ntok), I32([0, 1]), count, ptr(out), nq, nkv, 128, 16,
                                   cuda_stream_ptr())
@@ -787,8 +787,8 @@ def test_attn_prefill_wait_that_runs_out(lib, monkeypatch):
 
 @pytest.mark.parametrize("pos0", [0, 64])
 def test_attn_prefill_rows_meet_their_own_key_tiles_only(lib, pos0):
-    """A value that is not finite reaches the rows whose key tiles of 128 hold it (0 times an infinity is not 0) and no others, whatever shares their CTA: the second
-    sequence's units of 64 tokens are paired differently behind one unit and behind two."""
+    """A value that is not finite reaches the rows whose key tiles of 128 hold it (0 times an infinity is not 0) and no others, wherever the sequence stands in the
+    batch: behind one unit of 64 tokens and behind two."""
     nq, nkv = 8, 4
     n, bad = 2560, pos0 + 130      # row 66 to 130 of the second sequence: their tile ends before or with position 127, or holds `bad`
     for lead in (40, 100):

@@ -451,3 +451,31 @@ def test_bf16_rebuilt_keys_and_values(rot_dim):
                 assert np.abs(lg[at:at + c] - refs[r][done[r]:done[r] + c]).max() / scale < BF16_BAR, "request %d at %d" % (r, done[r])
                 at += c
                 done[r] += c
+
+
+def test_rebuilt_rows_meet_their_own_key_tiles_only():
+    """Two units of 128 tokens to a CTA (more units than SMs): a token whose key and value are not finite reaches the rows whose key tiles of 128 hold it and no others,
+    also where it shares the CTA with a unit in front of it: the second request's units are paired differently behind one unit and behind two."""
+    cfg = {"architecture": "Lerasun", "vocab": 211, "width": 96, "logit_scale": 1.0, "norm": {"eps": 1e-6}, "layers": [
+        layer(mixer(40, 128, 64, 128, 128, 0.05), None)]}
+    w = random_weights(cfg, seed=47)
+    w["embed"][210] = float("inf")
+    for lead in (128, 200):
+        a, b = [t % 210 for t in tokens(cfg, lead, 48)], [t % 210 for t in tokens(cfg, 640, 49)]
+        ref = Oracle(cfg, w).forward(b).numpy()
+        b[300] = 210
+        with engine(cfg, w, f32=False) as e:
+            got, _ = e.prefill_logits([e.seq_create(lead), e.seq_create(640)], [a, b], list(range(lead + 640)))
+        assert np.abs(got[lead:lead + 256] - ref[:256]).max() / np.abs(ref).max() < BF16_BAR
+        assert not np.isfinite(got[lead + 300:]).any()
+
+
+def test_rebuilt_form_reports_a_wait_that_ran_out(monkeypatch):
+    """One and two units to a CTA: a portion whose attention is given no time to wait makes the call an error."""
+    cfg = {"architecture": "Lerasun", "vocab": 211, "width": 96, "logit_scale": 1.0, "norm": {"eps": 1e-6}, "layers": [
+        layer(mixer(40, 128, 64, 128, 128, 0.05), None)]}
+    monkeypatch.setenv("B2_PREFILL_WAIT_MS", "0")
+    with engine(cfg, random_weights(cfg, seed=50), f32=False) as e:
+        for n in (130, 640):
+            with pytest.raises(pkg().B2Error, match="did not end within 0 ms"):
+                e.prefill([e.seq_create(n)], [tokens(cfg, n, 51)])
