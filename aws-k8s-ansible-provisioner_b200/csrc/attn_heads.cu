@@ -35,6 +35,8 @@
 //   talk_gate         that sum, times the gate, rounded to the operand type
 #include <mma.h>
 
+#include <type_traits>
+
 #include "kernels.h"
 
 #define B2_TRY_RC(expr)      \
@@ -728,8 +730,8 @@ __global__ void __launch_bounds__(HA_WARPS * 32) heads_attention_kernel(const fl
 // tokens of 8 heads whose values go to 4 key/value heads, 1.34 ms without that, against some 1 GFLOP of arithmetic.  Here 32 tokens share every key and
 // value row: a thread forms 2 x 2 scores (16-byte loads of four numbers of a row, packed multiply-adds on pairs of neighbouring dims), eight threads
 // share a row's maximum and sum, and a warp accumulates four rows of the output, four columns a lane.  K rows of the next tile arrive (cp.async) under
-// the products with V, V rows under the scores.  Everything is fp32; which keys a row sees is decided per (row, key).  The same two launches: 169 and
-// 103 us.
+// the products with V, V rows under the scores.  Everything is fp32; which keys a row sees is decided per (row, key).  The same two launches: 177 and
+// 99 us.
 // NV: value columns / 128, rounded up (with cross: columns of the run that this CTA weights).
 constexpr int HF_ROWS = 32, HF_KEYS = 32, HF_PLD = 36;
 __host__ __device__ inline int hf_row(int d) { return (d + 31) / 32 * 32 + 4; }   // row stride whose rows start four banks apart
@@ -807,6 +809,10 @@ __global__ void __launch_bounds__(256) heads_attention_f32_kernel(const float* _
   const int last_tile = pos_last / HF_KEYS, lo_tile = first_seen_key(pos0, g.window, g.chunk) / HF_KEYS;
   const int keep_tiles = g.window > 0 ? (g.keep_first + HF_KEYS - 1) / HF_KEYS : 0;
   auto next_tile = [&](int t) { return t >= lo_tile || t < keep_tiles ? t : lo_tile; };
+  auto visible = [&](int r, int key) {
+    const int pos = pos0 + r;
+    return r < nrows && key <= pos && (key >= first_seen_key(pos, g.window, g.chunk) || key < g.keep_first);
+  };
   const float slope = g.slopes ? (float)exp2(-(double)g.slope_exp * (double)(a + 1) / (double)g.heads) : 0.f;
   const int qy = tid >> 4, kx = tid & 15;     // scores: rows qy, qy + 16, keys kx, kx + 16
   const int srow = tid >> 3, spart = tid & 7; // softmax: eight threads a row, four keys each
@@ -841,8 +847,7 @@ __global__ void __launch_bounds__(256) heads_attention_f32_kernel(const float* _
         for (int j = 0; j < 2; ++j) {
           const float2 s = hf_split(s2[i][j]);
           const int r = qy + 16 * i, key = k0 + kx + 16 * j, pos = pos0 + r;
-          const bool vis = r < nrows && key <= pos && (key >= first_seen_key(pos, g.window, g.chunk) || key < g.keep_first);
-          Ps[r * HF_PLD + kx + 16 * j] = vis ? (s.x + s.y) * g.scale - slope * (float)(pos - key) : -INFINITY;
+          Ps[r * HF_PLD + kx + 16 * j] = visible(r, key) ? (s.x + s.y) * g.scale - slope * (float)(pos - key) : -INFINITY;
         }
     }
     __syncthreads();
@@ -879,28 +884,42 @@ __global__ void __launch_bounds__(256) heads_attention_f32_kernel(const float* _
         acc[i][n][1] = hf_fma(acc[i][n][1], f2, 0ull);
       }
     }
+    // Keys that a row does not see add nothing to it, whatever their values are (0 times an infinity is not 0): tiles that some row of the warp sees
+    // in part pick key by key.
+    unsigned seen[4];
+    bool whole = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      seen[i] = __ballot_sync(0xffffffffu, visible(4 * warp + i, k0 + lane));
+      whole = whole && seen[i] == 0xffffffffu;
+    }
+    auto add_values = [&](auto all) {
 #pragma unroll 2
-    for (int k4 = 0; k4 < HF_KEYS; k4 += 4) {
-      float4 p[4];
+      for (int k4 = 0; k4 < HF_KEYS; k4 += 4) {
+        float4 p[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (4 * warp + i) * HF_PLD + k4);
+        for (int i = 0; i < 4; ++i) p[i] = *reinterpret_cast<const float4*>(Ps + (4 * warp + i) * HF_PLD + k4);
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        ulonglong2 v[NV];
+        for (int kk = 0; kk < 4; ++kk) {
+          ulonglong2 v[NV];
 #pragma unroll
-        for (int n = 0; n < NV; ++n) v[n] = *reinterpret_cast<const ulonglong2*>(Vs + (k4 + kk) * VP + 128 * n + 4 * lane);
+          for (int n = 0; n < NV; ++n) v[n] = *reinterpret_cast<const ulonglong2*>(Vs + (k4 + kk) * VP + 128 * n + 4 * lane);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float w = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
-          const hf_x2 w2 = hf_pair(w, w);
+          for (int i = 0; i < 4; ++i) {
+            if (!decltype(all)::value && !(seen[i] >> (k4 + kk) & 1u)) continue;   // (the same for the whole warp)
+            const float w = kk == 0 ? p[i].x : kk == 1 ? p[i].y : kk == 2 ? p[i].z : p[i].w;
+            const hf_x2 w2 = hf_pair(w, w);
 #pragma unroll
-          for (int n = 0; n < NV; ++n) {
-            acc[i][n][0] = hf_fma(w2, v[n].x, acc[i][n][0]);
-            acc[i][n][1] = hf_fma(w2, v[n].y, acc[i][n][1]);
+            for (int n = 0; n < NV; ++n) {
+              acc[i][n][0] = hf_fma(w2, v[n].x, acc[i][n][0]);
+              acc[i][n][1] = hf_fma(w2, v[n].y, acc[i][n][1]);
+            }
           }
         }
       }
-    }
+    };
+    if (whole) add_values(std::true_type{});
+    else add_values(std::false_type{});
     __syncthreads();   // V, weights and factors are free
     t = tn;
   }

@@ -589,3 +589,20 @@ def test_projection_finish_in_groups_of_tokens(n, f32):
         bar = F32_BAR if f32 else BF16_BAR
         assert err(np.concatenate([x[:2], y[6:]]), ra) < bar
         assert err(np.concatenate([x[2:], y[:6]]), rb) < bar
+
+
+@pytest.mark.parametrize("mixer,bad,clean", [(att(4, 2, 20, 12, 0.3, rot=4), 40, range(0, 40)), (att(2, 1, 9, 131, 0.3), 70, range(0, 70)),
+                                             (att2(4, 2, 12, 20, 1.1, 2, window=9, keep=0), 3, [*range(0, 3), *range(13, 90)])])
+def test_fp32_prompt_rows_take_nothing_from_what_they_do_not_see(mixer, bad, clean):
+    """A token whose keys and values are not finite: positions before it, and those whose window it has left, are what they are with any other token in its place.
+    (Position `bad` and the next one, which the convolution's second tap reaches, are out of sight of a window of 9 from 13 on.)"""
+    cfg = model([(mixer, None)], vocab=61, width=48, groups=3)
+    w = random_weights(cfg, seed=97)
+    w["embed"][60] = float("inf")
+    toks = [t % 60 for t in tokens(cfg, 90, 98)]
+    ref = ref_logits(cfg, w, toks)
+    toks[bad] = 60
+    with engine(cfg, w) as e:
+        got, _ = e.prefill_logits([e.seq_create(90)], [toks], list(range(90)))
+        assert err(got[list(clean)], ref[list(clean)]) < F32_BAR
+        assert not np.isfinite(got[bad]).any()
