@@ -115,6 +115,7 @@ struct ListLayer {
   float *bias1 = nullptr, *bias1b = nullptr, *bias2 = nullptr, *bias2b = nullptr, *latq_gain = nullptr;
   void* uq = nullptr;
   bf16* router_op = nullptr;  // the router (and the gate's row) as a bf16 operand
+  bool uv_in_ukv = false;     // uv is the second half of ukv
   bf16* ukv = nullptr;        // key and value up-projections as one matrix [heads (dim + vdim)][kv_rank]: layers that rebuild keys and values
   int32_t* table = nullptr;
   // Norms behind the sublayers only (Tolanex): gain1b / gain2b.  Its delta mixer projects q | k | v | beta | decay | gate in `wqd` (off_sg = the
@@ -1142,12 +1143,14 @@ bool latent_rebuild_ok(const b2_engine* e, const b2_layer_spec& sp) {
          (c.max_model_len + 15) / 16 <= 1024 && c.max_batch_tokens >= LATENT_REBUILD_ROWS;
 }
 
-// Scratch for the contexts of one group: as many pages as a step brings at least, one full-length context at most needs
+// Rows of the scratch for the contexts of one group: as many pages as a step brings at least, one full-length context at most needs
+size_t latent_rebuild_rows(const b2_engine* e, size_t Tc) {
+  return 16 * std::max((size_t)(e->cfg.max_model_len + 15) / 16, Tc / 16 + (size_t)e->cfg.max_seqs);
+}
+
 int latent_rebuild_alloc(b2_engine* e, size_t Tc, size_t max_rank, size_t max_nq, bool rot) {
   const b2_config& c = e->cfg;
-  const size_t ctx_pages = (size_t)(c.max_model_len + 15) / 16;
-  e->lx_pages_cap = (int)std::max(ctx_pages, Tc / 16 + (size_t)c.max_seqs);
-  const size_t rows = (size_t)e->lx_pages_cap * 16;
+  const size_t ctx_pages = (size_t)(c.max_model_len + 15) / 16, rows = latent_rebuild_rows(e, Tc);
   B2_TRY(dalloc(&e->lx_rows, rows * max_rank));
   B2_TRY(dalloc(&e->lx_kv, rows * 2 * max_nq));
   B2_TRY(dalloc(&e->lx_k, rows * max_nq));
@@ -1165,6 +1168,59 @@ int latent_rebuild_alloc(b2_engine* e, size_t Tc, size_t max_rank, size_t max_nq
   B2_CUDA_OK(cudaMallocHost(&e->h_xtiles, (size_t)e->xtiles_cap * sizeof(PrefillTile)));
   B2_CUDA_OK(cudaMallocHost(&e->h_xctx, (size_t)c.max_seqs * sizeof(LatentContext)));
   B2_CUDA_OK(cudaMallocHost(&e->h_xtable, (size_t)c.max_seqs * ctx_pages * sizeof(int32_t)));
+  e->lx_pages_cap = (int)(rows / 16);
+  return 0;
+}
+
+void latent_rebuild_free(b2_engine* e) {
+  auto drop = [](auto*& p) {
+    if (p) cudaFree(p);
+    p = nullptr;
+  };
+  auto drop_host = [](auto*& p) {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+  };
+  drop(e->lx_rows); drop(e->lx_kv); drop(e->lx_k); drop(e->lx_v); drop(e->lx_r); drop(e->d_xtiles); drop(e->d_xctx); drop(e->d_xtable);
+  drop_host(e->h_xtiles); drop_host(e->h_xctx); drop_host(e->h_xtable);
+}
+
+// A Lerasun engine takes what the rebuilt form needs -- a layer's up-projections as one matrix (the key part a second time: 2 MB at 16 heads and a latent of
+// 512), the scratch of a group (8 192 tokens, 16 heads: 143 MB; 16 384 tokens: 286 MB) -- last, behind the cache, and only where it leaves 512 MB free, as much
+// as the cache's own sizing leaves: an engine that fits without it is not refused, its portions all take the absorbed form then.
+int latent_rebuild_setup(b2_engine* e) {
+  size_t nq = 0, rank = 0, weights = 0;
+  for (const ListLayer& L : e->ll)
+    if (latent_rebuild_ok(e, L.sp)) {
+      nq = std::max(nq, (size_t)L.sp.heads * 128);
+      rank = std::max(rank, (size_t)L.sp.kv_rank);
+      weights += (size_t)2 * L.sp.heads * 128 * L.sp.kv_rank * sizeof(bf16);
+    }
+  if (nq == 0) return 0;
+  const size_t need = weights + latent_rebuild_rows(e, e->cap_tokens) * (rank + 4 * nq + 64) * sizeof(bf16);
+  size_t free_b = 0, total_b = 0;
+  B2_CUDA_OK(cudaMemGetInfo(&free_b, &total_b));
+  if (need + ((size_t)512 << 20) > free_b) return 0;
+  int rc = latent_rebuild_alloc(e, e->cap_tokens, rank, nq, true);
+  std::vector<bf16*> ukv(e->ll.size(), nullptr);
+  for (size_t l = 0; l < e->ll.size() && rc == 0; ++l)
+    if (latent_rebuild_ok(e, e->ll[l].sp)) rc = dalloc(&ukv[l], (size_t)2 * e->ll[l].sp.heads * 128 * e->ll[l].sp.kv_rank);
+  if (rc != 0) {   // (another process was quicker)
+    cudaGetLastError();
+    for (bf16* p : ukv)
+      if (p) cudaFree(p);
+    latent_rebuild_free(e);
+    e->lx_pages_cap = 0;
+    return 0;
+  }
+  for (size_t l = 0; l < e->ll.size(); ++l) {
+    ListLayer& L = e->ll[l];
+    if (ukv[l] == nullptr) continue;
+    cudaFree(L.uv);   // (the value part serves both forms)
+    L.ukv = ukv[l];
+    L.uv = L.ukv + (size_t)L.sp.heads * 128 * L.sp.kv_rank;
+    L.uv_in_ukv = true;
+  }
   return 0;
 }
 
@@ -3075,11 +3131,7 @@ int list_tensor(b2_engine* e, const std::string& name, const void* host, size_t 
     if (L.ukv) B2_TRY(put_operand(e, L.ukv, 0, src, H * dn * r));
     return done(put_key_up(e, L.ukT, src, H, dn, r));
   }
-  if (rest == "mix.uv") {
-    B2_TRY(want(H * dv * r));
-    if (L.ukv) B2_TRY(put_operand(e, L.ukv, H * dn * r, src, H * dv * r));
-    return done(put_operand(e, L.uv, 0, src, H * dv * r));
-  }
+  if (rest == "mix.uv") { B2_TRY(want(H * dv * r)); return done(put_operand(e, L.uv, 0, src, H * dv * r)); }
   if (rest == "mix.sink") { B2_TRY(want(H)); return done(put_f32(L.sink, src, H, 0.0f)); }
   if (rest == "mix.o") { B2_TRY(want(W * H * dv)); return done(put_operand(e, L.wo, 0, src, W * H * dv)); }
   if (sp.ff == B2_FF_ROUTED_EXPERTS) {
@@ -4390,7 +4442,7 @@ int list_engine_alloc(b2_engine* e) {
   B2_TRY(falloc(&e->l_embed_gain, W));
   B2_TRY(falloc(&e->l_final_gain, W));
   e->ll.resize(c.num_layers);
-  size_t max_nqd = 1, max_hn = 1, max_hr = 1, max_hrot = 1, max_hv = 1, max_ff = 1, max_rebuild_nq = 0, max_rebuild_rank = 0;
+  size_t max_nqd = 1, max_hn = 1, max_hr = 1, max_hrot = 1, max_hv = 1, max_ff = 1;
   int max_top = 1, max_exp = 1;
   for (int l = 0; l < c.num_layers; ++l) {
     ListLayer& L = e->ll[l];
@@ -4410,13 +4462,6 @@ int list_engine_alloc(b2_engine* e) {
     B2_TRY(xalloc(&L.wqd, (size_t)L.nqd * W));
     B2_TRY(xalloc(&L.ukT, (size_t)sp.heads * sp.kv_rank * sp.dim));
     B2_TRY(xalloc(&L.uv, (size_t)sp.heads * sp.vdim * sp.kv_rank));
-    if (latent_rebuild_ok(e, sp)) {
-      void* q = nullptr;
-      B2_TRY(xalloc(&q, (size_t)2 * sp.heads * 128 * sp.kv_rank));
-      L.ukv = reinterpret_cast<bf16*>(q);
-      max_rebuild_nq = std::max(max_rebuild_nq, (size_t)sp.heads * 128);
-      max_rebuild_rank = std::max(max_rebuild_rank, (size_t)sp.kv_rank);
-    }
     B2_TRY(xalloc(&L.wo, W * sp.heads * sp.vdim));
     B2_TRY(falloc(&L.gain1, W));
     B2_TRY(falloc(&L.sink, sp.heads));
@@ -4491,7 +4536,6 @@ int list_engine_alloc(b2_engine* e) {
       B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
     }
   }
-  if (max_rebuild_nq > 0) B2_TRY(latent_rebuild_alloc(e, Tc, max_rebuild_rank, max_rebuild_nq, true));
   B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));
   B2_CUDA_OK(cudaMemset(e->l_pair_slot, 0, Tc * max_top * 4));
   return 0;
@@ -5129,6 +5173,7 @@ extern "C" int b2_engine_create(const b2_config* cfg, const char* safetensors_pa
         for (int r = 0; r < 2 * c.num_layers; ++r)
           e->regions.push_back({reinterpret_cast<char*>(e->kv_pool + (size_t)r * e->layer_kv_elems), blk_elems * 2});
       }
+      if (c.arch == B2_ARCH_LERASUN) E_TRY(latent_rebuild_setup(e));
       e->free_blocks.reserve(nb);
       for (int64_t b = nb - 1; b >= 1; --b) e->free_blocks.push_back((int32_t)b);  // page 0 = null page
       e->blk_ref.assign(nb, 0);
@@ -5236,10 +5281,7 @@ extern "C" void b2_engine_free(b2_engine* e) {
   if (e->ev_tok) cudaEventDestroy(e->ev_tok);
   F(e->partial2); F(e->attn_scratch2); F(e->ssq);
   if (e->l_head == e->l_embed) e->l_head = nullptr;   // (a tied head is the embedding table)
-  F(e->lx_rows); F(e->lx_kv); F(e->lx_k); F(e->lx_v); F(e->lx_r); F(e->d_xtiles); F(e->d_xctx); F(e->d_xtable);
-  if (e->h_xtiles) cudaFreeHost(e->h_xtiles);
-  if (e->h_xctx) cudaFreeHost(e->h_xctx);
-  if (e->h_xtable) cudaFreeHost(e->h_xtable);
+  latent_rebuild_free(e);
   for (auto& t : e->rot_tables) F(t.table);
   F(e->l_shift); F(e->l_ao); F(e->l_rkvg); F(e->l_lr); F(e->l_cv);
   F(e->l_final_bias); F(e->l_bigram); F(e->l_pos); F(e->l_tok_ring); F(e->l_sg); F(e->l_rz);
@@ -5249,7 +5291,8 @@ extern "C" void b2_engine_free(b2_engine* e) {
   F(e->l_mix); F(e->l_y); F(e->l_rw); F(e->l_logits); F(e->l_x1); F(e->l_x2); F(e->l_qnope); F(e->l_olat); F(e->l_av); F(e->l_act); F(e->l_xl);
   F(e->l_attn_scratch); F(e->l_idx); F(e->l_offsets); F(e->l_slot_token); F(e->l_pair_slot); F(e->l_tile_group); F(e->l_tile_row0); F(e->l_ntiles); F(e->dbg_hidden_f32);
   for (auto& L : e->ll) {
-    F(L.wqd); F(L.ukT); F(L.uv); F(L.wo); F(L.up); F(L.down); F(L.gain1); F(L.gain2); F(L.lat_gain); F(L.sink); F(L.router); F(L.corr);
+    if (!L.uv_in_ukv) F(L.uv);
+    F(L.wqd); F(L.ukT); F(L.wo); F(L.up); F(L.down); F(L.gain1); F(L.gain2); F(L.lat_gain); F(L.sink); F(L.router); F(L.corr);
     F(L.gain1b); F(L.gain2b); F(L.qkv_bias); F(L.o_bias); F(L.conv_w); F(L.talk); F(L.vmix); F(L.conv_ring);
     F(L.wo2); F(L.sh_up); F(L.sh_down); F(L.qk_gain); F(L.head_gain); F(L.a2); F(L.a2_bias); F(L.g2); F(L.a_log); F(L.out_gain_l); F(L.out_gain_r); F(L.poly);
     F(L.bias1); F(L.bias1b); F(L.bias2); F(L.bias2b); F(L.latq_gain); F(L.uq); F(L.ukv); F(L.router_op); F(L.table);

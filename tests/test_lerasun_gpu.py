@@ -479,3 +479,30 @@ def test_rebuilt_form_reports_a_wait_that_ran_out(monkeypatch):
         for n in (130, 640):
             with pytest.raises(pkg().B2Error, match="did not end within 0 ms"):
                 e.prefill([e.seq_create(n)], [tokens(cfg, n, 51)])
+
+
+def wide(heads, kv_from=None, rot=64, scale=0.05):
+    return layer(mixer(heads, 128, rot, 128, 128, scale, kv_from=kv_from), None)
+
+
+def test_too_little_memory_for_the_rebuilt_form():
+    """An engine that fits without the rebuilt form's buffers is not refused: its long portions take the absorbed form, whose logits do not depend on the cut."""
+    cfg = {"architecture": "Lerasun", "vocab": 211, "width": 96, "logit_scale": 1.0, "norm": {"eps": 1e-6}, "layers": [wide(160)]}
+    w = random_weights(cfg, seed=45)
+    toks = tokens(cfg, 150, 46)
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    room = 1536 << 20     # the buffers for contexts of 16384 tokens: 2.7 GB; all else about 0.2
+    held = torch.empty(max(0, free - room), dtype=torch.uint8, device="cuda")
+    try:
+        with engine(cfg, w, f32=False, max_model_len=16384, num_blocks=40, max_seqs=2, max_batch_tokens=256) as e:
+            whole, _ = e.prefill_logits([e.seq_create(150)], [toks], list(range(150)))
+            sid = e.seq_create(150)
+            x, _ = e.prefill_logits([sid], [toks[:80]], list(range(80)))
+            y, _ = e.prefill_logits([sid], [toks[80:]], list(range(70)))
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    assert (np.concatenate([x, y]) == whole).all()
+    ref = Oracle(cfg, w).forward(toks).numpy()
+    assert np.abs(whole - ref).max() / np.abs(ref).max() < BF16_BAR
