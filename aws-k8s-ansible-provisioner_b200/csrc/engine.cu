@@ -5472,7 +5472,9 @@ void latent_context_add(b2_engine* e, int i, int len, int n, int row0) {
   const int x = g.ctx0 + g.nctx++;
   e->h_xctx[x] = LatentContext{i, len + n, g.pages, pages};
   int32_t* bt = e->h_xtable + (size_t)x * e->bt_stride;
-  for (int p = 0; p < e->bt_stride; ++p) bt[p] = p < pages ? g.pages + p : 0;   // (past the end: the group's first page, masked)
+  // past the end: a page that no group's pools have, whose copies bring zeros (another request's page would reach this one's rows: its values are multiplied by
+  // weights of 0, which is not 0 for an infinity)
+  for (int p = 0; p < e->bt_stride; ++p) bt[p] = p < pages ? g.pages + p : e->lx_pages_cap;
   for (int j = 0; j < n; j += 64) e->h_xtiles[g.tile0 + g.ntiles++] = PrefillTile{row0 + j, len + j, std::min(64, n - j), x};
   if (g.ntiles & 1) e->h_xtiles[g.tile0 + g.ntiles++] = PrefillTile{row0, len + n, 0, x};   // tiles 2i and 2i + 1 belong to one sequence
   g.pages += pages;

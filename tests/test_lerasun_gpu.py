@@ -506,3 +506,16 @@ def test_too_little_memory_for_the_rebuilt_form():
     assert (np.concatenate([x, y]) == whole).all()
     ref = Oracle(cfg, w).forward(toks).numpy()
     assert np.abs(whole - ref).max() / np.abs(ref).max() < BF16_BAR
+
+
+def test_rebuilt_contexts_of_one_step_stay_apart():
+    """Two long portions in one step, keys and values of both rebuilt side by side: what is behind a context's end belongs to nobody, so a request whose first token is
+    not finite changes nothing in the other's logits."""
+    cfg = {"architecture": "Lerasun", "vocab": 211, "width": 96, "logit_scale": 1.0, "norm": {"eps": 1e-6}, "layers": [wide(4)]}
+    w = random_weights(cfg, seed=40)
+    w["embed"][210] = float("inf")
+    a, b = [210] + [t % 210 for t in tokens(cfg, 149, 41)], [t % 210 for t in tokens(cfg, 130, 42)]
+    with engine(cfg, w, f32=False) as e:
+        both, _ = e.prefill_logits([e.seq_create(150), e.seq_create(130)], [a, b], list(range(280)))
+        assert err(both[150:], Oracle(cfg, w).forward(b).numpy()) < BF16_BAR
+        assert not np.isfinite(both[:150]).any()
