@@ -1989,10 +1989,9 @@ __global__ void __launch_bounds__(PX_THREADS, NC == 8 ? 2 : 1) heads_attention_p
   auto cache_row = [&](int kp) { return kp <= pos_hi ? bt[kp / a.block_size] * a.block_size + kp % a.block_size : -1; };
   if (tid < PX_KEYS) key_row[tid] = cache_row(k_first + tid);
   float m_run = -INFINITY, l_run = 0.f;   // of row `warp`, head lane mod PC_HEADS
-  const float exp_scale = g.softcap > 0.f ? g.scale * 2.0f * 1.4426950408889634f / g.softcap : 0.f, minus_two_cap = -2.0f * g.softcap;
-  auto finish_score = [&](float v) {   // scale, cap: cap * tanh(s / cap) as cap - 2 cap / (2^(s * 2 log2(e) / cap) + 1)
-    if (g.softcap > 0.f) return g.softcap + __fdividef(minus_two_cap, fast_exp2(v * exp_scale) + 1.0f);
-    return v * g.scale;
+  const float per_cap = g.softcap > 0.f ? g.scale / g.softcap : 0.f;
+  auto finish_score = [&](float v) {   // scale, cap (cap - 2 cap / (e^(2 s / cap) + 1) would lose the small scores of a high cap: 0.001 at a cap of 10 000)
+    return g.softcap > 0.f ? g.softcap * tanhf(v * per_cap) : v * g.scale;
   };
   int cur = 0;
   for (int k0 = k_first; k0 <= pos_hi; k0 += PX_KEYS, cur ^= 1) {

@@ -604,3 +604,15 @@ def test_a_trace_replayed_through_the_command_line(tmp_path):
     rd = lambda i: np.fromfile(str(out / ("%d.f32" % i)), dtype="<f4").reshape(-1, cfg["vocab"])
     assert err(rd(0), ra[[0, 69]]) < F32_BAR and err(rd(1), rb[[19]]) < F32_BAR
     assert err(rd(2), np.stack([ra[72], rb[20]])) < F32_BAR and err(rd(3), ra[[89]]) < F32_BAR and err(rd(4), rb[[20]]) < F32_BAR
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(24, 8, 48, 96), (20, 4, 64, 128)])
+@pytest.mark.parametrize("cap,rot,factor", [(None, None, 1.0), (None, (3000.0, 16, 2.0), 3.0), (2.0, (3000.0, 16, None), 6.0), (1e8, None, 1.0)])
+def test_bf16_head_mixed_attention_on_clusters_caps(heads, kv, dim, vdim, cap, rot, factor):
+    """The cluster form without a cap and without rotation, with scores far beyond a low cap, and with a cap so high that it must change nothing."""
+    cfg = model([(att(heads, kv, dim, vdim, dim ** -0.5, rot=rot, cap=cap), None)], vocab=211, width=96)
+    w = sharpen(cfg, random_weights(cfg, seed=60), factor=factor)
+    w["l0.mix.talk"] = (torch.randn(heads, heads, generator=torch.Generator().manual_seed(61)) * heads ** -0.5).to(torch.bfloat16).float()
+    toks = tokens(cfg, 70, 62)
+    with engine(cfg, w, f32=False) as e:
+        run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), BF16_BAR, [41, 27], 68)
