@@ -2541,12 +2541,14 @@ int launch_heads_finish(const float* proj, int ld, const HeadsGeom& g, const flo
   const int C = g.heads * g.dim + g.kv_heads * (g.dim + g.vdim);
   const size_t smem = ((size_t)4 * std::max(g.dim, g.vdim) + std::max(g.rot_dims, 2)) * sizeof(float);
   B2_REQUIRE(smem <= 200 * 1024, "heads_finish: a head of %d numbers exceeds shared memory", std::max(g.dim, g.vdim));
-  // Sizes and addresses that the 16-byte form can read; everything else takes a number at a time.  Prompt-sized steps: four tokens per CTA of eight warps,
-  // a head per warp until the tokens alone give every SM several CTAs; short steps: a token and four heads per CTA.
+  // Sizes and addresses that the 16-byte form can read; everything else takes a number at a time.  Long steps: four tokens per CTA of eight warps, a head per
+  // warp, from 2048 tokens on all heads in one CTA; short steps: a token and four heads per CTA.  32 heads of 128, us for a token and four heads / four tokens and
+  // eight heads / four tokens and all: 256 tokens 11.9 / 14.5 / 18.2; 512: 15.7 / 19.0 / 23.6; 1024: 20.3 / 18.7 / 26.1; 2048: 46.2 / 27.8 / 25.8;
+  // 4096: 95.5 / 41.5 / 38.0.
   auto ok16 = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (g.dim % 4 == 0 && g.vdim % 4 == 0 && g.dim <= 128 && g.vdim <= 128 && ld % 4 == 0 && (g.conv_taps == 0 || g.conv_taps == 4) && ok16(proj) && ok16(bias) &&
       ok16(conv_w) && ok16(ring) && ok16(v_first) && ok16(q_out) && ok16(k_cache) && ok16(v_cache) && ok16(q_bf16)) {
-    const int vunits = g.heads + 2 * g.kv_heads, tpc = T >= 256 ? 4 : 1, vupc = tpc == 1 ? 4 : T >= 4096 ? vunits : 8;
+    const int vunits = g.heads + 2 * g.kv_heads, tpc = T >= 1024 ? 4 : 1, vupc = tpc == 1 ? 4 : T >= 2048 ? vunits : 8;
     const dim3 vgrid((T + tpc - 1) / tpc, (vunits + vupc - 1) / vupc);
     const size_t vsmem = (size_t)tpc * g.rot_dims * sizeof(float);   // (at most 2 KB)
 #define HV_LAUNCH(TC, TAPS, TPC, Q16)                                                                                                                    \

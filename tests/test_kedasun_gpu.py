@@ -574,15 +574,15 @@ def test_fp32_prompt_attention_tiles(mixer, T):
 
 
 @pytest.mark.parametrize("f32", [True, False])
-@pytest.mark.parametrize("n", [1, 130, 255, 256, 257, 262])
+@pytest.mark.parametrize("n", [1, 130, 255, 256, 257, 262, 1017, 1018, 1019, 1020, 1021, 2045])
 def test_projection_finish_in_groups_of_tokens(n, f32):
-    """What follows the fused projection, at the edges of its groups of four tokens (from 256 rows on): a convolution that looks back into the portion before, into
+    """What follows the fused projection, a token per CTA and (from 1024 rows on) in groups of four, at the edges of a group: a convolution that looks back into the portion before, into
     the state of another sequence's slot and past a sequence's first token inside a group; heads that fill a warp and heads that do not."""
     cfg = model([(att2(4, 2, 128, 128, 0.5, 4, window=40, keep=3), None), (att(4, 2, 20, 128, 0.2, rot=6), None), (att(4, 2, 128, 128, 0.09, rot=64), None)], vocab=61, width=96, groups=3)
     w = random_weights(cfg, seed=94)
     a, b = tokens(cfg, 2 + n, 95), tokens(cfg, 7, 96)
     ra, rb = ref_logits(cfg, w, a), ref_logits(cfg, w, b)
-    with engine(cfg, w, f32=f32) as e:
+    with engine(cfg, w, f32=f32, max_batch_tokens=2064, max_model_len=2064, num_blocks=160) as e:
         sa, sb = e.seq_create(len(a)), e.seq_create(len(b))
         x, _ = e.prefill_logits([sa, sb], [a[:2], b[:1]], [0, 1, 2])
         y, _ = e.prefill_logits([sb, sa], [b[1:], a[2:]], list(range(6 + n)))
