@@ -271,8 +271,9 @@ int launch_f32_tile(const AnyGemm& g, dim3 grid, cudaStream_t s) {
 int launch_gemm_f32(const AnyGemm& g, int batch, int max_tiles, cudaStream_t s) {
   if (g.tile_group != nullptr) return launch_f32_tile<64, 128>(g, dim3(max_tiles, (g.N + 127) / 128, 1), s);
   const int z = batch > 0 ? batch : 1;
+  static const int sms = device_num_sms();
   auto cost = [&](int tm, int tn, double handicap) {
-    const long tiles = (long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * z, per_sm = (tiles + 147) / 148;
+    const long tiles = (long)((g.M + tm - 1) / tm) * ((g.N + tn - 1) / tn) * z, per_sm = (tiles + sms - 1) / sms;
     return handicap * (double)tm * tn * (double)(tm * tn == 64 * 64 && per_sm < 2 ? 2 : per_sm);
   };
   const double big = cost(128, 128, 1.0), mid = cost(64, 128, 1.03), small = cost(64, 64, 1.1);
