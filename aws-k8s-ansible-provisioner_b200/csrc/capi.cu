@@ -63,12 +63,27 @@ extern "C" int b2k_linear(const void* x, const void* w, void* out, int out_is_f3
   return launch_linear_tc(a, (cudaStream_t)stream);
 }
 
+// The kernel hooks below do not synchronise: a wait that ran out is reported by the next call of such a hook.
+static int hook_waits(B2WaitLimit* w) {
+  static uint32_t* word = [] {
+    uint32_t* p = nullptr;
+    if (cudaMallocHost(&p, sizeof(uint32_t)) == cudaSuccess) *p = 0;
+    return p;
+  }();
+  B2_REQUIRE(word != nullptr, "no pinned memory for the kernels' wait word");
+  B2_REQUIRE(*(volatile uint32_t*)word == 0, "a wait of an earlier call's kernel ran out");
+  *w = B2WaitLimit{word, 2000};
+  return 0;
+}
+
 extern "C" int b2k_linear_multicast(const void* x, const void* w, void* out, int T, int N, int K, void* stream) {
   B2_REQUIRE(x && w && out, "b2k_linear_multicast: null pointer");
+  B2WaitLimit wait;
+  CAPI_TRY(hook_waits(&wait));
   CUtensorMap tw, tx;
   CAPI_TRY(b2_make_tmap_bf16(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)K, 128));
   CAPI_TRY(b2_make_tmap_bf16(&tx, x, (uint64_t)T, (uint64_t)K, (uint64_t)K, 128));
-  return launch_linear_mc(tw, tx, (bf16*)out, T, N, K, 0, (cudaStream_t)stream);
+  return launch_linear_mc(tw, tx, (bf16*)out, T, N, K, 0, wait, (cudaStream_t)stream);
 }
 
 extern "C" int b2k_linear_add(const void* x, const void* w, void* h, int T, int N, int K, void* stream) {
@@ -116,9 +131,11 @@ extern "C" int b2k_qkv_rope(const void* x, const void* w_qkv, const void* qnorm_
   CAPI_TRY(b2_make_tmap_bf16(&tm, w_qkv, (uint64_t)(nq + 2 * nkv) * 128, (uint64_t)K, (uint64_t)K, 128));
   if (T > 64) {  // prefill-sized: gemm_mc.cu, ROPE variant
     CUtensorMap tx;
+    B2WaitLimit wait;
+    CAPI_TRY(hook_waits(&wait));
     CAPI_TRY(b2_make_tmap_bf16(&tx, x, (uint64_t)T, (uint64_t)K, (uint64_t)K, 128));
     return launch_qkv_rope_prefill(tm, tx, (const bf16*)qnorm_w, (const bf16*)knorm_w, (const bf16*)cos_sin, positions, slots, (bf16*)q_out,
-                                   (bf16*)k_pages, (bf16*)v_pages, T, nq, nkv, K, block_size, eps, 0, (cudaStream_t)stream);
+                                   (bf16*)k_pages, (bf16*)v_pages, T, nq, nkv, K, block_size, eps, 0, wait, (cudaStream_t)stream);
   }
   return launch_qkv_rope(tm, (const bf16*)x, (const bf16*)qnorm_w, (const bf16*)knorm_w, (const bf16*)cos_sin, positions, slots, (bf16*)q_out,
                          (bf16*)k_pages, (bf16*)v_pages, T, nq, nkv, K, block_size, eps, (cudaStream_t)stream);

@@ -308,11 +308,11 @@ struct b2_engine {
   int l2_weight_prefetch = 0;  // B2_WPF: resid path, see forward_layers (measured slower: off)
   int prefill_resid_fused = 0;  // B2_RESID_FUSED: prefill O / down projections add into the residual stream in their epilogue (measured slower: off)
   int qkv_rope_prefill_fused = 1;  // B2_QKV_ROPE_FUSED: prefill QKV projection finishes norm / RoPE / page write itself
-  uint32_t* h_ran_out = nullptr;     // host word that the prompt attention sets when one of its waits ran out
+  uint32_t* h_ran_out = nullptr;     // host word that a prompt kernel sets when one of its waits ran out
   int prefill_wait_ms = 2000;        // B2_PREFILL_WAIT_MS: how long such a wait may last (0: none may, for tests)
   B2WaitLimit wait_limit() const { return B2WaitLimit{h_ran_out, prefill_wait_ms}; }
   int prefill_pairs = 1;  // B2_PREFILL_PAIRS: see prefill_tile_pairs()
-  int prefill_mc = 1;  // B2_MC: prefill projections as multicast CTA pairs (gemm_mc.cu)
+  int prefill_mc = 1;  // B2_MC: prefill projections on pairs of CTAs (gemm_mc.cu)
   int gu_prefill_fused = 1;  // B2_GU_FUSED: prefill-sized gate/up projection with SwiGLU in its epilogue (gemm_gateup.cu)
   int use_pair = 1;   // B2_PAIR: bit 0 gate/up + SwiGLU, bit 1 QKV + QK-norm/RoPE/KV write as fused cluster-pair launches (gemm_pair.cu)
 
@@ -533,7 +533,7 @@ ActIn linear(b2_engine* e, const Lane& ln, int cls, XBuf xb, const bf16* xptr, c
     }
     if (e->prefill_mc && a.bn == 256 && linear_mc_shapes_ok(T, N, K) && !pf.k_pages) {
       // prefill shapes: pairs of CTAs share the token tile (gemm_mc.cu); same arithmetic, a third less L2 -> shared-memory traffic
-      if (!k.skip()) *rc = launch_linear_mc(tm_w, e->tm_x[xb][bn_index(128)], out_bf16, T, N, K, ln.row0, ln.stream);
+      if (!k.skip()) *rc = launch_linear_mc(tm_w, e->tm_x[xb][bn_index(128)], out_bf16, T, N, K, ln.row0, e->wait_limit(), ln.stream);
       return act_bf16(out_bf16);
     }
     if (!k.skip()) *rc = launch_linear_tc(a, ln.stream);
@@ -860,7 +860,7 @@ int forward_layers(b2_engine* e, const Lane& ln, int T, int ntiles) {
     if (qkv_prefill_fused) {
       KL k(e, B2K_GEMM_QKV);  // prefill: QK-norm + RoPE + page write in the QKV projection's epilogue (gemm_mc.cu)
       B2_TRY(launch_qkv_rope_prefill(L.tm_qkv, e->tm_x[XB_X][bn_index(128)], L.qnorm, L.knorm, e->cos_sin, positions, slots, qrot, kp, vp, T, e->nq,
-                                     e->nkv, H, c.block_size, c.rms_eps, ln.row0, st));
+                                     e->nkv, H, c.block_size, c.rms_eps, ln.row0, e->wait_limit(), st));
     } else if (qkv_pair) {
       KL k(e, B2K_GEMM_QKV);
       if (!k.skip())
@@ -5532,6 +5532,14 @@ int read_bf16_rows(b2_engine* e, float* dst, const bf16* src, size_t n) {
   return 0;
 }
 
+// After the stream was synchronised: did a wait of a kernel run out?
+int check_waits(b2_engine* e, const char* what) {
+  if (*(volatile uint32_t*)e->h_ran_out == 0) return 0;
+  *(volatile uint32_t*)e->h_ran_out = 0;
+  b2_set_error("%s: a wait of a kernel did not end within %d ms; the results are not valid", what, e->prefill_wait_ms);
+  return -110;
+}
+
 int prefill_impl(b2_engine* e, const int32_t* ids, const int32_t* seq_offsets, int32_t nseq, const int32_t* seq_ids, const int32_t* rows,
                  int32_t nrows, float* out_logits, int32_t* out_tokens) {
   B2_REQUIRE(e && ids && seq_offsets && seq_ids && nseq >= 1, "b2_prefill: bad arguments");
@@ -5655,11 +5663,7 @@ int prefill_impl(b2_engine* e, const int32_t* ids, const int32_t* seq_offsets, i
     B2_CUDA_OK(cudaMemcpyAsync(out_logits, e->l_logits + (size_t)nseq * e->cfg.vocab, (size_t)nrows * e->cfg.vocab * 4, cudaMemcpyDeviceToHost,
                                e->stream));
   B2_CUDA_OK(cudaStreamSynchronize(e->stream));
-  if (*(volatile uint32_t*)e->h_ran_out != 0) {   // (none of the portions counts as written, none is registered in the prefix cache: the caller frees its sequences)
-    *(volatile uint32_t*)e->h_ran_out = 0;
-    b2_set_error("b2_prefill: a wait of the prompt attention did not end within %d ms; the call's results are not valid", e->prefill_wait_ms);
-    return -110;
-  }
+  B2_TRY(check_waits(e, "b2_prefill"));   // (none of the portions counts as written then, none is registered in the prefix cache: the caller frees its sequences)
   for (int i = 0; i < nseq; ++i) {
     Seq& s = e->seqs[seq_ids[i]];
     const int n = seq_offsets[i + 1] - seq_offsets[i] - skip[i];
@@ -5749,6 +5753,7 @@ extern "C" int b2_decode_step(b2_engine* e, int32_t nseq, const int32_t* seq_ids
   if (out_tokens) {
     B2_CUDA_OK(cudaMemcpyAsync(e->h_out, e->d_out_tokens, nseq * 4, cudaMemcpyDeviceToHost, e->stream));
     B2_CUDA_OK(cudaStreamSynchronize(e->stream));
+    B2_TRY(check_waits(e, "b2_decode_step"));   // (steps of 512 sequences and more take prompt kernels)
     memcpy(out_tokens, e->h_out, nseq * 4);
     for (int i = 0; i < nseq; ++i) {
       e->seqs[seq_ids[i]].next_token = e->h_out[i];
@@ -5786,6 +5791,7 @@ extern "C" int b2_decode_run(b2_engine* e, int32_t nseq, const int32_t* seq_ids,
   for (; done < steps; ++done) B2_TRY(run_decode_step(e, B, split));
   B2_CUDA_OK(cudaEventRecord(ev1, e->stream));
   B2_CUDA_OK(cudaStreamSynchronize(e->stream));
+  B2_TRY(check_waits(e, "b2_decode_run"));
   if (elapsed_ms) B2_CUDA_OK(cudaEventElapsedTime(elapsed_ms, ev0, ev1));
   for (int i = 0; i < nseq; ++i) e->seqs[seq_ids[i]].len += steps;
   e->last_n = nseq;

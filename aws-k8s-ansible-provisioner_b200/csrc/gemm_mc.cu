@@ -1,17 +1,16 @@
-// gemm_mc.cu -- prefill-sized projection y[T][N] = x[T][K] . W[N][K]^T (bf16 out) with the token operand SHARED between
-// the two CTAs of a cluster (HF nn.Linear, models/qwen3/modeling_qwen3.py:236-247).
+// gemm_mc.cu -- prefill-sized projection y[T][N] = x[T][K] . W[N][K]^T (bf16 out) on PAIRS of CTAs that multiply one
+// 256 x 256 tile together (HF nn.Linear, models/qwen3/modeling_qwen3.py:236-247).
 //
 // Why: the persistent 128 x 256 tile kernel of gemm_tc.cu moves 48 KB from L2 into shared memory per 64-wide k-block
 // (16 KB of weights + 32 KB of tokens) for 532 cycles of tcgen05.mma: 90 bytes per cycle and SM, more than an SM gets
 // from L2 when all 148 ask at once -- ncu shows the tensor pipe 52-68 % active and the share rising with K, i.e. with the
-// weight of the main loop (profiles/qwen3_b_prefill_full_raw.csv).  Here two CTAs take two ADJACENT weight-row tiles of the same
-// 256-token tile: each loads its own 16 KB of weights and only HALF of the token rows (16 KB), and the TMA engine writes that
-// half into BOTH CTAs' shared memory (cp.async.bulk.tensor ... .multicast::cluster; the tensor maps cover this GPU's memory
-// only).  32 KB per k-block and SM instead of 48.
-//   * full barrier of a stage (per CTA): one arrive.expect_tx of 48 KB by the CTA's own producer; bytes arrive from its own
-//     weight load, its own token half and the peer's token half
-//   * empty barrier of a stage (per CTA): TWO arrivals -- the stage is rewritten by the peer's multicast too, so both CTAs'
-//     MMAs must have read it: each MMA thread commits with .multicast::cluster to the barrier of both CTAs
+// weight of the main loop (profiles/qwen3_b_prefill_full_raw.csv).  Here the two CTAs of a cluster take two ADJACENT weight-row
+// tiles of the same 256-token tile: each loads its own 16 KB of weights and HALF of the token rows (16 KB), and the MMA of the
+// pair (cta_group::2, M = 256) reads both halves where they are.  32 KB per k-block and SM instead of 48, every byte loaded once.
+//   * full barrier of a stage (the first CTA's): one arrive.expect_tx of 64 KB by its producer; the bytes of both CTAs' loads
+//     are counted there
+//   * empty barrier of a stage (per CTA) and "accumulator full" (per CTA): one arrival, the first CTA's MMA thread commits to both
+//   * "accumulator empty" (the first CTA's): a lane of every epilogue warp of both CTAs
 // Everything else is gemm_tc.cu's plain bf16 path: swap-AB (weight rows on MMA-M, tokens on MMA-N), double-buffered TMEM
 // accumulator, four epilogue warps, same k order -> the same bits (tests/test_kernels_gpu.py::test_linear_multicast).
 #include "kernels.h"
@@ -23,8 +22,8 @@ namespace {
 constexpr int MC_BM = 128, MC_BN = 256, MC_BK = 64;
 constexpr int MC_W_BYTES = MC_BM * MC_BK * 2;       // 16 KB
 constexpr int MC_XH_BYTES = (MC_BN / 2) * MC_BK * 2;  // 16 KB: one CTA's half of the token tile
-constexpr int MC_STAGE_BYTES = MC_W_BYTES + 2 * MC_XH_BYTES;
-constexpr int MC_STAGES = 4;
+constexpr int MC_STAGE_BYTES = MC_W_BYTES + MC_XH_BYTES;
+constexpr int MC_STAGES = 6;
 constexpr int MC_OUT_ROWS = 32;                               // tokens per output staging buffer
 constexpr int MC_OUT_BYTES = MC_OUT_ROWS * MC_BM * 2;         // 8 KB: [32 tokens][128 features] bf16
 constexpr int MC_SMEM_BYTES = MC_STAGES * MC_STAGE_BYTES + 2 * MC_OUT_BYTES + 1024;
@@ -37,16 +36,33 @@ __device__ __forceinline__ uint32_t mc_cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void mc_tma_load_2d_multicast(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, uint32_t bar, uint16_t mask) {
+__device__ __forceinline__ uint32_t mc_first_cta(uint32_t addr) {   // the same place in the first CTA's shared memory
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+// into this CTA's shared memory; the bytes are counted on a barrier of either CTA of the pair
+__device__ __forceinline__ void mc_tma_load_2d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst_smem), "l"(tmap), "r"(bar),
+               "r"(c0), "r"(c1)
+               : "memory");
+}
+// D[256 x 256, 128 rows in each CTA's TMEM] (+)= A[256] * B[256]: each CTA's shared memory holds 128 rows of A and 128 of B
+__device__ __forceinline__ void mc_mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%3, %4}], [%2], %5;" ::"r"(
-          dst_smem),
-      "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "h"(mask)
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+      "}\n" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ void mc_commit_multicast(uint32_t bar, uint16_t mask) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"(mask)
-               : "memory");
+__device__ __forceinline__ void mc_commit(uint32_t bar) {   // to the barrier of both CTAs
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void mc_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ void mc_cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -71,13 +87,15 @@ struct McRope {
 template <bool ROPE>
 __global__ void __launch_bounds__(ROPE ? MC_ROPE_THREADS : 192, 1)
 linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_out,
-                 int T, int N, int K, int m_pairs, int n_tiles, int x_row0, const McRope rp) {
+                 int T, int N, int K, int m_pairs, int n_tiles, int x_row0, const McRope rp, const B2WaitLimit limit) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[MC_STAGES];
   __shared__ __align__(8) uint64_t empty_bar[MC_STAGES];
   __shared__ __align__(8) uint64_t tmem_full_bar[2];
   __shared__ __align__(8) uint64_t tmem_empty_bar[2];
+  __shared__ __align__(8) uint64_t drained;
   __shared__ uint32_t tmem_slot;
+  __shared__ volatile uint32_t gave_up;
   __shared__ int s_pos[ROPE ? MC_BN : 1], s_slot[ROPE ? MC_BN : 1];  // positions / cache slots of the tile's tokens
   __shared__ __align__(16) bf16 s_gain[ROPE ? 256 : 8];             // QK-norm gains, q then k
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -90,74 +108,79 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < MC_STAGES; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
-      mbar_init(smem_u32(&empty_bar[s]), 2);  // this CTA's MMAs and the peer's
+      mbar_init(smem_u32(&empty_bar[s]), 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(smem_u32(&tmem_full_bar[a]), 1);
-      mbar_init(smem_u32(&tmem_empty_bar[a]), ROPE ? MC_ROPE_THREADS - 64 : 128);
+      mbar_init(smem_u32(&tmem_empty_bar[a]), 2 * (ROPE ? MC_ROPE_THREADS - 64 : 128) / 32);
     }
+    mbar_init(smem_u32(&drained), 1);
+    gave_up = 0;
     mbar_fence_init();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_slot), 512);
-    tmem_relinquish();
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_slot)) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
-  mc_cluster_sync();  // the peer's barriers exist before anything of mine can arrive on them
+  const B2Waits wait{&gave_up, limit};
+  mc_cluster_sync();  // the peer's barriers exist before anything of mine can arrive on them, and its TMEM is taken
   pdl_wait();
   if (threadIdx.x == 0) pdl_launch_dependents();
+  int sent = 0;   // (producer: stages filled)
 
-  if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmap_w);
-      tma_prefetch_desc(&tmap_x);
-      int it = 0;
-      for (int p = cluster; p < total; p += clusters) {
-        const int m_tile = 2 * (p % m_pairs) + (int)rank, n_tile = p / m_pairs;
-        for (int kb = 0; kb < kb_total; ++kb, ++it) {
-          const int s = it % MC_STAGES;
-          mbar_wait(smem_u32(&empty_bar[s]), ((it / MC_STAGES) & 1) ^ 1);  // both CTAs are done with this stage
-          const uint32_t fb = smem_u32(&full_bar[s]);
-          mbar_arrive_expect_tx(fb, MC_STAGE_BYTES);
-          const uint32_t ws = smem_base + s * MC_STAGE_BYTES;
-          tma_load_2d(ws, &tmap_w, kb * MC_BK, m_tile * MC_BM, fb);
-          // my half of the token rows, into the same place of both CTAs' stage; the bytes are counted on both full barriers
-          mc_tma_load_2d_multicast(ws + MC_W_BYTES + rank * MC_XH_BYTES, &tmap_x, kb * MC_BK, n_tile * MC_BN + (int)rank * (MC_BN / 2) + x_row0, fb,
-                                   (uint16_t)3);
-        }
+  auto produce = [&]() {   // (one thread)
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+    for (int p = cluster; p < total; p += clusters) {
+      const int m_tile = 2 * (p % m_pairs) + (int)rank, n_tile = p / m_pairs;
+      for (int kb = 0; kb < kb_total; ++kb) {
+        const int s = sent % MC_STAGES;
+        if (!wait(empty_bar[s], ((sent / MC_STAGES) & 1) ^ 1)) return;  // the pair's MMAs are done with this stage
+        const uint32_t fb = mc_first_cta(smem_u32(&full_bar[s]));
+        if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * MC_STAGE_BYTES);
+        const uint32_t ws = smem_base + s * MC_STAGE_BYTES;
+        mc_tma_load_2d(ws, &tmap_w, kb * MC_BK, m_tile * MC_BM, fb);
+        mc_tma_load_2d(ws + MC_W_BYTES, &tmap_x, kb * MC_BK, n_tile * MC_BN + (int)rank * (MC_BN / 2) + x_row0, fb);   // this CTA's half of the token rows
+        ++sent;
       }
-      // tail: the releases of the last stages (this CTA's MMAs and the PEER's, which arrive through the cluster network) have
-      // landed on my barriers before this CTA goes to the final cluster barrier and exits
-      for (int j = it > MC_STAGES ? it - MC_STAGES : 0; j < it; ++j) mbar_wait(smem_u32(&empty_bar[j % MC_STAGES]), (j / MC_STAGES) & 1);
     }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = umma_idesc_bf16(MC_BM, MC_BN);
-      int it = 0, lt = 0;
-      for (int p = cluster; p < total; p += clusters, ++lt) {
-        const int as = lt & 1;
-        mbar_wait(smem_u32(&tmem_empty_bar[as]), ((lt >> 1) & 1) ^ 1);
+    // tail: the releases of the last stages have landed on this CTA's barriers before it goes to the final cluster barrier and exits
+    for (int j = max(0, sent - MC_STAGES); j < sent; ++j)
+      if (!wait(empty_bar[j % MC_STAGES], (j / MC_STAGES) & 1)) return;
+  };
+  auto multiply = [&]() {   // (one thread of the first CTA)
+    constexpr uint32_t idesc = umma_idesc_bf16(2 * MC_BM, MC_BN);
+    int it = 0, lt = 0;
+    for (int p = cluster; p < total; p += clusters, ++lt) {
+      const int as = lt & 1;
+      if (!wait(tmem_empty_bar[as], ((lt >> 1) & 1) ^ 1)) return;
+      tc_fence_after();
+      const uint32_t tmem_d = tmem_base + (uint32_t)(as * MC_BN);
+      for (int kb = 0; kb < kb_total; ++kb, ++it) {
+        const int s = it % MC_STAGES;
+        if (!wait(full_bar[s], (it / MC_STAGES) & 1)) return;
         tc_fence_after();
-        const uint32_t tmem_d = tmem_base + (uint32_t)(as * MC_BN);
-        for (int kb = 0; kb < kb_total; ++kb, ++it) {
-          const int s = it % MC_STAGES;
-          mbar_wait(smem_u32(&full_bar[s]), (it / MC_STAGES) & 1);
-          tc_fence_after();
-          const uint32_t ws = smem_base + s * MC_STAGE_BYTES;
-          const uint64_t da = umma_desc_sw128(ws);
-          const uint64_t db = umma_desc_sw128(ws + MC_W_BYTES);  // 256 token rows: the two halves are contiguous
+        const uint32_t ws = smem_base + s * MC_STAGE_BYTES;
+        const uint64_t da = umma_desc_sw128(ws), db = umma_desc_sw128(ws + MC_W_BYTES);
 #pragma unroll
-          for (int k = 0; k < MC_BK / 16; ++k)
-            tc_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-          mc_commit_multicast(smem_u32(&empty_bar[s]), (uint16_t)3);
-        }
-        tc_commit(smem_u32(&tmem_full_bar[as]));
+        for (int k = 0; k < MC_BK / 16; ++k)
+          mc_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        mc_commit(smem_u32(&empty_bar[s]));
       }
+      mc_commit(smem_u32(&tmem_full_bar[as]));
     }
-  } else {
+  };
+  // a warp's share of the accumulator is in registers: back to the MMA thread, which waits for both CTAs' warps
+  auto hand_back = [&](int as) {
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mc_arrive_cluster(mc_first_cta(smem_u32(&tmem_empty_bar[as])));
+  };
+  auto finish = [&]() {
     if constexpr (!ROPE) {
     // ---- epilogue: the tile leaves through shared memory and TMA stores, 32 tokens x 128 features (8 KB) at a time ----
     // Thread = weight row (TMEM lane), registers = tokens, memory = [token][feature]: written directly, a tile is 32 768
@@ -174,7 +197,7 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     for (int p = cluster; p < total; p += clusters, ++lt) {
       const int m_tile = 2 * (p % m_pairs) + (int)rank, n_tile = p / m_pairs;
       const int as = lt & 1;
-      mbar_wait(smem_u32(&tmem_full_bar[as]), (lt >> 1) & 1);
+      wait.warp(tmem_full_bar[as], (lt >> 1) & 1);   // (run out: the warps go on to the end together, past their barriers)
       tc_fence_after();
       const int tok0 = n_tile * MC_BN;
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * MC_BN);
@@ -184,8 +207,7 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         tmem_ld32(tbase + (uint32_t)c0, r);
         tmem_ld_wait();
         if (c0 + MC_OUT_ROWS == MC_BN) {  // the whole accumulator is in registers or out: hand it back to the MMA warp
-          tc_fence_before();
-          mbar_arrive(smem_u32(&tmem_empty_bar[as]));
+          hand_back(as);
         }
         const int b = chunk & 1;
         // buffer b was last read by the store issued two chunks ago
@@ -232,7 +254,7 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       }
       asm volatile("bar.sync 5, %0;" ::"n"(NE) : "memory");
       const int as = lt & 1;
-      mbar_wait(smem_u32(&tmem_full_bar[as]), (lt >> 1) & 1);
+      wait.warp(tmem_full_bar[as], (lt >> 1) & 1);   // (run out: the warps go on to the end together, past their barriers)
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * MC_BN);
 #pragma unroll 1
@@ -251,8 +273,7 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         tmem_ld16(tbase + (uint32_t)c0, r);
         tmem_ld_wait();
         if (c0 + NG * RB >= MC_BN) {  // this group's last block of the tile: its share of the accumulator is out
-          tc_fence_before();
-          mbar_arrive(smem_u32(&tmem_empty_bar[as]));
+          hand_back(as);
         }
         if (eg == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the group's previous q store has read the buffer
         asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
@@ -331,14 +352,30 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
     }
     if (eg == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
+  };
+  if (warp == 0) {
+    if (lane == 0) produce();
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) multiply();
+  } else {
+    finish();
   }
   tc_fence_before();
   __syncthreads();
-  // no CTA leaves while its peer may still write into its shared memory or arrive on its barriers
+  if (gave_up != 0 && rank == 0 && lane == 0) {   // copies and MMAs of the pair that are under way end before shared memory and TMEM are given back
+    if (warp == 0) {
+      for (int k = max(0, sent - MC_STAGES); k < sent; ++k) b2_drain(full_bar[k % MC_STAGES], (k / MC_STAGES) & 1);
+    } else if (warp == 1) {
+      asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(&drained)) : "memory");
+      b2_drain(drained, 0);
+    }
+  }
+  // no CTA leaves while its peer's loads may still be counted on its barriers, or the pair's MMAs read its shared memory
+  __syncwarp();
   mc_cluster_sync();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
   }
 }
 
@@ -348,7 +385,7 @@ bool linear_mc_shapes_ok(int T, int N, int K) { return T >= 512 && N % (2 * MC_B
 
 template <bool ROPE>
 static int launch_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, const CUtensorMap& tm_out, int T, int N, int K, int x_row0,
-                     const McRope& rp, cudaStream_t s) {
+                     const McRope& rp, const B2WaitLimit& wait, cudaStream_t s) {
   static B2PerDeviceOnce attr_once;
   if (attr_once.need()) B2_CUDA_OK(cudaFuncSetAttribute(linear_mc_kernel<ROPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MC_SMEM_BYTES));
   const int m_pairs = N / (2 * MC_BM), n_tiles = (T + MC_BN - 1) / MC_BN;
@@ -369,12 +406,12 @@ static int launch_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, const 
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = b2_pdl_enabled() ? 2 : 1;
-  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_mc_kernel<ROPE>, tm_w, tm_x128, tm_out, T, N, K, m_pairs, n_tiles, x_row0, rp));
+  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_mc_kernel<ROPE>, tm_w, tm_x128, tm_out, T, N, K, m_pairs, n_tiles, x_row0, rp, wait));
   return 0;
 }
 
 // tm_w: W [N][K], 128-row x 64-column box; tm_x128: X with a 128-row box (NOT the 256-row one of the single-CTA kernel).
-int launch_linear_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* out, int T, int N, int K, int x_row0, cudaStream_t s) {
+int launch_linear_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* out, int T, int N, int K, int x_row0, const B2WaitLimit& wait, cudaStream_t s) {
   if (T <= 0) return 0;
   B2_REQUIRE(linear_mc_shapes_ok(T, N, K), "linear_mc: shape T=%d N=%d K=%d not built", T, N, K);
   CUtensorMap tm_out;  // out [T][N], box 128 features x 32 tokens, no swizzle: the staging buffer's layout
@@ -382,7 +419,7 @@ int launch_linear_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* 
     const int rc = b2_make_tmap_bf16_ex(&tm_out, out, (uint64_t)T, (uint64_t)N, (uint64_t)N, MC_BM, MC_OUT_ROWS, /*swizzle128=*/0);
     if (rc != 0) return rc;
   }
-  return launch_mc<false>(tm_w, tm_x128, tm_out, T, N, K, x_row0, McRope(), s);
+  return launch_mc<false>(tm_w, tm_x128, tm_out, T, N, K, x_row0, McRope(), wait, s);
 }
 
 // Prefill-sized QKV projection + QK-norm + RoPE + K/V page write (Qwen3 geometry: 128-wide heads, norm gains given).
@@ -390,7 +427,7 @@ int launch_linear_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* 
 // q_out are already offset to that row.
 int launch_qkv_rope_prefill(const CUtensorMap& tm_qkv, const CUtensorMap& tm_x128, const bf16* qw, const bf16* kw, const bf16* cos_sin,
                             const int32_t* positions, const int32_t* slots, bf16* q_out, bf16* k_pages, bf16* v_pages, int T, int nq, int nkv,
-                            int K, int block_size, float eps, int x_row0, cudaStream_t s) {
+                            int K, int block_size, float eps, int x_row0, const B2WaitLimit& wait, cudaStream_t s) {
   if (T <= 0) return 0;
   const int N = (nq + 2 * nkv) * 128;
   B2_REQUIRE(linear_mc_shapes_ok(T, N, K) && qw != nullptr && kw != nullptr, "qkv_rope_prefill: T=%d N=%d K=%d not built, or no QK-norm gains", T, N, K);
@@ -400,7 +437,7 @@ int launch_qkv_rope_prefill(const CUtensorMap& tm_qkv, const CUtensorMap& tm_x12
     if (rc != 0) return rc;
   }
   McRope rp = {qw, kw, cos_sin, positions, slots, k_pages, v_pages, nq, nkv, block_size, eps};
-  return launch_mc<true>(tm_qkv, tm_x128, tm_q, T, N, K, x_row0, rp, s);
+  return launch_mc<true>(tm_qkv, tm_x128, tm_q, T, N, K, x_row0, rp, wait, s);
 }
 
 }  // namespace b2

@@ -566,19 +566,21 @@ def test_logits_of_few_and_many_rows(P, nseq):
     eng.close()
 
 
-def test_prefill_reports_a_wait_that_ran_out(P, tiny, monkeypatch):
-    """A prompt attention whose waits run out (here: are given no time) makes the call an error; the caller's other engines are not touched by it."""
+@pytest.mark.parametrize("n", [199, 700])
+def test_prefill_reports_a_wait_that_ran_out(P, tiny, monkeypatch, n):
+    """A prompt kernel whose waits run out (here: are given no time) makes the call an error; the caller's other engines are not touched by it.  Long prompts have their
+    projections on pairs of CTAs."""
     _, sd = tiny
-    prompt = [list(range(1, 200))]
+    prompt = [[1 + i % 300 for i in range(n)]]
     monkeypatch.setenv("B2_PREFILL_WAIT_MS", "0")
-    bad = make_engine(P, QWEN3_TINY, sd, max_model_len=256, num_blocks=32, max_seqs=2, max_batch_tokens=256)
+    bad = make_engine(P, QWEN3_TINY, sd, max_model_len=1024, num_blocks=140, max_seqs=2, max_batch_tokens=1024)
     monkeypatch.delenv("B2_PREFILL_WAIT_MS")
-    good = make_engine(P, QWEN3_TINY, sd, max_model_len=256, num_blocks=32, max_seqs=2, max_batch_tokens=256)
-    want = good.prefill([good.seq_create(200)], prompt)
-    sid = bad.seq_create(200)
+    good = make_engine(P, QWEN3_TINY, sd, max_model_len=1024, num_blocks=140, max_seqs=2, max_batch_tokens=1024)
+    want = good.prefill([good.seq_create(n + 1)], prompt)
+    sid = bad.seq_create(n + 1)
     with pytest.raises(P.B2Error, match="did not end within 0 ms"):
         bad.prefill([sid], prompt)
     bad.seq_free(sid)
-    assert (good.prefill([good.seq_create(200)], prompt) == want).all()
+    assert (good.prefill([good.seq_create(n + 1)], prompt) == want).all()
     bad.close()
     good.close()
