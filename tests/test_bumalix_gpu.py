@@ -610,3 +610,16 @@ def test_rows_held_in_registers(width, ff):
         e.prefill_logits([sid], [toks[:700]], [0])
         part, _ = e.prefill_logits([sid], [toks[700:]], [r - 700 for r in rows])
         assert err(whole, part) < F32_BAR
+
+
+@pytest.mark.parametrize("width,ff", [(512, 4096), (516, 4100), (1020, 8192), (2048, 8196), (2052, 12288), (4096, 12292), (90, 16388)])
+def test_rows_held_in_registers_bf16(width, ff):
+    """The same edges with bf16 operands behind the activation and the add, and the forms for many tokens against the restatement."""
+    cfg = model([(par(2, 1, 8, 4, 0.5, 11, 1, 4, 4, 5.0, rank=2), dense(ff)), (delta(1, 1, 8, 8, 2, rank=2), dense(24))], vocab=61, width=width)
+    w = random_weights(cfg, seed=73)
+    toks = tokens(cfg, 1030, 74)
+    ref = ref_logits(cfg, w, toks)
+    with engine(cfg, w, f32=False, max_batch_tokens=1040, max_model_len=1040, num_blocks=160) as e:
+        for n in (9, 1030):
+            got, _ = e.prefill_logits([e.seq_create(n)], [toks[:n]], list(range(n)))
+            assert err(got, ref[:n]) < BF16_BAR

@@ -519,3 +519,19 @@ def test_rebuilt_contexts_of_one_step_stay_apart():
         both, _ = e.prefill_logits([e.seq_create(150), e.seq_create(130)], [a, b], list(range(280)))
         assert err(both[150:], Oracle(cfg, w).forward(b).numpy()) < BF16_BAR
         assert not np.isfinite(both[:150]).any()
+
+
+def test_layers_with_and_without_the_rebuilt_form():
+    """A layer whose sizes take the rebuilt form between two whose sizes do not, long and short portions in one step."""
+    cfg = {"architecture": "Lerasun", "vocab": 211, "width": 96, "logit_scale": 1.0, "norm": {"eps": 1e-6}, "layers": [
+        layer(mixer(3, 12, 6, 20, 40, 0.3), None), wide(5, rot=24), layer(mixer(2, 32, 16, 32, 128, 0.15), None)]}
+    w = random_weights(cfg, seed=43)
+    p = [tokens(cfg, n, 44 + n) for n in (300, 40)]
+    refs = [Oracle(cfg, w).forward(x).numpy() for x in p]
+    scale = max(np.abs(r).max() for r in refs)
+    with engine(cfg, w, f32=False) as e:
+        s = [e.seq_create(len(x)) for x in p]
+        x, _ = e.prefill_logits(s, [p[0][:140], p[1][:20]], list(range(160)))
+        y, _ = e.prefill_logits([s[1], s[0]], [p[1][20:], p[0][140:]], list(range(180)))
+        for got, ref in ((x[:140], refs[0][:140]), (x[140:], refs[1][:20]), (y[:20], refs[1][20:]), (y[20:], refs[0][140:])):
+            assert np.abs(got - ref).max() / scale < BF16_BAR
