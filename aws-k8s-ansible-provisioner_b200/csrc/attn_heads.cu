@@ -1874,8 +1874,8 @@ bool premix_mma_fits(const HeadsGeom& g) {
 // lanes) stay in registers, the mixed scores are never written, and the only other barrier among the CTAs -- nobody overwrites its slab before the
 // others have read it -- is an arrival behind the reads and a wait a whole K copy later.
 // The plain kernel kept queries and weights in fp32, so both enter the tensor-core products here as two bf16 numbers (value, and what its rounding left:
-// 16 bits of mantissa against bf16 K and V rows that are exact): the distance from the 64-bit result stays what it was.  The 4 x 1024 tokens: 1.88 ms, bound
-// by instruction issue (half the issue slots busy) and the reads of other CTAs' scores.
+// 16 bits of mantissa against bf16 K and V rows that are exact): the distance from the 64-bit result stays what it was.  The 4 x 1024 tokens: 1.93 ms.
+// Every row sees all keys up to its own, and the scores are always mixed: no layer asks for a window or for unmixed scores at these sizes.
 struct PremixClusterLayout {
   int HC, GC, QP, KP, OP;
   size_t k_off, s_off, p_off, misc_off, cs_off, total;   // bytes; the queries start at 0
@@ -1956,7 +1956,7 @@ __global__ void __launch_bounds__(PX_THREADS, NC == 8 ? 2 : 1) heads_attention_p
   }
   for (int i = tid; i < H * PC_HEADS; i += PX_THREADS) {
     const int b = i / PC_HEADS, h = i - b * PC_HEADS;
-    Tk[i] = h >= HC ? 0.f : a.mix != nullptr ? a.mix[(h0 + h) * H + b] : (h0 + h == b ? 1.f : 0.f);
+    Tk[i] = h >= HC ? 0.f : a.mix[(h0 + h) * H + b];
   }
   if (tid < PX_ROWS) row_pos[tid] = tid < ntok ? pos_lo + tid : -1;
   float oacc[NU][2][4];   // unit u = head * (vdim / 16) + column block: a 16 x 16 block as two m16n8 accumulators
@@ -1985,16 +1985,15 @@ __global__ void __launch_bounds__(PX_THREADS, NC == 8 ? 2 : 1) heads_attention_p
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   auto stage_wait = [&]() { asm volatile("cp.async.wait_group 0;" ::: "memory"); };
-  const int k_first = g.window > 0 ? max(0, pos_lo - g.window + 1) / PX_KEYS * PX_KEYS : 0;
   auto cache_row = [&](int kp) { return kp <= pos_hi ? bt[kp / a.block_size] * a.block_size + kp % a.block_size : -1; };
-  if (tid < PX_KEYS) key_row[tid] = cache_row(k_first + tid);
+  if (tid < PX_KEYS) key_row[tid] = cache_row(tid);
   float m_run = -INFINITY, l_run = 0.f;   // of row `warp`, head lane mod PC_HEADS
   const float per_cap = g.softcap > 0.f ? g.scale / g.softcap : 0.f;
   auto finish_score = [&](float v) {   // scale, cap (cap - 2 cap / (e^(2 s / cap) + 1) would lose the small scores of a high cap: 0.001 at a cap of 10 000)
     return g.softcap > 0.f ? g.softcap * tanhf(v * per_cap) : v * g.scale;
   };
   int cur = 0;
-  for (int k0 = k_first; k0 <= pos_hi; k0 += PX_KEYS, cur ^= 1) {
+  for (int k0 = 0; k0 <= pos_hi; k0 += PX_KEYS, cur ^= 1) {
     const int* rows_now = key_row + cur * PX_KEYS;
     __syncthreads();   // the tile before is consumed; this tile's cache rows are in place
     stage_rows(a.k_cache, D, cpr_k, mk_key, mk_cpr, rows_now);
@@ -2047,7 +2046,7 @@ __global__ void __launch_bounds__(PX_THREADS, NC == 8 ? 2 : 1) heads_attention_p
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[n][i] = finish_score(acc[n][i]);
       }
-      if (k0 != k_first) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // the other CTAs have read the last tile's slab
+      if (k0 != 0) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");   // the other CTAs have read the last tile's slab
       if (h < HC) {
         float* srow = Ss + ((size_t)h * PX_ROWS + fg) * PX_SLD + key0 + 2 * ft;
 #pragma unroll
@@ -2098,8 +2097,7 @@ __global__ void __launch_bounds__(PX_THREADS, NC == 8 ? 2 : 1) heads_attention_p
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");   // this CTA has read every slab
     // ---- softmax of row `warp`, every head of the CTA ----
     {
-      const int kp = k0 + lane, p0 = row_pos[warp];
-      const bool vis = kp <= p0 && (g.window <= 0 || p0 - kp < g.window);
+      const bool vis = k0 + lane <= row_pos[warp];
       float m_new = m_run;
 #pragma unroll
       for (int h = 0; h < PC_HEADS; ++h) {
@@ -2489,7 +2487,7 @@ int launch_heads_attention_premix(const float* q, const void* k_cache, const voi
   B2_REQUIRE(g.heads >= 1 && g.kv_heads >= 1 && g.heads % g.kv_heads == 0, "heads_attention_premix: %d heads over %d key/value heads", g.heads, g.kv_heads);
   B2_REQUIRE(cache_f32 == out_f32, "heads_attention_premix: cache and output have one element type");
   static const bool use_mma = [] { const char* e = getenv("B2_PREMIX_MMA"); return !(e && *e == '0'); }();
-  if (use_mma && !cache_f32 && tiles != nullptr && !premix_mma_fits(g) && premix_cluster_fits(g)) {
+  if (use_mma && !cache_f32 && tiles != nullptr && mix != nullptr && g.window <= 0 && !premix_mma_fits(g) && premix_cluster_fits(g)) {
     const PremixMmaArgs a{q, (const bf16*)k_cache, (const bf16*)v_cache, g, mix, block_table, bt_stride, block_size, tiles, (bf16*)out};
     return premix_cluster_ctas(g) == 8 ? launch_premix_cluster<8>(a, ntiles, s) : launch_premix_cluster<4>(a, ntiles, s);
   }
