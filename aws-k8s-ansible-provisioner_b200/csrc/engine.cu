@@ -308,7 +308,7 @@ struct b2_engine {
   int l2_weight_prefetch = 0;  // B2_WPF: resid path, see forward_layers (measured slower: off)
   int prefill_resid_fused = 0;  // B2_RESID_FUSED: prefill O / down projections add into the residual stream in their epilogue (measured slower: off)
   int qkv_rope_prefill_fused = 1;  // B2_QKV_ROPE_FUSED: prefill QKV projection finishes norm / RoPE / page write itself
-  uint32_t* h_ran_out = nullptr;     // host word that a prompt kernel sets when one of its waits ran out
+  uint32_t* h_ran_out = nullptr;     // host word (behind h_tok) that a prompt kernel sets when one of its waits ran out
   int prefill_wait_ms = 2000;        // B2_PREFILL_WAIT_MS: how long such a wait may last (0: none may, for tests)
   B2WaitLimit wait_limit() const { return B2WaitLimit{h_ran_out, prefill_wait_ms}; }
   int prefill_pairs = 1;  // B2_PREFILL_PAIRS: see prefill_tile_pairs()
@@ -5059,8 +5059,8 @@ extern "C" int b2_engine_create(const b2_config* cfg, const char* safetensors_pa
     E_CUDA(cudaMallocHost(&e->h_stage, e->h_stage_ints * sizeof(int32_t)));
     E_CUDA(cudaMallocHost(&e->h_tiles, (size_t)e->tiles_cap * sizeof(PrefillTile)));
     E_CUDA(cudaMallocHost(&e->h_out, (size_t)e->log_cap_steps * c.max_seqs * sizeof(int32_t)));
-    E_CUDA(cudaMallocHost(&e->h_tok, Bcap * sizeof(int32_t)));
-    E_CUDA(cudaMallocHost(&e->h_ran_out, sizeof(uint32_t)));
+    E_CUDA(cudaMallocHost(&e->h_tok, (Bcap + 1) * sizeof(int32_t)));
+    e->h_ran_out = reinterpret_cast<uint32_t*>(e->h_tok + Bcap);
     *e->h_ran_out = 0;
     E_CUDA(cudaEventCreateWithFlags(&e->ev_tok, cudaEventDisableTiming));
     e->seqs.resize(c.max_seqs);
@@ -5277,7 +5277,6 @@ extern "C" void b2_engine_free(b2_engine* e) {
   if (e->h_tiles) cudaFreeHost(e->h_tiles);
   if (e->h_out) cudaFreeHost(e->h_out);
   if (e->h_tok) cudaFreeHost(e->h_tok);
-  if (e->h_ran_out) cudaFreeHost(e->h_ran_out);
   if (e->ev_tok) cudaEventDestroy(e->ev_tok);
   F(e->partial2); F(e->attn_scratch2); F(e->ssq);
   if (e->l_head == e->l_embed) e->l_head = nullptr;   // (a tied head is the embedding table)
