@@ -1,4 +1,4 @@
-"""ctypes binding of include/b2_engine.h (the same stub INTEGRATION.md shows a maintainer)."""
+"""ctypes binding of include/b2_engine.h (a stub of the same kind is all a maintainer needs)."""
 from __future__ import annotations
 
 import ctypes as C

@@ -1,7 +1,7 @@
 // attn_decode.cu -- paged GQA decode attention
 // (HF:integrations/sdpa_attention.py:40-104 at T == 1; eager form HF:models/qwen3/
 // modeling_qwen3.py:196-218).  This is the HBM-dominant kernel of batch-64 decode: per step and
-// layer it reads every resident K and V page exactly once (SURVEY.md section 8d).
+// layer it reads every resident K and V page exactly once.
 //
 // Work distribution ("stream-K" over pages): the pages of all (sequence, kv head) units are laid
 // end to end, and each of the grid's persistent warps (8 per SM) takes one contiguous run of that

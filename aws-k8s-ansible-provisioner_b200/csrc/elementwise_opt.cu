@@ -1,5 +1,5 @@
-// elementwise_opt.cu -- the small kernels of the OPT variant of the hot path (SURVEY.md 8a row a13,
-// HF:models/opt/modeling_opt.py): learned positions, LayerNorm with bias, biased projections and a
+// elementwise_opt.cu -- the small kernels of the OPT variant of the hot path
+// (HF:models/opt/modeling_opt.py): learned positions, LayerNorm with bias, biased projections and a
 // ReLU feed-forward.  The GEMMs and the attention kernels are shared with the other model families;
 // these kernels consume the GEMMs' fp32 split-K partials, so every nn.Linear bias is added in fp32
 // BEFORE the one rounding to bf16 that nn.Linear performs (the parity contract's rounding point).

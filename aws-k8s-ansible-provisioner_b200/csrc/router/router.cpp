@@ -1,9 +1,9 @@
-// b2route -- load- and prefix-aware HTTP front for N model-server replicas (SURVEY.md 8f rank 2).
+// b2route -- load- and prefix-aware HTTP front for N model-server replicas.
 //
 // In the reference's cluster this job belongs to the llm-d gateway's endpoint picker, which the
-// reference's test reaches the model through (llm-d-test.yaml:14-26); on a bare 8-GPU box (BASELINE
-// config 5: one b2serve per GPU, ports 8000+i) something has to do it.  The replicas never talk to each
-// other (DESIGN.md section 1, row e), so the router is the only place where "which GPU" is decided:
+// reference's test reaches the model through (llm-d-test.yaml:14-26); on a bare 8-GPU machine (one
+// b2serve per GPU, ports 8000+i) something has to do it.  The replicas never talk to each
+// other (each holds the whole model), so the router is the only place where "which GPU" is decided:
 //   * load: every replica's /metrics is scraped (vllm:num_requests_running / _waiting, the same series
 //     the endpoint picker reads) and combined with the router's own count of requests in flight;
 //   * prefix affinity: requests whose prompt starts with the same text (or ids) go to the replica that

@@ -140,7 +140,7 @@ static bool has_layer_list(const b2_config& c) {
 static void fill_config(const Options& o, b2_config& c) {
   memset(&c, 0, sizeof c);
   c.abi_version = B2_ABI_VERSION;
-  // Qwen3-0.6B (BASELINE.json north_star) unless the model directory carries a config.json
+  // Qwen3-0.6B unless the model directory carries a config.json
   c.num_layers = 28; c.hidden = 1024; c.num_q_heads = 16; c.num_kv_heads = 8; c.head_dim = 128; c.intermediate = 3072;
   c.vocab = 151936; c.tie_embeddings = 1; c.rms_eps = 1e-6f; c.rope_theta = 1e6f;
   // the model registry of the engine library reads the directory's config.json and picks the family

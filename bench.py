@@ -1,10 +1,10 @@
 #!/usr/bin/env python
-"""bench.py -- BASELINE.json's metric: Qwen3-0.6B bf16 greedy decode throughput (tok/s) on B200.
+"""bench.py -- Qwen3-0.6B bf16 greedy decode throughput (tok/s) on B200.
 
     python bench.py [--gpus N] [--steps K] [--warmup W]            our engine (CUDA, sm_100a)
     python bench.py --impl reference [--gpus N] [--steps K] ...     HF transformers on the host cores
 
-Workload (config.workload = "C2"): BASELINE.json configs[1] -- batch 64, 512-token prompts,
+Workload (config.workload = "C2"): batch 64, 512-token prompts,
 256 generated tokens, paged KV.  One "step" = one decode forward over the whole batch
 (64 tokens).  The workload does NOT shrink with --steps: whatever K and W are, the K timed steps
 are centred on the middle of C2's decode window (mean context 640.5; `config.timed_context` gives the
@@ -53,7 +53,7 @@ OUT_TOKENS = 256
 REPEATS = 3
 NUM_LAYERS = 28
 KV_BYTES_PER_TOKEN = 2 * NUM_LAYERS * 8 * 128 * 2          # K+V, 28 layers, 8 kv heads x 128 dims, bf16
-WEIGHT_BYTES = 1_192_099_840                                 # SURVEY.md section 8d (tied head counted once)
+WEIGHT_BYTES = 1_192_099_840                                 # the tied head counted once
 
 
 def timed_window(K: int, W: int):
@@ -389,7 +389,7 @@ def run_b200(args, rank, world, local, dist):
         pass
     prof_total = sum(v["ms"] for v in prof.values()) / 3.0
     kernel_ms = {k: round(v["ms"] / 3.0, 4) for k, v in prof.items() if v["launches"]}
-    # whole-step algorithmic bytes (SURVEY.md 8d): W + B*S*kv + B*kv at the mean context of the timed region
+    # whole-step algorithmic bytes: W + B*S*kv + B*kv at the mean context of the timed region
     step_bytes = WEIGHT_BYTES + BATCH * s_mean * KV_BYTES_PER_TOKEN + BATCH * KV_BYTES_PER_TOKEN
     step_frac = (step_bytes / (ms_max / K / 1e3) / 1e9) / peak
 

@@ -7,7 +7,7 @@
  * over HTTP by llm-d-test.yaml:32-43,61-73.  The arithmetic contract is HF transformers'
  * Qwen3 forward (models/qwen3/modeling_qwen3.py, cited per entry point below as "HF:").
  * This header is the in-process boundary the C++ server (b2serve) and the Python host mirror
- * (aws-k8s-ansible-provisioner_b200/engine.py) both bind; INTEGRATION.md shows the ctypes stub.
+ * (aws-k8s-ansible-provisioner_b200/engine.py) both bind.
  *
  * Conventions: plain pointers and sizes only.  Every function returns 0 on success or a
  * negative errno-style code; b2_last_error() returns the message for the calling thread.

@@ -3,7 +3,7 @@
 Runs the real HF transformers Qwen3 (the arithmetic behind the model the reference deploys,
 `llm-d-deploy.yaml:118`) on CPU and writes small JSON/npz fixtures:
 
-  qwen3_0p6b_c1.json     config 1 of BASELINE.json: Qwen3-0.6B arch, HF default init under
+  qwen3_0p6b_c1.json     Qwen3-0.6B arch, HF default init under
                          torch.manual_seed(0), bf16, sdpa, batch 1, 128 random prompt ids
                          (generator seed 1) -> 128 greedy tokens; per-step top-1/top-2 logits
                          (tie-aware evidence) and per-layer digests of a teacher-forced pass.

@@ -1,4 +1,4 @@
-"""CPU oracle for the OPT variant of the hot path (SURVEY.md section 8a row a13) -- TEST INFRASTRUCTURE.
+"""CPU oracle for the OPT variant of the hot path -- TEST INFRASTRUCTURE.
 
 Only tests/, __graft_entry__.smoke() and bench.py's CPU legs may import this package; nothing the
 product ships goes through it.
@@ -36,7 +36,7 @@ class OptArch(ArchConfig):
         return 2 * self.num_layers * self.kv_size * 2
 
 
-# facebook/opt-125m shapes (BASELINE.json config 3)
+# facebook/opt-125m shapes
 OPT_125M = OptArch(name="facebook/opt-125m", num_layers=12, hidden=768, num_q_heads=12, num_kv_heads=12, head_dim=64,
                    intermediate=3072, vocab=50272, rms_eps=1e-5, max_position=2048, tie_embeddings=True)
 # same structure, CPU-cheap

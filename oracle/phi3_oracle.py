@@ -1,4 +1,4 @@
-"""CPU oracle for the Phi-3 variant of the hot path (SURVEY.md section 8a row a14) -- TEST INFRASTRUCTURE.
+"""CPU oracle for the Phi-3 variant of the hot path -- TEST INFRASTRUCTURE.
 
 Only tests/, __graft_entry__.smoke() and bench.py's CPU legs may import this package; nothing the
 product ships goes through it.
@@ -41,7 +41,7 @@ class Phi3Arch(ArchConfig):
         return self.rotary_dim or self.head_dim
 
 
-# microsoft/Phi-3-mini-4k-instruct shapes (BASELINE.json config 4)
+# microsoft/Phi-3-mini-4k-instruct shapes
 PHI3_MINI = Phi3Arch(name="microsoft/Phi-3-mini-4k-instruct", num_layers=32, hidden=3072, num_q_heads=32, num_kv_heads=32,
                      head_dim=96, intermediate=8192, vocab=32064, rms_eps=1e-5, rope_theta=10000.0, max_position=4096,
                      tie_embeddings=False, sliding_window=2047)
@@ -56,7 +56,7 @@ PHI3_MINI_2L = Phi3Arch(name="phi3-mini-2-layers", num_layers=2, hidden=3072, nu
 PHI3_TINY_WINDOW = Phi3Arch(name="phi3-tiny-sliding-window", num_layers=2, hidden=768, num_q_heads=8, num_kv_heads=8, head_dim=96,
                             intermediate=1024, vocab=1024, rms_eps=1e-5, rope_theta=10000.0, max_position=4096,
                             tie_embeddings=False, sliding_window=24)
-# partial rotary (the "partial-rotary support" of SURVEY.md a14): 64 of 96 dims rotate
+# partial rotary: 64 of 96 dims rotate
 PHI3_TINY_PARTIAL = Phi3Arch(name="phi3-tiny-partial-rotary", num_layers=2, hidden=768, num_q_heads=8, num_kv_heads=8, head_dim=96,
                              intermediate=1024, vocab=1024, rms_eps=1e-5, rope_theta=10000.0, max_position=4096,
                              tie_embeddings=False, rotary_dim=64)

@@ -30,7 +30,7 @@ import torch.nn.functional as F
 
 
 # --------------------------------------------------------------------------------------
-# Model constants (BASELINE.json north_star; SURVEY.md section 8)
+# Model constants
 # --------------------------------------------------------------------------------------
 @dataclass
 class ArchConfig:
@@ -106,7 +106,7 @@ def hf_config(arch: ArchConfig):
 
 def hf_model(arch: ArchConfig = QWEN3_0_6B, seed: int = 0, attn: str = "sdpa"):
     """The graded oracle: HF Qwen3ForCausalLM, default init under `torch.manual_seed(seed)`,
-    cast to bf16, eval mode, on CPU (SURVEY.md section 8c)."""
+    cast to bf16, eval mode, on CPU."""
     from transformers import Qwen3ForCausalLM
 
     cfg = hf_config(arch)
@@ -164,7 +164,7 @@ def perturb_norm_weights(sd: dict[str, torch.Tensor], seed: int = 7) -> None:
 
 
 def make_prompts(batch: int, prompt_len: int, vocab: int, seed: int = 1) -> torch.Tensor:
-    """Uniform random token ids, generator seed 1 (SURVEY.md section 8d)."""
+    """Uniform random token ids, generator seed 1."""
     g = torch.Generator().manual_seed(seed)
     return torch.randint(0, vocab, (batch, prompt_len), generator=g, dtype=torch.int64)
 
@@ -367,7 +367,7 @@ class Restated:
 
 
 def top2_gap(logits: torch.Tensor) -> torch.Tensor:
-    """Gap between the best and second-best logit (tie-aware evidence, SURVEY.md 7.2-1)."""
+    """Gap between the best and second-best logit (tie-aware evidence)."""
     t = logits.to(torch.float32).topk(2, dim=-1).values
     return t[..., 0] - t[..., 1]
 
