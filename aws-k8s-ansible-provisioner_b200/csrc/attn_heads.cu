@@ -1874,7 +1874,8 @@ bool premix_mma_fits(const HeadsGeom& g) {
 // lanes) stay in registers, the mixed scores are never written, and the only other barrier among the CTAs -- nobody overwrites its slab before the
 // others have read it -- is an arrival behind the reads and a wait a whole K copy later.
 // The plain kernel kept queries and weights in fp32, so both enter the tensor-core products here as two bf16 numbers (value, and what its rounding left:
-// 16 bits of mantissa against bf16 K and V rows that are exact): the distance from the 64-bit result stays what it was.  The 4 x 1024 tokens: 1.93 ms.
+// 16 bits of mantissa against bf16 K and V rows that are exact): the distance from the 64-bit result stays what it was.  The 4 x 1024 tokens: 1.93 ms.  No
+// pipe is near its limit (42 % of the issue slots, the LSU at 43 %): copies, the scores of other CTAs and the barriers are waited for.
 // Every row sees all keys up to its own, and the scores are always mixed: no layer asks for a window or for unmixed scores at these sizes.
 struct PremixClusterLayout {
   int HC, GC, QP, KP, OP;
