@@ -35,11 +35,12 @@
 //   conv_unit_rows     the same for prompt-sized steps (a CTA walks down sixteen rows of one head)
 //   conv_ring_store    the ring update, after every token of the step has read the ring (a decode step's tokens do it themselves)
 //   conv_act           state-space mixer: causal convolution with bias + silu on x | B | C, step sizes and decays
-//   state_scan         the recurrence; state_scan_head: the delta rule with one decay per head on packed fp32 pairs
-//   state_scan_sum     the state-space and time-mixing rules on packed fp32 pairs
+//   state_scan         the recurrence, any sizes; state_scan_packed: on packed fp32 pairs
 //   state_out_gate     per-head RMS norm of the read-out with a gain, times the gate (silu or given), operand type out
 //   gate_part_norm     the read-out times silu(gate), RMS-normed in equal parts, operand type out
 #include "kernels.h"
+
+#include <type_traits>
 
 namespace b2 {
 
@@ -851,23 +852,43 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const float* __restrict
   }
 }
 
-// ---- the delta rule with one decay per head, packed: the same grid, lanes and staging as state_scan_kernel with NC = 4, the state of a lane held
-// as pairs of neighbouring channels so that every multiply-add works on two of them (fma.rn.f32x2, two independent fp32 operations).  The state is
-// kept as a factor times a matrix: a decay multiplies the factor only, u enters divided by it, and the matrix takes the factor in (and the factor
-// becomes one) before it could run out of range, so a decay of any size down to zero is exact to rounding.  The
-// keys of a token stay in registers between the two sums that read them; the read-out's sum over the eight lanes leaves each column with
-// one lane pair.
-template <int DPT>   // channels per lane: 4, 8 or 16 (dim <= 8 DPT); lane j owns channels 32 m + 4 j + (0..3): rows are staged as they are, 16 bytes a copy
-__global__ void __launch_bounds__(256) state_scan_head_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
-                                                              const float* __restrict__ v, int ldv, const float* __restrict__ decay,
-                                                              const float* __restrict__ beta, StateGeom g, float qscale, float* __restrict__ state,
-                                                              const int32_t* __restrict__ last_rows, const int32_t* __restrict__ row_seq,
-                                                              const int32_t* __restrict__ row_first, const int32_t* __restrict__ row_end,
-                                                              const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
-                                                              float* __restrict__ out, int cols) {
-  constexpr int NC = 4, CH = SC_CHUNK, DP = DPT * SC_LANES, MAXC = 32 * NC, HP = DPT / 2;
-  __shared__ __align__(16) float qs[2][CH][DP], ks[2][CH][DP];
-  __shared__ __align__(16) float vs[2][CH][MAXC];
+// ---- all rules, packed: sixteen lanes share NC neighbouring columns and split the key channels, lane j owns channels 64 m + 4 j + (0..3), held as pairs of
+// neighbouring channels so that one instruction works on two of them (fma.rn.f32x2, two independent fp32 operations: 123 multiply-adds a cycle and SM, as
+// with scalar ones, for half the issue slots).  Rows are staged as they are, 16 bytes a copy, eight tokens ahead.  The eight tokens of a chunk are
+// unrolled, and sixteen sums (16 / NC tokens of NC columns) cross the sixteen lanes together: each exchange halves what a lane still holds, and every lane
+// ends with one of them.  The sum of a column runs over the channels of a lane, then over lanes 1, 2, 4 and 8 apart, whatever NC, the tile or the cut of
+// the prompt.
+//   one decay per head (DELTA_HEAD, DECAY_HEAD): the state is kept as a factor times a matrix -- a decay multiplies the factor only, the write enters
+//     divided by it, and the matrix takes the factor in (and the factor becomes one) before it could run out of range, so a decay of any size down to zero is
+//     exact to rounding
+//   DELTA   S^T (a k) is summed over the state as it is while the decay is applied beside the sum: the chain from token to token is the sum, the exchange
+//     over the lanes and one multiply-add
+//   BONUS   the read-out sees the state before the write, and the bonus of a token is the number sum_d q_d u_d k_d times its value
+// What bounds it: the way from shared memory into registers (128 bytes a cycle and SM: k, q and the decays of a lane's channels, per token) beside the FMA
+// pipe, and, with few heads and sequences, the latency of one warp per scheduler -- hence sixteen lanes (eight lanes of sixteen channels: 686 us for the 629
+// above, and 134 for the 111 us below), and two columns per lane instead of four where there are few of them, see launch_scan_packed.
+// Before (eight lanes, scalar or without the unrolled chunk): 16 x 1024 tokens, DECAY, 8 heads of 128 x 256 918 -> 629 us; one prompt of 1011 tokens, 32 heads,
+// DECAY_HEAD of 128 x 64 306 -> 111 us, BONUS of 64 x 64 176 -> 87 us; four of up to 300 tokens, DELTA_HEAD, 16 heads of 128 x 128 172 -> 100 us.
+template <int NC>
+struct ScanTile {
+  static constexpr int LANES = 16, THREADS = 128;
+  static constexpr int COLS = THREADS / LANES * NC;
+  static constexpr int PER_SM = 4;   // CTAs: 128 registers a thread (NC 4, 16 x 1024 tokens of 8 heads of 128 x 256: 629 us; five CTAs of 96 registers 657, seven of 72 687)
+};
+template <int DPT, int RULE, int NC>   // channels per lane: 4 or 8 (dim <= 16 DPT)
+__global__ void __launch_bounds__(ScanTile<NC>::THREADS, ScanTile<NC>::PER_SM)
+state_scan_packed_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk, const float* __restrict__ v, int ldv,
+                         const float* __restrict__ decay, const float* __restrict__ beta, StateGeom g, float qscale, float* __restrict__ state,
+                         const int32_t* __restrict__ last_rows, const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
+                         const int32_t* __restrict__ row_end, const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
+                         float* __restrict__ out) {
+  constexpr int NT = ScanTile<NC>::THREADS, COLS = ScanTile<NC>::COLS, L = ScanTile<NC>::LANES, CH = SC_CHUNK, DP = DPT * L, HP = DPT / 2, TB = L / NC;
+  constexpr int PIECES = DP / 4, RSTEP = NT / PIECES, VP = COLS / 4;   // 16-byte pieces of a row; rows that the CTA copies at a time
+  constexpr bool HEAD = RULE == STATE_RULE_DELTA_HEAD || RULE == STATE_RULE_DECAY_HEAD;
+  constexpr bool DELTA = RULE == STATE_RULE_DELTA_HEAD || RULE == STATE_RULE_DELTA;
+  constexpr bool BETA = DELTA || RULE == STATE_RULE_DECAY_HEAD;
+  __shared__ __align__(16) float qs[2][CH][DP], ks[2][CH][DP], as[HEAD ? 1 : 2][HEAD ? 1 : CH][HEAD ? 4 : DP];
+  __shared__ __align__(16) float vs[2][CH][COLS];
   __shared__ float bs[2][CH], ds[2][CH];
   pdl_wait();
   pdl_launch_dependents();
@@ -875,314 +896,224 @@ __global__ void __launch_bounds__(256) state_scan_head_kernel(const float* __res
   const int first = row_first[r_last], end = row_end[r_last];
   if (slots[first] < 0) return;   // padding row of a decode bucket
   const int a = blockIdx.y, kh = a / (g.heads / g.kv_heads);
-  const int col0 = blockIdx.z * cols;
-  const int grp = threadIdx.x / SC_LANES, j = threadIdx.x % SC_LANES, cl = grp * NC;
+  const int col0 = blockIdx.z * COLS;
+  const int tid = threadIdx.x, j = tid % L, cl = tid / L * NC;
   const int pos0 = positions[first], n = end - first;
-  const int nthreads = blockDim.x;
   const size_t head_floats = (size_t)g.dim * g.vdim;
   float* sbase = state + ((size_t)row_seq[first] * 2 * g.heads) * head_floats;
   const float* s_in = sbase + ((size_t)((pos0 + 1) & 1) * g.heads + a) * head_floats;
   float* s_out = sbase + ((size_t)((pos0 + n - 1) & 1) * g.heads + a) * head_floats;
-  // channels past dim and columns past vdim never change: zero keys, queries and values
-  for (int i = threadIdx.x; i < 2 * CH * (DP - g.dim); i += nthreads) {
+  // channels past dim and columns past vdim never change: zero keys, queries, decays and values (what no copy ever writes)
+  for (int i = tid; i < 2 * CH * (DP - g.dim); i += NT) {
     const int st = i / (CH * (DP - g.dim)), rem = i % (CH * (DP - g.dim)), tt = rem / (DP - g.dim), d = g.dim + rem % (DP - g.dim);
     qs[st][tt][d] = 0.f;
     ks[st][tt][d] = 0.f;
+    if (!HEAD) as[HEAD ? 0 : st][HEAD ? 0 : tt][HEAD ? 0 : d] = 0.f;
   }
-  const int vcols = min(cols, g.vdim - col0);
-  if (vcols < cols) {
-    for (int i = threadIdx.x; i < 2 * CH * (cols - vcols); i += nthreads) {
-      const int row = i / (cols - vcols), c = vcols + i % (cols - vcols);
+  const int vcols = min(COLS, g.vdim - col0);
+  if (vcols < COLS) {
+    for (int i = tid; i < 2 * CH * (COLS - vcols); i += NT) {
+      const int row = i / (COLS - vcols), c = vcols + i % (COLS - vcols);
       vs[row / CH][row % CH][c] = 0.f;
     }
   }
   __syncthreads();
-  const int dq = g.dim >> 2, vq4 = vcols >> 2;   // 16-byte pieces of a row
-  const int dsh = (dq & (dq - 1)) == 0 ? 31 - __clz(dq) : -1, vsh = (vq4 & (vq4 - 1)) == 0 ? 31 - __clz(vq4) : -1;
-  const float* qb = q + (size_t)first * ldq + kh * g.dim;
-  const float* kb = k + (size_t)first * ldk + kh * g.dim;
-  const float* vb = v + (size_t)first * ldv + a * g.vdim + col0;
-  auto issue = [&](int c0, int st) {
-    const int cn = min(CH, n - c0);
-    for (int i = threadIdx.x; i < cn * dq; i += nthreads) {
-      const int tt = dsh >= 0 ? i >> dsh : i / dq, d = (i - tt * dq) * 4;
-      cp_async_16(&qs[st][tt][d], qb + (size_t)(c0 + tt) * ldq + d);
-      cp_async_16(&ks[st][tt][d], kb + (size_t)(c0 + tt) * ldk + d);
+  // this thread's pieces: row d_row of every RSTEP rows, columns d_at
+  const int d_row = tid / PIECES, d_at = tid % PIECES * 4, v_row = tid / VP, v_at = tid % VP * 4;
+  const bool d_on = d_at < g.dim, v_on = v_at < vcols;
+  const int lda = g.heads * g.dim;
+  const float* qsrc = q + (size_t)(first + d_row) * ldq + kh * g.dim + d_at;
+  const float* ksrc = k + (size_t)(first + d_row) * ldk + kh * g.dim + d_at;
+  const float* asrc = HEAD ? decay : decay + (size_t)(first + d_row) * lda + a * g.dim + d_at;
+  const float* vsrc = v + (size_t)(first + v_row) * ldv + a * g.vdim + col0 + v_at;
+  const float* bsrc = BETA ? beta + (size_t)(first + tid) * g.heads + a : nullptr;
+  const float* dsrc = HEAD ? decay + (size_t)(first + tid) * g.heads + a : nullptr;
+  auto issue = [&](int cn, int st) {   // the next cn tokens
+    if (d_on) {
+#pragma unroll
+      for (int x = 0; x < (CH + RSTEP - 1) / RSTEP; ++x) {
+        const int tt = d_row + x * RSTEP;
+        if (tt < cn) {
+          cp_async_16(&qs[st][tt][d_at], qsrc + (size_t)(x * RSTEP) * ldq);
+          cp_async_16(&ks[st][tt][d_at], ksrc + (size_t)(x * RSTEP) * ldk);
+          if constexpr (!HEAD) cp_async_16(&as[st][tt][d_at], asrc + (size_t)(x * RSTEP) * lda);
+        }
+      }
+      qsrc += (size_t)CH * ldq;
+      ksrc += (size_t)CH * ldk;
+      if (!HEAD) asrc += (size_t)CH * lda;
     }
-    for (int i = threadIdx.x; i < cn * vq4; i += nthreads) {
-      const int tt = vsh >= 0 ? i >> vsh : i / vq4, c = (i - tt * vq4) * 4;
-      cp_async_16(&vs[st][tt][c], vb + (size_t)(c0 + tt) * ldv + c);
+    if (v_on && v_row < cn) cp_async_16(&vs[st][v_row < CH ? v_row : 0][v_at], vsrc);
+    vsrc += (size_t)CH * ldv;
+    if (BETA && tid < cn) {
+      cp_async_f32(&bs[st][tid < CH ? tid : 0], bsrc);
+      if (HEAD) cp_async_f32(&ds[st][tid < CH ? tid : 0], dsrc);
     }
-    for (int i = threadIdx.x; i < cn; i += nthreads) {
-      cp_async_f32(&bs[st][i], beta + (size_t)(first + c0 + i) * g.heads + a);
-      cp_async_f32(&ds[st][i], decay + (size_t)(first + c0 + i) * g.heads + a);
-    }
+    if (BETA) bsrc += (size_t)CH * g.heads;
+    if (HEAD) dsrc += (size_t)CH * g.heads;
   };
-  issue(0, 0);
-  const bool live = col0 + cl + NC <= g.vdim;   // this group's four columns (vdim is a multiple of four)
-  auto channel = [&](int i) { return (i >> 2) * 32 + 4 * j + (i & 3); };
-  f32x2_t s[HP][NC];
+  static_assert(NT / VP >= CH && NT >= PIECES, "a chunk's values are one copy per thread");
+  issue(min(CH, n), 0);
+  const bool live = col0 + cl < g.vdim;   // this group's columns (vdim is a multiple of four)
+  auto channel = [&](int i) { return (i >> 2) * 64 + 4 * j + (i & 3); };
+  f32x2_t s[HP][NC], bonus[RULE == STATE_RULE_BONUS ? HP : 1];
 #pragma unroll
   for (int i = 0; i < HP; ++i) {
-    float lo[NC], hi[NC];
+    float w[2][NC];
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
       const int d = channel(2 * i + x);
-      float* dst = x ? hi : lo;
-      float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live && pos0 > 0 && d < g.dim) w = *reinterpret_cast<const float4*>(s_in + (size_t)d * g.vdim + col0 + cl);
-      dst[0] = w.x; dst[1] = w.y; dst[2] = w.z; dst[3] = w.w;
+      const float* src = s_in + (size_t)d * g.vdim + col0 + cl;
+      const bool in = live && pos0 > 0 && d < g.dim;
+      if constexpr (NC == 4) {
+        const float4 r = in ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+        w[x][0] = r.x; w[x][1] = r.y; w[x][2] = r.z; w[x][3] = r.w;
+      } else {
+        const float2 r = in ? *reinterpret_cast<const float2*>(src) : make_float2(0.f, 0.f);
+        w[x][0] = r.x; w[x][1] = r.y;
+      }
     }
 #pragma unroll
-    for (int c = 0; c < NC; ++c) s[i][c] = x2_pack(lo[c], hi[c]);
+    for (int c = 0; c < NC; ++c) s[i][c] = x2_pack(w[0][c], w[1][c]);
+    if constexpr (RULE == STATE_RULE_BONUS) {
+      const int d0 = channel(2 * i), d1 = channel(2 * i + 1);
+      bonus[i] = x2_pack(d0 < g.dim ? g.bonus[a * g.dim + d0] : 0.f, d1 < g.dim ? g.bonus[a * g.dim + d1] : 0.f);
+    }
   }
-  float fac = 1.0f;   // the state is fac * s: a decay multiplies one number
+  const float skip = RULE == STATE_RULE_DECAY_HEAD ? g.skip[a] : 0.f;
+  const bool b0 = (j & 1) != 0, b1 = (j & 2) != 0, b2 = (j & 4) != 0, b3 = (j & 8) != 0;
+  const int mine = (b0 ? 8 : 0) + (b1 ? 4 : 0) + (b2 ? 2 : 0) + (b3 ? 1 : 0);   // which of sixteen sums this lane ends with
+  const int mtok = mine / NC, mcol = mine % NC;
+  const int ucol = NC == 4 ? (mine >> 2) : (mine >> 3);     // DELTA: the column whose u this lane forms
+  const size_t ostep = (size_t)g.heads * g.vdim;
+  float* optr = out + (size_t)(first + mtok) * ostep + a * g.vdim + col0 + cl + mcol;
+  float fac = 1.0f;   // HEAD: the state is fac * s
   int st = 0;
-  for (int c0 = 0; c0 < n; c0 += CH, st ^= 1) {
-    const int cn = min(CH, n - c0);
-    cp_async_wait_all();                         // this chunk's copies (the only ones in flight)
-    __syncthreads();                             // ... of every thread; and every thread has left the other stage
-    if (c0 + CH < n) issue(c0 + CH, st ^ 1);     // the next chunk's copies run beside this chunk's arithmetic
-    for (int tt = 0; tt < cn; ++tt) {
-      const float4 vq = *reinterpret_cast<const float4*>(&vs[st][tt][cl]);
-      const float vc[NC] = {vq.x, vq.y, vq.z, vq.w};
-      const float bt = bs[st][tt];
-      fac *= ds[st][tt];
-      if (fac < 1e-12f) {   // (the same in every thread of the CTA)
-        const f32x2_t f2 = x2_pack(fac, fac);
+  auto rescale = [&] {   // the factor goes into the state
+    const f32x2_t f2 = x2_pack(fac, fac);
 #pragma unroll
-        for (int i = 0; i < HP; ++i)
+    for (int i = 0; i < HP; ++i)
 #pragma unroll
-          for (int c = 0; c < NC; ++c) s[i][c] = x2_mul(f2, s[i][c]);
-        fac = 1.0f;
+      for (int c = 0; c < NC; ++c) s[i][c] = x2_mul(f2, s[i][c]);
+    fac = 1.0f;
+  };
+  // one token's write and this lane's part of its read-out
+  auto token = [&](int tt, float* o) {
+    float vc[NC];
+    if constexpr (!DELTA) {
+      if constexpr (NC == 2) {
+        const float2 x = *reinterpret_cast<const float2*>(&vs[st][tt][cl]);
+        vc[0] = x.x; vc[1] = x.y;
+      } else {
+        const float4 x = *reinterpret_cast<const float4*>(&vs[st][tt][cl]);
+        vc[0] = x.x; vc[1] = x.y; vc[2] = x.z; vc[3] = x.w;
       }
-      const float inv = __fdividef(1.0f, fac);   // (1e-12 <= fac <= 1)
-      const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(&ks[st][tt][4 * j]);   // (32 channels on: eight pieces of 16 bytes)
-      const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(&qs[st][tt][4 * j]);
-      f32x2_t kk[HP], sum[NC];
+    }
+    const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(&ks[st][tt][4 * j]);   // (64 channels on: sixteen pieces of 16 bytes)
+    const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(&qs[st][tt][4 * j]);
+    const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(&as[HEAD ? 0 : st][HEAD ? 0 : tt][HEAD ? 0 : 4 * j]);
+    const float inv = HEAD ? __fdividef(1.0f, fac) : 1.0f;   // (1e-12 <= fac <= 1)
+    f32x2_t sum[NC], w2[NC];
+    if constexpr (DELTA) {
+      const float bt = bs[st][tt];
+      f32x2_t kk[HP];
 #pragma unroll
       for (int i = 0; i < HP; i += 2) {
-        const ulonglong2 w = kp[(i >> 1) * 8];
+        const ulonglong2 w = kp[(i >> 1) * 16];
         kk[i] = w.x;
         kk[i + 1] = w.y;
       }
+      if constexpr (HEAD) {
 #pragma unroll
-      for (int c = 0; c < NC; ++c) sum[c] = x2_mul(s[0][c], kk[0]);
+        for (int c = 0; c < NC; ++c) sum[c] = x2_mul(s[0][c], kk[0]);
 #pragma unroll
-      for (int i = 1; i < HP; ++i)
+        for (int i = 1; i < HP; ++i)
 #pragma unroll
-        for (int c = 0; c < NC; ++c) sum[c] = x2_fma(s[i][c], kk[i], sum[c]);
-      f32x2_t u2[NC];
+          for (int c = 0; c < NC; ++c) sum[c] = x2_fma(s[i][c], kk[i], sum[c]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < HP; i += 2) {
+          const ulonglong2 aw = ap[(i >> 1) * 16];
+          const f32x2_t ak0 = x2_mul(aw.x, kk[i]), ak1 = x2_mul(aw.y, kk[i + 1]);
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            sum[c] = i == 0 ? x2_mul(s[0][c], ak0) : x2_fma(s[i][c], ak0, sum[c]);
+            sum[c] = x2_fma(s[i + 1][c], ak1, sum[c]);
+            s[i][c] = x2_mul(s[i][c], aw.x);
+            s[i + 1][c] = x2_mul(s[i + 1][c], aw.y);
+          }
+        }
+      }
+      float kv[NC];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
         float lo, hi;
         x2_unpack(sum[c], lo, hi);
-        float kv = lo + hi;
-        kv += __shfl_xor_sync(0xffffffffu, kv, 1);
-        kv += __shfl_xor_sync(0xffffffffu, kv, 2);
-        kv += __shfl_xor_sync(0xffffffffu, kv, 4);
-        const float u = bt * fmaf(vc[c], inv, -kv);   // beta (v - fac S^T k) / fac
-        u2[c] = x2_pack(u, u);
+        kv[c] = lo + hi;
+      }
+      // the lanes' sums: exchanges that halve the columns a lane holds, then full ones; a lane forms the u of one column, and all lanes take all of them
+#pragma unroll
+      for (int m = 1, w = NC / 2; m < L; m *= 2, w /= 2) {
+        const bool up = (j & m) != 0;
+        if (w >= 1) {
+#pragma unroll
+          for (int x = 0; x < (w > 0 ? w : 1); ++x) kv[x] = (up ? kv[x + w] : kv[x]) + __shfl_xor_sync(0xffffffffu, up ? kv[x] : kv[x + w], m);
+        } else {
+          kv[0] += __shfl_xor_sync(0xffffffffu, kv[0], m);
+        }
+      }
+      const float vu = vs[st][tt][cl + ucol];
+      const float u = HEAD ? bt * fmaf(vu, inv, -kv[0])   // beta (v - fac S^T k) / fac
+                           : bt * (vu - kv[0]);
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int from = NC == 4 ? ((c >> 1) & 1) | ((c & 1) << 1) : c;   // the lane with this column
+        const float uc = __shfl_sync(0xffffffffu, u, from, L);
+        w2[c] = x2_pack(uc, uc);
       }
 #pragma unroll
       for (int i = 0; i < HP; i += 2) {
-        const ulonglong2 w = qp[(i >> 1) * 8];
+        const ulonglong2 qw = qp[(i >> 1) * 16];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          s[i][c] = x2_fma(kk[i], u2[c], s[i][c]);
-          s[i + 1][c] = x2_fma(kk[i + 1], u2[c], s[i + 1][c]);
-          sum[c] = i == 0 ? x2_mul(s[0][c], w.x) : x2_fma(s[i][c], w.x, sum[c]);
-          sum[c] = x2_fma(s[i + 1][c], w.y, sum[c]);
+          s[i][c] = x2_fma(kk[i], w2[c], s[i][c]);
+          s[i + 1][c] = x2_fma(kk[i + 1], w2[c], s[i + 1][c]);
+          sum[c] = i == 0 ? x2_mul(s[0][c], qw.x) : x2_fma(s[i][c], qw.x, sum[c]);
+          sum[c] = x2_fma(s[i + 1][c], qw.y, sum[c]);
         }
       }
-      // sum over the eight lanes: each exchange halves the columns a lane still holds, then the last two lanes of a column add
-      float o[NC];
+    } else {
+      const float wr = HEAD ? bs[st][tt] * inv : 1.0f;
+      f32x2_t ruk = 0ull;
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
-        float lo, hi;
-        x2_unpack(sum[c], lo, hi);
-        o[c] = lo + hi;
+        const float w = HEAD ? vc[c] * wr : vc[c];
+        w2[c] = x2_pack(w, w);
       }
-      const bool up1 = (j & 1) != 0, up2 = (j & 2) != 0;
-      const float a0 = (up1 ? o[2] : o[0]) + __shfl_xor_sync(0xffffffffu, up1 ? o[0] : o[2], 1);
-      const float a1 = (up1 ? o[3] : o[1]) + __shfl_xor_sync(0xffffffffu, up1 ? o[1] : o[3], 1);
-      float r = (up2 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up2 ? a0 : a1, 2);
-      r += __shfl_xor_sync(0xffffffffu, r, 4);
-      const int c = (up1 ? 2 : 0) + (up2 ? 1 : 0);   // the column this lane ended with
-      if (j < 4 && live)
-        out[(size_t)(first + c0 + tt) * ((size_t)g.heads * g.vdim) + a * g.vdim + col0 + cl + c] = r * (qscale * fac);
-    }
-  }
-  const f32x2_t f2 = x2_pack(fac, fac);
 #pragma unroll
-  for (int i = 0; i < HP; ++i) {
-    float lo[NC], hi[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) x2_unpack(x2_mul(f2, s[i][c]), lo[c], hi[c]);
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      const int d = channel(2 * i + x);
-      const float* src = x ? hi : lo;
-      if (live && d < g.dim) *reinterpret_cast<float4*>(s_out + (size_t)d * g.vdim + col0 + cl) = make_float4(src[0], src[1], src[2], src[3]);
-    }
-  }
-}
-
-// ---- the rules whose write does not read the state (DECAY_HEAD, BONUS), packed the same way.  DECAY_HEAD: the state is a factor times a matrix, as above.
-// BONUS: decays per channel are staged beside the keys; the read-out sees the state before the write, and the bonus of a token is the number
-// sum_d q_d u_d k_d times its value.
-template <int DPT, int RULE>
-__global__ void __launch_bounds__(256) state_scan_sum_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
-                                                             const float* __restrict__ v, int ldv, const float* __restrict__ decay,
-                                                             const float* __restrict__ beta, StateGeom g, float qscale, float* __restrict__ state,
-                                                             const int32_t* __restrict__ last_rows, const int32_t* __restrict__ row_seq,
-                                                             const int32_t* __restrict__ row_first, const int32_t* __restrict__ row_end,
-                                                             const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
-                                                             float* __restrict__ out, int cols) {
-  constexpr int NC = 4, CH = SC_CHUNK, DP = DPT * SC_LANES, MAXC = 32 * NC, HP = DPT / 2;
-  constexpr bool HEAD = RULE == STATE_RULE_DECAY_HEAD;
-  __shared__ __align__(16) float qs[2][CH][DP], ks[2][CH][DP], as[HEAD ? 1 : 2][HEAD ? 1 : CH][HEAD ? 4 : DP];
-  __shared__ __align__(16) float vs[2][CH][MAXC];
-  __shared__ float bs[2][CH], ds[2][CH];
-  pdl_wait();
-  pdl_launch_dependents();
-  const int r_last = last_rows ? last_rows[blockIdx.x] : (int)blockIdx.x;
-  const int first = row_first[r_last], end = row_end[r_last];
-  if (slots[first] < 0) return;   // padding row of a decode bucket
-  const int a = blockIdx.y, kh = a / (g.heads / g.kv_heads);
-  const int col0 = blockIdx.z * cols;
-  const int grp = threadIdx.x / SC_LANES, j = threadIdx.x % SC_LANES, cl = grp * NC;
-  const int pos0 = positions[first], n = end - first;
-  const int nthreads = blockDim.x;
-  const size_t head_floats = (size_t)g.dim * g.vdim;
-  float* sbase = state + ((size_t)row_seq[first] * 2 * g.heads) * head_floats;
-  const float* s_in = sbase + ((size_t)((pos0 + 1) & 1) * g.heads + a) * head_floats;
-  float* s_out = sbase + ((size_t)((pos0 + n - 1) & 1) * g.heads + a) * head_floats;
-  // channels past dim and columns past vdim never change: zero keys, queries, decays and values
-  for (int i = threadIdx.x; i < 2 * CH * (DP - g.dim); i += nthreads) {
-    const int st = i / (CH * (DP - g.dim)), rem = i % (CH * (DP - g.dim)), tt = rem / (DP - g.dim), d = g.dim + rem % (DP - g.dim);
-    qs[st][tt][d] = 0.f;
-    ks[st][tt][d] = 0.f;
-    if (!HEAD) {
-      as[HEAD ? 0 : st][HEAD ? 0 : tt][HEAD ? 0 : d] = 0.f;
-    }
-  }
-  const int vcols = min(cols, g.vdim - col0);
-  if (vcols < cols) {
-    for (int i = threadIdx.x; i < 2 * CH * (cols - vcols); i += nthreads) {
-      const int row = i / (cols - vcols), c = vcols + i % (cols - vcols);
-      vs[row / CH][row % CH][c] = 0.f;
-    }
-  }
-  __syncthreads();
-  const int dq = g.dim >> 2, vq4 = vcols >> 2;   // 16-byte pieces of a row
-  const int dsh = (dq & (dq - 1)) == 0 ? 31 - __clz(dq) : -1, vsh = (vq4 & (vq4 - 1)) == 0 ? 31 - __clz(vq4) : -1;
-  const int lda = g.heads * g.dim;
-  const float* qb = q + (size_t)first * ldq + kh * g.dim;
-  const float* kb = k + (size_t)first * ldk + kh * g.dim;
-  const float* ab = HEAD ? decay : decay + (size_t)first * lda + a * g.dim;
-  const float* vb = v + (size_t)first * ldv + a * g.vdim + col0;
-  auto issue = [&](int c0, int st) {
-    const int cn = min(CH, n - c0);
-    for (int i = threadIdx.x; i < cn * dq; i += nthreads) {
-      const int tt = dsh >= 0 ? i >> dsh : i / dq, d = (i - tt * dq) * 4;
-      cp_async_16(&qs[st][tt][d], qb + (size_t)(c0 + tt) * ldq + d);
-      cp_async_16(&ks[st][tt][d], kb + (size_t)(c0 + tt) * ldk + d);
-      if (!HEAD) {
-        cp_async_16(&as[HEAD ? 0 : st][HEAD ? 0 : tt][HEAD ? 0 : d], ab + (size_t)(c0 + tt) * lda + d);
-      }
-    }
-    for (int i = threadIdx.x; i < cn * vq4; i += nthreads) {
-      const int tt = vsh >= 0 ? i >> vsh : i / vq4, c = (i - tt * vq4) * 4;
-      cp_async_16(&vs[st][tt][c], vb + (size_t)(c0 + tt) * ldv + c);
-    }
-    if (HEAD) {
-      for (int i = threadIdx.x; i < cn; i += nthreads) {
-        cp_async_f32(&bs[st][i], beta + (size_t)(first + c0 + i) * g.heads + a);
-        cp_async_f32(&ds[st][i], decay + (size_t)(first + c0 + i) * g.heads + a);
-      }
-    }
-  };
-  issue(0, 0);
-  const bool live = col0 + cl + NC <= g.vdim;   // this group's four columns (vdim is a multiple of four)
-  auto channel = [&](int i) { return (i >> 2) * 32 + 4 * j + (i & 3); };
-  f32x2_t s[HP][NC], bonus[HEAD ? 1 : HP];
-#pragma unroll
-  for (int i = 0; i < HP; ++i) {
-    float lo[NC], hi[NC];
-#pragma unroll
-    for (int x = 0; x < 2; ++x) {
-      const int d = channel(2 * i + x);
-      float* dst = x ? hi : lo;
-      float4 w = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (live && pos0 > 0 && d < g.dim) w = *reinterpret_cast<const float4*>(s_in + (size_t)d * g.vdim + col0 + cl);
-      dst[0] = w.x; dst[1] = w.y; dst[2] = w.z; dst[3] = w.w;
-    }
-#pragma unroll
-    for (int c = 0; c < NC; ++c) s[i][c] = x2_pack(lo[c], hi[c]);
-    if (!HEAD) {
-      const int d0 = channel(2 * i), d1 = channel(2 * i + 1);
-      bonus[HEAD ? 0 : i] = x2_pack(d0 < g.dim ? g.bonus[a * g.dim + d0] : 0.f, d1 < g.dim ? g.bonus[a * g.dim + d1] : 0.f);
-    }
-  }
-  const float skip = HEAD ? g.skip[a] : 0.f;
-  const bool up1 = (j & 1) != 0, up2 = (j & 2) != 0;
-  const int ccol = (up1 ? 2 : 0) + (up2 ? 1 : 0);   // the column this lane ends a token with
-  const size_t ostep = (size_t)g.heads * g.vdim;
-  float* optr = out + (size_t)first * ostep + a * g.vdim + col0 + cl + ccol;
-  float fac = 1.0f;
-  int st = 0;
-  for (int c0 = 0; c0 < n; c0 += CH, st ^= 1) {
-    const int cn = min(CH, n - c0);
-    cp_async_wait_all();                         // this chunk's copies (the only ones in flight)
-    __syncthreads();                             // ... of every thread; and every thread has left the other stage
-    if (c0 + CH < n) issue(c0 + CH, st ^ 1);     // the next chunk's copies run beside this chunk's arithmetic
-    // one token: wr is the write's factor (DECAY_HEAD), ofac the read-out's
-    auto token = [&](int tt, float wr, float ofac) {
-      const float4 vq = *reinterpret_cast<const float4*>(&vs[st][tt][cl]);
-      const float vc[NC] = {vq.x, vq.y, vq.z, vq.w};
-      const ulonglong2* kp = reinterpret_cast<const ulonglong2*>(&ks[st][tt][4 * j]);   // (32 channels on: eight pieces of 16 bytes)
-      const ulonglong2* qp = reinterpret_cast<const ulonglong2*>(&qs[st][tt][4 * j]);
-      f32x2_t sum[NC], w2[NC];
-      float o[NC];
-      if constexpr (HEAD) {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) w2[c] = x2_pack(vc[c] * wr, vc[c] * wr);
-#pragma unroll
-        for (int i = 0; i < HP; i += 2) {
-          const ulonglong2 kw = kp[(i >> 1) * 8], qw = qp[(i >> 1) * 8];
-#pragma unroll
-          for (int c = 0; c < NC; ++c) {
-            s[i][c] = x2_fma(kw.x, w2[c], s[i][c]);
-            s[i + 1][c] = x2_fma(kw.y, w2[c], s[i + 1][c]);
-            sum[c] = i == 0 ? x2_mul(s[0][c], qw.x) : x2_fma(s[i][c], qw.x, sum[c]);
-            sum[c] = x2_fma(s[i + 1][c], qw.y, sum[c]);
-          }
+      for (int i = 0; i < HP; i += 2) {
+        const ulonglong2 kw = kp[(i >> 1) * 16], qw = qp[(i >> 1) * 16];
+        ulonglong2 aw = make_ulonglong2(0ull, 0ull);
+        if constexpr (!HEAD) aw = ap[(i >> 1) * 16];
+        if constexpr (RULE == STATE_RULE_BONUS) {
+          ruk = x2_fma(x2_mul(qw.x, bonus[i]), kw.x, ruk);
+          ruk = x2_fma(x2_mul(qw.y, bonus[i + 1]), kw.y, ruk);
         }
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-          float lo, hi;
-          x2_unpack(sum[c], lo, hi);
-          o[c] = lo + hi;
-        }
-      } else {
-        const ulonglong2* ap = reinterpret_cast<const ulonglong2*>(&as[HEAD ? 0 : st][HEAD ? 0 : tt][HEAD ? 0 : 4 * j]);
-        f32x2_t ruk = 0ull;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) w2[c] = x2_pack(vc[c], vc[c]);
-#pragma unroll
-        for (int i = 0; i < HP; i += 2) {
-          const ulonglong2 kw = kp[(i >> 1) * 8], qw = qp[(i >> 1) * 8], aw = ap[(i >> 1) * 8];
-          ruk = x2_fma(x2_mul(qw.x, bonus[HEAD ? 0 : i]), kw.x, ruk);
-          ruk = x2_fma(x2_mul(qw.y, bonus[HEAD ? 0 : i + 1]), kw.y, ruk);
-#pragma unroll
-          for (int c = 0; c < NC; ++c) {
+          if constexpr (RULE == STATE_RULE_BONUS) {
             sum[c] = i == 0 ? x2_mul(s[0][c], qw.x) : x2_fma(s[i][c], qw.x, sum[c]);
             sum[c] = x2_fma(s[i + 1][c], qw.y, sum[c]);
-            s[i][c] = x2_fma(aw.x, s[i][c], x2_mul(kw.x, w2[c]));
-            s[i + 1][c] = x2_fma(aw.y, s[i + 1][c], x2_mul(kw.y, w2[c]));
+          }
+          s[i][c] = HEAD ? x2_fma(kw.x, w2[c], s[i][c]) : x2_fma(aw.x, s[i][c], x2_mul(kw.x, w2[c]));
+          s[i + 1][c] = HEAD ? x2_fma(kw.y, w2[c], s[i + 1][c]) : x2_fma(aw.y, s[i + 1][c], x2_mul(kw.y, w2[c]));
+          if constexpr (RULE != STATE_RULE_BONUS) {
+            sum[c] = i == 0 ? x2_mul(s[0][c], qw.x) : x2_fma(s[i][c], qw.x, sum[c]);
+            sum[c] = x2_fma(s[i + 1][c], qw.y, sum[c]);
           }
         }
+      }
+      if constexpr (RULE == STATE_RULE_BONUS) {
         float rl, rh;
         x2_unpack(ruk, rl, rh);
 #pragma unroll
@@ -1191,50 +1122,85 @@ __global__ void __launch_bounds__(256) state_scan_sum_kernel(const float* __rest
           x2_unpack(sum[c], lo, hi);
           o[c] = fmaf(rl + rh, vc[c], lo + hi);
         }
+        return;
       }
-      // sum over the eight lanes: each exchange halves the columns a lane still holds, then the last two lanes of a column add
-      const float a0 = (up1 ? o[2] : o[0]) + __shfl_xor_sync(0xffffffffu, up1 ? o[0] : o[2], 1);
-      const float a1 = (up1 ? o[3] : o[1]) + __shfl_xor_sync(0xffffffffu, up1 ? o[1] : o[3], 1);
-      float r = (up2 ? a1 : a0) + __shfl_xor_sync(0xffffffffu, up2 ? a0 : a1, 2);
-      r += __shfl_xor_sync(0xffffffffu, r, 4);
-      r *= ofac;
-      if (HEAD) r = fmaf(skip, up1 ? (up2 ? vc[3] : vc[2]) : (up2 ? vc[1] : vc[0]), r);
-      if (j < 4 && live) *optr = r;
-      optr += ostep;
-    };
-    if constexpr (HEAD) {
-#pragma unroll 1
-      for (int tt = 0; tt < cn; ++tt) {
-        fac *= ds[st][tt];
-        if (fac < 1e-12f) {   // (the same in every thread of the CTA)
-          const f32x2_t f2 = x2_pack(fac, fac);
+    }
 #pragma unroll
-          for (int i = 0; i < HP; ++i)
+    for (int c = 0; c < NC; ++c) {
+      float lo, hi;
+      x2_unpack(sum[c], lo, hi);
+      o[c] = lo + hi;
+    }
+  };
+  // tokens tt .. tt + TB - 1 of the chunk (ALL: all of them are there; else those below cn)
+  auto batch = [&](int tt, int cn, auto all) {
+    constexpr bool ALL = decltype(all)::value;
+    float o[16], of = qscale;
 #pragma unroll
-            for (int c = 0; c < NC; ++c) s[i][c] = x2_mul(f2, s[i][c]);
-          fac = 1.0f;
+    for (int x = 0; x < TB; ++x) {
+      if (ALL || tt + x < cn) {
+        if constexpr (HEAD) {
+          fac *= ds[st][tt + x];
+          if (!ALL && fac < 1e-12f) rescale();
+          of = x == mtok ? qscale * fac : of;
         }
-        token(tt, bs[st][tt] * __fdividef(1.0f, fac), qscale * fac);   // (1e-12 <= fac <= 1)
+        token(tt + x, o + x * NC);
+      } else {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) o[x * NC + c] = 0.f;
       }
-    } else if (cn == CH) {
-#pragma unroll 2
-      for (int tt = 0; tt < CH; ++tt) token(tt, 0.f, qscale);
-    } else {
+    }
+#pragma unroll
+    for (int x = 0; x < 8; ++x) o[x] = (b0 ? o[x + 8] : o[x]) + __shfl_xor_sync(0xffffffffu, b0 ? o[x] : o[x + 8], 1);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) o[x] = (b1 ? o[x + 4] : o[x]) + __shfl_xor_sync(0xffffffffu, b1 ? o[x] : o[x + 4], 2);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) o[x] = (b2 ? o[x + 2] : o[x]) + __shfl_xor_sync(0xffffffffu, b2 ? o[x] : o[x + 2], 4);
+    float r = (b3 ? o[1] : o[0]) + __shfl_xor_sync(0xffffffffu, b3 ? o[0] : o[1], 8);
+    r *= of;
+    if (live && (ALL || tt + mtok < cn)) {
+      if (RULE == STATE_RULE_DECAY_HEAD) r = fmaf(skip, vs[st][tt + mtok][cl + mcol], r);
+      *optr = r;
+    }
+    optr += TB * ostep;
+  };
+  for (int c0 = 0; c0 < n; c0 += CH, st ^= 1) {
+    const int cn = min(CH, n - c0);
+    cp_async_wait_all();                                            // this chunk's copies (the only ones in flight)
+    __syncthreads();                                                // ... of every thread; and every thread has left the other stage
+    if (c0 + CH < n) issue(min(CH, n - c0 - CH), st ^ 1);           // the next chunk's copies run beside this chunk's arithmetic
+    bool all = cn == CH;
+    if (HEAD && all) {   // decays are at most one, so the factor behind the chunk's last token is the smallest (the same in every thread of the CTA)
+      float d = ds[st][0];
+#pragma unroll
+      for (int tt = 1; tt < CH; ++tt) d *= ds[st][tt];
+      if (fac * d < 2e-12f) rescale();
+      all = !(fac * d < 2e-12f);
+    }
+    if (all) {
+#pragma unroll
+      for (int tt = 0; tt < CH; tt += TB) batch(tt, CH, std::true_type());
+    } else {   // the last tokens, or decays near zero
 #pragma unroll 1
-      for (int tt = 0; tt < cn; ++tt) token(tt, 0.f, qscale);
+      for (int tt = 0; tt < cn; tt += TB) batch(tt, cn, std::false_type());
     }
   }
-  const f32x2_t f2 = x2_pack(fac, fac);
+  if (HEAD) rescale();
 #pragma unroll
   for (int i = 0; i < HP; ++i) {
-    float lo[NC], hi[NC];
+    float w[2][NC];
 #pragma unroll
-    for (int c = 0; c < NC; ++c) x2_unpack(x2_mul(f2, s[i][c]), lo[c], hi[c]);
+    for (int c = 0; c < NC; ++c) x2_unpack(s[i][c], w[0][c], w[1][c]);
 #pragma unroll
     for (int x = 0; x < 2; ++x) {
       const int d = channel(2 * i + x);
-      const float* src = x ? hi : lo;
-      if (live && d < g.dim) *reinterpret_cast<float4*>(s_out + (size_t)d * g.vdim + col0 + cl) = make_float4(src[0], src[1], src[2], src[3]);
+      float* dst = s_out + (size_t)d * g.vdim + col0 + cl;
+      if (!live || d >= g.dim) continue;
+      if constexpr (NC == 4) {
+        *reinterpret_cast<float4*>(dst) = make_float4(w[x][0], w[x][1], w[x][2], w[x][3]);
+      } else {
+        *reinterpret_cast<float2*>(dst) = make_float2(w[x][0], w[x][1]);
+      }
     }
   }
 }
@@ -1449,6 +1415,33 @@ int launch_scan_rule(int dpt, dim3 grid, dim3 block, cudaStream_t s, const float
   return -22;
 }
 
+template <int RULE>
+static int launch_scan_packed(cudaStream_t s, const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay,
+                              const float* beta, const StateGeom& g, float qscale, float* state, int portions, const int32_t* last_rows,
+                              const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions, const int32_t* slots,
+                              float* out) {
+  // Columns per lane: four, or two where that leaves fewer than twelve warps of two columns per SM (one to six prompts of 512 tokens, 32 heads of 64 columns,
+  // state-space / time-mixing rules, us with two and with four: two prompts 76 / 84 and 58 / 61, three 96 / 109 and 75 / 80, four 120 / 110 and 94 / 81, six 188 / 144
+  // and 144 / 110; one token per sequence is bound by the states' bytes, and four columns are one sixteen-byte access).
+  // Prompts: a full dependency on the kernel in front.  Launched early, the CTAs, which last for the whole prompt, gather on the SMs that the product in front
+  // leaves free (1011 tokens: 173 and 145 us instead of 87 and 111).
+  const long groups = (long)portions * g.heads * ((g.vdim + 7) / 8);
+  const int nc = last_rows != nullptr && groups < 6L * device_num_sms() ? 2 : 4;
+  if (last_rows != nullptr) b2_pdl_skip_next();
+#define B2_SCAN_PACKED_CASE(D, N)                                                                                                                \
+  B2_CUDA_OK(b2_launch(state_scan_packed_kernel<D, RULE, N>, dim3(portions, g.heads, (g.vdim + ScanTile<N>::COLS - 1) / ScanTile<N>::COLS),      \
+                       dim3(ScanTile<N>::THREADS), 0, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq, row_first,  \
+                       row_end, positions, slots, out));                                                                                        \
+  return 0
+#define B2_SCAN_PACKED_NC(D)                    \
+  if (nc == 4) { B2_SCAN_PACKED_CASE(D, 4); }   \
+  B2_SCAN_PACKED_CASE(D, 2)
+  if (g.dim <= 64) { B2_SCAN_PACKED_NC(4); }
+  B2_SCAN_PACKED_NC(8);
+#undef B2_SCAN_PACKED_CASE
+#undef B2_SCAN_PACKED_NC
+}
+
 }  // namespace
 
 int launch_lowrank_act(const float* lr, int ld, int lr_off, int rank, const float* w2, const float* bias, int mode, float rate,
@@ -1523,49 +1516,31 @@ int launch_state_scan(const float* q, int ldq, const float* k, int ldk, const fl
   int cols = std::min(32 * nc, (g.vdim + step - 1) / step * step);
   while (cols > step && (long)portions * g.heads * ((g.vdim + cols - 1) / cols) < 2L * device_num_sms()) cols = (cols / 2 + step - 1) / step * step;
   const dim3 grid(portions, g.heads, (g.vdim + cols - 1) / cols), block(cols / nc * SC_LANES);
-  if (g.rule == STATE_RULE_DECAY)
-    return launch_scan_rule<STATE_RULE_DECAY>(dpt, grid, block, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq,
-                                              row_first, row_end, positions, slots, out, cols);
   static const bool packed = [] { const char* e = getenv("B2_SCAN_PACKED"); return !(e && *e == '0'); }();   // 0: the generic form (cross-check)
+  const bool head = g.rule == STATE_RULE_DECAY_HEAD || g.rule == STATE_RULE_DELTA_HEAD;
   const bool rows16 = g.dim % 4 == 0 && g.vdim % 4 == 0 && ldq % 4 == 0 && ldk % 4 == 0 && ldv % 4 == 0 &&
-                      ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v)) & 15) == 0;
-  if ((g.rule == STATE_RULE_DECAY_HEAD || g.rule == STATE_RULE_BONUS) && packed && rows16 && dpt <= 16 && (reinterpret_cast<uintptr_t>(decay) & 15) == 0) {
-#define B2_SCAN_SUM(D, R)                                                                                                                          \
-  B2_CUDA_OK(b2_launch(state_scan_sum_kernel<D, R>, grid, block, 0, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq,   \
-                       row_first, row_end, positions, slots, out, cols))
-    if (g.rule == STATE_RULE_DECAY_HEAD) {
-      if (dpt <= 4) B2_SCAN_SUM(4, STATE_RULE_DECAY_HEAD);
-      else if (dpt == 8) B2_SCAN_SUM(8, STATE_RULE_DECAY_HEAD);
-      else B2_SCAN_SUM(16, STATE_RULE_DECAY_HEAD);
-    } else {
-      if (dpt <= 4) B2_SCAN_SUM(4, STATE_RULE_BONUS);
-      else if (dpt == 8) B2_SCAN_SUM(8, STATE_RULE_BONUS);
-      else B2_SCAN_SUM(16, STATE_RULE_BONUS);
-    }
-#undef B2_SCAN_SUM
-    return 0;
+                      ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+                        reinterpret_cast<uintptr_t>(state) | (head ? 0 : reinterpret_cast<uintptr_t>(decay))) & 15) == 0;
+  const bool fits = packed && rows16 && g.dim <= 128;
+#define B2_SCAN_RULES(CALL)                                            \
+  switch (g.rule) {                                                    \
+    case STATE_RULE_DECAY: return CALL(STATE_RULE_DECAY);              \
+    case STATE_RULE_DECAY_HEAD: return CALL(STATE_RULE_DECAY_HEAD);    \
+    case STATE_RULE_BONUS: return CALL(STATE_RULE_BONUS);              \
+    case STATE_RULE_DELTA_HEAD: return CALL(STATE_RULE_DELTA_HEAD);    \
+    default: return CALL(STATE_RULE_DELTA);                            \
   }
-  if (g.rule == STATE_RULE_DECAY_HEAD)
-    return launch_scan_rule<STATE_RULE_DECAY_HEAD>(dpt, grid, block, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq,
-                                                   row_first, row_end, positions, slots, out, cols);
-  if (g.rule == STATE_RULE_BONUS)
-    return launch_scan_rule<STATE_RULE_BONUS>(dpt, grid, block, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq,
-                                              row_first, row_end, positions, slots, out, cols);
-  if (g.rule == STATE_RULE_DELTA_HEAD && packed && rows16 && dpt <= 16) {
-#define B2_SCAN_HEAD(D)                                                                                                                          \
-  B2_CUDA_OK(b2_launch(state_scan_head_kernel<D>, grid, block, 0, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq,   \
-                       row_first, row_end, positions, slots, out, cols))
-    if (dpt <= 4) B2_SCAN_HEAD(4);
-    else if (dpt == 8) B2_SCAN_HEAD(8);
-    else B2_SCAN_HEAD(16);
-#undef B2_SCAN_HEAD
-    return 0;
+#define B2_SCAN_GENERIC(R) \
+  launch_scan_rule<R>(dpt, grid, block, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq, row_first, row_end, positions, slots, out, cols)
+#define B2_SCAN_PACKED_RULE(R) \
+  launch_scan_packed<R>(s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, portions, last_rows, row_seq, row_first, row_end, positions, slots, out)
+  if (fits) {
+    B2_SCAN_RULES(B2_SCAN_PACKED_RULE)
   }
-  if (g.rule == STATE_RULE_DELTA_HEAD)
-    return launch_scan_rule<STATE_RULE_DELTA_HEAD>(dpt, grid, block, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq,
-                                                   row_first, row_end, positions, slots, out, cols);
-  return launch_scan_rule<STATE_RULE_DELTA>(dpt, grid, block, s, q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, last_rows, row_seq,
-                                            row_first, row_end, positions, slots, out, cols);
+  B2_SCAN_RULES(B2_SCAN_GENERIC)
+#undef B2_SCAN_RULES
+#undef B2_SCAN_GENERIC
+#undef B2_SCAN_PACKED_RULE
 }
 
 size_t state_floats_per_slot(const StateGeom& g) { return (size_t)2 * g.heads * g.dim * g.vdim; }

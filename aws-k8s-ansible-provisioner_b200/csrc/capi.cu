@@ -86,6 +86,18 @@ extern "C" int b2k_linear_multicast(const void* x, const void* w, void* out, int
   return launch_linear_mc(tw, tx, (bf16*)out, T, N, K, 0, wait, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
+                              const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
+                              const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,
+                              const int32_t* slots, float* out, void* stream) {
+  B2_REQUIRE(q && k && v && decay && state && row_seq && row_first && row_end && positions && slots && out, "b2k_state_scan: null pointer");
+  StateGeom g{heads, kv_heads, dim, vdim, rule};
+  g.skip = skip;
+  g.bonus = bonus;
+  return launch_state_scan(q, ldq, k, ldk, v, ldv, decay, beta, g, qscale, state, portions, last_rows, row_seq, row_first, row_end, positions, slots, out,
+                           (cudaStream_t)stream);
+}
+
 extern "C" int b2k_linear_add(const void* x, const void* w, void* h, int T, int N, int K, void* stream) {
   B2_REQUIRE(x && w && h, "b2k_linear_add: null pointer");
   TcGemmArgs a;

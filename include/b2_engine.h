@@ -420,9 +420,15 @@ int b2k_qkv_rope(const void* x_bf16, const void* w_qkv_bf16, const void* qnorm_w
  *   K <= 3072; ssq[N/16][ssq_ld] (fp32) receives per token column the sum of squares of each 16-feature piece of the new h.
  * b2k_gateup_swiglu_norm / b2k_qkv_rope_norm: b2k_gateup_swiglu / b2k_qkv_rope with x = bf16(norm_w * bf16(h * rstd)) formed
  *   on the fly, rstd = rsqrt(sum of the `pieces` pieces of ssq / K + eps). */
-/* Prefill-sized y[T][N] (bf16) = x[T][K] . W[N][K]^T by pairs of CTAs that share the token tile through TMA multicast (both
- * operands in this GPU's memory); T >= 512, N % 256 == 0, K % 64 == 0.  Bit-identical to b2k_linear's bf16 output. */
+/* Prefill-sized y[T][N] (bf16) = x[T][K] . W[N][K]^T by pairs of CTAs that multiply one tile together; T >= 512, N % 256 == 0, K % 64 == 0.  Bit-identical to b2k_linear's bf16 output. */
 int b2k_linear_multicast(const void* x_bf16, const void* w_bf16, void* out_bf16, int T, int N, int K, void* stream);
+/* The recurrence of the matrix-state mixers over `portions` portions (portion i ends at row last_rows[i]; last_rows null: every row is one of one token); rule as
+ * StateRule in csrc/kernels.h; all tensors fp32: q / k rows of kv_heads * dim, v rows of heads * vdim, decay [T][heads * dim] or [T][heads] by the rule, beta
+ * [T][heads], skip [heads], bonus [heads][dim] (null where the rule has none), state [slots][2][heads][dim][vdim], out [T][heads * vdim]. */
+int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
+                   const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
+                   const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,
+                   const int32_t* slots, float* out, void* stream);
 /* Prefill-sized residual add in the projection's epilogue: h[T][N] (bf16, in place) = bf16(h + bf16(x[T][K] . W[N][K]^T)), T > 16. */
 int b2k_linear_add(const void* x_bf16, const void* w_bf16, void* h_bf16, int T, int N, int K, void* stream);
 int b2k_linear_resid(const void* x_bf16, const void* w_bf16, void* h_bf16, float* ssq, int T, int N, int K, int ssq_ld, void* stream);

@@ -1,0 +1,143 @@
+"""Kernels of the layer-list families (GPU), called through the C ABI (include/b2_engine.h, b2k_*) and compared with the same arithmetic in 64 bits."""
+import pytest
+import torch
+
+from _util import cuda_stream_ptr, pkg, ptr
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return pkg().load_library()
+
+
+def chk(lib, rc):
+    assert rc == 0, lib.b2_last_error().decode()
+
+
+DECAY, DELTA, DELTA_HEAD, DECAY_HEAD, BONUS = range(5)
+
+
+def scan_inputs(lengths, heads, kv, dim, vdim, rule, seed):
+    g = torch.Generator().manual_seed(seed)
+    T = sum(lengths)
+    f = lambda *s: torch.randn(*s, generator=g)
+    head = rule in (DELTA_HEAD, DECAY_HEAD)
+    decay = torch.exp(-torch.exp(f(T, heads if head else heads * dim) - 2.0))
+    decay[torch.rand(decay.shape, generator=g) < 0.02] = 0.0        # a memory that is gone at once
+    decay[torch.rand(decay.shape, generator=g) < 0.02] = 1e-9
+    unit = lambda x: x / x.norm(dim=-1, keepdim=True)
+    k = f(T, kv, dim)
+    d = {"q": f(T, kv, dim), "k": unit(k) if rule in (DELTA, DELTA_HEAD) else k * dim ** -0.5, "v": f(T, heads, vdim), "decay": decay,
+         "beta": torch.rand(T, heads, generator=g), "skip": f(heads), "bonus": f(heads, dim)}
+    return {n: t.float() for n, t in d.items()}
+
+
+def scan_reference(x, lengths, heads, kv, dim, vdim, rule, qscale, s0):
+    """[T][heads][vdim] and the states behind the last tokens, in 64 bits."""
+    d = {n: t.double().cuda() for n, t in x.items()}
+    rep = heads // kv
+    out, states, at = [], [], 0
+    for i, n in enumerate(lengths):
+        S = s0[i].double().cuda().clone()          # [heads][dim][vdim]
+        for t in range(at, at + n):
+            q, k = d["q"][t].repeat_interleave(rep, 0), d["k"][t].repeat_interleave(rep, 0)
+            v, b = d["v"][t], d["beta"][t][:, None]
+            a = d["decay"][t].view(heads, -1)[:, :, None]
+            if rule == BONUS:
+                o = torch.einsum("hd,hdv->hv", q, S) + (q * d["bonus"] * k).sum(1, keepdim=True) * v
+                S = a * S + k[:, :, None] * v[:, None, :]
+            else:
+                S = a * S
+                w = v if rule == DECAY else b * v if rule == DECAY_HEAD else b * (v - torch.einsum("hd,hdv->hv", k, S))
+                S = S + k[:, :, None] * w[:, None, :]
+                o = torch.einsum("hd,hdv->hv", q, S)
+            o = o * qscale
+            out.append(o + d["skip"][:, None] * v if rule == DECAY_HEAD else o)
+        states.append(S)
+        at += n
+    return torch.stack(out), torch.stack(states)
+
+
+def run_scan(lib, x, lengths, heads, kv, dim, vdim, rule, qscale, state, starts, single=False):
+    """One launch over all portions; state [portions][2][heads][dim][vdim] on the GPU, updated in place."""
+    T, n = sum(lengths), len(lengths)
+    i32 = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")
+    seq, first, end, pos, last, at = [], [], [], [], [], 0
+    for i, m in enumerate(lengths):
+        seq += [i] * m
+        first += [at] * m
+        end += [at + m] * m
+        pos += list(range(starts[i], starts[i] + m))
+        at += m
+        last.append(at - 1)
+    d = {name: t.cuda().contiguous() for name, t in x.items()}
+    out = torch.full((T, heads * vdim), float("nan"), device="cuda")
+    idx = [i32(v) for v in (last, seq, first, end, pos, list(range(T)))]
+    chk(lib, lib.b2k_state_scan(ptr(d["q"]), kv * dim, ptr(d["k"]), kv * dim, ptr(d["v"]), heads * vdim, ptr(d["decay"]), ptr(d["beta"]), ptr(d["skip"]), ptr(d["bonus"]),
+                                heads, kv, dim, vdim, rule, qscale, ptr(state), n, None if single else ptr(idx[0]), *[ptr(t) for t in idx[1:]], ptr(out), cuda_stream_ptr()))
+    torch.cuda.synchronize()
+    return out.view(T, heads, vdim)
+
+
+def rel2(a, b):
+    return ((a.double() - b).norm() / b.norm().clamp_min(1e-30)).item()
+
+
+@pytest.mark.parametrize("rule", [DECAY, DELTA, DELTA_HEAD, DECAY_HEAD, BONUS])
+@pytest.mark.parametrize("dim,vdim", [(128, 64), (64, 36), (96, 20), (20, 128), (18, 10), (160, 24)])
+def test_state_scan(lib, rule, dim, vdim):
+    """Portions around the chunk of eight tokens, a state to start from, decays down to zero; the sizes that the packed form does not hold ((18, 10): rows that are
+    no multiples of 16 bytes, 160: wider keys) take the generic one.  Bound: a number of the result passes through at most dim + tokens roundings of 2^-24 each,
+    of which the sums' random signs leave a few; an eighth of that count is allowed in the 2-norm."""
+    heads, kv, lengths, starts, qscale = 4, 2, [1, 7, 8, 9, 33, 16], [0, 3, 0, 4, 6, 1], 0.37
+    x = scan_inputs(lengths, heads, kv, dim, vdim, rule, seed=dim * 1000 + vdim * 10 + rule)
+    g = torch.Generator().manual_seed(5)
+    state = torch.zeros(len(lengths), 2, heads, dim, vdim)
+    s0 = torch.zeros(len(lengths), heads, dim, vdim)
+    for i, p in enumerate(starts):
+        if p > 0:
+            s0[i] = torch.randn(heads, dim, vdim, generator=g)
+            state[i, (p - 1) & 1] = s0[i]
+    ref, ref_s = scan_reference(x, lengths, heads, kv, dim, vdim, rule, qscale, s0)
+    dev = state.cuda()
+    got = run_scan(lib, x, lengths, heads, kv, dim, vdim, rule, qscale, dev, starts)
+    got_s = torch.stack([dev[i, (p + n - 1) & 1] for i, (p, n) in enumerate(zip(starts, lengths))])
+    tol = (dim + max(lengths)) / 8 * 2.0 ** -24
+    assert rel2(got, ref) < tol and rel2(got_s, ref_s) < tol
+
+    # one token per launch: the same, and the same bits where no factor is carried through a portion
+    dev1 = state.cuda()
+    at, per = 0, []
+    for i, n in enumerate(lengths):
+        per.append((at, n))
+        at += n
+    one = torch.empty_like(got)
+    for step in range(max(lengths)):
+        who = [i for i, n in enumerate(lengths) if step < n]
+        sub = {name: t if name in ("skip", "bonus") else torch.stack([t[per[i][0] + step] for i in who]) for name, t in x.items()}
+        sel = dev1[who].contiguous()
+        o = run_scan(lib, sub, [1] * len(who), heads, kv, dim, vdim, rule, qscale, sel, [starts[i] + step for i in who], single=True)
+        for j, i in enumerate(who):
+            dev1[i] = sel[j]
+            one[per[i][0] + step] = o[j]
+    if rule in (DECAY, DELTA, BONUS):
+        assert torch.equal(one, got)
+    else:
+        assert rel2(one, ref) < tol
+
+
+@pytest.mark.parametrize("rule", [DECAY, DELTA, DELTA_HEAD, DECAY_HEAD, BONUS])
+def test_state_scan_many_portions(lib, rule):
+    """Enough portions for four columns per lane: the bits of a portion are those it has alone (two columns per lane)."""
+    heads, kv, dim, vdim, n = 4, 4, 64, 128, 19
+    one = scan_inputs([n], heads, kv, dim, vdim, rule, seed=rule)
+    zero = lambda p: torch.zeros(p, 2, heads, dim, vdim, device="cuda")
+    alone = run_scan(lib, one, [n], heads, kv, dim, vdim, rule, 1.0, zero(1), [0])
+    many = 24   # 24 * 4 * 16 groups of eight columns
+    x = {name: t if name in ("skip", "bonus") else torch.cat([t] * many) for name, t in one.items()}
+    got = run_scan(lib, x, [n] * many, heads, kv, dim, vdim, rule, 1.0, zero(many), [0] * many)
+    assert torch.equal(got, alone.repeat(many, 1, 1))
