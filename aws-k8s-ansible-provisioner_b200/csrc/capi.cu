@@ -86,6 +86,13 @@ extern "C" int b2k_linear_multicast(const void* x, const void* w, void* out, int
   return launch_linear_mc(tw, tx, (bf16*)out, T, N, K, 0, wait, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_linear_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, int tile, void* stream) {
+  B2_REQUIRE(x && w && out, "b2k_linear_sum: null pointer");
+  B2WaitLimit wait;
+  CAPI_TRY(hook_waits(&wait));
+  return launch_linear_sum(x, w, offsets, groups, rows, out, N, K, epilogue, wait, (cudaStream_t)stream, tile);
+}
+
 extern "C" int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
                               const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
                               const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,

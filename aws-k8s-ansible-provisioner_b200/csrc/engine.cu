@@ -944,7 +944,9 @@ int forward_layers(b2_engine* e, const Lane& ln, int T, int ntiles) {
 // layer share one statistic (one kernel).  Mixer = latent attention in absorbed form (attn_latent.cu); feed-forward =
 // routed squared-ReLU experts as ragged groups of gemm_any.cu.  `rows` (device, nlast entries; null = every row) selects
 // the positions that get logits.  Operands are bf16, or fp32 when the engine was created with compute_f32.
-constexpr int LIST_TC_EXPERT_ROWS = 2048;   // (token, choice) pairs of a step from which the experts' products go expert by expert to the tcgen05 kernel
+constexpr int LIST_SILU_EXPERT_ROWS = 2048;   // (token, choice) pairs of a step from which silu-gated experts go one by one to the product with the activation in its epilogue
+// ... and from which the experts' products run on the tcgen05 kernel of ragged groups: all that do not stream the experts' weights group by group
+int list_tc_expert_rows() { return any_gemm_ragged_rows_limit() + 1; }
 
 // C (fp32 [M][N]) = alpha * A (operand type [M][K]) . Wt^T for the layer-list families.  Prompt-sized bf16 products whose K the tcgen05
 // projection kernel can tile (gemm_tc.cu: TMA needs 16-byte rows, its k-block is 64) take that kernel, fp32 sums written directly;
@@ -958,6 +960,7 @@ int list_dense(b2_engine* e, const void* A, const void* Wt, float* C, int M, int
   cudaStream_t ls = stream ? stream : e->stream;
   const int f = e->f32 ? 1 : 0;
   if (alpha == 1.f && list_dense_tc(e, M, N, K)) {
+    if (M > 128 && linear_sum_pays(M, N)) return launch_linear_sum(A, Wt, nullptr, 1, M, C, N, K, SUM_EPI_F32, e->wait_limit(), ls);
     TcGemmArgs a;
     a.bn = tc_pick_bn(M);
     B2_TRY(b2_make_tmap_bf16(&a.tmap_w, Wt, (uint64_t)N, (uint64_t)K, (uint64_t)K, 128));
@@ -977,9 +980,10 @@ int list_dense(b2_engine* e, const void* A, const void* Wt, float* C, int M, int
 
 // The two products of a layer's routed experts around a gated activation, for the families whose experts have gate and up rows: l_x1 rows -> gate |
 // up sums (l_upf, fp32, expert order) -> act(operand is fp32?) -> l_act -> l_y (fp32, expert order).  The permutation (l_offsets,
-// l_slot_token) is in place.  Prompt-sized bf16 steps (prompt = true) run expert by expert on the tcgen05 projection kernel: rows gathered into
-// expert order, the experts' slot ranges read back (one small copy and a stream synchronisation per layer); everything else as ragged groups.
-// plain_silu: the activation is silu(gate) * up as it is, so the gate/up products that have it in their epilogue may be used.
+// l_slot_token) is in place.  Prompt-sized bf16 steps (prompt = true): rows gathered into expert order, then one tcgen05 launch per product over all
+// experts (gemm_sum.cu reads their slot ranges on the device); everything else as ragged groups of gemm_any.cu.
+// plain_silu: the activation is silu(gate) * up as it is, so long steps go expert by expert to the gate/up product that has it in its epilogue
+// (the slot ranges are read back: one small copy and a stream synchronisation per layer).
 bool list_gate_up_fused(int M, int F, int W) {
   static const bool on = [] { const char* v = getenv("B2_LIST_GU_FUSED"); return !(v && *v == '0'); }();
   return on && list_use_tc() && gateup_prefill_shapes_ok(M, F, W);
@@ -1021,8 +1025,26 @@ template <typename Act>
 int list_gated_experts(b2_engine* e, const ListLayer& L, int layer, int T, bool prompt, cudaStream_t s, Act act, bool plain_silu = false) {
   const b2_layer_spec& sp = L.sp;
   const int W = e->cfg.hidden, f = e->f32 ? 1 : 0, F = sp.ff_dim, pairs = T * sp.top;
-  const bool tc_experts = prompt && list_use_tc() && !f && e->l_xperm != nullptr && pairs >= LIST_TC_EXPERT_ROWS && W % 64 == 0 && F % 64 == 0 && W >= 128 &&
-                          F >= 64 && e->skip_mask == 0;
+  const bool grouped = prompt && list_use_tc() && !f && e->l_xperm != nullptr && pairs >= list_tc_expert_rows() && W % 64 == 0 && F % 64 == 0 && W >= 128 &&
+                       linear_sum_shapes_ok(pairs, sp.experts, 2 * F, W) && linear_sum_shapes_ok(pairs, sp.experts, W, F);
+  const bool tc_experts = grouped && plain_silu && pairs >= LIST_SILU_EXPERT_ROWS && T > 256 && e->skip_mask == 0;   // (no read-back where side streams run)
+  if (grouped && !tc_experts) {
+    {
+      KL k(e, B2K_MISC);
+      if (!k.skip()) B2_TRY(launch_gather_rows((const bf16*)e->l_x1, e->l_slot_token, e->l_xperm, pairs, W, s));
+    }
+    {
+      KL k(e, B2K_GEMM_GATEUP);
+      if (!k.skip()) B2_TRY(launch_linear_sum(e->l_xperm, L.up, e->l_offsets, sp.experts, pairs, e->l_upf, 2 * F, W, SUM_EPI_F32, e->wait_limit(), s));
+    }
+    {
+      KL k(e, B2K_ACT);
+      if (!k.skip()) B2_TRY(act(0));
+    }
+    KL k(e, B2K_GEMM_DOWN);
+    if (!k.skip()) B2_TRY(launch_linear_sum(e->l_act, L.down, e->l_offsets, sp.experts, pairs, e->l_y, W, F, SUM_EPI_F32, e->wait_limit(), s));
+    return 0;
+  }
   if (tc_experts) {
     B2_CUDA_OK(cudaMemcpyAsync(e->h_offsets, e->l_offsets, (size_t)(sp.experts + 1) * 4, cudaMemcpyDeviceToHost, s));
     {
@@ -1038,17 +1060,13 @@ int list_gated_experts(b2_engine* e, const ListLayer& L, int layer, int T, bool 
         const int n = off[x + 1] - off[x];
         const bf16 *xa = e->l_xperm + (size_t)off[x] * W, *wu = (const bf16*)L.up + (size_t)x * 2 * F * W;
         if (n == 0) continue;
-        if (plain_silu && list_gate_up_fused(n, F, W)) {
+        if (list_gate_up_fused(n, F, W)) {
           B2_TRY(list_gate_up(xa, wu, (bf16*)e->l_act + (size_t)off[x] * F, n, F, W, s));
           continue;
         }
         B2_TRY(list_dense(e, xa, wu, e->l_upf + (size_t)off[x] * 2 * F, n, 2 * F, W, 1.f, s));
-        if (plain_silu) B2_TRY(launch_silu_gate(e->l_upf + (size_t)off[x] * 2 * F, nullptr, nullptr, (bf16*)e->l_act + (size_t)off[x] * F, 0, n, F, s));
+        B2_TRY(launch_silu_gate(e->l_upf + (size_t)off[x] * 2 * F, nullptr, nullptr, (bf16*)e->l_act + (size_t)off[x] * F, 0, n, F, s));
       }
-    }
-    if (!plain_silu) {
-      KL k(e, B2K_ACT);
-      B2_TRY(act(0));
     }
     {
       KL k(e, B2K_GEMM_DOWN);
@@ -1302,38 +1320,25 @@ int forward_list(b2_engine* e, int T, int ntiles, int nlast) {
         KL k(e, B2K_MISC);
         if (!k.skip()) B2_TRY(launch_route_permute(e->l_idx, T, sp.top, sp.experts, e->l_offsets, e->l_offsets_stride, e->l_slot_token, e->l_pair_slot, st));
       }
-      // Prompt-sized bf16 steps: the rows are gathered into expert order, the experts' slot ranges are read back (one small
-      // copy and a stream synchronisation per layer: nothing beside a pass that takes milliseconds), and every expert's two
-      // products are plain dense projections on the tcgen05 kernel; the activation rounds the fp32 sums to the bf16 operand
-      // of the second product.  Everything else (decode steps, short portions, fp32, odd sizes) runs as ragged groups.
-      const bool tc_experts = use_tc && !f && ntiles > 0 && e->l_xperm != nullptr && T * sp.top >= LIST_TC_EXPERT_ROWS && W % 64 == 0 &&
-                              sp.ff_dim % 64 == 0 && W >= 128 && sp.ff_dim >= 128 && e->skip_mask == 0;
-      if (tc_experts) {
-        B2_CUDA_OK(cudaMemcpyAsync(e->h_offsets, e->l_offsets, (size_t)(sp.experts + 1) * 4, cudaMemcpyDeviceToHost, st));
+      // Prompt-sized bf16 steps: the rows are gathered into expert order, and each of the two products is one tcgen05 launch over all experts, which
+      // reads their slot ranges on the device; the first one's epilogue rounds the activation to the bf16 operand of the second.  (8 x 1024 tokens, 16 experts
+      // of 704, width 2048, both products: 520 us as a launch per expert behind a read-back of the ranges.)
+      // Everything else (decode steps, short portions, fp32, odd sizes) runs as ragged groups of gemm_any.cu.
+      const bool grouped = use_tc && !f && ntiles > 0 && e->l_xperm != nullptr && T * sp.top >= list_tc_expert_rows() && W % 64 == 0 &&
+                           sp.ff_dim % 64 == 0 && W >= 128 && sp.ff_dim >= 128 && linear_sum_shapes_ok(T * sp.top, sp.experts, sp.ff_dim, W) &&
+                           linear_sum_shapes_ok(T * sp.top, sp.experts, W, sp.ff_dim);
+      if (grouped) {
         {
           KL k(e, B2K_MISC);
-          B2_TRY(launch_gather_rows((const bf16*)e->l_x2, e->l_slot_token, e->l_xperm, T * sp.top, W, st));
+          if (!k.skip()) B2_TRY(launch_gather_rows((const bf16*)e->l_x2, e->l_slot_token, e->l_xperm, T * sp.top, W, st));
         }
-        B2_CUDA_OK(cudaStreamSynchronize(st));
-        const int32_t* off = e->h_offsets;
-        B2_REQUIRE(off[0] == 0 && off[sp.experts] == T * sp.top, "layer %d: the experts' slot ranges do not cover the step's %d pairs", l, T * sp.top);
         {
           KL k(e, B2K_GEMM_GATEUP);
-          for (int x = 0; x < sp.experts; ++x)
-            if (off[x + 1] > off[x])
-              B2_TRY(dense(e->l_xperm + (size_t)off[x] * W, (const bf16*)L.up + (size_t)x * sp.ff_dim * W, e->l_upf + (size_t)off[x] * sp.ff_dim,
-                           off[x + 1] - off[x], sp.ff_dim, W, 1.f));
-        }
-        {
-          KL k(e, B2K_ACT);
-          B2_TRY(launch_relu2_round(e->l_upf, (bf16*)e->l_act, (size_t)T * sp.top * sp.ff_dim, st));
+          if (!k.skip()) B2_TRY(launch_linear_sum(e->l_xperm, L.up, e->l_offsets, sp.experts, T * sp.top, e->l_act, sp.ff_dim, W, SUM_EPI_RELU2, e->wait_limit(), st));
         }
         {
           KL k(e, B2K_GEMM_DOWN);
-          for (int x = 0; x < sp.experts; ++x)
-            if (off[x + 1] > off[x])
-              B2_TRY(dense((const bf16*)e->l_act + (size_t)off[x] * sp.ff_dim, (const bf16*)L.down + (size_t)x * W * sp.ff_dim,
-                           e->l_y + (size_t)off[x] * W, off[x + 1] - off[x], W, sp.ff_dim, 1.f));
+          if (!k.skip()) B2_TRY(launch_linear_sum(e->l_act, L.down, e->l_offsets, sp.experts, T * sp.top, e->l_y, W, sp.ff_dim, SUM_EPI_F32, e->wait_limit(), st));
         }
       } else {
         const int max_tiles = std::min(e->l_tiles_cap, (T * sp.top + any_gemm_tile_rows() - 1) / any_gemm_tile_rows() + sp.experts);
@@ -1684,7 +1689,7 @@ int forward_state_list(b2_engine* e, int T, int ntiles, int nlast) {
         }
       }
       // The weight multiplies the expert's input: gate and up are linear in it, so it is applied to their fp32 sums inside the activation.
-      B2_TRY(list_gated_experts(e, L, R.layer, T, ntiles > 0 && !multi, sF,
+      B2_TRY(list_gated_experts(e, L, R.layer, T, ntiles > 0, sF,
                                 [&](int act_f32) { return launch_silu_gate(e->l_upf, e->l_slot_scale, nullptr, e->l_act, act_f32, pairs, F, sF); }));
       yr = e->l_y;
       if (sp.shared_ff > 0) {   // (buffers of its own: in short steps it runs beside the routed experts)
@@ -2059,7 +2064,7 @@ int forward_outnorm_list(b2_engine* e, int T, int ntiles, int nlast) {
         KL k(e, B2K_MISC);
         if (!k.skip()) B2_TRY(launch_route_permute(e->l_idx, T, sp.top, sp.experts, e->l_offsets, e->l_offsets_stride, e->l_slot_token, e->l_pair_slot, st));
       }
-      B2_TRY(list_gated_experts(e, L, l, T, ntiles > 0 && !multi, st,
+      B2_TRY(list_gated_experts(e, L, l, T, ntiles > 0, st,
                                 [&](int act_f32) { return launch_silu_gate(e->l_upf, nullptr, nullptr, e->l_act, act_f32, pairs, F, st); }, true));
       if (sS == st && shared) B2_TRY(shared_expert());
       if (sS != st) {
@@ -2289,7 +2294,7 @@ int forward_streams_list(b2_engine* e, int T, int ntiles, int nlast) {
         KL k(e, B2K_MISC);
         if (!k.skip()) B2_TRY(launch_route_permute(e->l_idx, T, sp.top, sp.experts, e->l_offsets, e->l_offsets_stride, e->l_slot_token, e->l_pair_slot, st));
       }
-      B2_TRY(list_gated_experts(e, L, R.layer, T, ntiles > 0 && !multi, st,
+      B2_TRY(list_gated_experts(e, L, R.layer, T, ntiles > 0, st,
                                 [&](int act_f32) { return launch_silu_gate(e->l_upf, nullptr, nullptr, e->l_act, act_f32, pairs, F, st); }, true));
       StreamBranch br;
       br.y = e->l_y;
@@ -3482,7 +3487,7 @@ int state_engine_alloc(b2_engine* e) {
   B2_TRY(dalloc(&e->l_tile_group, (size_t)e->l_tiles_cap));
   B2_TRY(dalloc(&e->l_tile_row0, (size_t)e->l_tiles_cap));
   B2_TRY(dalloc(&e->l_ntiles, (size_t)1));
-  if (!e->f32 && Tc * max_top >= (size_t)LIST_TC_EXPERT_ROWS && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
+  if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
     B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
     B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
   }
@@ -3788,7 +3793,7 @@ int mixed_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&e->l_tile_group, (size_t)e->l_tiles_cap));
     B2_TRY(dalloc(&e->l_tile_row0, (size_t)e->l_tiles_cap));
     B2_TRY(dalloc(&e->l_ntiles, (size_t)1));
-    if (!e->f32 && Tc * max_top >= (size_t)LIST_TC_EXPERT_ROWS && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
+    if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
       B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
     }
@@ -4045,7 +4050,7 @@ int outnorm_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&e->l_tile_row0, (size_t)e->l_tiles_cap));
     B2_TRY(dalloc(&e->l_ntiles, (size_t)1));
     B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));
-    if (!e->f32 && Tc * max_top >= (size_t)LIST_TC_EXPERT_ROWS && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
+    if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
       B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
     }
@@ -4351,7 +4356,7 @@ int streams_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&e->l_tile_row0, (size_t)e->l_tiles_cap));
     B2_TRY(dalloc(&e->l_ntiles, (size_t)1));
     B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));
-    if (!e->f32 && Tc * max_top >= (size_t)LIST_TC_EXPERT_ROWS && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
+    if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
       B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
     }
@@ -4530,7 +4535,7 @@ int list_engine_alloc(b2_engine* e) {
     }
     e->l_attn_scratch_floats = latent_attention_scratch_floats(bucket_batch(c.max_seqs), max_heads, max_rank);
     B2_TRY(dalloc(&e->l_attn_scratch, e->l_attn_scratch_floats));
-    if (max_top > 0 && Tc * max_top >= (size_t)LIST_TC_EXPERT_ROWS) {   // prompt-sized expert products on the tcgen05 projection kernel
+    if (max_top > 0 && Tc * max_top >= (size_t)list_tc_expert_rows()) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
       B2_TRY(dalloc(&e->l_upf, Tc * max_top * max_ff));
       B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));

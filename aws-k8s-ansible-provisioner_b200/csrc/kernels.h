@@ -100,6 +100,13 @@ int launch_linear_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* 
 int launch_qkv_rope_prefill(const CUtensorMap& tm_qkv, const CUtensorMap& tm_x128, const bf16* qw, const bf16* kw, const bf16* cos_sin,
                             const int32_t* positions, const int32_t* slots, bf16* q_out, bf16* k_pages, bf16* v_pages, int T, int nq, int nkv,
                             int K, int block_size, float eps, int x_row0, const B2WaitLimit& wait, cudaStream_t s);
+// gemm_sum.cu: prompt-sized products with fp32 sums out (or a squared-ReLU expert's bf16 activation), rows of one block or of the ragged blocks of
+// `groups` experts (offsets: [groups + 1] first rows, device memory; null: one block); w [groups * N][K]; bn: 0 = by the sizes
+enum { SUM_EPI_F32 = 0, SUM_EPI_RELU2 = 1 };
+bool linear_sum_shapes_ok(int rows, int groups, int N, int K);
+bool linear_sum_pays(int rows, int N);   // one block of rows: faster than launch_linear_tc
+int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, const B2WaitLimit& wait,
+                      cudaStream_t s, int bn = 0);
 // gemm_gateup.cu: the prefill-sized counterpart (two accumulators per tile, SwiGLU in the epilogue)
 bool gateup_prefill_shapes_ok(int T, int I, int K);
 int launch_gateup_swiglu_prefill(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* act, int T, int I, int K, int x_row0, cudaStream_t s);
@@ -555,8 +562,6 @@ int launch_route_permute(const int32_t* idx, int T, int top, int experts, int32_
                          int32_t* pair_slot, cudaStream_t s);
 // slot_weight[pair_slot[p]] = weight[p] for the T*top pairs
 int launch_route_slot_weights(const float* weight, const int32_t* pair_slot, float* slot_weight, int npairs, cudaStream_t s);
-// act[i] = bf16(max(up[i], 0)^2), n a multiple of 4
-int launch_relu2_round(const float* up, bf16* act, size_t n, cudaStream_t s);
 // h[t] += sum_k weight[t][k] * y[pair_slot[t*top + k]]   (+ mix[t] when given); fp32
 int launch_route_combine(float* h, const float* mix, const float* y, const float* weight, const int32_t* pair_slot, int T, int W, int top,
                          cudaStream_t s);

@@ -301,31 +301,7 @@ __global__ void __launch_bounds__(256) route_table_kernel(const int32_t* __restr
   weight[p] = 1.0f / (float)top;
 }
 
-// act = bf16(max(up, 0)^2): the experts' activation between the two dense products of a prompt-sized step
-__global__ void __launch_bounds__(256) relu2_round_kernel(const float4* __restrict__ up, uint2* __restrict__ act, size_t n4) {
-  pdl_wait();
-  pdl_launch_dependents();
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
-    const float4 v = up[i];
-    const float a = fmaxf(v.x, 0.f), b = fmaxf(v.y, 0.f), c = fmaxf(v.z, 0.f), d = fmaxf(v.w, 0.f);
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(a * a, b * b), hi = __floats2bfloat162_rn(c * c, d * d);
-    uint2 o;
-    o.x = *reinterpret_cast<const uint32_t*>(&lo);
-    o.y = *reinterpret_cast<const uint32_t*>(&hi);
-    act[i] = o;
-  }
-}
-
 }  // namespace
-
-int launch_relu2_round(const float* up, bf16* act, size_t n, cudaStream_t s) {
-  if (n == 0) return 0;
-  if (n % 4 != 0) return -22;   // (rows are multiples of 64 wide on this path)
-  const size_t n4 = n / 4;
-  const int grid = (int)std::min<size_t>((n4 + 255) / 256, 148 * 16);
-  B2_CUDA_OK(b2_launch(relu2_round_kernel, dim3(grid), dim3(256), 0, s, (const float4*)up, (uint2*)act, n4));
-  return 0;
-}
 
 int launch_route(const void* x, int x_f32, const float* router, const float* correction, const RouteGeom& g, int32_t* idx, float* weight,
                  int T, int W, cudaStream_t s, float* gate_out) {

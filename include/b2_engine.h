@@ -422,6 +422,10 @@ int b2k_qkv_rope(const void* x_bf16, const void* w_qkv_bf16, const void* qnorm_w
  *   on the fly, rstd = rsqrt(sum of the `pieces` pieces of ssq / K + eps). */
 /* Prefill-sized y[T][N] (bf16) = x[T][K] . W[N][K]^T by pairs of CTAs that multiply one tile together; T >= 512, N % 256 == 0, K % 64 == 0.  Bit-identical to b2k_linear's bf16 output. */
 int b2k_linear_multicast(const void* x_bf16, const void* w_bf16, void* out_bf16, int T, int N, int K, void* stream);
+/* Prompt-sized products of the layer-list families on pairs of CTAs, rows of one block (offsets null, groups 1) or of `groups` ragged blocks whose first
+ * rows the kernel reads from device memory (offsets [groups + 1], the last one = rows): out[row][N] = x[row][K] . w_g[N][K]^T as fp32 (epilogue 0) or
+ * bf16(max(sum, 0)^2) (1).  K % 64 == 0; tile: 0 (by the sizes), 128 or 256 rows of x. */
+int b2k_linear_sum(const void* x_bf16, const void* w_bf16, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, int tile, void* stream);
 /* The recurrence of the matrix-state mixers over `portions` portions (portion i ends at row last_rows[i]; last_rows null: every row is one of one token); rule as
  * StateRule in csrc/kernels.h; all tensors fp32: q / k rows of kv_heads * dim, v rows of heads * vdim, decay [T][heads * dim] or [T][heads] by the rule, beta
  * [T][heads], skip [heads], bonus [heads][dim] (null where the rule has none), state [slots][2][heads][dim][vdim], out [T][heads * vdim]. */

@@ -141,3 +141,37 @@ def test_state_scan_many_portions(lib, rule):
     x = {name: t if name in ("skip", "bonus") else torch.cat([t] * many) for name, t in one.items()}
     got = run_scan(lib, x, [n] * many, heads, kv, dim, vdim, rule, 1.0, zero(many), [0] * many)
     assert torch.equal(got, alone.repeat(many, 1, 1))
+
+
+@pytest.mark.parametrize("tile", [128, 256, 0])
+@pytest.mark.parametrize("N,K", [(128, 64), (64, 192), (704, 320), (256, 1024), (300, 128)])
+def test_linear_sum_groups(lib, tile, N, K):
+    """Ragged groups around the tiles of 128 and 256 rows, empty ones, weight rows that fill no pair of 256; nothing is written behind the last row.  Sums of K products
+    of bf16 numbers, exact in fp32, in fp32: K roundings of 2^-24 of the sum of their absolute values at most (the activation squares the sum and rounds to bf16)."""
+    sizes = [0, 1, 127, 128, 129, 255, 0, 256, 257, 300, 64]
+    g = torch.Generator().manual_seed(N + K)
+    rows, G = sum(sizes), len(sizes)
+    x = torch.randn(rows, K, generator=g).to(torch.bfloat16).cuda()
+    w = (torch.randn(G, N, K, generator=g) * K ** -0.5).to(torch.bfloat16).cuda()
+    off = torch.tensor([0] + list(torch.tensor(sizes).cumsum(0)), dtype=torch.int32, device="cuda")
+    ref, mag = torch.empty(rows, N, dtype=torch.float64, device="cuda"), torch.empty(rows, N, dtype=torch.float64, device="cuda")
+    for i in range(G):
+        a, b = int(off[i]), int(off[i + 1])
+        ref[a:b] = x[a:b].double() @ w[i].double().T
+        mag[a:b] = x[a:b].double().abs() @ w[i].double().abs().T
+    for epilogue, dtype in ((0, torch.float32), (1, torch.bfloat16)):
+        out = torch.full((rows + 8, N), 7.0, dtype=dtype, device="cuda")
+        chk(lib, lib.b2k_linear_sum(ptr(x), ptr(w), ptr(off), G, rows, ptr(out), N, K, epilogue, tile, cuda_stream_ptr()))
+        torch.cuda.synchronize()
+        assert (out[rows:] == 7.0).all()
+        got = out[:rows].double()
+        err = K * 2.0 ** -24 * mag
+        if epilogue == 0:
+            assert ((got - ref).abs() <= err).all()
+        else:
+            want = ref.clamp_min(0.0) ** 2
+            assert ((got - want).abs() <= 2.0 ** -8 * want + 2.1 * err * (ref.abs() + err)).all()
+    one = torch.full((rows, N), 7.0, device="cuda")   # one block
+    chk(lib, lib.b2k_linear_sum(ptr(x), ptr(w[0]), None, 1, rows, ptr(one), N, K, 0, tile, cuda_stream_ptr()))
+    torch.cuda.synchronize()
+    assert ((one.double() - x.double() @ w[0].double().T).abs() <= K * 2.0 ** -24 * (x.double().abs() @ w[0].double().abs().T)).all()
