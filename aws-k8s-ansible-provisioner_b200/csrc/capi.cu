@@ -93,6 +93,22 @@ extern "C" int b2k_linear_sum(const void* x, const void* w, const int32_t* offse
   return launch_linear_sum(x, w, offsets, groups, rows, out, N, K, epilogue, wait, (cudaStream_t)stream, tile);
 }
 
+extern "C" int b2k_few_linear(const void* w, const void* x, const void* gain, float eps, void* out, int T, int N, int K, int mode, void* stream) {
+  B2_REQUIRE(w && x && out && (mode == 1 || gain) && mode >= 0 && mode <= 2, "b2k_few_linear: bad arguments");
+  B2_REQUIRE(few_shapes_ok(T, K, K, K), "b2k_few_linear: T=%d N=%d K=%d not built", T, N, K);
+  if (mode == 0) return launch_few_qkv((const bf16*)w, (const bf16*)x, (const bf16*)gain, eps, (bf16*)out, T, N, K, (cudaStream_t)stream);
+  if (mode == 1) return launch_few_resid((const bf16*)w, (const bf16*)x, (bf16*)out, T, N, K, (cudaStream_t)stream);
+  return launch_few_gateup((const bf16*)w, (const bf16*)x, (const bf16*)gain, eps, (bf16*)out, T, N, K, (cudaStream_t)stream);
+}
+
+extern "C" int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* knorm_w, const void* cos_sin, const int32_t* positions, const int32_t* slots, void* k_pages,
+                            void* v_pages, const int32_t* block_table, int bt_stride, const int32_t* seq_lens, void* out, int B, int nq, int nkv, float eps, float scale,
+                            void* stream) {
+  B2_REQUIRE(qkv && qnorm_w && knorm_w && cos_sin && positions && slots && k_pages && v_pages && block_table && seq_lens && out, "b2k_few_attn: null pointer");
+  return launch_few_attn((const bf16*)qkv, (const bf16*)qnorm_w, (const bf16*)knorm_w, (const bf16*)cos_sin, positions, slots, (bf16*)k_pages, (bf16*)v_pages, block_table,
+                         bt_stride, seq_lens, (bf16*)out, B, nq, nkv, eps, scale, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
                               const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
                               const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,

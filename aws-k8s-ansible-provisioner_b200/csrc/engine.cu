@@ -314,6 +314,8 @@ struct b2_engine {
   int prefill_pairs = 1;  // B2_PREFILL_PAIRS: see prefill_tile_pairs()
   int prefill_mc = 1;  // B2_MC: prefill projections on pairs of CTAs (gemm_mc.cu)
   int gu_prefill_fused = 1;  // B2_GU_FUSED: prefill-sized gate/up projection with SwiGLU in its epilogue (gemm_gateup.cu)
+  bool step_long = false;   // the step's contexts are too long for those kernels (pick_attn_split)
+  int use_few = 1;    // B2_FEW: 0 = at most eight sequences take the kernels of larger batches (cross-check)
   int use_pair = 1;   // B2_PAIR: bit 0 gate/up + SwiGLU, bit 1 QKV + QK-norm/RoPE/KV write as fused cluster-pair launches (gemm_pair.cu)
 
   // two-lane decode (B2_MB, see forward()): second stream, its own partials and attention scratch, fork/join events
@@ -456,10 +458,12 @@ int bucket_batch(int B) {
 }
 
 int pick_attn_split(b2_engine* e, int B, int max_len) {
-  // The decode-attention kernel balances pages over its persistent warps by itself; there is no
-  // host-side split factor any more.  The slot of the graph key now tells the two step variants apart.
-  (void)B; (void)max_len;
-  return (e->debug_flags & 2) ? 2 : 1;
+  // The slot of the graph key tells the step variants apart: 1 arg-max only, 2 logits written too; + 2 where the contexts are too long for the kernels of few
+  // sequences (gemm_few.cu: a cluster per sequence and kv head, however long the sequence, against attn_decode.cu's even share of all pages per warp).
+  // 16 steps of 28 layers, ms, few / larger batches' kernels: 1 x 1500 tokens 10.4 / 22.6, 1 x 12000 25.6 / 31.9, 4 x 1500 12.7 / 22.4, 4 x 4000 17.7 / 24.3,
+  // 8 x 1500 17.9 / 20.7, 8 x 4000 28.1 / 27.1, 4 x 12000 34.4 / 32.9.
+  const bool long_contexts = B <= 8 && (long)B * max_len > 24576;
+  return ((e->debug_flags & 2) ? 2 : 1) + (long_contexts ? 2 : 0);
 }
 
 // ---- one Linear layer: picks SIMT GEMV or the tcgen05 kernel, bf16 or split-K partial output
@@ -832,6 +836,31 @@ int forward_layers(b2_engine* e, const Lane& ln, int T, int ntiles) {
     const bool resid = qkv_pair && gu_pair && (e->use_pair & 4) && e->ssq != nullptr && H / 16 <= 64 && resid_shapes_ok(T, H, e->q_size) &&
                        resid_shapes_ok(T, H, I) && !((e->skip_mask >> B2K_NORM) & 1u) && !((e->skip_mask >> B2K_GEMM_O) & 1u) &&
                        !((e->skip_mask >> B2K_GEMM_DOWN) & 1u) && !((e->skip_mask >> B2K_GEMM_QKV) & 1u) && !((e->skip_mask >> B2K_GEMM_GATEUP) & 1u);
+    // ... and at most eight sequences take the kernels of gemm_few.cu: five launches a layer too, for a chain that is bound by latencies
+    if (resid && few_shapes_ok(T, H, e->q_size, I) && e->nq == 2 * e->nkv && e->hd == 128 && c.block_size == 16 && c.sliding_window <= 0 && e->use_few && !e->step_long && e->skip_mask == 0 &&
+        !e->l2_weight_prefetch) {
+      {
+        KL k(e, B2K_GEMM_QKV);
+        B2_TRY(launch_few_qkv(L.wqkv, h, L.ln1, c.rms_eps, qkvb, T, e->qkv_size, H, st));
+      }
+      {
+        KL k(e, B2K_ATTN_DECODE);
+        B2_TRY(launch_few_attn(qkvb, L.qnorm, L.knorm, e->cos_sin, positions, slots, kp, vp, block_table, e->bt_stride, seq_lens, attn, T, e->nq, e->nkv, c.rms_eps,
+                               e->attn_scale, st));
+      }
+      {
+        KL k(e, B2K_GEMM_O);
+        B2_TRY(launch_few_resid(L.wo, attn, h, T, H, e->q_size, st));
+      }
+      {
+        KL k(e, B2K_GEMM_GATEUP);
+        B2_TRY(launch_few_gateup(L.wgu, h, L.ln2, c.rms_eps, act, T, I, H, st));
+      }
+      KL k(e, B2K_GEMM_DOWN);
+      B2_TRY(launch_few_resid(L.wd, act, h, T, H, I, st));
+      delta = act_bf16(nullptr);   // h is up to date
+      continue;
+    }
     PairNorm pn1, pn2;
     if (resid) {
       pn1.ssq = pn2.ssq = e->ssq;
@@ -2338,7 +2367,7 @@ bool two_lane_decode(const b2_engine* e, int T, int ntiles) {
 int forward(b2_engine* e, int T, int ntiles, int nlast, int attn_split) {
   const b2_config& c = e->cfg;
   const int H = c.hidden;
-  (void)attn_split;
+  e->step_long = attn_split > 2;
   if (c.arch == B2_ARCH_LERASUN) return forward_list(e, T, ntiles, nlast);
   if (c.arch == B2_ARCH_KEDASUN) return forward_heads_list(e, T, ntiles, nlast);
   if (c.arch == B2_ARCH_BUMALIX) return forward_state_list(e, T, ntiles, nlast);
@@ -2508,7 +2537,7 @@ int ensure_graph(b2_engine* e, int B, int attn_split) {
 }
 
 // hidden-state capture needs eager launches; the logits buffer is just another kernel argument, so it
-// only selects a different graph (attn_split slot of the key: 1 = argmax only, 2 = logits written too)
+// only selects a different graph (attn_split slot of the key, see pick_attn_split)
 bool graphs_enabled(b2_engine* e) { return e->cfg.use_cuda_graphs && !e->profiling && !(e->debug_flags & 1); }
 
 int run_decode_step(b2_engine* e, int B, int attn_split) {
@@ -4872,6 +4901,7 @@ extern "C" int b2_engine_create(const b2_config* cfg, const char* safetensors_pa
   // 0 separate kernels (default: fastest measured), 1 eight-step chain kernel (chain.cu), 2 fused four-step cluster
   // chain (chain_cluster.cu); 1 and 2 are kept as measured experiments with parity tests
   e->use_chain = env_int("B2_CHAIN", 0);
+  e->use_few = env_int("B2_FEW", 1);
   e->use_pair = env_int("B2_PAIR", 7);  // bit 2: O / down projections update the residual stream themselves (gemm_resid.cu)
   e->prefill_tc = env_int("B2_PREFILL_TC", 1);
   e->gu_prefill_fused = env_int("B2_GU_FUSED", 1);

@@ -100,6 +100,13 @@ int launch_linear_mc(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* 
 int launch_qkv_rope_prefill(const CUtensorMap& tm_qkv, const CUtensorMap& tm_x128, const bf16* qw, const bf16* kw, const bf16* cos_sin,
                             const int32_t* positions, const int32_t* slots, bf16* q_out, bf16* k_pages, bf16* v_pages, int T, int nq, int nkv,
                             int K, int block_size, float eps, int x_row0, const B2WaitLimit& wait, cudaStream_t s);
+// gemm_few.cu: the decode step of a Qwen3-geometry layer for at most eight sequences (bf16; qkv rows of (nq + 2 nkv) * 128, before norm and RoPE)
+bool few_shapes_ok(int T, int H, int q_size, int I);
+int launch_few_qkv(const bf16* w, const bf16* h, const bf16* gain, float eps, bf16* qkv, int T, int N, int K, cudaStream_t s);
+int launch_few_gateup(const bf16* wgu, const bf16* h, const bf16* gain, float eps, bf16* act, int T, int I, int K, cudaStream_t s);
+int launch_few_resid(const bf16* w, const bf16* x, bf16* h, int T, int N, int K, cudaStream_t s);
+int launch_few_attn(const bf16* qkv, const bf16* qw, const bf16* kw, const bf16* cos_sin, const int32_t* positions, const int32_t* slots, bf16* k_pages, bf16* v_pages,
+                    const int32_t* block_table, int bt_stride, const int32_t* seq_lens, bf16* out, int B, int nq, int nkv, float eps, float scale, cudaStream_t s);
 // gemm_sum.cu: prompt-sized products with fp32 sums out (or a squared-ReLU expert's bf16 activation), rows of one block or of the ragged blocks of
 // `groups` experts (offsets: [groups + 1] first rows, device memory; null: one block); w [groups * N][K]; bn: 0 = by the sizes
 enum { SUM_EPI_F32 = 0, SUM_EPI_RELU2 = 1 };

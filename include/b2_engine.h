@@ -426,6 +426,13 @@ int b2k_linear_multicast(const void* x_bf16, const void* w_bf16, void* out_bf16,
  * rows the kernel reads from device memory (offsets [groups + 1], the last one = rows): out[row][N] = x[row][K] . w_g[N][K]^T as fp32 (epilogue 0) or
  * bf16(max(sum, 0)^2) (1).  K % 64 == 0; tile: 0 (by the sizes), 128 or 256 rows of x. */
 int b2k_linear_sum(const void* x_bf16, const void* w_bf16, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, int tile, void* stream);
+/* A decode step's products for at most eight sequences (csrc/gemm_few.cu), K % 32 == 0, all bf16: mode 0: out[T][N] = RMSNorm(x) . w^T; 1: out += x . w^T (gain unused);
+ * 2: out[T][N] = silu(g) * u with g | u = RMSNorm(x) . w^T, w [2N][K] (gate rows, then up rows). */
+int b2k_few_linear(const void* w, const void* x, const void* gain, float eps, void* out, int T, int N, int K, int mode, void* stream);
+/* ... and its attention, nq == 2 * nkv, 128-wide heads, pages of sixteen tokens: qkv [B][(nq + 2 nkv) * 128] as the projection leaves it; QK-norm, RoPE and the page write
+ * of the new token (position seq_lens - 1, slot as in b2k_qknorm_rope_kv), then softmax(q k^T * scale) v over the pages. */
+int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* knorm_w, const void* cos_sin, const int32_t* positions, const int32_t* slots, void* k_pages, void* v_pages,
+                 const int32_t* block_table, int bt_stride, const int32_t* seq_lens, void* out, int B, int nq, int nkv, float eps, float scale, void* stream);
 /* The recurrence of the matrix-state mixers over `portions` portions (portion i ends at row last_rows[i]; last_rows null: every row is one of one token); rule as
  * StateRule in csrc/kernels.h; all tensors fp32: q / k rows of kv_heads * dim, v rows of heads * vdim, decay [T][heads * dim] or [T][heads] by the rule, beta
  * [T][heads], skip [heads], bonus [heads][dim] (null where the rule has none), state [slots][2][heads][dim][vdim], out [T][heads * vdim]. */

@@ -1,0 +1,97 @@
+"""The decode kernels of at most eight sequences (GPU), called through the C ABI: against the kernels that larger batches take (page writes bit for bit) and against
+the same arithmetic in 64 bits between the bf16 roundings."""
+import pytest
+import torch
+
+from _util import assert_bf16_close, cuda_stream_ptr, kv_swizzle, pkg, ptr
+
+pytestmark = pytest.mark.gpu
+HD, BS, EPS = 128, 16, 1e-6
+
+
+@pytest.fixture(scope="module")
+def lib():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    return pkg().load_library()
+
+
+def chk(lib, rc):
+    assert rc == 0, lib.b2_last_error().decode()
+
+
+def norm(x, gain):
+    """bf16(gain * bf16(x * rstd)); the statistic in 64 bits"""
+    rstd = (x.double().pow(2).mean(-1, keepdim=True) + EPS).rsqrt()
+    return (gain.double() * (x.double() * rstd).to(torch.bfloat16).double()).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("T", [1, 3, 8])
+@pytest.mark.parametrize("N,K", [(8, 32), (40, 96), (72, 256), (264, 1024), (1024, 2048), (100, 3072), (48, 3360)])
+def test_few_linear(lib, T, N, K):
+    """Weight rows that fill no CTA, a K that is not the warps' multiple of 256 or takes several rounds; nothing behind row T.  The sums differ from 64 bits by fp32
+    roundings, which move a bf16 result by one unit now and then (two where two roundings follow each other)."""
+    g = torch.Generator().manual_seed(N * 10 + T)
+    x = torch.randn(T, K, generator=g).to(torch.bfloat16)
+    gain = (1 + 0.2 * torch.randn(K, generator=g)).to(torch.bfloat16)
+    for mode in (0, 1, 2):
+        rows = 2 * N if mode == 2 else N
+        w = (torch.randn(rows, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+        h = torch.randn(8, N, generator=g).to(torch.bfloat16)
+        out = h.clone().cuda()
+        dw, dx, dg = w.cuda(), x.cuda(), gain.cuda()
+        chk(lib, lib.b2k_few_linear(ptr(dw), ptr(dx), ptr(dg), EPS, ptr(out), T, N, K, mode, cuda_stream_ptr()))
+        torch.cuda.synchronize()
+        y = ((x if mode == 1 else norm(x, gain)).double() @ w.double().T).to(torch.bfloat16)
+        if mode == 1:
+            ref = (h[:T].double() + y.double()).to(torch.bfloat16)
+        elif mode == 2:
+            gate, up = y[:, :N].double(), y[:, N:].double()
+            ref = ((gate / (1 + torch.exp(-gate))).to(torch.bfloat16).double() * up).to(torch.bfloat16)
+        else:
+            ref = y
+        assert_bf16_close(out[:T], ref, 3, 0.06, "mode %d" % mode, abs_floor=2.0 ** -8)
+        assert torch.equal(out[T:].cpu(), h[T:])
+
+
+@pytest.mark.parametrize("lens", [[1], [15, 16, 17, 2], [511, 512, 513, 0, 528], [1030, 33, 1024, 700, 1, 544, 496, 2000]])
+def test_few_attn(lib, lens):
+    """Contexts around a page, around the 32 pages of a cluster's first turn, several turns; a padding row.  Pages and rotated queries: those of b2k_qknorm_rope_kv."""
+    nq, nkv, B = 8, 4, len(lens)
+    g = torch.Generator().manual_seed(sum(lens))
+    width = max(1, max((n + BS - 1) // BS for n in lens))
+    blocks = B * width + 3
+    bt = torch.randperm(blocks, generator=g)[:B * width].view(B, width).to(torch.int32)
+    kp, vp = (torch.randn(blocks, nkv, BS, HD, generator=g).to(torch.bfloat16) for _ in range(2))
+    qkv = torch.randn(B, (nq + 2 * nkv) * HD, generator=g).to(torch.bfloat16)
+    qw, kw = ((1 + 0.25 * torch.randn(HD, generator=g)).to(torch.bfloat16) for _ in range(2))
+    ang = torch.arange(2048)[:, None] * (1e4 ** (-torch.arange(64) / 64.0))[None, :]
+    table = torch.cat([ang.cos(), ang.sin()], -1).to(torch.bfloat16)
+    pos = torch.tensor([n - 1 for n in lens], dtype=torch.int32)
+    slots = torch.tensor([-1 if n == 0 else int(bt[b, (n - 1) // BS]) * BS + (n - 1) % BS for b, n in enumerate(lens)], dtype=torch.int32)
+    d = [t.cuda() for t in (qkv, qw, kw, table, pos, slots, bt, torch.tensor(lens, dtype=torch.int32))]
+    pages = [[t.cuda() for t in (kp, vp)] for _ in range(2)]
+    q_out = torch.zeros(B, nq * HD, dtype=torch.bfloat16, device="cuda")
+    chk(lib, lib.b2k_qknorm_rope_kv(ptr(d[0]), 0, 1, ptr(d[1]), ptr(d[2]), ptr(d[3]), ptr(d[4].clamp_min(0)), ptr(d[5]), ptr(q_out), ptr(pages[0][0]), ptr(pages[0][1]), B, nq, nkv,
+                                    HD, BS, EPS, cuda_stream_ptr()))
+    out = torch.full((B, nq * HD), float("nan"), dtype=torch.bfloat16, device="cuda")
+    scale = HD ** -0.5
+    run = lambda dst: chk(lib, lib.b2k_few_attn(ptr(d[0]), ptr(d[1]), ptr(d[2]), ptr(d[3]), ptr(d[4]), ptr(d[5]), ptr(pages[1][0]), ptr(pages[1][1]), ptr(d[6]), width, ptr(d[7]), ptr(dst),
+                                                B, nq, nkv, EPS, scale, cuda_stream_ptr()))
+    run(out)
+    torch.cuda.synchronize()
+    for a, b in zip(pages[0], pages[1]):
+        assert torch.equal(a, b)
+    k, v = (kv_swizzle(t.cpu()).double() for t in pages[1])
+    for b, n in enumerate(lens):
+        if n == 0:
+            assert not out[b].any()
+            continue
+        idx = bt[b, :(n + BS - 1) // BS].long()
+        ks, vs = (t[idx].permute(1, 0, 2, 3).reshape(nkv, -1, HD)[:, :n] for t in (k, v))
+        q = q_out[b].cpu().double().view(nkv, 2, HD)
+        ref = torch.softmax(torch.einsum("gqd,gkd->gqk", q, ks) * scale, -1) @ vs
+        assert_bf16_close(out[b], ref.reshape(-1).to(torch.bfloat16), 2, 0.05, "sequence of %d" % n, abs_floor=2.0 ** -12)
+    again = torch.empty_like(out)
+    run(again)
+    assert torch.equal(out, again)
