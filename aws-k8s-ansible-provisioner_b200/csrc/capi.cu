@@ -109,6 +109,13 @@ extern "C" int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* kn
                          bt_stride, seq_lens, (bf16*)out, B, nq, nkv, eps, scale, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_linear_split3(const float* x, void* planes, const void* w, float* out, int rows, int N, int K, int tile, void* stream) {
+  B2_REQUIRE(x && planes && w && out, "b2k_linear_split3: null pointer");
+  B2WaitLimit wait;
+  CAPI_TRY(hook_waits(&wait));
+  return launch_linear_split3(x, (bf16*)planes, (const bf16*)w, out, rows, N, K, wait, (cudaStream_t)stream, tile);
+}
+
 extern "C" int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
                               const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
                               const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,

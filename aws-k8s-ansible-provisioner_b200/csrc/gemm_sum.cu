@@ -8,6 +8,9 @@
 //     the next group (or to nobody: zero-filled) and are not stored.
 //   * epilogue: fp32 sums straight from registers (a warp's 32 weight rows are 128 contiguous bytes of an output row), or, for squared-ReLU experts, their
 //     activation rounded to the bf16 operand of the second product.
+//   * SPLIT: x is fp32, given as three bf16 planes whose sum it is (split3_kernel: 8 + 8 + 8 bits of the 24), and the weights are bf16 numbers, so the three
+//     products are exact.  The tensor pipe's accumulator rounds every addition towards zero, so it holds only 128 of the K at a time, smallest plane first: the
+//     epilogue's warps keep the running sums of a tile in registers and add a chunk, rounded to nearest, while the next one is multiplied.
 // Bound: tensor pipe under the power cap, and the last wave.
 #include "kernels.h"
 
@@ -25,6 +28,7 @@ struct GsCfg {
   static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024;
   static constexpr int TMEM_COLS = 2 * BN;
 };
+constexpr int GS_CHUNK_KB = 2;   // SPLIT: k-blocks per chunk
 constexpr int GS_EPI_WARPS = 8, GS_THREADS = 64 + 32 * GS_EPI_WARPS;
 
 __device__ __forceinline__ uint32_t gs_cluster_rank() {
@@ -88,7 +92,7 @@ struct GsWalk {
 };
 
 // offsets: [groups + 1] first rows of the groups in device memory, or null: one group of `rows_total` rows
-template <int BN, int EPI>
+template <int BN, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(GS_THREADS, 1)
 linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const int32_t* __restrict__ offsets, int groups,
                   int rows_total, void* __restrict__ out, int N, int K, const B2WaitLimit limit) {
@@ -106,7 +110,8 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = gs_cluster_rank();
   const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
-  const int kb_total = K / GS_BK, m_pairs = (N + 2 * GS_BM - 1) / (2 * GS_BM);
+  constexpr int PLANES = SPLIT ? 3 : 1;
+  const int kb_total = K / GS_BK, chunk_kb = SPLIT ? GS_CHUNK_KB : kb_total, m_pairs = (N + 2 * GS_BM - 1) / (2 * GS_BM);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -147,16 +152,18 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int p = cluster; w.at(p); p += clusters) {
       const int wrow = w.g * N + (2 * w.pair + (int)rank) * GS_BM;   // (rows past the group's N: the next group's or zeros, not stored)
       const int xrow = w.row0 + (int)rank * (BN / 2);
-      for (int kb = 0; kb < kb_total; ++kb) {
-        const int s = sent % C::STAGES;
-        if (!wait(empty_bar[s], ((sent / C::STAGES) & 1) ^ 1)) return;  // the pair's MMAs are done with this stage
-        const uint32_t fb = gs_first_cta(smem_u32(&full_bar[s]));
-        if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * C::STAGE_BYTES);
-        const uint32_t ws = smem_base + s * C::STAGE_BYTES;
-        gs_tma_load_2d(ws, &tmap_w, kb * GS_BK, wrow, fb);
-        gs_tma_load_2d(ws + GS_W_BYTES, &tmap_x, kb * GS_BK, xrow, fb);
-        ++sent;
-      }
+      for (int c0 = 0; c0 < kb_total; c0 += chunk_kb)
+        for (int plane = PLANES - 1; plane >= 0; --plane)
+          for (int kb = c0; kb < min(kb_total, c0 + chunk_kb); ++kb) {
+            const int s = sent % C::STAGES;
+            if (!wait(empty_bar[s], ((sent / C::STAGES) & 1) ^ 1)) return;  // the pair's MMAs are done with this stage
+            const uint32_t fb = gs_first_cta(smem_u32(&full_bar[s]));
+            if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * C::STAGE_BYTES);
+            const uint32_t ws = smem_base + s * C::STAGE_BYTES;
+            gs_tma_load_2d(ws, &tmap_w, kb * GS_BK, wrow, fb);
+            gs_tma_load_2d(ws + GS_W_BYTES, &tmap_x, kb * GS_BK, plane * rows_total + xrow, fb);   // (rows behind a plane's end: the next plane's, not stored)
+            ++sent;
+          }
     }
     // the releases of the last stages have landed on this CTA's barriers before it goes to the final cluster barrier and exits
     for (int j = max(0, sent - C::STAGES); j < sent; ++j)
@@ -166,68 +173,98 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     constexpr uint32_t idesc = umma_idesc_bf16(2 * GS_BM, BN);
     int it = 0, lt = 0;
     GsWalk<BN> w(s_off, groups, m_pairs);
-    for (int p = cluster; w.at(p); p += clusters, ++lt) {
-      const int as = lt & 1;
-      if (!wait(tmem_empty_bar[as], ((lt >> 1) & 1) ^ 1)) return;
-      tc_fence_after();
-      const uint32_t tmem_d = tmem_base + (uint32_t)(as * BN);
-      for (int kb = 0; kb < kb_total; ++kb, ++it) {
-        const int s = it % C::STAGES;
-        if (!wait(full_bar[s], (it / C::STAGES) & 1)) return;
+    for (int p = cluster; w.at(p); p += clusters)
+      for (int c0 = 0; c0 < kb_total; c0 += chunk_kb, ++lt) {
+        const int as = lt & 1, steps = PLANES * min(chunk_kb, kb_total - c0);
+        if (!wait(tmem_empty_bar[as], ((lt >> 1) & 1) ^ 1)) return;
         tc_fence_after();
-        const uint32_t ws = smem_base + s * C::STAGE_BYTES;
-        const uint64_t da = umma_desc_sw128(ws), db = umma_desc_sw128(ws + GS_W_BYTES);
+        const uint32_t tmem_d = tmem_base + (uint32_t)(as * BN);
+        for (int i = 0; i < steps; ++i, ++it) {
+          const int s = it % C::STAGES;
+          if (!wait(full_bar[s], (it / C::STAGES) & 1)) return;
+          tc_fence_after();
+          const uint32_t ws = smem_base + s * C::STAGE_BYTES;
+          const uint64_t da = umma_desc_sw128(ws), db = umma_desc_sw128(ws + GS_W_BYTES);
 #pragma unroll
-        for (int k = 0; k < GS_BK / 16; ++k)
-          gs_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-        gs_commit(smem_u32(&empty_bar[s]));
+          for (int k = 0; k < GS_BK / 16; ++k)
+            gs_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
+          gs_commit(smem_u32(&empty_bar[s]));
+        }
+        gs_commit(smem_u32(&tmem_full_bar[as]));
       }
-      gs_commit(smem_u32(&tmem_full_bar[as]));
-    }
   };
   auto finish = [&]() {
     // thread = weight row (TMEM lane), two warps per lane quarter that take every other 32 rows of x
     const int q = warp & 3, half = (warp - 2) >> 2;
     int lt = 0;
     GsWalk<BN> w(s_off, groups, m_pairs);
-    for (int p = cluster; w.at(p); p += clusters, ++lt) {
-      const int as = lt & 1;
-      if (!wait.warp(tmem_full_bar[as], (lt >> 1) & 1)) return;
-      tc_fence_after();
-      const int col = (2 * w.pair + (int)rank) * GS_BM + q * 32 + lane;
-      const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(as * BN);
-#pragma unroll 1
-      for (int c0 = half * 32; c0 < BN; c0 += 64) {
-        uint32_t r[32];
-        tmem_ld32(tbase + (uint32_t)c0, r);
-        tmem_ld_wait();
-        if (c0 + 64 >= BN) {   // this warp's share of the accumulator is in registers: back to the MMA thread, which waits for both CTAs' warps
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0)
-            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(gs_first_cta(smem_u32(&tmem_empty_bar[as]))) : "memory");
-        }
-        if (col >= N) continue;
-        const size_t at = (size_t)(w.row0 + c0) * N + col;
-        const int have = w.rows - c0;   // rows of this block that are the group's
-        if constexpr (EPI == SUM_EPI_F32) {
-          float* d = reinterpret_cast<float*>(out) + at;
-          if (have >= 32) {
+    auto hand_back = [&](int as) {   // this warp's share of the accumulator is in registers: back to the MMA thread, which waits for both CTAs' warps
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(gs_first_cta(smem_u32(&tmem_empty_bar[as]))) : "memory");
+    };
+    auto store = [&](int c0, int col, const uint32_t (&r)[32]) {   // 32 rows of x from c0 of the tile on, this thread's weight row
+      if (col >= N) return;
+      const size_t at = (size_t)(w.row0 + c0) * N + col;
+      const int have = w.rows - c0;   // rows of this block that are the group's
+      if constexpr (EPI == SUM_EPI_F32) {
+        float* d = reinterpret_cast<float*>(out) + at;
+        if (have >= 32) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) d[(size_t)j * N] = __uint_as_float(r[j]);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (j < have) d[(size_t)j * N] = __uint_as_float(r[j]);
-          }
+          for (int j = 0; j < 32; ++j) d[(size_t)j * N] = __uint_as_float(r[j]);
         } else {
-          bf16* d = reinterpret_cast<bf16*>(out) + at;
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float a = fmaxf(__uint_as_float(r[j]), 0.f);
-            if (j < have) d[(size_t)j * N] = __float2bfloat16_rn(a * a);
+          for (int j = 0; j < 32; ++j)
+            if (j < have) d[(size_t)j * N] = __uint_as_float(r[j]);
+        }
+      } else {
+        bf16* d = reinterpret_cast<bf16*>(out) + at;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const float a = fmaxf(__uint_as_float(r[j]), 0.f);
+          if (j < have) d[(size_t)j * N] = __float2bfloat16_rn(a * a);
+        }
+      }
+    };
+    for (int p = cluster; w.at(p); p += clusters) {
+      const int col = (2 * w.pair + (int)rank) * GS_BM + q * 32 + lane;
+      const uint32_t tq = tmem_base + ((uint32_t)(q * 32) << 16);
+      if constexpr (SPLIT) {
+        uint32_t sum[BN / 64][32];
+#pragma unroll
+        for (int b = 0; b < BN / 64; ++b)
+#pragma unroll
+          for (int j = 0; j < 32; ++j) sum[b][j] = 0u;
+        for (int c0 = 0; c0 < kb_total; c0 += chunk_kb, ++lt) {
+          const int as = lt & 1;
+          if (!wait.warp(tmem_full_bar[as], (lt >> 1) & 1)) return;
+          tc_fence_after();
+#pragma unroll
+          for (int b = 0; b < BN / 64; ++b) {
+            uint32_t r[32];
+            tmem_ld32(tq + (uint32_t)(as * BN + half * 32 + b * 64), r);
+            tmem_ld_wait();
+            if (b == BN / 64 - 1) hand_back(as);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) sum[b][j] = __float_as_uint(__uint_as_float(sum[b][j]) + __uint_as_float(r[j]));
           }
         }
+#pragma unroll
+        for (int b = 0; b < BN / 64; ++b) store(half * 32 + b * 64, col, sum[b]);
+      } else {
+        const int as = lt & 1;
+        if (!wait.warp(tmem_full_bar[as], (lt >> 1) & 1)) return;
+        tc_fence_after();
+#pragma unroll 1
+        for (int c0 = half * 32; c0 < BN; c0 += 64) {
+          uint32_t r[32];
+          tmem_ld32(tq + (uint32_t)(as * BN + c0), r);
+          tmem_ld_wait();
+          if (c0 + 64 >= BN) hand_back(as);
+          store(c0, col, r);
+        }
+        ++lt;
       }
     }
   };
@@ -258,14 +295,50 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
 }
 
-template <int BN, int EPI>
+// planes [3][n] bf16 whose sum is x: every plane the nearest bf16 to what is left (a value that rounds to infinity is cut instead; infinities and NaN stay in the first)
+__global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ x, uint2* __restrict__ planes, size_t n4) {
+  pdl_wait();
+  pdl_launch_dependents();
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
+    const float4 v = x[i];
+    const float in[4] = {v.x, v.y, v.z, v.w};
+    uint32_t h[3][4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float left = in[c];
+      const bool finite = fabsf(left) < INFINITY;
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        uint32_t b = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(left));
+        if (finite && (b & 0x7fffu) == 0x7f80u) b = __float_as_uint(left) >> 16;
+        h[p][c] = b;
+        left = finite ? left - __uint_as_float(b << 16) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < 3; ++p) planes[(size_t)p * n4 + i] = make_uint2(h[p][0] | h[p][1] << 16, h[p][2] | h[p][3] << 16);
+  }
+}
+
+// bf16 copies of fp32 numbers; *inexact becomes 1 when one of them is not a bf16 number
+__global__ void __launch_bounds__(256) bf16_copy_kernel(const uint32_t* __restrict__ w, uint16_t* __restrict__ out, size_t n, uint32_t* inexact) {
+  bool bad = false;
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+    const uint32_t b = w[i];
+    bad = bad || (b & 0xffffu) != 0;
+    out[i] = (uint16_t)(b >> 16);
+  }
+  if (bad) *inexact = 1;
+}
+
+template <int BN, int EPI, bool SPLIT = false>
 int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, const B2WaitLimit& wait, cudaStream_t s) {
   using C = GsCfg<BN>;
   static B2PerDeviceOnce attr_once;
-  if (attr_once.need()) B2_CUDA_OK(cudaFuncSetAttribute(linear_sum_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+  if (attr_once.need()) B2_CUDA_OK(cudaFuncSetAttribute(linear_sum_kernel<BN, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
   CUtensorMap tw, tx;
   int rc = b2_make_tmap_bf16(&tw, w, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K, GS_BM);
-  if (rc == 0) rc = b2_make_tmap_bf16(&tx, x, (uint64_t)rows, (uint64_t)K, (uint64_t)K, BN / 2);
+  if (rc == 0) rc = b2_make_tmap_bf16(&tx, x, (uint64_t)rows * (SPLIT ? 3 : 1), (uint64_t)K, (uint64_t)K, BN / 2);
   if (rc != 0) return rc;
   const int m_pairs = (N + 2 * GS_BM - 1) / (2 * GS_BM);
   const long most = ((long)rows / BN + groups) * m_pairs;   // tiles at most
@@ -284,7 +357,7 @@ int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = b2_pdl_enabled() ? 2 : 1;
-  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_sum_kernel<BN, EPI>, tw, tx, offsets, groups, rows, out, N, K, wait));
+  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_sum_kernel<BN, EPI, SPLIT>, tw, tx, offsets, groups, rows, out, N, K, wait));
   return 0;
 }
 
@@ -321,6 +394,23 @@ int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int 
 #undef B2_SUM_CASE
   b2_set_error("linear_sum: tile %d, epilogue %d not built", bn, epilogue);
   return -22;
+}
+
+int launch_linear_split3(const float* x, bf16* planes, const bf16* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int bn) {
+  if (rows <= 0) return 0;
+  B2_REQUIRE(linear_sum_shapes_ok(rows, 1, N, K) && (reinterpret_cast<uintptr_t>(x) & 15) == 0, "linear_split3: %d rows, N=%d K=%d not built", rows, N, K);
+  const size_t n4 = (size_t)rows * K / 4;
+  B2_CUDA_OK(b2_launch(split3_kernel, dim3((unsigned)std::min<size_t>((n4 + 255) / 256, (size_t)device_num_sms() * 16)), dim3(256), 0, s, (const float4*)x, (uint2*)planes, n4));
+  if (bn == 0) bn = sum_pick_bn(rows, 1, N);
+  return bn == 128 ? launch_sum<128, SUM_EPI_F32, true>(planes, w, nullptr, 1, rows, out, N, K, wait, s)
+                   : launch_sum<256, SUM_EPI_F32, true>(planes, w, nullptr, 1, rows, out, N, K, wait, s);
+}
+
+int launch_bf16_copy(const float* w, bf16* out, size_t n, uint32_t* inexact, cudaStream_t s) {
+  if (n == 0) return 0;
+  bf16_copy_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)device_num_sms() * 16), 256, 0, s>>>((const uint32_t*)w, (uint16_t*)out, n, inexact);
+  B2_CUDA_OK(cudaGetLastError());
+  return 0;
 }
 
 }  // namespace b2

@@ -114,6 +114,10 @@ bool linear_sum_shapes_ok(int rows, int groups, int N, int K);
 bool linear_sum_pays(int rows, int N);   // one block of rows: faster than launch_linear_tc
 int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, const B2WaitLimit& wait,
                       cudaStream_t s, int bn = 0);
+// the same for fp32 x [rows][K] and bf16 weights, fp32 precision: x goes to three bf16 planes ([3][rows][K], scratch) whose sum it is
+int launch_linear_split3(const float* x, bf16* planes, const bf16* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int bn = 0);
+// bf16 copy of n fp32 numbers; *inexact (device) becomes 1 when one of them is not a bf16 number
+int launch_bf16_copy(const float* w, bf16* out, size_t n, uint32_t* inexact, cudaStream_t s);
 // gemm_gateup.cu: the prefill-sized counterpart (two accumulators per tile, SwiGLU in the epilogue)
 bool gateup_prefill_shapes_ok(int T, int I, int K);
 int launch_gateup_swiglu_prefill(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* act, int T, int I, int K, int x_row0, cudaStream_t s);

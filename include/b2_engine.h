@@ -433,6 +433,8 @@ int b2k_few_linear(const void* w, const void* x, const void* gain, float eps, vo
  * of the new token (position seq_lens - 1, slot as in b2k_qknorm_rope_kv), then softmax(q k^T * scale) v over the pages. */
 int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* knorm_w, const void* cos_sin, const int32_t* positions, const int32_t* slots, void* k_pages, void* v_pages,
                  const int32_t* block_table, int bt_stride, const int32_t* seq_lens, void* out, int B, int nq, int nkv, float eps, float scale, void* stream);
+/* out[rows][N] = x[rows][K] . w[N][K]^T at fp32 precision for fp32 x and bf16 w, as three exact bf16 products; planes: bf16 scratch [3][rows][K]. */
+int b2k_linear_split3(const float* x, void* planes_bf16, const void* w_bf16, float* out, int rows, int N, int K, int tile, void* stream);
 /* The recurrence of the matrix-state mixers over `portions` portions (portion i ends at row last_rows[i]; last_rows null: every row is one of one token); rule as
  * StateRule in csrc/kernels.h; all tensors fp32: q / k rows of kv_heads * dim, v rows of heads * vdim, decay [T][heads * dim] or [T][heads] by the rule, beta
  * [T][heads], skip [heads], bonus [heads][dim] (null where the rule has none), state [slots][2][heads][dim][vdim], out [T][heads * vdim]. */

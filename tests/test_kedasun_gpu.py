@@ -606,3 +606,19 @@ def test_fp32_prompt_rows_take_nothing_from_what_they_do_not_see(mixer, bad, cle
         got, _ = e.prefill_logits([e.seq_create(90)], [toks], list(range(90)))
         assert err(got[list(clean)], ref[list(clean)]) < F32_BAR
         assert not np.isfinite(got[bad]).any()
+
+
+def test_fp32_products_follow_a_reloaded_weight():
+    """The fp32 products of prompt size read bf16 copies of the weights: a tensor that is loaded again behind the finalisation counts from the next step on."""
+    import ctypes as C
+    cfg = cfg_c()
+    w = random_weights(cfg, seed=5)
+    new = dict(w)
+    new["l0.mlp.down"] = random_weights(cfg, seed=6)["l0.mlp.down"]
+    toks = tokens(cfg, 200, 7)
+    with engine(cfg, w) as e:
+        e.prefill([e.seq_create(256)], [toks])
+        t = new["l0.mlp.down"].to(torch.bfloat16).contiguous()
+        assert e.lib.b2_engine_load_tensor(e.h, b"l0.mlp.down", C.c_void_p(t.data_ptr()), t.numel() * 2) == 0
+        got, _ = e.prefill_logits([e.seq_create(256)], [toks], [199])
+    assert err(got[0], ref_logits(cfg, new, toks)[199]) < F32_BAR

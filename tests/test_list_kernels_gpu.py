@@ -175,3 +175,38 @@ def test_linear_sum_groups(lib, tile, N, K):
     chk(lib, lib.b2k_linear_sum(ptr(x), ptr(w[0]), None, 1, rows, ptr(one), N, K, 0, tile, cuda_stream_ptr()))
     torch.cuda.synchronize()
     assert ((one.double() - x.double() @ w[0].double().T).abs() <= K * 2.0 ** -24 * (x.double().abs() @ w[0].double().abs().T)).all()
+
+
+@pytest.mark.parametrize("tile", [128, 256, 0])
+@pytest.mark.parametrize("rows,N,K", [(1, 64, 64), (5, 300, 128), (127, 128, 192), (129, 200, 320), (300, 704, 1024), (257, 256, 3072)])
+def test_linear_split3(lib, tile, rows, N, K):
+    """fp32 rows as three bf16 planes: numbers of all sizes, the largest ones, infinities and NaN.  Products are exact; every addition inside a chunk of 128 (three
+    times 128 products, sixteen at a time, summed with at most one unit in the last place lost) and between chunks costs at most 2^-23 of the sum of absolute values."""
+    g = torch.Generator().manual_seed(rows + N + K)
+    x = torch.randn(rows, K, generator=g) * torch.exp2(torch.randint(-20, 20, (rows, K), generator=g).float())
+    w = (torch.randn(N, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    dx, dw, planes = x.cuda(), w.cuda(), torch.empty(3, rows, K, dtype=torch.bfloat16, device="cuda")
+    def run(xs):
+        out = torch.full((rows + 3, N), 7.0, device="cuda")
+        chk(lib, lib.b2k_linear_split3(ptr(xs), ptr(planes), ptr(dw), ptr(out), rows, N, K, tile, cuda_stream_ptr()))
+        torch.cuda.synchronize()
+        assert (out[rows:] == 7.0).all()
+        return out[:rows].double()
+    got = run(dx)
+    assert torch.equal(planes.double().sum(0), dx.double())
+    ref, mag = dx.double() @ dw.double().T, dx.double().abs() @ dw.double().abs().T
+    assert ((got - ref).abs() <= (24 + K / 128) * 2.0 ** -23 * mag).all()
+    odd = x.clone()
+    odd[0, :4] = torch.tensor([3.4028234e38, 1e-42, -3.4e38, 0.0])    # rounds to infinity in bf16; below bf16's normal numbers
+    if rows > 4:
+        odd[2, 1], odd[4, 2] = float("inf"), float("nan")
+    got = run(odd.cuda())
+    if rows > 4:
+        fine = w[:, 1].float() != 0
+        assert torch.equal(got[2].cpu()[fine], (w[:, 1].double() * float("inf"))[fine]) and torch.isnan(got[4]).all()
+    keep = [r for r in range(rows) if r not in (0, 2, 4)]
+    if keep:
+        assert ((got[keep] - ref[keep]).abs() <= (24 + K / 128) * 2.0 ** -23 * mag[keep]).all()
+    big = odd[0].double().cuda() @ dw.double().T
+    sure = big.abs() < 1e38                                           # (partial sums may pass the largest number on the way)
+    assert torch.isfinite(planes[:, 0].float()).all() and ((got[0] - big).abs() <= 2.0 ** -15 * (odd[0].double().abs().cuda() @ dw.double().abs().T))[sure & torch.isfinite(got[0])].all()
