@@ -116,6 +116,17 @@ extern "C" int b2k_linear_split3(const float* x, void* planes, const void* w, fl
   return launch_linear_split3(x, (bf16*)planes, (const bf16*)w, out, rows, N, K, wait, (cudaStream_t)stream, tile);
 }
 
+extern "C" int b2k_heads_postmix(const float* q, const void* k_cache, const void* v_cache, int heads, int kv_heads, int dim, int vdim, float scale, float slope_exp,
+                                 int window, int keep_first, const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, int ntiles, const float* talk,
+                                 const float* gate, int gate_ld, void* out, void* stream) {
+  B2_REQUIRE(q && k_cache && v_cache && block_table && tiles && talk && out, "b2k_heads_postmix: null pointer");
+  HeadsGeom g{};
+  g.heads = heads; g.kv_heads = kv_heads; g.dim = dim; g.vdim = vdim; g.scale = scale;
+  g.slopes = slope_exp > 0.f ? 1 : 0; g.slope_exp = slope_exp; g.window = window; g.keep_first = keep_first; g.cross = 1;
+  return launch_heads_postmix(q, (const bf16*)k_cache, (const bf16*)v_cache, g, block_table, bt_stride, block_size, (const PrefillTile*)tiles, ntiles, talk, gate, gate_ld,
+                              (bf16*)out, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
                               const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
                               const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,

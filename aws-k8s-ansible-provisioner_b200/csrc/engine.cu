@@ -1481,7 +1481,16 @@ int forward_heads_list(b2_engine* e, int T, int ntiles, int nlast) {
                                                 e->d_positions, e->d_slots, L.vmix_mode, L.vmix, e->l_vfirst, e->l_q, kc, vc, f, T, st,
                                                 L.gqa_tc ? e->l_qb : nullptr));
     }
-    if (L.gqa_tc) {   // the framework's GQA kernels: tcgen05 for prompt portions, the page-balanced stream for decode steps
+    const float* gates = e->l_qd + (L.nq + L.nk + L.nv);
+    static const bool use_postmix = [] { const char* v = getenv("B2_HEADS_POSTMIX"); return !(v && *v == '0'); }();   // 0: outputs mixed (cross-check)
+    // (few queries leave its one CTA per SM and sixteen queries alone with the barriers; whole calls, us, outputs mixed / weights mixed: 16 heads 1 x 300 tokens
+    // 575 / 583, 1 x 600 721 / 698, 12 x 100 1232 / 1124; 8 heads 1 x 600 463 / 497, 6 x 200 725 / 697)
+    const bool postmix = use_postmix && conv && tiles != nullptr && !f && (long)T * sp.heads >= 8192 && heads_postmix_ok(g, c.block_size);
+    if (postmix) {   // prompt portions: the weights mixed over the heads, and the head gates
+      KL k(e, B2K_MISC);
+      if (!k.skip()) B2_TRY(launch_heads_postmix(e->l_q, (const bf16*)kc, (const bf16*)vc, g, e->d_block_table, e->bt_stride, c.block_size, tiles, ntiles, L.talk, gates,
+                                                 L.nqd, (bf16*)e->l_av, st));
+    } else if (L.gqa_tc) {   // the framework's GQA kernels: tcgen05 for prompt portions, the page-balanced stream for decode steps
       KL k(e, ntiles > 0 ? B2K_MISC : B2K_ATTN_DECODE);
       if (!k.skip()) {
         if (ntiles > 0)
@@ -1496,9 +1505,9 @@ int forward_heads_list(b2_engine* e, int T, int ntiles, int nlast) {
       if (!k.skip()) B2_TRY(launch_heads_attention(e->l_q, kc, vc, f, g, e->d_block_table, e->bt_stride, c.block_size, tiles, ntiles, e->d_positions,
                                                    e->d_seq_lens, conv ? (void*)e->l_cross : e->l_av, conv ? 1 : f, T, st));
     }
-    if (conv) {
+    if (conv && !postmix) {
       KL k(e, B2K_ACT);  // the heads' weights mixed (as sums over the per-head outputs) and the head gates
-      if (!k.skip()) B2_TRY(launch_talk_gate(e->l_cross, L.talk, e->l_qd + (L.nq + L.nk + L.nv), L.nqd, e->l_av, f, sp.heads, sp.kv_heads, sp.vdim, T, st));
+      if (!k.skip()) B2_TRY(launch_talk_gate(e->l_cross, L.talk, gates, L.nqd, e->l_av, f, sp.heads, sp.kv_heads, sp.vdim, T, st));
     }
     {
       KL k(e, B2K_GEMM_O);

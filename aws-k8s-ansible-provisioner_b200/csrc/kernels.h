@@ -443,6 +443,10 @@ int launch_heads_attention_premix(const float* q, const void* k_cache, const voi
 size_t heads_attention_premix_scratch_floats(int max_rows, int heads, int vdim);
 int launch_talk_gate(const float* cross, const float* talk, const float* gate, int gate_ld, void* out, int out_f32, int heads, int kv_heads,
                      int vdim, int T, cudaStream_t s);
+// attn_postmix.cu: both in one for prompt portions over a bf16 cache, the weights mixed instead of the outputs; out bf16 [T][heads * vdim]
+bool heads_postmix_ok(const HeadsGeom& g, int block_size);
+int launch_heads_postmix(const float* q, const bf16* k_cache, const bf16* v_cache, const HeadsGeom& g, const int32_t* block_table, int bt_stride, int block_size,
+                         const PrefillTile* tiles, int ntiles, const float* talk, const float* gate, int gate_ld, bf16* out, cudaStream_t s);
 
 // ---- attn_state.cu: mixers with a matrix state per head (gated linear attention, gated delta rule) ----
 enum StateRule {

@@ -435,6 +435,12 @@ int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* knorm_w, cons
                  const int32_t* block_table, int bt_stride, const int32_t* seq_lens, void* out, int B, int nq, int nkv, float eps, float scale, void* stream);
 /* out[rows][N] = x[rows][K] . w[N][K]^T at fp32 precision for fp32 x and bf16 w, as three exact bf16 products; planes: bf16 scratch [3][rows][K]. */
 int b2k_linear_split3(const float* x, void* planes_bf16, const void* w_bf16, float* out, int rows, int N, int K, int tile, void* stream);
+/* Prompt attention whose softmax weights are mixed over at most sixteen heads (csrc/attn_postmix.cu): out[t][a] = sigmoid(gate[t][a]) * sum_j (sum_b talk[a][b] P_b[t][j])
+ * v_{kv(a)}[j], P_b = softmax(scale q_b k - slope_b distance), slope_b = 2^(-slope_exp (b + 1) / heads) (slope_exp 0: none).  q fp32 [T][heads * dim]; caches bf16
+ * [pages][block_size][kv_heads * dim or vdim]; tiles: {first row, its position, rows <= 64, block-table row}; gate may be null; out bf16 [T][heads * vdim]. */
+int b2k_heads_postmix(const float* q, const void* k_cache, const void* v_cache, int heads, int kv_heads, int dim, int vdim, float scale, float slope_exp, int window,
+                      int keep_first, const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, int ntiles, const float* talk, const float* gate,
+                      int gate_ld, void* out, void* stream);
 /* The recurrence of the matrix-state mixers over `portions` portions (portion i ends at row last_rows[i]; last_rows null: every row is one of one token); rule as
  * StateRule in csrc/kernels.h; all tensors fp32: q / k rows of kv_heads * dim, v rows of heads * vdim, decay [T][heads * dim] or [T][heads] by the rule, beta
  * [T][heads], skip [heads], bonus [heads][dim] (null where the rule has none), state [slots][2][heads][dim][vdim], out [T][heads * vdim]. */

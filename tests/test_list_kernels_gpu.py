@@ -210,3 +210,48 @@ def test_linear_split3(lib, tile, rows, N, K):
     big = odd[0].double().cuda() @ dw.double().T
     sure = big.abs() < 1e38                                           # (partial sums may pass the largest number on the way)
     assert torch.isfinite(planes[:, 0].float()).all() and ((got[0] - big).abs() <= 2.0 ** -15 * (odd[0].double().abs().cuda() @ dw.double().abs().T))[sure & torch.isfinite(got[0])].all()
+
+
+@pytest.mark.parametrize("heads,kv,dim,vdim,window,keep,bs", [(16, 8, 128, 128, 70, 9, 16), (16, 16, 64, 64, 0, 0, 32), (5, 1, 128, 64, 33, 0, 48), (8, 4, 64, 128, 16, 40, 16),
+                                                              (1, 1, 128, 128, 1, 5, 16), (12, 4, 128, 128, 100, 16, 64)])
+def test_heads_postmix(lib, heads, kv, dim, vdim, window, keep, bs):
+    """Portions around the tiles of sixteen, some behind earlier tokens, windows and kept tokens around them, fewer heads than the mix's sixteen.  Against 64 bits over
+    the same bf16 queries, keys and values: the weights carry sixteen bits into the products, so what is left is fp32 sums and the bf16 result (2^-9 of it).  A weight and
+    a mixed one are off by 2^-17 of themselves, a score of a few units by as much: 2^-14 of the sum of absolute values holds them."""
+    g = torch.Generator().manual_seed(heads * 100 + window)
+    portions = [(0, 1), (0, 17), (100, 64), (3, 33), (200, 130), (0, 256)]            # (earlier tokens, tokens)
+    T, width = sum(n for _, n in portions), max((p + n + bs - 1) // bs for p, n in portions)
+    pages = len(portions) * width + 2
+    bt = torch.randperm(pages, generator=g)[:len(portions) * width].view(-1, width).to(torch.int32)
+    q = torch.randn(T, heads * dim, generator=g)
+    kc, vc = (torch.randn(pages, bs, kv * d, generator=g).to(torch.bfloat16) for d in (dim, vdim))
+    talk = torch.eye(heads) + 0.3 * torch.randn(heads, heads, generator=g)
+    gate = torch.randn(T, heads + 3, generator=g)
+    tiles, at = [], 0
+    for b, (p, n) in enumerate(portions):
+        tiles += [(at + i, p + i, min(64, n - i), b) for i in range(0, n, 64)]
+        at += n
+    scale, slope_exp = dim ** -0.5, 8.0
+    dev = [t.cuda() for t in (q, kc, vc, bt, torch.tensor(tiles, dtype=torch.int32), talk, gate)]
+    out = torch.full((T + 1, heads * vdim), float("nan"), dtype=torch.bfloat16, device="cuda")
+    chk(lib, lib.b2k_heads_postmix(ptr(dev[0]), ptr(dev[1]), ptr(dev[2]), heads, kv, dim, vdim, scale, slope_exp, window, keep, ptr(dev[3]), width, bs, ptr(dev[4]), len(tiles),
+                                   ptr(dev[5]), ptr(dev[6]), heads + 3, ptr(out), cuda_stream_ptr()))
+    torch.cuda.synchronize()
+    assert torch.isnan(out[T]).all()
+    at, rep = 0, heads // kv
+    slope = torch.tensor([2.0 ** (-slope_exp * (a + 1) / heads) for a in range(heads)], dtype=torch.float64)[:, None, None]
+    for b, (p, n) in enumerate(portions):
+        idx, S = bt[b].long(), p + n
+        k = kc[idx].reshape(-1, kv, dim)[:S].double().repeat_interleave(rep, 1)
+        v = vc[idx].reshape(-1, kv, vdim)[:S].double().repeat_interleave(rep, 1)
+        qq = q[at:at + n].to(torch.bfloat16).double().view(n, heads, dim)
+        i, j = torch.arange(p, S)[:, None], torch.arange(S)[None, :]
+        seen = (j <= i) & ((i - j < window) | (j < keep)) if window else j <= i
+        s = torch.einsum("ihd,jhd->hij", qq, k) * scale - slope * (i - j)
+        pr = torch.softmax(s.masked_fill(~seen, float("-inf")), -1)
+        w = torch.einsum("ab,bij->aij", talk.double(), pr)
+        ref = torch.einsum("hij,jhd->ihd", w, v) * torch.sigmoid(gate[at:at + n, :heads].double())[:, :, None]
+        got = out[at:at + n].cpu().double().view(n, heads, vdim)
+        mag = torch.einsum("hij,jhd->ihd", torch.einsum("ab,bij->aij", talk.double().abs(), pr), v.abs())
+        assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -14 * mag + 1e-6).all(), (b, (got - ref).abs().max())
+        at += n
