@@ -46,9 +46,9 @@ __device__ __forceinline__ void px_split(float a, float b, uint32_t& hi, uint32_
 // grid (query tiles * 4 of sixteen rows); block 32 * heads
 template <int D, int DV>
 __global__ void __launch_bounds__(32 * PX_HEADS, 1)
-heads_postmix_kernel(const float* __restrict__ q, const bf16* __restrict__ k_cache, const bf16* __restrict__ v_cache, HeadsGeom g, const int32_t* __restrict__ block_table,
-                     int bt_stride, int block_size, const PrefillTile* __restrict__ tiles, const float* __restrict__ talk, const float* __restrict__ gate, int gate_ld,
-                     bf16* __restrict__ out) {
+heads_postmix_kernel(const float* q, const bf16* k_cache, const bf16* v_cache, HeadsGeom g, const int32_t* __restrict__ block_table,
+                     int bt_stride, int block_size, const PrefillTile* __restrict__ tiles, const float* __restrict__ talk, const float* gate, int gate_ld,
+                     bf16* out) {
   extern __shared__ __align__(128) unsigned char px_smem[];
   constexpr int KC = D / 8, VC = DV / 8;                                         // 16-byte chunks of a row; chunk c of row r lies at c ^ (r & 7)
   bf16* Qs = reinterpret_cast<bf16*>(px_smem);                                   // [heads][16][D]

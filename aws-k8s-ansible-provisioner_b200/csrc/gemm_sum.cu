@@ -94,8 +94,8 @@ struct GsWalk {
 // offsets: [groups + 1] first rows of the groups in device memory, or null: one group of `rows_total` rows
 template <int BN, int EPI, bool SPLIT>
 __global__ void __launch_bounds__(GS_THREADS, 1)
-linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const int32_t* __restrict__ offsets, int groups,
-                  int rows_total, void* __restrict__ out, int N, int K, const B2WaitLimit limit) {
+linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const int32_t* offsets, int groups,
+                  int rows_total, void* out, int N, int K, const B2WaitLimit limit) {
   using C = GsCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::STAGES];
@@ -296,7 +296,7 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
 }
 
 // planes [3][n] bf16 whose sum is x: every plane the nearest bf16 to what is left (a value that rounds to infinity is cut instead; infinities and NaN stay in the first)
-__global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ x, uint2* __restrict__ planes, size_t n4) {
+__global__ void __launch_bounds__(256) split3_kernel(const float4* x, uint2* planes, size_t n4) {
   pdl_wait();
   pdl_launch_dependents();
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
