@@ -101,6 +101,12 @@ extern "C" int b2k_few_linear(const void* w, const void* x, const void* gain, fl
   return launch_few_gateup((const bf16*)w, (const bf16*)x, (const bf16*)gain, eps, (bf16*)out, T, N, K, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_few_head(const void* w, const void* x, float* out, int T, int N, int K, float alpha, void* stream) {
+  B2_REQUIRE(w && x && out, "b2k_few_head: null pointer");
+  B2_REQUIRE(few_head_ok(T, N, K), "b2k_few_head: T=%d N=%d K=%d not built", T, N, K);
+  return launch_few_head((const bf16*)w, (const bf16*)x, out, T, N, K, alpha, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* knorm_w, const void* cos_sin, const int32_t* positions, const int32_t* slots, void* k_pages,
                             void* v_pages, const int32_t* block_table, int bt_stride, const int32_t* seq_lens, void* out, int B, int nq, int nkv, float eps, float scale,
                             void* stream) {

@@ -1010,6 +1010,8 @@ int list_dense(b2_engine* e, const void* A, const void* Wt, float* C, int M, int
   if (alpha == 1.f) {
     if (const bf16* wb = list_f32_copy(e, A, Wt, M, N, K, ls)) return launch_linear_split3((const float*)A, e->f32_planes, wb, C, M, N, K, e->wait_limit(), ls);
   }
+  static const bool few_head = [] { const char* v = getenv("B2_FEW_HEAD"); return !(v && *v == '0'); }();
+  if (few_head && !f && N >= 16384 && few_head_ok(M, N, K)) return launch_few_head((const bf16*)Wt, (const bf16*)A, C, M, N, K, alpha, ls);
   if (alpha == 1.f && list_dense_tc(e, M, N, K)) {
     if (M > 128 && linear_sum_pays(M, N)) return launch_linear_sum(A, Wt, nullptr, 1, M, C, N, K, SUM_EPI_F32, e->wait_limit(), ls);
     TcGemmArgs a;
@@ -2474,18 +2476,21 @@ int lm_head_and_argmax(b2_engine* e, int nlast, const bf16* xl, XBuf xb) {
     KL k2(e, B2K_MISC);
     if (!k2.skip()) B2_TRY(launch_argmax_rows(e->logits, e->d_out_tokens, nlast, c.vocab, e->stream));
   } else {
-    TcGemmArgs a;
-    // operands trade places for the fused arg-max: tokens on MMA-M (128-row box of X), 128 vocabulary
-    // rows per tile on MMA-N
-    a.bn = 128;
-    a.tmap_w = e->tm_x[xb][bn_index(128)];
-    a.tmap_x = e->tm_lm_head;
-    a.T = nlast; a.N = c.vocab; a.K = H;
-    a.nsplit = 1;
-    a.epilogue = TC_EPI_ARGMAX_ROWS;
-    a.out = logits;
-    a.argmax_packed = e->d_argmax;
-    {
+    if (e->force_gemm_impl < 0 && e->use_few && few_head_ok(nlast, c.vocab, H)) {   // at most sixteen rows: the weights stream through registers
+      KL k(e, B2K_LMHEAD);
+      if (!k.skip()) B2_TRY(launch_few_head_argmax(e->lm_head, xl, logits, e->d_argmax, nlast, c.vocab, H, e->stream));
+    } else {
+      TcGemmArgs a;
+      // operands trade places for the fused arg-max: tokens on MMA-M (128-row box of X), 128 vocabulary
+      // rows per tile on MMA-N
+      a.bn = 128;
+      a.tmap_w = e->tm_x[xb][bn_index(128)];
+      a.tmap_x = e->tm_lm_head;
+      a.T = nlast; a.N = c.vocab; a.K = H;
+      a.nsplit = 1;
+      a.epilogue = TC_EPI_ARGMAX_ROWS;
+      a.out = logits;
+      a.argmax_packed = e->d_argmax;
       KL k(e, B2K_LMHEAD);
       if (!k.skip()) B2_TRY(launch_linear_tc(a, e->stream));
     }

@@ -9,7 +9,8 @@
 // of which about 2 are the hand-off).  So:
 //   * a CTA's share of the weights sits in its REGISTERS before the kernel in front has ended: it is requested before the dependency wait, and every kernel lets
 //     the next one start at its own start, so the weight streams of two or three kernels run beside the one that computes.  (Constants and page tables only:
-//     everything that a kernel in front writes is read behind the wait, and a kernel that is through its wait has all kernels before it complete.)
+//     everything that a kernel in front writes is read behind the wait, through pointers that are not __restrict__: read-only loads may be moved across it. A
+//     kernel that is through its wait has all kernels before it complete.)
 //   * 128 CTAs of 8 warps; a CTA owns whole weight rows (no sums between CTAs), its warps split K.  Inside a 32-wide k chunk lane (n, c) = (lane / 4, lane % 4)
 //     takes elements [8c, 8c + 8) of weight row n and of token n; elements 0..3 feed one m16n8k16 (tokens on M, weight rows on N; an MMA does not care which
 //     physical k sits behind its logical k as long as both operands agree), elements 4..7 the next: operands go from global memory into the fragments as they are.
@@ -173,15 +174,103 @@ __global__ void __launch_bounds__(FEW_THREADS) few_kernel(const bf16* __restrict
   }
 }
 
+// ---- heads: at most sixteen rows against many weight rows ----
+// out [T][N] fp32 = alpha * x [T][K] . w [N][K]^T, or (ARGMAX) bf16 logits, written where out is given, and the largest with the lowest index per row.  A CTA per SM walks the tiles of eight weight rows with stride gridDim.x; its warps split K as above, the rows of x stay
+// in fragments (HALVES: one or two times eight of them), and while a tile is multiplied the next DEPTH - 1 are under way into registers, the first ones before the
+// dependency wait.  Bound: HBM.  What a launch adds to a step, us, the tcgen05 kernel with its 16-row tiles before and this one: 32000 x 2048, 4 rows 27.7 -> 21.8 (6.0 TB/s),
+// 16 rows 29.5 -> 25.3; 151936 x 1024, 1 row 60 -> 47.5 (6.5 TB/s).
+template <int CH, int HALVES, int DEPTH, bool ARGMAX>
+__global__ void __launch_bounds__(FEW_THREADS, CH <= 4 ? 2 : 1) few_head_kernel(const bf16* __restrict__ w, const bf16* x, void* out, int T, int N,
+                                                                                  int K, float alpha, unsigned long long* best_packed) {
+  __shared__ float red[2][FEW_WARPS][HALVES * FEW_T][8 + 1];
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+  const int chunks = K / 32, tiles = (N + 7) / 8;
+  uint4 wr[DEPTH][CH];
+  auto load = [&](int tile, uint4 (&r)[CH]) {
+    const bf16* p = w + (size_t)min(tile * 8 + g, N - 1) * K + c * 8;   // (rows past N: computed and dropped)
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const int k = warp + i * FEW_WARPS;
+      r[i] = tile < tiles && k < chunks ? few_ldw(p + k * 32) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  };
+#pragma unroll
+  for (int d = 0; d < DEPTH - 1; ++d) load(blockIdx.x + d * gridDim.x, wr[d]);
+  pdl_wait();
+  uint4 xr[HALVES][CH];
+#pragma unroll
+  for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const int k = warp + i * FEW_WARPS, t = h * 8 + g;
+      xr[h][i] = k < chunks && t < T ? *reinterpret_cast<const uint4*>(x + (size_t)t * K + k * 32 + c * 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
+  int parity = 0;
+  unsigned long long best = 0ull;   // ARGMAX: (value, -index) of this thread's row, as gemm_tc.cu packs it
+  for (int t0 = blockIdx.x; t0 < tiles; t0 += DEPTH * gridDim.x) {
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d) {
+      const int tile = t0 + d * gridDim.x;
+      if (tile >= tiles) break;
+      load(tile + (DEPTH - 1) * gridDim.x, wr[(d + DEPTH - 1) % DEPTH]);
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const uint4 b = wr[d][i], a0 = xr[0][i], a1 = HALVES == 2 ? xr[HALVES - 1][i] : make_uint4(0u, 0u, 0u, 0u);
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+                     : "r"(a0.x), "r"(a1.x), "r"(a0.y), "r"(a1.y), "r"(b.x), "r"(b.y));
+        asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                     : "+f"(acc[0]), "+f"(acc[1]), "+f"(acc[2]), "+f"(acc[3])
+                     : "r"(a0.z), "r"(a1.z), "r"(a0.w), "r"(a1.w), "r"(b.z), "r"(b.w));
+      }
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h) {
+        red[parity][warp][h * 8 + g][2 * c] = acc[2 * h];
+        red[parity][warp][h * 8 + g][2 * c + 1] = acc[2 * h + 1];
+      }
+      __syncthreads();   // (the other parity's sums were read before this tile's were written by every warp: one barrier a tile)
+      if (threadIdx.x < HALVES * 64) {
+        const int row = threadIdx.x & 7, t = threadIdx.x >> 3, col = tile * 8 + row;
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < FEW_WARPS; ++k) v += red[parity][k][t][row];
+        if (t < T && col < N) {
+          if constexpr (ARGMAX) {
+            const bf16 b = __float2bfloat16_rn(v);
+            if (out != nullptr) reinterpret_cast<bf16*>(out)[(size_t)t * N + col] = b;
+            const float lv = __bfloat162float(b);
+            const uint32_t u = __float_as_uint(lv), key = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+            const unsigned long long p = lv == lv ? ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)col) : 0ull;
+            best = p > best ? p : best;
+          } else {
+            reinterpret_cast<float*>(out)[(size_t)t * N + col] = v * alpha;
+          }
+        }
+      }
+      parity ^= 1;
+    }
+  }
+  if (ARGMAX && threadIdx.x < HALVES * 64) {   // (whole warps; eight lanes hold a row)
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+      best = other > best ? other : best;
+    }
+    if ((threadIdx.x & 7) == 0 && best != 0ull) atomicMax(best_packed + (threadIdx.x >> 3), best);
+  }
+}
+
 // ---- attention ----
 constexpr int FA_CTAS = 8, FA_WARPS = 4, FA_SHARES = FA_CTAS * FA_WARPS, FA_HD = 128, FA_BS = 16;
 struct FaRecord { float o[2][FA_HD], m[2], l[2]; };   // one share: unnormalised output, maximum and sum of the two query heads
 
 // grid (8, kv heads, sequences), clusters of eight along x; qkv: bf16 rows of (nq + 2 nkv) * 128
 __global__ void __launch_bounds__(32 * FA_WARPS) __cluster_dims__(FA_CTAS, 1, 1)
-few_attn_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw, const bf16* __restrict__ cos_sin,
+few_attn_kernel(const bf16* qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw, const bf16* __restrict__ cos_sin,
                 const int32_t* __restrict__ positions, const int32_t* __restrict__ slots, bf16* k_pages, bf16* v_pages,
-                const int32_t* __restrict__ block_table, int bt_stride, const int32_t* __restrict__ seq_lens, bf16* __restrict__ out, int nq, int nkv, float eps,
+                const int32_t* __restrict__ block_table, int bt_stride, const int32_t* __restrict__ seq_lens, bf16* out, int nq, int nkv, float eps,
                 float scale) {
   __shared__ __align__(16) float qs[2][FA_HD];            // the two query heads, scaled
   __shared__ __align__(16) bf16 kv_new[2][FA_HD];         // the new token's key and value
@@ -380,6 +469,29 @@ int launch_few_gateup(const bf16* wgu, const bf16* h, const bf16* gain, float ep
 int launch_few_resid(const bf16* w, const bf16* x, bf16* h, int T, int N, int K, cudaStream_t s) {
   if (K > 2048) return launch_few<12, 1, FEW_RESID>(w, x, nullptr, 0.f, h, T, N, K, 0, s);
   return launch_few<8, 1, FEW_RESID>(w, x, nullptr, 0.f, h, T, N, K, 0, s);
+}
+// K up to 2048 for sixteen rows, up to 4096 for eight (the fragments of x and of the tiles under way are registers)
+bool few_head_ok(int T, int N, int K) { return T >= 1 && N >= 1 && K % 32 == 0 && K >= 32 && (T <= 8 ? K <= 4096 : T <= 16 && K <= 2048); }
+template <bool ARGMAX>
+static int launch_head(const bf16* w, const bf16* x, void* out, int T, int N, int K, float alpha, unsigned long long* best, cudaStream_t s) {
+  const dim3 grid(std::min((N + 7) / 8, device_num_sms() * (K <= 1024 ? 2 : 1)));   // (a tile of 16 KB is done before its barrier: two CTAs per SM)
+#define B2_FEW_HEAD(C, H, D)                                                                                                   \
+  do {                                                                                                                         \
+    B2_CUDA_OK(b2_launch(few_head_kernel<C, H, D, ARGMAX>, grid, dim3(FEW_THREADS), 0, s, w, x, out, T, N, K, alpha, best));   \
+    return 0;                                                                                                                  \
+  } while (0)
+  if (T <= 8) {
+    if (K <= 1024) B2_FEW_HEAD(4, 1, 4);
+    if (K <= 2048) B2_FEW_HEAD(8, 1, 4);
+    B2_FEW_HEAD(16, 1, 2);
+  }
+  if (K <= 1024) B2_FEW_HEAD(4, 2, 4);
+  B2_FEW_HEAD(8, 2, 3);
+#undef B2_FEW_HEAD
+}
+int launch_few_head(const bf16* w, const bf16* x, float* out, int T, int N, int K, float alpha, cudaStream_t s) { return launch_head<false>(w, x, out, T, N, K, alpha, nullptr, s); }
+int launch_few_head_argmax(const bf16* w, const bf16* x, bf16* logits, unsigned long long* best, int T, int N, int K, cudaStream_t s) {
+  return launch_head<true>(w, x, logits, T, N, K, 1.f, best, s);
 }
 int launch_few_attn(const bf16* qkv, const bf16* qw, const bf16* kw, const bf16* cos_sin, const int32_t* positions, const int32_t* slots, bf16* k_pages, bf16* v_pages,
                     const int32_t* block_table, int bt_stride, const int32_t* seq_lens, bf16* out, int B, int nq, int nkv, float eps, float scale, cudaStream_t s) {

@@ -105,6 +105,11 @@ bool few_shapes_ok(int T, int H, int q_size, int I);
 int launch_few_qkv(const bf16* w, const bf16* h, const bf16* gain, float eps, bf16* qkv, int T, int N, int K, cudaStream_t s);
 int launch_few_gateup(const bf16* wgu, const bf16* h, const bf16* gain, float eps, bf16* act, int T, int I, int K, cudaStream_t s);
 int launch_few_resid(const bf16* w, const bf16* x, bf16* h, int T, int N, int K, cudaStream_t s);
+// out fp32 [T][N] = alpha * x [T][K] . w [N][K]^T for at most sixteen rows and many weight rows (the layer-list families' heads)
+bool few_head_ok(int T, int N, int K);
+int launch_few_head(const bf16* w, const bf16* x, float* out, int T, int N, int K, float alpha, cudaStream_t s);
+// bf16 logits (null: not written) and the packed arg-max of every row (TC_EPI_ARGMAX_ROWS' words, zero before the launch)
+int launch_few_head_argmax(const bf16* w, const bf16* x, bf16* logits, unsigned long long* best, int T, int N, int K, cudaStream_t s);
 int launch_few_attn(const bf16* qkv, const bf16* qw, const bf16* kw, const bf16* cos_sin, const int32_t* positions, const int32_t* slots, bf16* k_pages, bf16* v_pages,
                     const int32_t* block_table, int bt_stride, const int32_t* seq_lens, bf16* out, int B, int nq, int nkv, float eps, float scale, cudaStream_t s);
 // gemm_sum.cu: prompt-sized products with fp32 sums out (or a squared-ReLU expert's bf16 activation), rows of one block or of the ragged blocks of

@@ -429,7 +429,9 @@ int b2k_linear_sum(const void* x_bf16, const void* w_bf16, const int32_t* offset
 /* A decode step's products for at most eight sequences (csrc/gemm_few.cu), K % 32 == 0, all bf16: mode 0: out[T][N] = RMSNorm(x) . w^T; 1: out += x . w^T (gain unused);
  * 2: out[T][N] = silu(g) * u with g | u = RMSNorm(x) . w^T, w [2N][K] (gate rows, then up rows). */
 int b2k_few_linear(const void* w, const void* x, const void* gain, float eps, void* out, int T, int N, int K, int mode, void* stream);
-/* ... and its attention, nq == 2 * nkv, 128-wide heads, pages of sixteen tokens: qkv [B][(nq + 2 nkv) * 128] as the projection leaves it; QK-norm, RoPE and the page write
+/* out[T][N] (fp32) = alpha * x[T][K] . w[N][K]^T for at most sixteen rows (K <= 2048; eight: K <= 4096), K % 32 == 0. */
+int b2k_few_head(const void* w, const void* x, float* out, int T, int N, int K, float alpha, void* stream);
+/* The decode attention of at most eight sequences, nq == 2 * nkv, 128-wide heads, pages of sixteen tokens: qkv [B][(nq + 2 nkv) * 128] as the projection leaves it; QK-norm, RoPE and the page write
  * of the new token (position seq_lens - 1, slot as in b2k_qknorm_rope_kv), then softmax(q k^T * scale) v over the pages. */
 int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* knorm_w, const void* cos_sin, const int32_t* positions, const int32_t* slots, void* k_pages, void* v_pages,
                  const int32_t* block_table, int bt_stride, const int32_t* seq_lens, void* out, int B, int nq, int nkv, float eps, float scale, void* stream);

@@ -95,3 +95,47 @@ def test_few_attn(lib, lens):
     again = torch.empty_like(out)
     run(again)
     assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("T", [1, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(5, 32), (8, 1024), (9001, 96), (20003, 2048), (1189, 4096), (148 * 8 * 4 + 1, 256)])
+def test_few_head(lib, T, N, K):
+    """Fewer tiles than SMs, a last tile that is not whole, tiles under way behind the end, K that leaves warps without a chunk.  Sums of exact products in fp32: K
+    roundings of 2^-24 of the sum of absolute values at most, and one of the scaling."""
+    if T > 8 and K > 2048:
+        assert lib.b2k_few_head(ptr(torch.zeros(1, device="cuda")), ptr(torch.zeros(1, device="cuda")), ptr(torch.zeros(1, device="cuda")), T, N, K, 1.0, cuda_stream_ptr()) != 0
+        return
+    g = torch.Generator().manual_seed(N + T)
+    x, w = torch.randn(T, K, generator=g).to(torch.bfloat16).cuda(), torch.randn(N, K, generator=g).to(torch.bfloat16).cuda()
+    out = torch.full((T + 1, N), 7.0, device="cuda")
+    chk(lib, lib.b2k_few_head(ptr(w), ptr(x), ptr(out), T, N, K, 0.3, cuda_stream_ptr()))
+    torch.cuda.synchronize()
+    ref, mag = 0.3 * (x.double() @ w.double().T), 0.3 * (x.double().abs() @ w.double().abs().T)
+    assert ((out[:T].double() - ref).abs() <= (K + 4) * 2.0 ** -24 * mag).all() and (out[T] == 7.0).all()
+
+
+def test_few_head_argmax_against_the_tile_kernel(lib):
+    """The lm head of at most sixteen rows through the engine's own entry: bf16 logits and tokens of a prompt and of decode steps against the kernels of larger batches."""
+    P = pkg()
+    import numpy as np
+    torch.manual_seed(0)
+    cfg = P.EngineConfig(num_layers=1, hidden=256, num_q_heads=4, num_kv_heads=2, head_dim=128, intermediate=512, vocab=20003, max_model_len=64, num_blocks=40, max_seqs=8,
+                         max_batch_tokens=128)
+    names = {"model.embed_tokens.weight": (20003, 256), "model.norm.weight": (256,), "model.layers.0.input_layernorm.weight": (256,),
+             "model.layers.0.post_attention_layernorm.weight": (256,), "model.layers.0.self_attn.q_proj.weight": (512, 256), "model.layers.0.self_attn.k_proj.weight": (256, 256),
+             "model.layers.0.self_attn.v_proj.weight": (256, 256), "model.layers.0.self_attn.o_proj.weight": (256, 512), "model.layers.0.self_attn.q_norm.weight": (128,),
+             "model.layers.0.self_attn.k_norm.weight": (128,), "model.layers.0.mlp.gate_proj.weight": (512, 256), "model.layers.0.mlp.up_proj.weight": (512, 256),
+             "model.layers.0.mlp.down_proj.weight": (256, 512)}
+    sd = {n: (torch.ones(s) if len(s) == 1 else 0.05 * torch.randn(s)).to(torch.bfloat16) for n, s in names.items()}
+    with P.Engine(cfg) as e:
+        e.load_state_dict(sd)
+        e.set_debug(logits=True)
+        sids = [e.seq_create(32) for _ in range(5)]
+        toks = e.prefill(sids, [list(range(3 + i, 9 + 2 * i)) for i in range(5)])
+        for _ in range(3):
+            logits = np.asarray(e.get_logits(5))
+            assert np.isfinite(logits).all()
+            best = logits.max(1)
+            for i in range(5):   # the lowest index of the largest bf16 value
+                assert int(np.flatnonzero(logits[i] == best[i])[0]) == int(toks[i])
+            toks = e.decode_step(sids, toks)
