@@ -90,6 +90,10 @@ extern "C" int b2k_linear_sum(const void* x, const void* w, const int32_t* offse
   B2_REQUIRE(x && w && out, "b2k_linear_sum: null pointer");
   B2WaitLimit wait;
   CAPI_TRY(hook_waits(&wait));
+  if (epilogue == 2) {
+    B2_REQUIRE(offsets == nullptr && groups == 1, "b2k_linear_sum: the fine sums are built for one block");
+    return launch_linear_sum_fine(x, w, (float*)out, rows, N, K, wait, (cudaStream_t)stream);
+  }
   return launch_linear_sum(x, w, offsets, groups, rows, out, N, K, epilogue, wait, (cudaStream_t)stream, tile);
 }
 

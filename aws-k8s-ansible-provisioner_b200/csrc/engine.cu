@@ -382,6 +382,7 @@ struct b2_engine {
   void *l_bigram = nullptr, *l_pos = nullptr;
   int32_t* l_tok_ring = nullptr;     // [sequence slots][2]: the token at a position, by the position's parity (a sequence's previous token)
   float* l_rz = nullptr;             // a prompt-sized step's router logits
+  size_t l_rz_cols = 0;              // their columns (families that allocate the buffer behind their layers)
   float* l_sg = nullptr;             // the shared expert's gate, one number per token row
   // several residual streams (Resitar; l_h is then [T][streams][W])
   int n_streams = 1;
@@ -1161,6 +1162,19 @@ int list_gated_experts(b2_engine* e, const ListLayer& L, int layer, int T, bool 
   return 0;
 }
 
+// A step's experts and their weights.  Prompt-sized bf16 steps form the logits as one product (a checkpoint's router is bf16: every product of two operands is exact,
+// and the sums are rounded to nearest every 128 of the width, closer to 64 bits than route_kernel's chains), then select per token: 8192 rows of 2048, 16 experts,
+// 87 -> 27 + 11 us; 560 rows 12 -> 21 us (a product of one tile and a launch more), hence the line.
+constexpr int LIST_ROUTE_ROWS = 2560;
+int list_route(b2_engine* e, const ListLayer& L, const void* x, const float* corr, const RouteGeom& g, int T, cudaStream_t s) {
+  const int W = e->cfg.hidden, er = std::max(128, g.experts);
+  if (L.router_op != nullptr && T >= LIST_ROUTE_ROWS && list_use_tc()) {
+    B2_TRY(launch_linear_sum_fine(x, L.router_op, e->l_rz, T, er, W, e->wait_limit(), s));
+    return launch_route_select(e->l_rz, er, corr, g, e->l_idx, e->l_rw, T, s);
+  }
+  return launch_route(x, e->f32 ? 1 : 0, L.router, corr, g, e->l_idx, e->l_rw, T, W, s);
+}
+
 constexpr int LATENT_REBUILD_ROWS = 128;    // portions of at least this many tokens attend over rebuilt keys and values
 
 // C (bf16 [M][N]) = A (bf16 [M][K]) . Wt^T on the tcgen05 projection kernel (K a multiple of 64, N at least 128)
@@ -1367,7 +1381,7 @@ int forward_list(b2_engine* e, int T, int ntiles, int nlast) {
       RouteGeom rg{sp.experts, sp.top, sp.groups, sp.groups_keep};
       {
         KL k(e, B2K_ACT);
-        if (!k.skip()) B2_TRY(launch_route(e->l_x2, f, L.router, L.corr, rg, e->l_idx, e->l_rw, T, W, st));
+        if (!k.skip()) B2_TRY(list_route(e, L, e->l_x2, L.corr, rg, T, st));
       }
       {
         KL k(e, B2K_MISC);
@@ -1741,7 +1755,7 @@ int forward_state_list(b2_engine* e, int T, int ntiles, int nlast) {
       const int F = sp.ff_dim, pairs = T * sp.top;
       {
         KL k(e, B2K_ACT);
-        if (!k.skip()) B2_TRY(launch_route(e->l_x1, f, L.router, nullptr, rg, e->l_idx, e->l_rw, T, W, sF));
+        if (!k.skip()) B2_TRY(list_route(e, L, e->l_x1, nullptr, rg, T, sF));
       }
       {
         KL k(e, B2K_MISC);
@@ -2776,6 +2790,18 @@ int put_f32(float* dst, const uint16_t* src, size_t n, float add) {
   return 0;
 }
 
+// The router as a bf16 operand of list_route's product (zero rows fill it up to the kernel's tile), and the logits' columns
+int router_operand(b2_engine* e, ListLayer& L) {
+  const size_t W = e->cfg.hidden, rows = (size_t)std::max(128, L.sp.experts);
+  if (e->f32 || W % 64 != 0) return 0;
+  char* q = nullptr;
+  B2_TRY(dalloc(&q, rows * W * 2));
+  B2_CUDA_OK(cudaMemset(q, 0, rows * W * 2));
+  L.router_op = reinterpret_cast<bf16*>(q);
+  e->l_rz_cols = std::max(e->l_rz_cols, rows);
+  return 0;
+}
+
 // A key up-projection stored [heads * dim][rank], kept per head as [rank][dim]: the layout the absorbed-query product reads
 int put_key_up(b2_engine* e, void* dst, const uint16_t* src, size_t heads, size_t dim, size_t rank) {
   std::vector<uint16_t> tr(heads * dim * rank);
@@ -2908,7 +2934,11 @@ int list_tensor(b2_engine* e, const std::string& name, const void* host, size_t 
       if (rest == "mlp.act") { B2_TRY(want(4)); return done(put_f32(L.poly, src, 4, 0.0f)); }
     } else if (sp.ff == B2_FF_SCALED_GATED_EXPERTS) {
       const size_t sf = sp.shared_ff;
-      if (rest == "mlp.router") { B2_TRY(want((size_t)sp.experts * W)); return done(put_f32(L.router, src, (size_t)sp.experts * W, 0.0f)); }
+      if (rest == "mlp.router") {
+      B2_TRY(want((size_t)sp.experts * W));
+      if (L.router_op) B2_TRY(put_operand(e, L.router_op, 0, src, (size_t)sp.experts * W));
+      return done(put_f32(L.router, src, (size_t)sp.experts * W, 0.0f));
+    }
       if (sf > 0 && rest == "mlp.shared.gate") { B2_TRY(want(sf * W)); return done(put_operand(e, L.sh_up, 0, src, sf * W)); }
       if (sf > 0 && rest == "mlp.shared.up") { B2_TRY(want(sf * W)); return done(put_operand(e, L.sh_up, sf * W, src, sf * W)); }
       if (sf > 0 && rest == "mlp.shared.down") { B2_TRY(want(W * sf)); return done(put_operand(e, L.sh_down, 0, src, W * sf)); }
@@ -3205,7 +3235,11 @@ int list_tensor(b2_engine* e, const std::string& name, const void* host, size_t 
   if (rest == "mix.sink") { B2_TRY(want(H)); return done(put_f32(L.sink, src, H, 0.0f)); }
   if (rest == "mix.o") { B2_TRY(want(W * H * dv)); return done(put_operand(e, L.wo, 0, src, W * H * dv)); }
   if (sp.ff == B2_FF_ROUTED_EXPERTS) {
-    if (rest == "mlp.router") { B2_TRY(want((size_t)sp.experts * W)); return done(put_f32(L.router, src, (size_t)sp.experts * W, 0.0f)); }
+    if (rest == "mlp.router") {
+      B2_TRY(want((size_t)sp.experts * W));
+      if (L.router_op) B2_TRY(put_operand(e, L.router_op, 0, src, (size_t)sp.experts * W));
+      return done(put_f32(L.router, src, (size_t)sp.experts * W, 0.0f));
+    }
     if (rest == "mlp.correction") { B2_TRY(want((size_t)sp.experts)); return done(put_f32(L.corr, src, (size_t)sp.experts, 0.0f)); }
     if (rest.compare(0, 5, "mlp.e") == 0) {
       size_t d2 = rest.find('.', 5);
@@ -3456,6 +3490,7 @@ int state_engine_alloc(b2_engine* e) {
       B2_REQUIRE(sp.experts >= 1 && sp.top >= 1 && sp.top <= sp.experts && sp.ff_dim >= 1 && sp.shared_ff >= 0,
                  "layer %d: bad router sizes (experts %d, top %d, ff %d)", l, sp.experts, sp.top, sp.ff_dim);
       B2_TRY(falloc(&L.router, (size_t)sp.experts * W));
+      B2_TRY(router_operand(e, L));
       B2_TRY(xalloc(&L.up, (size_t)sp.experts * 2 * sp.ff_dim * W));
       B2_TRY(xalloc(&L.down, (size_t)sp.experts * W * sp.ff_dim));
       if (sp.shared_ff > 0) {
@@ -3548,6 +3583,7 @@ int state_engine_alloc(b2_engine* e) {
   e->l_offsets_stride = max_exp + 1;
   B2_TRY(dalloc(&e->l_offsets, (size_t)3 * (max_exp + 1)));
   B2_CUDA_OK(cudaMemset(e->l_offsets, 0, (size_t)3 * (max_exp + 1) * 4));
+  if (e->l_rz_cols > 0 && Tc >= (size_t)LIST_ROUTE_ROWS) B2_TRY(dalloc(&e->l_rz, Tc * e->l_rz_cols));
   B2_TRY(dalloc(&e->l_slot_token, Tc * max_top));
   B2_TRY(dalloc(&e->l_pair_slot, Tc * max_top));
   e->l_tiles_cap = (int)(Tc * max_top / any_gemm_tile_rows() + max_exp + 1);
@@ -4549,6 +4585,7 @@ int list_engine_alloc(b2_engine* e) {
       B2_TRY(falloc(&L.gain2, W));
       B2_TRY(falloc(&L.router, (size_t)sp.experts * W));
       B2_TRY(falloc(&L.corr, sp.experts));
+      B2_TRY(router_operand(e, L));
       B2_TRY(xalloc(&L.up, (size_t)sp.experts * sp.ff_dim * W));
       B2_TRY(xalloc(&L.down, (size_t)sp.experts * W * sp.ff_dim));
       max_top = std::max(max_top, sp.top);
@@ -4592,6 +4629,7 @@ int list_engine_alloc(b2_engine* e) {
   e->l_offsets_stride = max_exp + 1;
   B2_TRY(dalloc(&e->l_offsets, (size_t)3 * (max_exp + 1)));
   B2_CUDA_OK(cudaMemset(e->l_offsets, 0, (size_t)3 * (max_exp + 1) * 4));
+  if (e->l_rz_cols > 0 && Tc >= (size_t)LIST_ROUTE_ROWS) B2_TRY(dalloc(&e->l_rz, Tc * e->l_rz_cols));
   B2_TRY(dalloc(&e->l_slot_token, Tc * max_top));
   B2_TRY(dalloc(&e->l_pair_slot, Tc * max_top));
   e->l_tiles_cap = (int)(Tc * max_top / any_gemm_tile_rows() + max_exp + 1);

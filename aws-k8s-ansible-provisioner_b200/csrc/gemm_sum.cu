@@ -8,7 +8,7 @@
 //     the next group (or to nobody: zero-filled) and are not stored.
 //   * epilogue: fp32 sums straight from registers (a warp's 32 weight rows are 128 contiguous bytes of an output row), or, for squared-ReLU experts, their
 //     activation rounded to the bf16 operand of the second product.
-//   * SPLIT: x is fp32, given as three bf16 planes whose sum it is (split3_kernel: 8 + 8 + 8 bits of the 24), and the weights are bf16 numbers, so the three
+//   * SPLIT (3; 1: the same sums for bf16 x): x is fp32, given as three bf16 planes whose sum it is (split3_kernel: 8 + 8 + 8 bits of the 24), and the weights are bf16 numbers, so the three
 //     products are exact.  The tensor pipe's accumulator rounds every addition towards zero, so it holds only 128 of the K at a time, smallest plane first: the
 //     epilogue's warps keep the running sums of a tile in registers and add a chunk, rounded to nearest, while the next one is multiplied.
 // Bound: tensor pipe under the power cap, and the last wave.
@@ -92,7 +92,7 @@ struct GsWalk {
 };
 
 // offsets: [groups + 1] first rows of the groups in device memory, or null: one group of `rows_total` rows
-template <int BN, int EPI, bool SPLIT>
+template <int BN, int EPI, int SPLIT>   // SPLIT: planes of x (0: x as it is, its whole K in the accumulator)
 __global__ void __launch_bounds__(GS_THREADS, 1)
 linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const int32_t* offsets, int groups,
                   int rows_total, void* out, int N, int K, const B2WaitLimit limit) {
@@ -110,8 +110,8 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = gs_cluster_rank();
   const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
-  constexpr int PLANES = SPLIT ? 3 : 1;
-  const int kb_total = K / GS_BK, chunk_kb = SPLIT ? GS_CHUNK_KB : kb_total, m_pairs = (N + 2 * GS_BM - 1) / (2 * GS_BM);
+  constexpr int PLANES = SPLIT > 0 ? SPLIT : 1;
+  const int kb_total = K / GS_BK, chunk_kb = SPLIT > 0 ? GS_CHUNK_KB : kb_total, m_pairs = (N + 2 * GS_BM - 1) / (2 * GS_BM);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -230,7 +230,7 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     for (int p = cluster; w.at(p); p += clusters) {
       const int col = (2 * w.pair + (int)rank) * GS_BM + q * 32 + lane;
       const uint32_t tq = tmem_base + ((uint32_t)(q * 32) << 16);
-      if constexpr (SPLIT) {
+      if constexpr (SPLIT > 0) {
         uint32_t sum[BN / 64][32];
 #pragma unroll
         for (int b = 0; b < BN / 64; ++b)
@@ -331,14 +331,14 @@ __global__ void __launch_bounds__(256) bf16_copy_kernel(const uint32_t* __restri
   if (bad) *inexact = 1;
 }
 
-template <int BN, int EPI, bool SPLIT = false>
+template <int BN, int EPI, int SPLIT = 0>
 int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, const B2WaitLimit& wait, cudaStream_t s) {
   using C = GsCfg<BN>;
   static B2PerDeviceOnce attr_once;
   if (attr_once.need()) B2_CUDA_OK(cudaFuncSetAttribute(linear_sum_kernel<BN, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
   CUtensorMap tw, tx;
   int rc = b2_make_tmap_bf16(&tw, w, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K, GS_BM);
-  if (rc == 0) rc = b2_make_tmap_bf16(&tx, x, (uint64_t)rows * (SPLIT ? 3 : 1), (uint64_t)K, (uint64_t)K, BN / 2);
+  if (rc == 0) rc = b2_make_tmap_bf16(&tx, x, (uint64_t)rows * (SPLIT > 0 ? SPLIT : 1), (uint64_t)K, (uint64_t)K, BN / 2);
   if (rc != 0) return rc;
   const int m_pairs = (N + 2 * GS_BM - 1) / (2 * GS_BM);
   const long most = ((long)rows / BN + groups) * m_pairs;   // tiles at most
@@ -402,8 +402,14 @@ int launch_linear_split3(const float* x, bf16* planes, const bf16* w, float* out
   const size_t n4 = (size_t)rows * K / 4;
   B2_CUDA_OK(b2_launch(split3_kernel, dim3((unsigned)std::min<size_t>((n4 + 255) / 256, (size_t)device_num_sms() * 16)), dim3(256), 0, s, (const float4*)x, (uint2*)planes, n4));
   if (bn == 0) bn = sum_pick_bn(rows, 1, N);
-  return bn == 128 ? launch_sum<128, SUM_EPI_F32, true>(planes, w, nullptr, 1, rows, out, N, K, wait, s)
-                   : launch_sum<256, SUM_EPI_F32, true>(planes, w, nullptr, 1, rows, out, N, K, wait, s);
+  return bn == 128 ? launch_sum<128, SUM_EPI_F32, 3>(planes, w, nullptr, 1, rows, out, N, K, wait, s)
+                   : launch_sum<256, SUM_EPI_F32, 3>(planes, w, nullptr, 1, rows, out, N, K, wait, s);
+}
+
+int launch_linear_sum_fine(const void* x, const void* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s) {
+  if (rows <= 0) return 0;
+  B2_REQUIRE(linear_sum_shapes_ok(rows, 1, N, K), "linear_sum_fine: %d rows, N=%d K=%d not built", rows, N, K);
+  return launch_sum<128, SUM_EPI_F32, 1>(x, w, nullptr, 1, rows, out, N, K, wait, s);
 }
 
 int launch_bf16_copy(const float* w, bf16* out, size_t n, uint32_t* inexact, cudaStream_t s) {

@@ -121,6 +121,8 @@ int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int 
                       cudaStream_t s, int bn = 0);
 // the same for fp32 x [rows][K] and bf16 weights, fp32 precision: x goes to three bf16 planes ([3][rows][K], scratch) whose sum it is
 int launch_linear_split3(const float* x, bf16* planes, const bf16* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int bn = 0);
+// bf16 x with the same sums (128 of the K in the accumulator at a time, rounded to nearest between them): router logits
+int launch_linear_sum_fine(const void* x, const void* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s);
 // bf16 copy of n fp32 numbers; *inexact (device) becomes 1 when one of them is not a bf16 number
 int launch_bf16_copy(const float* w, bf16* out, size_t n, uint32_t* inexact, cudaStream_t s);
 // gemm_gateup.cu: the prefill-sized counterpart (two accumulators per tile, SwiGLU in the epilogue)

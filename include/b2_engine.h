@@ -424,7 +424,7 @@ int b2k_qkv_rope(const void* x_bf16, const void* w_qkv_bf16, const void* qnorm_w
 int b2k_linear_multicast(const void* x_bf16, const void* w_bf16, void* out_bf16, int T, int N, int K, void* stream);
 /* Prompt-sized products of the layer-list families on pairs of CTAs, rows of one block (offsets null, groups 1) or of `groups` ragged blocks whose first
  * rows the kernel reads from device memory (offsets [groups + 1], the last one = rows): out[row][N] = x[row][K] . w_g[N][K]^T as fp32 (epilogue 0) or
- * bf16(max(sum, 0)^2) (1).  K % 64 == 0; tile: 0 (by the sizes), 128 or 256 rows of x. */
+ * bf16(max(sum, 0)^2) (1), or, for one block, fp32 with the sums rounded to nearest every 128 of K (2).  K % 64 == 0; tile: 0 (by the sizes), 128 or 256 rows of x. */
 int b2k_linear_sum(const void* x_bf16, const void* w_bf16, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, int tile, void* stream);
 /* A decode step's products for at most eight sequences (csrc/gemm_few.cu), K % 32 == 0, all bf16: mode 0: out[T][N] = RMSNorm(x) . w^T; 1: out += x . w^T (gain unused);
  * 2: out[T][N] = silu(g) * u with g | u = RMSNorm(x) . w^T, w [2N][K] (gate rows, then up rows). */

@@ -175,6 +175,21 @@ def test_bf16_expert_products_of_a_long_step():
         assert rows_over(np.concatenate(short), long_step, BF16_BAR) <= 1
 
 
+@pytest.mark.parametrize("experts,top", [(5, 2), (130, 3)])
+def test_bf16_router_of_a_long_step(experts, top):
+    """bf16: a step of 2560 tokens and more forms the router's logits as one product (fewer experts than its tile of 128 rows, and more); the same prompts in shorter
+    steps take a kernel that sums them token by token."""
+    cfg = {"architecture": "Lerasun", "vocab": 211, "width": 128, "logit_scale": 0.5, "norm": {"eps": 1e-6},
+           "layers": [layer(mixer(2, 32, 16, 32, 64, 0.2), moe(128, experts, top, 1, 1))]}
+    w = random_weights(cfg, seed=51)
+    prompts = [tokens(cfg, 900, 52 + i) for i in range(3)]
+    rows = [i * 900 + p for i in range(3) for p in range(500, 900, 9)]
+    with engine(cfg, w, f32=False, max_batch_tokens=2816, num_blocks=400, max_seqs=8) as e:
+        one, _ = e.prefill_logits([e.seq_create(900) for _ in prompts], prompts, rows)
+        each = [e.prefill_logits([e.seq_create(900)], [p], list(range(500, 900, 9)))[0] for p in prompts]
+    assert rows_over(one, np.concatenate(each), BF16_BAR) <= 1
+
+
 @pytest.mark.parametrize("experts,groups,keep,top", [(1, 1, 1, 1), (3, 1, 1, 2), (5, 5, 3, 2), (7, 1, 1, 7), (9, 3, 2, 4), (15, 5, 2, 1), (34, 2, 1, 17)])
 def test_router_of_any_expert_count(experts, groups, keep, top):
     """Expert counts that are odd, prime, one, or more than a warp's lanes, with a width the router reads four numbers at a time:

@@ -174,7 +174,13 @@ def test_linear_sum_groups(lib, tile, N, K):
     one = torch.full((rows, N), 7.0, device="cuda")   # one block
     chk(lib, lib.b2k_linear_sum(ptr(x), ptr(w[0]), None, 1, rows, ptr(one), N, K, 0, tile, cuda_stream_ptr()))
     torch.cuda.synchronize()
-    assert ((one.double() - x.double() @ w[0].double().T).abs() <= K * 2.0 ** -24 * (x.double().abs() @ w[0].double().abs().T)).all()
+    want, mag = x.double() @ w[0].double().T, x.double().abs() @ w[0].double().abs().T
+    assert ((one.double() - want).abs() <= K * 2.0 ** -24 * mag).all()
+    # sums of 128, eight additions of sixteen products with at most a unit in the last place lost, joined by additions to nearest
+    fine = torch.full((rows + 1, N), 7.0, device="cuda")
+    chk(lib, lib.b2k_linear_sum(ptr(x), ptr(w[0]), None, 1, rows, ptr(fine), N, K, 2, tile, cuda_stream_ptr()))
+    torch.cuda.synchronize()
+    assert (fine[rows] == 7.0).all() and ((fine[:rows].double() - want).abs() <= (8 + K / 128) * 2.0 ** -23 * mag).all()
 
 
 @pytest.mark.parametrize("tile", [128, 256, 0])
