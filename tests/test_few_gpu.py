@@ -1,5 +1,6 @@
 """The decode kernels of at most eight sequences (GPU), called through the C ABI: against the kernels that larger batches take (page writes bit for bit) and against
 the same arithmetic in 64 bits between the bf16 roundings."""
+import numpy as np
 import pytest
 import torch
 
@@ -114,10 +115,8 @@ def test_few_head(lib, T, N, K):
     assert ((out[:T].double() - ref).abs() <= (K + 4) * 2.0 ** -24 * mag).all() and (out[T] == 7.0).all()
 
 
-def test_few_head_argmax_against_the_tile_kernel(lib):
-    """The lm head of at most sixteen rows through the engine's own entry: bf16 logits and tokens of a prompt and of decode steps against the kernels of larger batches."""
+def small_model():
     P = pkg()
-    import numpy as np
     torch.manual_seed(0)
     cfg = P.EngineConfig(num_layers=1, hidden=256, num_q_heads=4, num_kv_heads=2, head_dim=128, intermediate=512, vocab=20003, max_model_len=64, num_blocks=40, max_seqs=8,
                          max_batch_tokens=128)
@@ -127,6 +126,12 @@ def test_few_head_argmax_against_the_tile_kernel(lib):
              "model.layers.0.self_attn.k_norm.weight": (128,), "model.layers.0.mlp.gate_proj.weight": (512, 256), "model.layers.0.mlp.up_proj.weight": (512, 256),
              "model.layers.0.mlp.down_proj.weight": (256, 512)}
     sd = {n: (torch.ones(s) if len(s) == 1 else 0.05 * torch.randn(s)).to(torch.bfloat16) for n, s in names.items()}
+    return P, cfg, sd
+
+
+def test_few_head_argmax_against_the_tile_kernel(lib):
+    """The lm head of at most sixteen rows through the engine's own entry: bf16 logits and tokens of a prompt and of decode steps against the kernels of larger batches."""
+    P, cfg, sd = small_model()
     with P.Engine(cfg) as e:
         e.load_state_dict(sd)
         e.set_debug(logits=True)
@@ -139,3 +144,34 @@ def test_few_head_argmax_against_the_tile_kernel(lib):
             for i in range(5):   # the lowest index of the largest bf16 value
                 assert int(np.flatnonzero(logits[i] == best[i])[0]) == int(toks[i])
             toks = e.decode_step(sids, toks)
+
+
+def test_decode_steps_whose_tokens_nobody_reads():
+    """Steps with and without their tokens in turn, a batch that changes between them, given tokens and the engine's own, a run of several steps: the same tokens as from
+    steps that are all read, one after the other."""
+    P, cfg, sd = small_model()
+    prompts = [list(range(3 + i, 9 + 2 * i)) for i in range(3)]
+    with P.Engine(cfg) as e:
+        e.load_state_dict(sd)
+        sids = [e.seq_create(48) for _ in prompts]
+        want = [list(map(int, e.prefill(sids, prompts)))]
+        for _ in range(14):
+            want.append(list(map(int, e.decode_step(sids))))
+    with P.Engine(cfg) as e:
+        e.load_state_dict(sd)
+        sids = [e.seq_create(48) for _ in prompts]
+        assert list(map(int, e.prefill(sids, prompts))) == want[0]
+        e.decode_step(sids, want_output=False)
+        e.decode_step(sids, want_output=False)
+        assert list(map(int, e.decode_step(sids))) == want[3]
+        assert list(map(int, e.decode_step(sids, want[3]))) == want[4]
+        e.decode_step(sids, want[4], want_output=False)
+        e.decode_step(sids, want[5], want_output=False)
+        assert list(map(int, e.decode_step(sids, want[6]))) == want[7]
+        for i in (2, 0, 1):                                   # each alone, then together again
+            assert int(e.decode_step([sids[i]], [want[7][i]])[0]) == want[8][i]
+        assert list(map(int, e.decode_step(sids, want[8]))) == want[9]
+        toks, _ = e.decode_run(sids, 3)
+        assert [list(map(int, r)) for r in np.asarray(toks)] == want[10:13]
+        assert list(map(int, e.decode_step(sids))) == want[13]
+        assert list(map(int, e.decode_step(sids))) == want[14]
