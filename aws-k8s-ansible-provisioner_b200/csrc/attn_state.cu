@@ -25,7 +25,7 @@
 //
 // The scan is sequential in time and parallel over (sequence, head, value column): a CTA owns up to 128 columns of one
 // head's state for one portion, eight lanes share four neighbouring columns and split the key channels (channel i * 8 + j
-// belongs to lane j), each lane keeps its channels of its columns in registers for the whole portion.  Tokens are staged through shared memory by asynchronous copies, a chunk ahead.  The arithmetic of a token does
+// belongs to lane j; the packed form, which all usual sizes take: see state_scan_packed_kernel), each lane keeps its channels of its columns in registers for the whole portion.  Tokens are staged through shared memory by asynchronous copies, a chunk ahead.  The arithmetic of a token does
 // not depend on where the portion was cut, so prefill, chunked prefill and token-by-token decoding give the same bits.
 //
 // Kernels:
