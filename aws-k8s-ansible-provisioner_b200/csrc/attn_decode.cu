@@ -67,9 +67,9 @@ struct AdPos {  // a position on the page line
 #endif
 template <int AD_WARPS, int AD_STAGES>
 __global__ void __launch_bounds__(AD_WARPS * 32, 1)
-attn_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
-                   const int32_t* __restrict__ block_table, int bt_stride, const int32_t* __restrict__ seq_lens,
-                   float* __restrict__ scratch, bf16* __restrict__ out, int B, int nq, int nkv, float scale, int early,
+attn_decode_kernel(const bf16* q, const bf16* k_pages, const bf16* v_pages,
+                   const int32_t* __restrict__ block_table, int bt_stride, const int32_t* seq_lens,
+                   float* scratch, bf16* __restrict__ out, int B, int nq, int nkv, float scale, int early,
                    int window, int tag, int chunk) {
   extern __shared__ __align__(128) uint8_t smem[];
   // Sliding-window attention (Phi-3, HF:models/phi3/modeling_phi3.py:265 sliding_window): a query at position

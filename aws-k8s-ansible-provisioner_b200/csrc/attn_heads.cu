@@ -81,11 +81,11 @@ __device__ __forceinline__ size_t swizzled_index(int slot, int kvh, int kv_heads
 // head at a time: all of them for prompt-sized steps (the token's cosines and sines are formed once), four when the step has few
 // tokens.  proj [T][ld] fp32: q (heads * dim) | k (kv_heads * dim) | v (kv_heads * vdim) | anything else.
 template <typename TC>
-__global__ void __launch_bounds__(128) heads_finish_kernel(const float* __restrict__ proj, int ld, HeadsGeom g, const float* __restrict__ bias,
-                                                           const float* __restrict__ conv_w, const float* __restrict__ ring,
+__global__ void __launch_bounds__(128) heads_finish_kernel(const float* proj, int ld, HeadsGeom g, const float* __restrict__ bias,
+                                                           const float* __restrict__ conv_w, const float* ring,
                                                            const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
-                                                           const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
-                                                           int vmix_mode, const float* __restrict__ vmix_lambda, float* __restrict__ v_first,
+                                                           const int32_t* positions, const int32_t* slots,
+                                                           int vmix_mode, const float* __restrict__ vmix_lambda, float* v_first,
                                                            float* __restrict__ q_out, TC* __restrict__ k_cache, TC* __restrict__ v_cache, int upc,
                                                            bf16* __restrict__ q_bf16) {
   extern __shared__ float sm[];
@@ -196,11 +196,11 @@ __device__ __forceinline__ void store4<bf16>(bf16* p, const float (&v)[4]) { *re
 // registers -- the form above reads every row and the taps (64 KB at 4096 channels) once per token and tap.
 // 3680 tokens of 32 heads of 128, bf16 caches: with the convolution and without it 196 us together, a number at a time -> 57 + 25 us.
 template <typename TC, int TAPS, int TPC>
-__global__ void __launch_bounds__(256) heads_finish_vec_kernel(const float* __restrict__ proj, int ld, HeadsGeom g, const float* __restrict__ bias,
-                                                               const float* __restrict__ conv_w, const float* __restrict__ ring,
+__global__ void __launch_bounds__(256) heads_finish_vec_kernel(const float* proj, int ld, HeadsGeom g, const float* __restrict__ bias,
+                                                               const float* __restrict__ conv_w, const float* ring,
                                                                const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
-                                                               const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
-                                                               int vmix_mode, const float* __restrict__ vmix_lambda, float* __restrict__ v_first,
+                                                               const int32_t* positions, const int32_t* slots,
+                                                               int vmix_mode, const float* __restrict__ vmix_lambda, float* v_first,
                                                                float* __restrict__ q_out, TC* __restrict__ k_cache, TC* __restrict__ v_cache, int upc,
                                                                bf16* __restrict__ q_bf16, int T) {
   constexpr int H = TAPS > 0 ? TAPS - 1 : 0;   // rows in front of the first token
@@ -319,8 +319,8 @@ __global__ void __launch_bounds__(256) heads_finish_vec_kernel(const float* __re
 // Whole-row norms: q (all heads at once) and k (all key heads at once) are each divided by the root mean square of the row and
 // multiplied by a gain per entry; v passes.  One CTA of NT threads per token (wide CTAs for steps of few tokens).
 template <typename TC, int NT>
-__global__ void __launch_bounds__(NT) heads_finish_rownorm_kernel(const float* __restrict__ proj, int ld, HeadsGeom g, const float* __restrict__ bias,
-                                                                   const float* __restrict__ qk_gain, const int32_t* __restrict__ slots,
+__global__ void __launch_bounds__(NT) heads_finish_rownorm_kernel(const float* proj, int ld, HeadsGeom g, const float* __restrict__ bias,
+                                                                   const float* __restrict__ qk_gain, const int32_t* slots,
                                                                    float* __restrict__ q_out, TC* __restrict__ k_cache, TC* __restrict__ v_cache,
                                                                    bf16* __restrict__ q_bf16) {
   __shared__ float red[2][NT / 32];
@@ -367,10 +367,10 @@ __global__ void __launch_bounds__(NT) heads_finish_rownorm_kernel(const float* _
   for (int i = threadIdx.x; i < nv; i += NT) stf(v_cache + (size_t)slot * nv + i, row[nq + nk + i] + (bias ? bias[nq + nk + i] : 0.f));
 }
 
-__global__ void __launch_bounds__(128) conv_tail_store_kernel(const float* __restrict__ proj, int ld, int C, int taps,
-                                                              const float* __restrict__ bias, float* __restrict__ ring,
+__global__ void __launch_bounds__(128) conv_tail_store_kernel(const float* proj, int ld, int C, int taps,
+                                                              const float* __restrict__ bias, float* ring,
                                                               const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_end,
-                                                              const int32_t* __restrict__ positions, const int32_t* __restrict__ slots) {
+                                                              const int32_t* positions, const int32_t* slots) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -384,9 +384,9 @@ __global__ void __launch_bounds__(128) conv_tail_store_kernel(const float* __res
 // Rotary positions from a table, interleaved or half-split pairs.  A CTA takes `upc` heads of one token (query heads, key heads, value heads; without
 // v in the projection the key heads write both caches), one warp per head at a time.
 template <typename TC>
-__global__ void __launch_bounds__(256) heads_finish_table_kernel(const float* __restrict__ proj, int ld, HeadsGeom g, const float* __restrict__ bias,
+__global__ void __launch_bounds__(256) heads_finish_table_kernel(const float* proj, int ld, HeadsGeom g, const float* __restrict__ bias,
                                                                  const float* __restrict__ table, int halves, int keys_as_values,
-                                                                 const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
+                                                                 const int32_t* positions, const int32_t* slots,
                                                                  float* __restrict__ q_out, bf16* __restrict__ q_bf16, TC* __restrict__ k_cache,
                                                                  TC* __restrict__ v_cache, int upc) {
   pdl_wait();
@@ -443,9 +443,9 @@ __device__ __forceinline__ void put4(bf16* p, const float* v) {
   *reinterpret_cast<uint2*>(p) = pk;
 }
 template <typename TC>
-__global__ void __launch_bounds__(256) heads_finish_table4_kernel(const float* __restrict__ proj, int ld, HeadsGeom g, const float* __restrict__ bias,
+__global__ void __launch_bounds__(256) heads_finish_table4_kernel(const float* proj, int ld, HeadsGeom g, const float* __restrict__ bias,
                                                                   const float* __restrict__ table, int halves, int keys_as_values,
-                                                                  const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
+                                                                  const int32_t* positions, const int32_t* slots,
                                                                   float* __restrict__ q_out, bf16* __restrict__ q_bf16, TC* __restrict__ k_cache,
                                                                   TC* __restrict__ v_cache) {
   pdl_wait();
@@ -557,11 +557,11 @@ template <bool VEC>
 __device__ __forceinline__ int ha_col(int n, int lane) { return VEC ? 64 * (n >> 1) + 2 * lane + (n & 1) : lane + 32 * n; }
 
 template <typename TC, typename TO, int NV, bool DECODE, bool VEC>
-__global__ void __launch_bounds__(HA_WARPS * 32) heads_attention_kernel(const float* __restrict__ q, const TC* __restrict__ k_cache,
-                                                                        const TC* __restrict__ v_cache, HeadsGeom g,
+__global__ void __launch_bounds__(HA_WARPS * 32) heads_attention_kernel(const float* q, const TC* k_cache,
+                                                                        const TC* v_cache, HeadsGeom g,
                                                                         const int32_t* __restrict__ block_table, int bt_stride, int block_size,
-                                                                        const PrefillTile* __restrict__ tiles, const int32_t* __restrict__ positions,
-                                                                        const int32_t* __restrict__ seq_lens, TO* __restrict__ out, int cross_cols) {
+                                                                        const PrefillTile* __restrict__ tiles, const int32_t* positions,
+                                                                        const int32_t* seq_lens, TO* __restrict__ out, int cross_cols) {
   extern __shared__ float sm[];
   pdl_wait();
   pdl_launch_dependents();
@@ -755,7 +755,7 @@ __device__ __forceinline__ float2 hf_split(hf_x2 v) {
 }
 
 template <int NV>
-__global__ void __launch_bounds__(256) heads_attention_f32_kernel(const float* __restrict__ q, const float* __restrict__ k_cache, const float* __restrict__ v_cache,
+__global__ void __launch_bounds__(256) heads_attention_f32_kernel(const float* q, const float* k_cache, const float* v_cache,
                                                                   HeadsGeom g, const int32_t* __restrict__ block_table, int bt_stride, int block_size,
                                                                   const PrefillTile* __restrict__ tiles, float* __restrict__ out, int cross_cols) {
   extern __shared__ __align__(16) float hf_sm[];
@@ -969,8 +969,8 @@ int launch_heads_attention_f32(const float* q, const float* k, const float* v, c
 
 // out[t][a][d] = sigmoid(gate[t][a]) * sum_b talk[a][b] * cross[t][b][kv(a) * vdim + d]
 template <typename TX>
-__global__ void __launch_bounds__(128) talk_gate_kernel(const float* __restrict__ cross, const float* __restrict__ talk,
-                                                        const float* __restrict__ gate, int gate_ld, TX* __restrict__ out, int heads,
+__global__ void __launch_bounds__(128) talk_gate_kernel(const float* cross, const float* __restrict__ talk,
+                                                        const float* gate, int gate_ld, TX* __restrict__ out, int heads,
                                                         int kv_heads, int vdim) {
   pdl_wait();
   pdl_launch_dependents();
@@ -1010,8 +1010,8 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t* r, uint32_t addr) {
 
 // HPC query heads of one key/value head per CTA (four warps each) share the staged key and value tiles.
 template <int KD, int NO, int HPC, typename TO>
-__global__ void __launch_bounds__(128 * HPC, 2) heads_attention_mma_kernel(const float* __restrict__ q, const bf16* __restrict__ k_cache,
-                                                                  const bf16* __restrict__ v_cache, HeadsGeom g,
+__global__ void __launch_bounds__(128 * HPC, 2) heads_attention_mma_kernel(const float* q, const bf16* k_cache,
+                                                                  const bf16* v_cache, HeadsGeom g,
                                                                   const int32_t* __restrict__ block_table, int bt_stride, int block_size,
                                                                   const PrefillTile* __restrict__ tiles, TO* __restrict__ out) {
   constexpr int D = KD * 16, DV = NO * 8, QS = D + HM_PAD, VS = DV + HM_PAD;
@@ -1286,9 +1286,9 @@ int launch_attention_t(const float* q, const void* k, const void* v, const Heads
 // at a time (query heads, then key heads, then value heads).  The token's cosines and
 // sines are formed once: [rot_dims/2] for q and k (angles divided by rot_factor), [vdim/2] for the values.
 template <typename TC>
-__global__ void __launch_bounds__(512) heads_finish_halves_kernel(const float* __restrict__ proj, int ld, HeadsGeom g, const float* __restrict__ q_gain,
-                                                                  const float* __restrict__ k_gain, const int32_t* __restrict__ positions,
-                                                                  const int32_t* __restrict__ slots, float* __restrict__ q_out, TC* __restrict__ k_cache,
+__global__ void __launch_bounds__(512) heads_finish_halves_kernel(const float* proj, int ld, HeadsGeom g, const float* __restrict__ q_gain,
+                                                                  const float* __restrict__ k_gain, const int32_t* positions,
+                                                                  const int32_t* slots, float* __restrict__ q_out, TC* __restrict__ k_cache,
                                                                   TC* __restrict__ v_cache) {
   extern __shared__ float cs[];   // qk: cos [half] | sin [half]; then v: cos [vhalf] | sin [vhalf]
   pdl_wait();
@@ -1597,7 +1597,7 @@ __global__ void __launch_bounds__(PX_THREADS, 1) heads_attention_premix_mma_kern
   for (int idx = tid; idx < H * PX_ROWS * (D / 4); idx += PX_THREADS) {
     const int c = idx % (D / 4), r = (idx / (D / 4)) % PX_ROWS, h = idx / ((D / 4) * PX_ROWS);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < ntok) v = __ldg(reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h) * D) + c);
+    if (r < ntok) v = reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h) * D)[c];
     __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
     uint2 pk;
     pk.x = *reinterpret_cast<unsigned*>(&lo);
@@ -1946,7 +1946,7 @@ __global__ void __launch_bounds__(PX_THREADS, NC == 8 ? 2 : 1) heads_attention_p
   for (int idx = tid; idx < HC * PX_ROWS * (D / 4); idx += PX_THREADS) {
     const int c = idx % (D / 4), r = (idx / (D / 4)) % PX_ROWS, h = idx / ((D / 4) * PX_ROWS);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < ntok) v = __ldg(reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h0 + h) * D) + c);
+    if (r < ntok) v = reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h0 + h) * D)[c];
     uint2 hi, lo;
     hi.x = pack_bf16x2(v.x, v.y);
     hi.y = pack_bf16x2(v.z, v.w);
@@ -2364,8 +2364,8 @@ __global__ void __launch_bounds__(1024) heads_attention_premix_decode_kernel(Pre
 // per head at a time (lane s holds split s: at most 32 splits; the CTA has as many warps as heads, up to sixteen, so that every head's
 // partial sums are in flight at once, eight splits a batch); the row's cosines and sines are formed once for all heads
 template <typename TX>
-__global__ void __launch_bounds__(512) premix_merge_kernel(const float* __restrict__ partial, int nsplit, HeadsGeom g, const int32_t* __restrict__ positions,
-                                                           const int32_t* __restrict__ seq_lens, TX* __restrict__ out) {
+__global__ void __launch_bounds__(512) premix_merge_kernel(const float* partial, int nsplit, HeadsGeom g, const int32_t* positions,
+                                                           const int32_t* seq_lens, TX* __restrict__ out) {
   extern __shared__ float sm[];   // [warps][vdim], then cos [vdim/2] | sin [vdim/2]
   pdl_wait();
   pdl_launch_dependents();

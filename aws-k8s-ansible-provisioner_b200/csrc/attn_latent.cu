@@ -64,9 +64,9 @@ __device__ __forceinline__ void pair_cos_sin(int pos, int i, int dims, float bas
 }
 
 template <typename TX, typename TC>
-__global__ void __launch_bounds__(128) latent_finish_kernel(const float* __restrict__ qd, int ld, LatentGeom g, int has_kv,
-                                                            const float* __restrict__ latent_gain, const int32_t* __restrict__ positions,
-                                                            const int32_t* __restrict__ slots, TX* __restrict__ q_nope,
+__global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int ld, LatentGeom g, int has_kv,
+                                                            const float* __restrict__ latent_gain, const int32_t* positions,
+                                                            const int32_t* slots, TX* __restrict__ q_nope,
                                                             float* __restrict__ q_rot, TC* __restrict__ cache) {
   extern __shared__ float cs[];  // [rot_dims / 2] cos | sin
   __shared__ float red[4];
@@ -131,9 +131,9 @@ __global__ void __launch_bounds__(128) latent_finish_kernel(const float* __restr
 // q_rank entries at column off_q, the other of kv_rank entries at off_c): both are RMS-normed with a plain gain; the first goes out as the
 // operand of the query up-projection, the second is the token's cache row.  One CTA of 128 threads per token.
 template <typename TX, typename TC>
-__global__ void __launch_bounds__(128) latent_pair_finish_kernel(const float* __restrict__ proj, int ld, int off_q, int q_rank, int off_c, int kv_rank,
+__global__ void __launch_bounds__(128) latent_pair_finish_kernel(const float* proj, int ld, int off_q, int q_rank, int off_c, int kv_rank,
                                                                  const float* __restrict__ gain_q, const float* __restrict__ gain_c, float eps,
-                                                                 const int32_t* __restrict__ slots, TX* __restrict__ xq, TC* __restrict__ cache) {
+                                                                 const int32_t* slots, TX* __restrict__ xq, TC* __restrict__ cache) {
   __shared__ float red[2][4];
   pdl_wait();
   pdl_launch_dependents();
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(128) latent_pair_finish_kernel(const float* __
 
 // One CTA per (page, context): 16 cached rows of `rank` numbers and `rot` more (multiples of 8).  The first go out side by side, the others (r_pages not null)
 // into rows of 64, zeros behind them, chunks swizzled as a K row's.
-__global__ void __launch_bounds__(256) latent_gather_kernel(const bf16* __restrict__ cache, int rank, int rot, const int32_t* __restrict__ block_table, int bt_stride,
+__global__ void __launch_bounds__(256) latent_gather_kernel(const bf16* cache, int rank, int rot, const int32_t* __restrict__ block_table, int bt_stride,
                                                             const LatentContext* __restrict__ ctx, bf16* __restrict__ rows, bf16* __restrict__ r_pages) {
   pdl_wait();
   pdl_launch_dependents();
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) latent_gather_kernel(const bf16* __restri
 }
 
 // One CTA per (page, head): the head's 16 key rows and 16 value rows, 128 wide, into the page layout of the GQA kernels.
-__global__ void __launch_bounds__(256) latent_store_pages_kernel(const bf16* __restrict__ kv, int heads, bf16* __restrict__ k_pages, bf16* __restrict__ v_pages) {
+__global__ void __launch_bounds__(256) latent_store_pages_kernel(const bf16* kv, int heads, bf16* __restrict__ k_pages, bf16* __restrict__ v_pages) {
   pdl_wait();
   pdl_launch_dependents();
   const int pg = blockIdx.x, a = blockIdx.y, r = threadIdx.x >> 4, c = threadIdx.x & 15;
@@ -199,11 +199,11 @@ constexpr int LA_WARPS = 8, LA_KEYS = 32;
 
 // NR = ceil(kv_rank / 32): latent dims per lane
 template <typename TC, typename TX, int NR>
-__global__ void __launch_bounds__(LA_WARPS * 32) latent_attention_kernel(const float* __restrict__ q_abs, const float* __restrict__ q_rot,
-                                                                         const TC* __restrict__ cache, LatentGeom g,
+__global__ void __launch_bounds__(LA_WARPS * 32) latent_attention_kernel(const float* q_abs, const float* q_rot,
+                                                                         const TC* cache, LatentGeom g,
                                                                          const int32_t* __restrict__ block_table, int bt_stride, int block_size,
-                                                                         const PrefillTile* __restrict__ tiles, const int32_t* __restrict__ positions,
-                                                                         const int32_t* __restrict__ seq_lens, const float* __restrict__ sink,
+                                                                         const PrefillTile* __restrict__ tiles, const int32_t* positions,
+                                                                         const int32_t* seq_lens, const float* __restrict__ sink,
                                                                          TX* __restrict__ out_lat) {
   extern __shared__ float sm[];
   pdl_wait();
@@ -362,8 +362,8 @@ __global__ void __launch_bounds__(MA_THREADS, 1) latent_attention_mma_kernel(Mma
       if (row < total) {
         const int tok = row / g.heads, head = row - tok * g.heads;
         const size_t base = (size_t)(q_row0 + tok) * g.heads + head;
-        v = c < qc ? __ldg(reinterpret_cast<const float4*>(a.q_abs + base * R) + c)
-                   : __ldg(reinterpret_cast<const float4*>(a.q_rot + base * g.rot_dim) + (c - qc));
+        v = c < qc ? reinterpret_cast<const float4*>(a.q_abs + base * R)[c]
+                   : reinterpret_cast<const float4*>(a.q_rot + base * g.rot_dim)[c - qc];
       }
       __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
       uint2 pk;
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(MA_THREADS, 1) latent_attention_mma_kernel(Mma
         const int j = idx / cpr, c = idx - j * cpr;
         const int kr = key_row[j];
         uint4 v = make_uint4(0, 0, 0, 0);
-        if (kr >= 0) v = ld_stream(a.cache + (size_t)kr * D + c * 8);
+        if (kr >= 0) v = ld_stream_written(a.cache + (size_t)kr * D + c * 8);
         *reinterpret_cast<uint4*>(Ks + j * DP + c * 8) = v;
       }
     } else {
@@ -589,8 +589,8 @@ __global__ void __launch_bounds__(MA_THREADS, 1) latent_attention_mma_kernel(Mma
 }
 
 // folds the splits of every (token, head) row and the sink into the output; one CTA per row, thread d owns latent dims d, d + 128, ...
-__global__ void __launch_bounds__(128) latent_merge_kernel(const float* __restrict__ partial, int nsplit, int R, int heads,
-                                                           const int32_t* __restrict__ seq_lens, const float* __restrict__ sink,
+__global__ void __launch_bounds__(128) latent_merge_kernel(const float* partial, int nsplit, int R, int heads,
+                                                           const int32_t* seq_lens, const float* __restrict__ sink,
                                                            bf16* __restrict__ out_lat, int nrows) {
   __shared__ float w_s[32];
   __shared__ float inv_s;

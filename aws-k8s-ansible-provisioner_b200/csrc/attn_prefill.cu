@@ -44,7 +44,7 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, uint32_t b
 }
 
 __global__ void __launch_bounds__(128)
-attn_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pages, const bf16* __restrict__ v_pages,
+attn_prefill_kernel(const bf16* q, const bf16* k_pages, const bf16* v_pages,
                     const int32_t* __restrict__ block_table, int bt_stride, const PrefillTile* __restrict__ tiles,
                     bf16* __restrict__ out, int nq, int nkv, int block_size, float scale_log2, int window) {
   extern __shared__ __align__(128) uint8_t smem[];

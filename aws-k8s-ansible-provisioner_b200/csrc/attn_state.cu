@@ -79,7 +79,7 @@ __device__ __forceinline__ float lowrank_value(float z, int mode, float rate) {
 // time) and applies it to every token of the tile.  lr [T][ld] fp32 (rank numbers per token at column lr_off), staged in shared memory.
 constexpr int LR_TOKENS = 8;
 template <int NT>
-__global__ void __launch_bounds__(NT) lowrank_act_kernel(const float* __restrict__ lr, int ld, int lr_off, int rank, const float* __restrict__ w2,
+__global__ void __launch_bounds__(NT) lowrank_act_kernel(const float* lr, int ld, int lr_off, int rank, const float* __restrict__ w2,
                                                           const float* __restrict__ bias, const float* __restrict__ rate_log, float rate,
                                                           int per_head, int mode, float* __restrict__ out, int C, int T) {
   extern __shared__ __align__(16) float lrs[];   // [LR_TOKENS][rank]
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(NT) lowrank_act_kernel(const float* __restrict
 // tokens' values are staged once (tanh applied there), then the CTA walks over its share of the channel tiles.  A channel's sum runs over the rank in
 // order, as above.
 constexpr int LT_T = 64, LT_C = 128, LT_K = 32, LT_MAX_RANK = 128;
-__global__ void __launch_bounds__(256) lowrank_act_tile_kernel(const float* __restrict__ lr, int ld, int lr_off, int rank, const float* __restrict__ w2,
+__global__ void __launch_bounds__(256) lowrank_act_tile_kernel(const float* lr, int ld, int lr_off, int rank, const float* __restrict__ w2,
                                                                const float* __restrict__ bias, const float* __restrict__ rate_log, float rate, int per_head,
                                                                int mode, float* __restrict__ out, int C, int T, int tiles_per_cta) {
   extern __shared__ __align__(16) float lt_smem[];
@@ -239,10 +239,10 @@ __global__ void __launch_bounds__(256) lowrank_act_tile_kernel(const float* __re
 // proj [T][ld] fp32 = q (kv_heads*dim) | k (kv_heads*dim) | v (heads*vdim) | beta logits (heads) | ...; out [T][C] = the finished q | k | v,
 // beta_out [T][heads]; with a_log one decay per head, exp(-exp(a_log) softplus(logit + dt_bias)), from the logits behind beta's.
 template <int TAPS>   // 0: any number of taps
-__global__ void __launch_bounds__(256) conv_unit_finish_kernel(const float* __restrict__ proj, int ld, StateGeom g, int taps_any,
-                                                               const float* __restrict__ conv_w, const float* __restrict__ ring,
+__global__ void __launch_bounds__(256) conv_unit_finish_kernel(const float* proj, int ld, StateGeom g, int taps_any,
+                                                               const float* __restrict__ conv_w, const float* ring,
                                                                const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
-                                                               const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
+                                                               const int32_t* positions, const int32_t* slots,
                                                                float unit_eps, float* __restrict__ out, float* __restrict__ beta_out, int upc,
                                                                const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                                                                float* __restrict__ decay_out, float* __restrict__ ring_store) {
@@ -306,10 +306,10 @@ __global__ void __launch_bounds__(256) conv_unit_finish_kernel(const float* __re
 // their unit vectors (a warp per row).
 constexpr int CR_ROWS = 16;
 template <int TAPS>
-__global__ void __launch_bounds__(128) conv_unit_rows_kernel(const float* __restrict__ proj, int ld, StateGeom g, const float* __restrict__ conv_w,
-                                                             const float* __restrict__ ring, const int32_t* __restrict__ row_seq,
-                                                             const int32_t* __restrict__ row_first, const int32_t* __restrict__ positions,
-                                                             const int32_t* __restrict__ slots, float unit_eps, float* __restrict__ out,
+__global__ void __launch_bounds__(128) conv_unit_rows_kernel(const float* proj, int ld, StateGeom g, const float* __restrict__ conv_w,
+                                                             const float* ring, const int32_t* __restrict__ row_seq,
+                                                             const int32_t* __restrict__ row_first, const int32_t* positions,
+                                                             const int32_t* slots, float unit_eps, float* __restrict__ out,
                                                              float* __restrict__ beta_out, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
                                                              float* __restrict__ decay_out, int T) {
   extern __shared__ float tile[];   // [CR_ROWS][dim] of a query or key head
@@ -391,11 +391,11 @@ __global__ void __launch_bounds__(128) conv_unit_rows_kernel(const float* __rest
 // A thread owns a channel of x | B | C and walks down `rows` neighbouring token rows with the last inputs in registers (rows = 1 in short steps).  proj
 // [T][ld] fp32 = x | B | C | step logits.  The first CTA column also forms the step sizes and decays.
 template <int TAPS>   // 0: any number of taps
-__global__ void __launch_bounds__(128) conv_act_kernel(const float* __restrict__ proj, int ld, int C, int heads, int taps_any, const float* __restrict__ conv_w,
+__global__ void __launch_bounds__(128) conv_act_kernel(const float* proj, int ld, int C, int heads, int taps_any, const float* __restrict__ conv_w,
                                                        const float* __restrict__ conv_b, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
-                                                       const float* __restrict__ ring, float* __restrict__ ring_store, const int32_t* __restrict__ row_seq,
-                                                       const int32_t* __restrict__ row_first, const int32_t* __restrict__ positions,
-                                                       const int32_t* __restrict__ slots, float* __restrict__ out, float* __restrict__ step,
+                                                       const float* ring, float* __restrict__ ring_store, const int32_t* __restrict__ row_seq,
+                                                       const int32_t* __restrict__ row_first, const int32_t* positions,
+                                                       const int32_t* slots, float* __restrict__ out, float* __restrict__ step,
                                                        float* __restrict__ decay, int rows, int T) {
   const int t0 = blockIdx.x * rows, tn = min(rows, T - t0), c = blockIdx.y * 128 + threadIdx.x;
   const int taps = TAPS > 0 ? TAPS : taps_any;
@@ -473,10 +473,10 @@ __global__ void __launch_bounds__(128) conv_act_kernel(const float* __restrict__
 
 // The same with four neighbouring channels per thread (prompt-sized steps; channels in multiples of four, rows on 16-byte boundaries).
 template <int TAPS>
-__global__ void __launch_bounds__(128) conv_act4_kernel(const float* __restrict__ proj, int ld, int C, int heads, const float* __restrict__ conv_w,
+__global__ void __launch_bounds__(128) conv_act4_kernel(const float* proj, int ld, int C, int heads, const float* __restrict__ conv_w,
                                                         const float* __restrict__ conv_b, const float* __restrict__ a_log, const float* __restrict__ dt_bias,
-                                                        const float* __restrict__ ring, const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
-                                                        const int32_t* __restrict__ positions, const int32_t* __restrict__ slots, float* __restrict__ out,
+                                                        const float* ring, const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
+                                                        const int32_t* positions, const int32_t* slots, float* __restrict__ out,
                                                         float* __restrict__ step, float* __restrict__ decay, int rows, int T) {
   const int t0 = blockIdx.x * rows, tn = min(rows, T - t0), c = (blockIdx.y * 128 + threadIdx.x) * 4;
   float4 w[TAPS], bias = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -543,9 +543,9 @@ __global__ void __launch_bounds__(128) conv_act4_kernel(const float* __restrict_
 // A CTA takes 32 tokens and RS_CHANNELS channels: the few rows to store are a chain of load and store for whoever walks them (16 single-token portions of
 // 6144 channels in one CTA: 45 us; 16 CTAs: 5).
 constexpr int RS_CHANNELS = 512;
-__global__ void __launch_bounds__(128) conv_ring_store_kernel(const float* __restrict__ proj, int ld, int C, int taps, float* __restrict__ ring,
+__global__ void __launch_bounds__(128) conv_ring_store_kernel(const float* proj, int ld, int C, int taps, float* ring,
                                                               const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_end,
-                                                              const int32_t* __restrict__ positions, const int32_t* __restrict__ slots, int T) {
+                                                              const int32_t* positions, const int32_t* slots, int T) {
   pdl_wait();
   pdl_launch_dependents();
   const int mine = blockIdx.x * 32 + (threadIdx.x & 31), at = mine < T ? mine : 0;
@@ -577,12 +577,12 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // eight lanes over the banks) and are read sixteen bytes at a time.  Tokens arrive by asynchronous copies, the chunk after the one being
 // worked on always in flight.  q is scaled at the read-out (S^T (c q) = c S^T q).
 template <int DPT, int NC, int RULE>
-__global__ void __launch_bounds__(256) state_scan_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk,
-                                                         const float* __restrict__ v, int ldv, const float* __restrict__ decay,
-                                                         const float* __restrict__ beta, StateGeom g, float qscale, float* __restrict__ state,
+__global__ void __launch_bounds__(256) state_scan_kernel(const float* q, int ldq, const float* k, int ldk,
+                                                         const float* v, int ldv, const float* decay,
+                                                         const float* beta, StateGeom g, float qscale, float* state,
                                                          const int32_t* __restrict__ last_rows, const int32_t* __restrict__ row_seq,
                                                          const int32_t* __restrict__ row_first, const int32_t* __restrict__ row_end,
-                                                         const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
+                                                         const int32_t* positions, const int32_t* slots,
                                                          float* __restrict__ out, int cols) {
   constexpr int LS = DPT + 4;               // words of one lane's channels in a staged row
   constexpr int RS = LS * SC_LANES;         // words of a staged row
@@ -877,10 +877,10 @@ struct ScanTile {
 };
 template <int DPT, int RULE, int NC>   // channels per lane: 4 or 8 (dim <= 16 DPT)
 __global__ void __launch_bounds__(ScanTile<NC>::THREADS, ScanTile<NC>::PER_SM)
-state_scan_packed_kernel(const float* __restrict__ q, int ldq, const float* __restrict__ k, int ldk, const float* __restrict__ v, int ldv,
-                         const float* __restrict__ decay, const float* __restrict__ beta, StateGeom g, float qscale, float* __restrict__ state,
+state_scan_packed_kernel(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv,
+                         const float* decay, const float* beta, StateGeom g, float qscale, float* state,
                          const int32_t* __restrict__ last_rows, const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
-                         const int32_t* __restrict__ row_end, const int32_t* __restrict__ positions, const int32_t* __restrict__ slots,
+                         const int32_t* __restrict__ row_end, const int32_t* positions, const int32_t* slots,
                          float* __restrict__ out) {
   constexpr int NT = ScanTile<NC>::THREADS, COLS = ScanTile<NC>::COLS, L = ScanTile<NC>::LANES, CH = SC_CHUNK, DP = DPT * L, HP = DPT / 2, TB = L / NC;
   constexpr int PIECES = DP / 4, RSTEP = NT / PIECES, VP = COLS / 4;   // 16-byte pieces of a row; rows that the CTA copies at a time
@@ -1207,8 +1207,8 @@ state_scan_packed_kernel(const float* __restrict__ q, int ldq, const float* __re
 
 // One warp per (token, head): y = o / sqrt(mean(o^2) + eps) * gain * gate, gate = silu(gate_in) or gate_in as it is.
 template <typename TX>
-__global__ void __launch_bounds__(128) state_out_gate_kernel(const float* __restrict__ o, const float* __restrict__ gain,
-                                                             const float* __restrict__ gate, int gate_ld, int gate_silu, TX* __restrict__ out,
+__global__ void __launch_bounds__(128) state_out_gate_kernel(const float* o, const float* __restrict__ gain,
+                                                             const float* gate, int gate_ld, int gate_silu, TX* __restrict__ out,
                                                              int heads, int vdim, float eps, int T, int gain_per_head, float scale, int out_ld) {
   pdl_wait();
   pdl_launch_dependents();
@@ -1252,7 +1252,7 @@ __global__ void __launch_bounds__(128) state_out_gate_kernel(const float* __rest
 // One CTA of NT threads per (token, part): v = o * silu(gate) is formed once and kept in registers (R groups of four numbers a thread) or, for other
 // sizes (R = 0), in shared memory.
 template <typename TX, int NT, int R>
-__global__ void __launch_bounds__(NT) gate_part_norm_kernel(const float* __restrict__ o, const float* __restrict__ gate, int gate_ld,
+__global__ void __launch_bounds__(NT) gate_part_norm_kernel(const float* o, const float* gate, int gate_ld,
                                                             const float* __restrict__ gain, float scale, TX* __restrict__ out, int out_ld, int N, int part,
                                                             float eps) {
   extern __shared__ float vrow[];
@@ -1341,8 +1341,8 @@ int gate_part_norm_typed(const float* o, const float* gate, int gate_ld, const f
 
 // The same for heads of 4 L numbers (L = 4 .. 32 lanes per head): a lane keeps its four numbers in registers.
 template <typename TX, int L>
-__global__ void __launch_bounds__(256) state_out_gate_lanes_kernel(const float* __restrict__ o, const float* __restrict__ gain,
-                                                                   const float* __restrict__ gate, int gate_ld, int gate_silu, TX* __restrict__ out,
+__global__ void __launch_bounds__(256) state_out_gate_lanes_kernel(const float* o, const float* __restrict__ gain,
+                                                                   const float* gate, int gate_ld, int gate_silu, TX* __restrict__ out,
                                                                    int heads, float eps, int T, int gain_per_head, float scale, int out_ld) {
   constexpr int V = 4 * L;
   pdl_wait();

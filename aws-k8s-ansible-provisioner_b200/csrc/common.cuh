@@ -64,7 +64,7 @@ __device__ __forceinline__ float warp_max(float v) {
   return v;
 }
 
-// streaming 128-bit load that does not allocate in L1 (weights / KV are read once per step)
+// streaming 128-bit load of constants that does not allocate in L1 (weights are read once per step)
 __device__ __forceinline__ uint4 ld_stream(const void* p) {
   uint4 r;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -73,18 +73,31 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
   return r;
 }
 
+// the same for what a kernel of the step wrote (cache rows)
+__device__ __forceinline__ uint4 ld_stream_written(const void* p) {
+  uint4 r;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  return r;
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
 // ---------------------------------------------------------------------------------------
-// Programmatic dependent launch (PDL): every kernel is launched with the programmatic stream
-// serialization attribute.  Discipline used throughout: a kernel calls pdl_wait() before it touches
-// anything its IMMEDIATE predecessor wrote, and only then pdl_launch_dependents().  So when a kernel
-// starts, its predecessor has already passed its own wait, i.e. everything older than the immediate
-// predecessor is complete and visible: code before pdl_wait() may read constants (weights, tables)
-// AND anything produced two or more kernels earlier (block tables, sequence lengths, the residual
-// stream, all K/V pages except the slots the previous kernel is writing).
+// Programmatic dependent launch (PDL): every kernel is launched with the programmatic stream serialization attribute, so it may start while
+// the kernel in front still runs.
+//   * What another kernel of the step writes is read behind pdl_wait().  When that returns, every kernel in front is complete and visible:
+//     the one right before, and, since each of them waits before it ends, all older ones.
+//   * It is read through plain pointers.  A load through a __restrict__ pointer may be moved across the wait (nothing that the compiler sees
+//     writes there), and a read-only load (const __restrict__, __ldg, ld.global.nc) asks for data that nobody writes while the kernel runs.  So
+//     __restrict__ is for weights, tables, what the host uploads before the step, and outputs that the kernel does not read.
+//   * In front of the wait a kernel reads weights, tables and uploads.  It may read older results too (attn_decode.cu, attn_latent_decode.cu,
+//     add_rmsnorm_kernel's residual stream, positions and slots in qknorm_rope_kv_kernel) only where the kernel in front releases it behind its OWN
+//     wait: then everything older than that kernel is complete.  add_rmsnorm_kernel, silu_mul_kernel and the kernels of gemm_few.cu release at
+//     their start.  Behind a row of those nothing is complete but what was when the first of them started: few_attn_kernel reads lengths,
+//     positions and the pages of earlier steps there, which decode_advance_kernel and the step before it wrote, and the embedding kernel between
+//     them releases behind its wait.
 // ---------------------------------------------------------------------------------------
 // A kernel's idle lanes ask for the NEXT kernel's weights to be brought into L2 (cp.async.bulk.prefetch.L2, 4 KB per
 // request): the next kernel's TMA stream then starts from L2 instead of HBM even when its CTAs could not become

@@ -11,7 +11,7 @@ B2_STEP_TRACE_DEFINE(step_trace_set_elementwise)
 // ---------------------------------------------------------------------------------------
 // a1: nn.Embedding lookup, HF:models/qwen3/modeling_qwen3.py:363,392
 // ---------------------------------------------------------------------------------------
-__global__ void embed_kernel(const int32_t* __restrict__ ids, const bf16* __restrict__ table, bf16* __restrict__ h,
+__global__ void embed_kernel(const int32_t* ids, const bf16* __restrict__ table, bf16* h,
                              int H, int vocab, unsigned long long* __restrict__ zero_buf, int nzero) {
   B2_STAMP_BEGIN();
   pdl_wait();
@@ -38,7 +38,7 @@ int launch_embed(const int32_t* ids, const bf16* table, bf16* h, int T, int H, i
   return 0;
 }
 
-__global__ void gather_rows_kernel(const bf16* __restrict__ src, const int32_t* __restrict__ rows, bf16* __restrict__ dst,
+__global__ void gather_rows_kernel(const bf16* src, const int32_t* __restrict__ rows, bf16* __restrict__ dst,
                                    int H) {
   pdl_wait();
   pdl_launch_dependents();
@@ -61,7 +61,7 @@ int launch_gather_rows(const bf16* src, const int32_t* rows, bf16* dst, int n, i
 // One CTA per token, H/8 threads, one 16-byte vector per thread.
 // ---------------------------------------------------------------------------------------
 template <int MODE>  // 0: no delta, 1: bf16 delta, 2: fp32 partials
-__global__ void add_rmsnorm_kernel(bf16* __restrict__ h, const void* __restrict__ delta, int nsplit, size_t split_stride,
+__global__ void add_rmsnorm_kernel(bf16* h, const void* delta, int nsplit, size_t split_stride,
                                    const bf16* __restrict__ w, bf16* __restrict__ x, int H, float eps, int early, int tag) {
   __shared__ float red[32];
   B2_STAMP_BEGIN();
@@ -69,8 +69,8 @@ __global__ void add_rmsnorm_kernel(bf16* __restrict__ h, const void* __restrict_
   // start the TMA stream of its weight tiles (constants).  Releasing it at the very start of this kernel -- before
   // this kernel's own wait -- gives that stream the whole hand-off + norm time instead of the ~1.5 us it had, which
   // was less than a 64-96 KB weight slice takes to arrive (the projection then issued its last MMA ~2 us after its
-  // wait; tools/step_timeline.py).  The projection triggers ITS dependents only after its own wait, so the
-  // discipline stated in common.cuh still holds for every other kernel.
+  // wait).  The kernels of gemm_tc.cu, gemm_pair.cu and gemm_resid.cu release THEIR dependents behind their own wait; gemm_few.cu's release
+  // at their start, and what stands behind those reads nothing of a step's kernels in front of its wait (common.cuh).
   if (early & 2) pdl_launch_dependents();
   if (!(early & 1)) pdl_wait();
   const int t = blockIdx.x;
@@ -171,10 +171,10 @@ int launch_add_rmsnorm(bf16* h, ActIn delta, const bf16* w, bf16* x, int T, int 
 // projections and a pre-scaled query: v = bf16(partials + bias), q = bf16(v * q_mul).
 // ---------------------------------------------------------------------------------------
 template <bool F32IN>
-__global__ void qknorm_rope_kv_kernel(const void* __restrict__ qkv, int nsplit, size_t split_stride,
+__global__ void qknorm_rope_kv_kernel(const void* qkv, int nsplit, size_t split_stride,
                                       const bf16* __restrict__ qw, const bf16* __restrict__ kw,
-                                      const bf16* __restrict__ cos_sin, const int32_t* __restrict__ positions,
-                                      const int32_t* __restrict__ slots, bf16* __restrict__ q_out,
+                                      const bf16* __restrict__ cos_sin, const int32_t* positions,
+                                      const int32_t* slots, bf16* __restrict__ q_out,
                                       bf16* __restrict__ k_pages, bf16* __restrict__ v_pages, int T, int nq, int nkv,
                                       int block_size, float eps, int early, int rot_quads, const bf16* __restrict__ bias, float q_mul, int tag) {
   constexpr int HD = 128;
@@ -287,9 +287,9 @@ __global__ void qknorm_rope_kv_kernel(const void* __restrict__ qkv, int nsplit, 
 // measured 82 us for 8192 tokens, 134 MB moved).  Here a warp takes FOUR consecutive heads of one token: position,
 // slot and the cos/sin row are fetched once, the four rows are requested together, then processed one by one.
 // bf16 input only (a prefill-sized projection is never split along K); needs (nq + 2 nkv) % 4 == 0.
-__global__ void qknorm_rope_kv_prefill_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
-                                              const bf16* __restrict__ cos_sin, const int32_t* __restrict__ positions,
-                                              const int32_t* __restrict__ slots, bf16* __restrict__ q_out,
+__global__ void qknorm_rope_kv_prefill_kernel(const bf16* qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
+                                              const bf16* __restrict__ cos_sin, const int32_t* positions,
+                                              const int32_t* slots, bf16* __restrict__ q_out,
                                               bf16* __restrict__ k_pages, bf16* __restrict__ v_pages, int T, int nq, int nkv,
                                               int block_size, float eps, int rot_quads) {
   constexpr int HD = 128;
@@ -364,9 +364,9 @@ __global__ void qknorm_rope_kv_prefill_kernel(const bf16* __restrict__ qkv, cons
 // at a third of the HBM rate (61 us for 8192 tokens x 32 heads); this one is bound by the 134 MB it moves.
 // A half-warp walks four heads of one token; rot16 = rotary_dim / 16 lanes hold each half of the rotated span.
 __global__ void __launch_bounds__(128)
-qknorm_rope_kv_prefill16_kernel(const bf16* __restrict__ qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
-                                const bf16* __restrict__ cos_sin, const int32_t* __restrict__ positions,
-                                const int32_t* __restrict__ slots, bf16* __restrict__ q_out, bf16* __restrict__ k_pages,
+qknorm_rope_kv_prefill16_kernel(const bf16* qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw,
+                                const bf16* __restrict__ cos_sin, const int32_t* positions,
+                                const int32_t* slots, bf16* __restrict__ q_out, bf16* __restrict__ k_pages,
                                 bf16* __restrict__ v_pages, int T, int nq, int nkv, int block_size, float eps, int rot16) {
   constexpr int HD = 128;
   pdl_wait();
@@ -490,7 +490,7 @@ int launch_qknorm_rope_kv(ActIn qkv, const bf16* qw, const bf16* kw, const bf16*
 // outputs of their Linear layers; silu is evaluated in fp32 as x / (1 + exp(-x)).
 // ---------------------------------------------------------------------------------------
 template <bool F32IN>
-__global__ void silu_mul_kernel(const void* __restrict__ gu, int nsplit, size_t split_stride, bf16* __restrict__ act,
+__global__ void silu_mul_kernel(const void* gu, int nsplit, size_t split_stride, bf16* __restrict__ act,
                                 int T, int I, int tag, int trigger_early) {
   B2_STAMP_BEGIN();
   if (trigger_early) pdl_launch_dependents();  // the down projection starts streaming its weights (see add_rmsnorm_kernel)
@@ -575,7 +575,7 @@ __device__ __forceinline__ unsigned long long argmax_pack(float v, int idx) {
   return ((unsigned long long)key << 32) | (unsigned long long)(0xffffffffu - (uint32_t)idx);
 }
 
-__global__ void argmax_rows_kernel(const bf16* __restrict__ logits, int32_t* __restrict__ out, int V) {
+__global__ void argmax_rows_kernel(const bf16* logits, int32_t* __restrict__ out, int V) {
   __shared__ unsigned long long red[32];
   pdl_wait();
   pdl_launch_dependents();
@@ -606,7 +606,7 @@ int launch_argmax_rows(const bf16* logits, int32_t* out, int T, int V, cudaStrea
   return 0;
 }
 
-__global__ void argmax_finalize_kernel(const unsigned long long* __restrict__ packed, int32_t* __restrict__ out, int T) {
+__global__ void argmax_finalize_kernel(const unsigned long long* packed, int32_t* __restrict__ out, int T) {
   pdl_wait();
   pdl_launch_dependents();
   int t = blockIdx.x * blockDim.x + threadIdx.x;

@@ -11,8 +11,8 @@ namespace b2 {
 // OPTDecoder.forward, HF:...:363-368: h = embed_tokens[id] + embed_positions[position + 2]
 // (OPTLearnedPositionalEmbedding, HF:...:45-70: the table is offset by 2), one bf16 add.
 // ---------------------------------------------------------------------------------------
-__global__ void embed_pos_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ positions,
-                                 const bf16* __restrict__ table, const bf16* __restrict__ pos_table, bf16* __restrict__ h, int H,
+__global__ void embed_pos_kernel(const int32_t* ids, const int32_t* positions,
+                                 const bf16* __restrict__ table, const bf16* __restrict__ pos_table, bf16* h, int H,
                                  int vocab, int pos_rows, unsigned long long* __restrict__ zero_buf, int nzero) {
   pdl_wait();
   pdl_launch_dependents();
@@ -55,7 +55,7 @@ int launch_embed_pos(const int32_t* ids, const int32_t* positions, const bf16* t
 // One CTA per token, H/8 threads, one 16-byte vector per thread.
 // ---------------------------------------------------------------------------------------
 template <bool HAS_DELTA>
-__global__ void add_layernorm_kernel(bf16* __restrict__ h, const float* __restrict__ delta, int nsplit, size_t split_stride,
+__global__ void add_layernorm_kernel(bf16* h, const float* delta, int nsplit, size_t split_stride,
                                      const bf16* __restrict__ delta_bias, const bf16* __restrict__ w, const bf16* __restrict__ b,
                                      bf16* __restrict__ x, int H, float eps) {
   __shared__ float red[2][32];
@@ -127,7 +127,7 @@ int launch_add_layernorm(bf16* h, ActIn delta, const bf16* delta_bias, const bf1
 // ---------------------------------------------------------------------------------------
 // fc1 + activation, HF:...:241-242: act = bf16(relu(bf16(sum of partials + bias)))
 // ---------------------------------------------------------------------------------------
-__global__ void bias_relu_kernel(const float* __restrict__ part, int nsplit, size_t split_stride, const bf16* __restrict__ bias,
+__global__ void bias_relu_kernel(const float* part, int nsplit, size_t split_stride, const bf16* __restrict__ bias,
                                  bf16* __restrict__ act, int T, int I) {
   const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;  // vector of 8 over [T][I]
   const size_t nvec = (size_t)T * I / 8;

@@ -2516,7 +2516,7 @@ int lm_head_and_argmax(b2_engine* e, int nlast, const bf16* xl, XBuf xb) {
   return 0;
 }
 
-__global__ void publish_tokens_kernel(const int32_t* __restrict__ out_tokens, int32_t* __restrict__ next_in,
+__global__ void publish_tokens_kernel(const int32_t* out_tokens, int32_t* __restrict__ next_in,
                                       int32_t* __restrict__ log, int32_t* step, int B, int log_cap_steps, int stride, volatile int32_t* host) {
   pdl_wait();
   pdl_launch_dependents();

@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(32 * NW) gemm_any_rows_mma_kernel(AnyGemm g) {
         const bool in = k + c * 8 < K;
 #pragma unroll
         for (int t = 0; t < NT; ++t)
-          tv[u][t] = (in && tok[t] != nullptr) ? __ldg(reinterpret_cast<const uint4*>(tok[t] + k)) : make_uint4(0, 0, 0, 0);
+          tv[u][t] = (in && tok[t] != nullptr) ? *reinterpret_cast<const uint4*>(tok[t] + k) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -754,7 +754,7 @@ int launch_rows_mma(const AnyGemm& g, int groups, int batch, cudaStream_t s) {
 }
 
 // One CTA: tiles of the ragged groups.  group_offsets [G + 1] -> (tile_group, tile_row0, n_tiles).
-__global__ void ragged_tiles_kernel(const int* __restrict__ group_offsets, int G, int* __restrict__ tile_group, int* __restrict__ tile_row0,
+__global__ void ragged_tiles_kernel(const int* group_offsets, int G, int* __restrict__ tile_group, int* __restrict__ tile_row0,
                                     int* __restrict__ n_tiles, int cap) {
   pdl_wait();
   pdl_launch_dependents();

@@ -269,8 +269,8 @@ struct FaRecord { float o[2][FA_HD], m[2], l[2]; };   // one share: unnormalised
 // grid (8, kv heads, sequences), clusters of eight along x; qkv: bf16 rows of (nq + 2 nkv) * 128
 __global__ void __launch_bounds__(32 * FA_WARPS) __cluster_dims__(FA_CTAS, 1, 1)
 few_attn_kernel(const bf16* qkv, const bf16* __restrict__ qw, const bf16* __restrict__ kw, const bf16* __restrict__ cos_sin,
-                const int32_t* __restrict__ positions, const int32_t* __restrict__ slots, bf16* k_pages, bf16* v_pages,
-                const int32_t* __restrict__ block_table, int bt_stride, const int32_t* __restrict__ seq_lens, bf16* out, int nq, int nkv, float eps,
+                const int32_t* positions, const int32_t* slots, bf16* k_pages, bf16* v_pages,
+                const int32_t* __restrict__ block_table, int bt_stride, const int32_t* seq_lens, bf16* out, int nq, int nkv, float eps,
                 float scale) {
   __shared__ __align__(16) float qs[2][FA_HD];            // the two query heads, scaled
   __shared__ __align__(16) bf16 kv_new[2][FA_HD];         // the new token's key and value

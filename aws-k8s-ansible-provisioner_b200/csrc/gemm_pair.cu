@@ -84,7 +84,7 @@ __device__ __forceinline__ void gp_st_cluster_f32(uint32_t addr, float v) {
 // exchange / finish the accumulator.
 template <int BN, int MODE>
 __global__ void __launch_bounds__(GP_THREADS, 1)
-linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const bf16* __restrict__ x, bf16* __restrict__ out, int T, int N, int K,
+linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const bf16* x, bf16* __restrict__ out, int T, int N, int K,
                    int up_row0, int m_tiles, const GpRope rp, const GpNorm nm, int tag) {
   using C = GpCfg<BN>;
   extern __shared__ uint8_t smem_raw[];

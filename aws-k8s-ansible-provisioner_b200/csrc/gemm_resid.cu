@@ -56,7 +56,7 @@ __device__ __forceinline__ void gr_st_cluster_v4(uint32_t addr, float a, float b
 // issuer, warps 2-5 fetch X with cp.async, scatter the accumulator, finish 16 rows.
 template <int BN>
 __global__ void __launch_bounds__(192, 1)
-linear_resid_kernel(const __grid_constant__ CUtensorMap tmap_w, const bf16* __restrict__ x, bf16* __restrict__ h, float* __restrict__ ssq,
+linear_resid_kernel(const __grid_constant__ CUtensorMap tmap_w, const bf16* x, bf16* h, float* __restrict__ ssq,
                     int T, int N, int K, int ssq_ld, const L2Prefetch pf, int tag) {
   using C = GrCfg<BN>;
   extern __shared__ uint8_t smem_raw[];

@@ -9,7 +9,7 @@
 namespace b2 {
 
 template <int TB, bool OUT_F32>
-__global__ void __launch_bounds__(128) linear_simt_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w,
+__global__ void __launch_bounds__(128) linear_simt_kernel(const bf16* x, const bf16* __restrict__ w,
                                                           void* __restrict__ out, int T, int N, int K) {
   pdl_wait();
   pdl_launch_dependents();

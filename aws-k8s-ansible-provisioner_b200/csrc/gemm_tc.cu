@@ -75,9 +75,9 @@ __device__ __forceinline__ unsigned long long tc_argmax_pack(float v, int idx) {
 template <int BN, int EPI, int SMALL = 0, int XCP = 0>
 __global__ void __launch_bounds__(192, SMALL ? 6 : 1)
 linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
-                 void* out, unsigned long long* __restrict__ argmax_packed, int T, int N, int K,
+                 void* out, unsigned long long* argmax_packed, int T, int N, int K,
                  int kb_per_split, int m_tiles, int n_tiles, int nsplit, const KvPrefetch pf, int x_row0,
-                 const bf16* __restrict__ x_raw, const bf16* resid) {
+                 const bf16* x_raw, const bf16* resid) {
   using C = TcCfg<BN, SMALL>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::STAGES];

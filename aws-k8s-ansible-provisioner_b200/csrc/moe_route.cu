@@ -93,7 +93,7 @@ __device__ void route_pick(float* s, float* ch, float* gs, const RouteGeom& g, c
 // A CTA takes NTOK tokens: their rows are staged once as fp32, warp w takes router rows w, w + 16, ... (a row is read once for all tokens of
 // the CTA), then one warp per token forms the scores and selects.  A token's arithmetic does not depend on NTOK.
 template <typename TX, int NTOK, int RT_WARPS>
-__global__ void __launch_bounds__(RT_WARPS * 32) route_kernel(const TX* __restrict__ x, const float* __restrict__ router,
+__global__ void __launch_bounds__(RT_WARPS * 32) route_kernel(const TX* x, const float* __restrict__ router,
                                                               const float* __restrict__ correction, RouteGeom g, int32_t* __restrict__ idx,
                                                               float* __restrict__ weight, int T, int W, float* __restrict__ gate_out) {
   extern __shared__ __align__(16) float sm[];  // x rows [NTOK][W rounded up to 4] (read as float4), then per token: s [E + 1], choice [E], group scores [groups]
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(RT_WARPS * 32) route_kernel(const TX* __restri
 }
 
 // The same behind a product that has formed the logits z [T][ld] already (experts, then the gate's): one warp per token.
-__global__ void __launch_bounds__(256) route_select_kernel(const float* __restrict__ z, int ld, const float* __restrict__ correction, RouteGeom g,
+__global__ void __launch_bounds__(256) route_select_kernel(const float* z, int ld, const float* __restrict__ correction, RouteGeom g,
                                                            int32_t* __restrict__ idx, float* __restrict__ weight, int T, float* __restrict__ gate_out) {
   extern __shared__ __align__(16) float sm[];
   pdl_wait();
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256) route_select_kernel(const float* __restri
 }
 
 // the permutation in three steps: histogram (any number of CTAs), scan (one thread; experts are few), placement
-__global__ void __launch_bounds__(256) route_count_kernel(const int32_t* __restrict__ idx, int npairs, int E, int* __restrict__ counts) {
+__global__ void __launch_bounds__(256) route_count_kernel(const int32_t* idx, int npairs, int E, int* counts) {
   extern __shared__ int hist[];
   pdl_wait();
   pdl_launch_dependents();
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) route_count_kernel(const int32_t* __restr
   for (int e = threadIdx.x; e < E; e += 256)
     if (hist[e]) atomicAdd(&counts[e], hist[e]);
 }
-__global__ void route_scan_kernel(int* __restrict__ counts, int E, int32_t* __restrict__ offsets, int* __restrict__ cursor) {
+__global__ void route_scan_kernel(int* counts, int E, int32_t* offsets, int* cursor) {
   pdl_wait();
   pdl_launch_dependents();
   if (threadIdx.x != 0) return;
@@ -196,7 +196,7 @@ __global__ void route_scan_kernel(int* __restrict__ counts, int E, int32_t* __re
   }
   offsets[E] = run;
 }
-__global__ void __launch_bounds__(256) route_place_kernel(const int32_t* __restrict__ idx, int npairs, int top, int* __restrict__ cursor,
+__global__ void __launch_bounds__(256) route_place_kernel(const int32_t* idx, int npairs, int top, int* cursor,
                                                           int32_t* __restrict__ slot_token, int32_t* __restrict__ pair_slot) {
   pdl_wait();
   pdl_launch_dependents();
@@ -208,8 +208,8 @@ __global__ void __launch_bounds__(256) route_place_kernel(const int32_t* __restr
 }
 
 // few pairs (a decode step): the three steps in one CTA, histogram and cursors in shared memory
-__global__ void __launch_bounds__(1024) route_permute_small_kernel(const int32_t* __restrict__ idx, int npairs, int top, int E,
-                                                                   int32_t* __restrict__ offsets, int32_t* __restrict__ slot_token,
+__global__ void __launch_bounds__(1024) route_permute_small_kernel(const int32_t* idx, int npairs, int top, int E,
+                                                                   int32_t* offsets, int32_t* __restrict__ slot_token,
                                                                    int32_t* __restrict__ pair_slot) {
   extern __shared__ int cur[];  // [E]
   pdl_wait();
@@ -239,8 +239,8 @@ __global__ void __launch_bounds__(1024) route_permute_small_kernel(const int32_t
 }
 
 constexpr int COMBINE_MAX_TOP = 16;   // choices staged in shared memory; wider routers read them from global memory
-__global__ void __launch_bounds__(256) route_combine_kernel(float* __restrict__ h, const float* __restrict__ mix, const float* __restrict__ y,
-                                                            const float* __restrict__ weight, const int32_t* __restrict__ pair_slot, int W,
+__global__ void __launch_bounds__(256) route_combine_kernel(float* h, const float* mix, const float* y,
+                                                            const float* weight, const int32_t* pair_slot, int W,
                                                             int top) {
   __shared__ float w_s[COMBINE_MAX_TOP];
   __shared__ int slot_s[COMBINE_MAX_TOP];
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(256) route_combine_kernel(float* __restrict__ 
 }
 
 // slot_weight[pair_slot[p]] = weight[p]: the pairs' weights in expert (slot) order, for experts whose INPUT the weight multiplies
-__global__ void __launch_bounds__(256) route_slot_weights_kernel(const float* __restrict__ weight, const int32_t* __restrict__ pair_slot,
+__global__ void __launch_bounds__(256) route_slot_weights_kernel(const float* weight, const int32_t* pair_slot,
                                                                  float* __restrict__ slot_weight, int npairs) {
   pdl_wait();
   pdl_launch_dependents();
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(256) route_slot_weights_kernel(const float* __
 }
 
 // No router: a table row per token id names the token's experts, each weighted 1 / top.  idx [T][top], weight [T][top].
-__global__ void __launch_bounds__(256) route_table_kernel(const int32_t* __restrict__ ids, const int32_t* __restrict__ table, int vocab, int experts,
+__global__ void __launch_bounds__(256) route_table_kernel(const int32_t* ids, const int32_t* __restrict__ table, int vocab, int experts,
                                                           int top, int32_t* __restrict__ idx, float* __restrict__ weight, int npairs) {
   pdl_wait();
   pdl_launch_dependents();

@@ -35,8 +35,8 @@ __device__ __forceinline__ float block_sum_n(float v, float* red) {
 }
 
 template <typename TT>
-__global__ void __launch_bounds__(128) embed_unit_norm_kernel(const int32_t* __restrict__ ids, const TT* __restrict__ table,
-                                                              const float* __restrict__ gain1p, float* __restrict__ h, int W, int vocab,
+__global__ void __launch_bounds__(128) embed_unit_norm_kernel(const int32_t* ids, const TT* __restrict__ table,
+                                                              const float* __restrict__ gain1p, float* h, int W, int vocab,
                                                               float eps) {
   __shared__ float red[4];
   pdl_wait();
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(128) embed_unit_norm_kernel(const int32_t* __r
 }
 
 template <typename TX>
-__global__ void __launch_bounds__(128) unit_norm2_kernel(const float* __restrict__ h, const float* __restrict__ gain_a,
+__global__ void __launch_bounds__(128) unit_norm2_kernel(const float* h, const float* __restrict__ gain_a,
                                                          const float* __restrict__ gain_b, TX* __restrict__ x1, TX* __restrict__ x2, int W,
                                                          float eps, const int32_t* __restrict__ rows) {
   __shared__ float red[4];
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(128) unit_norm2_kernel(const float* __restrict
   }
 }
 
-__global__ void __launch_bounds__(1024) logits_finish_kernel(const float* __restrict__ logits, int32_t* __restrict__ out_tokens,
+__global__ void __launch_bounds__(1024) logits_finish_kernel(const float* logits, int32_t* __restrict__ out_tokens,
                                                             bf16* __restrict__ lb, int lb_rows, int V, int v_pad) {
   __shared__ float bv[32];
   __shared__ int bi[32];
@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(1024) logits_finish_kernel(const float* __rest
   if (V % 4 == 0 && lb == nullptr) {   // greedy only: sixteen bytes at a time, many loads in flight
 #pragma unroll 8
     for (int i = threadIdx.x; i < (V >> 2); i += 1024) {
-      const float4 q = __ldg(reinterpret_cast<const float4*>(row) + i);
+      const float4 q = reinterpret_cast<const float4*>(row)[i];
       const float v[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
       for (int x = 0; x < 4; ++x)
@@ -136,8 +136,8 @@ __global__ void __launch_bounds__(1024) logits_finish_kernel(const float* __rest
 
 // ---- grouped RMS norm with a plain gain (Kedasun): the vector is `groups` equal pieces, each with its own statistic ----
 template <typename TT>
-__global__ void __launch_bounds__(128) embed_scaled_kernel(const int32_t* __restrict__ ids, const TT* __restrict__ table, float scale,
-                                                           float* __restrict__ h, int W, int vocab) {
+__global__ void __launch_bounds__(128) embed_scaled_kernel(const int32_t* ids, const TT* __restrict__ table, float scale,
+                                                           float* h, int W, int vocab) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -154,8 +154,8 @@ constexpr int GN_REG = 16;   // values of a piece a lane keeps in registers (pie
 // EARLY (steps of few tokens, where a launch is all latency): every operand is loaded before the first reduction -- one round trip
 // to memory instead of one per phase; prompt-sized steps load late and keep the registers for occupancy.
 template <typename TX, bool ADD, bool EARLY>
-__global__ void __launch_bounds__(128) group_norm_kernel(const float* __restrict__ src, const float* __restrict__ bias,
-                                                         const float* __restrict__ gain, TX* __restrict__ x, float* __restrict__ h, int W,
+__global__ void __launch_bounds__(128) group_norm_kernel(const float* src, const float* __restrict__ bias,
+                                                         const float* __restrict__ gain, TX* __restrict__ x, float* h, int W,
                                                          int groups, float eps, const int32_t* __restrict__ rows,
                                                          const float* __restrict__ gain_next) {
   pdl_wait();
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(128) group_norm_kernel(const float* __restrict
 }
 
 template <typename TX>
-__global__ void __launch_bounds__(256) clamped_gate_kernel(const float* __restrict__ gu, TX* __restrict__ act, int F, float limit, float sharp) {
+__global__ void __launch_bounds__(256) clamped_gate_kernel(const float* gu, TX* __restrict__ act, int F, float limit, float sharp) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(256) clamped_gate_kernel(const float* __restri
 
 // ---- a parallel layer with ONE norm and several branches (Bumalix) ----
 template <typename TX>
-__global__ void __launch_bounds__(256) store_rows_kernel(const float* __restrict__ src, TX* __restrict__ x, int ldx, int col0, int W) {
+__global__ void __launch_bounds__(256) store_rows_kernel(const float* src, TX* __restrict__ x, int ldx, int col0, int W) {
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x;
@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256) store_rows_kernel(const float* __restrict
 
 // One CTA of 128 threads per token row: three power sums in one pass, then the polynomial of the three unit-RMS vectors.
 template <typename TX>
-__global__ void __launch_bounds__(128) poly_norm_kernel(const float* __restrict__ z, const float* __restrict__ coef, TX* __restrict__ act, int F,
+__global__ void __launch_bounds__(128) poly_norm_kernel(const float* z, const float* __restrict__ coef, TX* __restrict__ act, int F,
                                                         float eps) {
   __shared__ float red[4];
   pdl_wait();
@@ -311,7 +311,7 @@ __device__ __forceinline__ void st4(bf16* p, const float (&v)[4]) { *reinterpret
 // The same with the row held in registers (NV runs of 1024 numbers) and 16-byte accesses: the row is read once.  Bound by memory.
 // 16384 rows of 9216, bf16 out: 215 -> 175 us (906 MB: 5.2 TB/s).
 template <typename TX, int NV>
-__global__ void __launch_bounds__(256) poly_norm_vec_kernel(const float* __restrict__ z, const float* __restrict__ coef, TX* __restrict__ act, int F,
+__global__ void __launch_bounds__(256) poly_norm_vec_kernel(const float* z, const float* __restrict__ coef, TX* __restrict__ act, int F,
                                                             float eps) {
   __shared__ float red[3][8];
   pdl_wait();
@@ -366,8 +366,8 @@ __global__ void __launch_bounds__(256) poly_norm_vec_kernel(const float* __restr
 }
 
 template <typename TX>
-__global__ void __launch_bounds__(256) silu_gate_kernel(const float* __restrict__ gu, const float* __restrict__ row_scale,
-                                                        const int32_t* __restrict__ row_of, TX* __restrict__ act, int F) {
+__global__ void __launch_bounds__(256) silu_gate_kernel(const float* gu, const float* row_scale,
+                                                        const int32_t* row_of, TX* __restrict__ act, int F) {
   pdl_wait();
   pdl_launch_dependents();
   const int r = blockIdx.x;
@@ -402,10 +402,10 @@ __global__ void __launch_bounds__(256) silu_gate_kernel(const float* __restrict_
 // (steps of few tokens take wide CTAs: a row is then two or three rounds of loads instead of sixteen).
 constexpr int BA_MAX_TOP = 16;
 template <typename TX, int NT>
-__global__ void __launch_bounds__(NT) branch_add_kernel(float* __restrict__ h, const float* __restrict__ a, const float* __restrict__ gain_a,
-                                                        const float* __restrict__ b, const float* __restrict__ gain_b, float coef,
-                                                        const float* __restrict__ d1, const float* __restrict__ y,
-                                                        const int32_t* __restrict__ pair_slot, int top, int W, float eps,
+__global__ void __launch_bounds__(NT) branch_add_kernel(float* h, const float* a, const float* __restrict__ gain_a,
+                                                        const float* b, const float* __restrict__ gain_b, float coef,
+                                                        const float* d1, const float* y,
+                                                        const int32_t* pair_slot, int top, int W, float eps,
                                                         const float* __restrict__ gain_next, TX* __restrict__ x_next) {
   __shared__ float red[NT / 32];
   __shared__ int slot_s[BA_MAX_TOP];
@@ -450,10 +450,10 @@ __global__ void __launch_bounds__(NT) branch_add_kernel(float* __restrict__ h, c
 // The same with the row held in registers (NV runs of 4 NT numbers) and 16-byte accesses: both branches and the stream are read once.  Bound by memory.
 // 16384 rows of 2048 with two branches, a feed-forward's rows and no following norm: 169 -> 97 us (671 MB: 6.9 TB/s).
 template <typename TX, int NT, int NV>
-__global__ void __launch_bounds__(NT) branch_add_vec_kernel(float* __restrict__ h, const float* __restrict__ a, const float* __restrict__ gain_a,
-                                                            const float* __restrict__ b, const float* __restrict__ gain_b, float coef,
-                                                            const float* __restrict__ d1, const float* __restrict__ y,
-                                                            const int32_t* __restrict__ pair_slot, int top, int W, float eps,
+__global__ void __launch_bounds__(NT) branch_add_vec_kernel(float* h, const float* a, const float* __restrict__ gain_a,
+                                                            const float* b, const float* __restrict__ gain_b, float coef,
+                                                            const float* d1, const float* y,
+                                                            const int32_t* pair_slot, int top, int W, float eps,
                                                             const float* __restrict__ gain_next, TX* __restrict__ x_next) {
   __shared__ float red[NT / 32];
   __shared__ int slot_s[BA_MAX_TOP];
@@ -526,7 +526,7 @@ __global__ void __launch_bounds__(NT) branch_add_vec_kernel(float* __restrict__ 
   }
 }
 
-__global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ logits, size_t n, float cap) {
+__global__ void __launch_bounds__(256) softcap_kernel(float* logits, size_t n, float cap) {
   pdl_wait();
   pdl_launch_dependents();
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) logits[i] = cap * tanhf(logits[i] / cap);
@@ -536,7 +536,7 @@ __global__ void __launch_bounds__(256) softcap_kernel(float* __restrict__ logits
 // (x - mean) / sqrt(variance + eps) * w + b, the variance as the mean of the squared deviations (two passes over a row staged in shared
 // memory).  One CTA of 128 threads per row, any width.
 template <typename TX>
-__global__ void __launch_bounds__(128) layer_norm_kernel(const float* __restrict__ h, const float* __restrict__ w, const float* __restrict__ b,
+__global__ void __launch_bounds__(128) layer_norm_kernel(const float* h, const float* __restrict__ w, const float* __restrict__ b,
                                                          TX* __restrict__ x, int W, float eps, const int32_t* __restrict__ rows) {
   extern __shared__ float lrow[];
   __shared__ float red[4];
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(128) layer_norm_kernel(const float* __restrict
 // h[t] += ln(y[t]) (gain w, bias b); with pair_slot the sublayer's output is the sum of the token's `top` routed rows times coef,
 // y[t] = coef * sum_k y[pair_slot[t * top + k]].  With w_next the norm in front of the next sublayer follows, x_next[t] = ln(h[t]).
 template <typename TX>
-__global__ void __launch_bounds__(128) layer_norm_add_kernel(float* __restrict__ h, const float* __restrict__ y, const int32_t* __restrict__ pair_slot,
+__global__ void __launch_bounds__(128) layer_norm_add_kernel(float* h, const float* y, const int32_t* pair_slot,
                                                              int top, float coef, const float* __restrict__ w, const float* __restrict__ b, int W,
                                                              float eps, const float* __restrict__ w_next, const float* __restrict__ b_next,
                                                              TX* __restrict__ x_next) {
@@ -614,7 +614,7 @@ __device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log
 
 // act = a(z), a(z) = softplus(p) z^2 + z / 2 for z > 0 and (1/2 + softplus(q)) (exp(z) - 1 - z) + z / 2 otherwise; pq (device) = p, q
 template <typename TX>
-__global__ void __launch_bounds__(256) xielu_kernel(const float* __restrict__ z, const float* __restrict__ pq, TX* __restrict__ act, size_t n) {
+__global__ void __launch_bounds__(256) xielu_kernel(const float* z, const float* __restrict__ pq, TX* __restrict__ act, size_t n) {
   pdl_wait();
   pdl_launch_dependents();
   const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
@@ -641,7 +641,7 @@ __device__ __forceinline__ void store4(bf16* p, const float* v) {
   *reinterpret_cast<uint2*>(p) = pk;
 }
 template <typename TA, typename TX, bool VEC>
-__global__ void __launch_bounds__(256) sigmoid_gate_kernel(const TA* __restrict__ a, const float* __restrict__ gate, int gate_ld, TX* __restrict__ out,
+__global__ void __launch_bounds__(256) sigmoid_gate_kernel(const TA* a, const float* gate, int gate_ld, TX* __restrict__ out,
                                                            int out_ld, float scale, int N) {
   pdl_wait();
   pdl_launch_dependents();
@@ -665,8 +665,8 @@ __global__ void __launch_bounds__(256) sigmoid_gate_kernel(const TA* __restrict_
 
 // ---- several residual streams with learned mixes (Resitar): h [T][n][W] ----
 template <typename TT>
-__global__ void __launch_bounds__(256) embed_streams_kernel(const int32_t* __restrict__ ids, const TT* __restrict__ table, const float* __restrict__ gain,
-                                                            float* __restrict__ h, int n, int W, int vocab, float eps) {
+__global__ void __launch_bounds__(256) embed_streams_kernel(const int32_t* ids, const TT* __restrict__ table, const float* __restrict__ gain,
+                                                            float* h, int n, int W, int vocab, float eps) {
   __shared__ float red[8];
   pdl_wait();
   pdl_launch_dependents();
@@ -875,7 +875,7 @@ int streams_step_typed(const StreamsArgs& p, int n, TX* x, int T, cudaStream_t s
   return 0;
 }
 
-__global__ void __launch_bounds__(256) streams_sum_kernel(const float* __restrict__ h, int n, float* __restrict__ out, int W) {
+__global__ void __launch_bounds__(256) streams_sum_kernel(const float* h, int n, float* __restrict__ out, int W) {
   pdl_wait();
   pdl_launch_dependents();
   const float* hr = h + (size_t)blockIdx.x * n * W;
@@ -889,10 +889,10 @@ __global__ void __launch_bounds__(256) streams_sum_kernel(const float* __restric
 // Blends of a row with the row before it.  A thread owns columns; in a portion's first row it reads the sequence's ring entry and then leaves the
 // portion's last row there, read and write in one thread: the two may be the same entry.
 template <typename TX, bool VEC>
-__global__ void __launch_bounds__(256) token_shift_kernel(const TX* __restrict__ x, const float* __restrict__ mu, TX* __restrict__ ring, TX* __restrict__ out,
+__global__ void __launch_bounds__(256) token_shift_kernel(const TX* x, const float* __restrict__ mu, TX* ring, TX* __restrict__ out,
                                                           int T, int W, const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
-                                                          const int32_t* __restrict__ row_end, const int32_t* __restrict__ positions,
-                                                          const int32_t* __restrict__ slots) {
+                                                          const int32_t* __restrict__ row_end, const int32_t* positions,
+                                                          const int32_t* slots) {
   constexpr int V = VEC ? 4 : 1;
   pdl_wait();
   pdl_launch_dependents();
@@ -947,12 +947,12 @@ __global__ void __launch_bounds__(256) token_shift_kernel(const TX* __restrict__
 // here) and, in the portion's first row, leaves the portion's last token in the ring: read and write sit in one thread, so a portion
 // whose last token lands on the entry that its first row reads is safe.
 template <typename TX>
-__global__ void __launch_bounds__(128) embed_sum_kernel(const int32_t* __restrict__ ids, const TX* __restrict__ table, const TX* __restrict__ bigram,
-                                                        int buckets, long long mul_prev, long long mul_cur, int32_t* __restrict__ tok_ring,
-                                                        const TX* __restrict__ pos_table, int pos_rows, float* __restrict__ h, TX* __restrict__ x, int W,
+__global__ void __launch_bounds__(128) embed_sum_kernel(const int32_t* ids, const TX* __restrict__ table, const TX* __restrict__ bigram,
+                                                        int buckets, long long mul_prev, long long mul_cur, int32_t* tok_ring,
+                                                        const TX* __restrict__ pos_table, int pos_rows, float* h, TX* __restrict__ x, int W,
                                                         int vocab, const int32_t* __restrict__ row_seq, const int32_t* __restrict__ row_first,
-                                                        const int32_t* __restrict__ row_end, const int32_t* __restrict__ positions,
-                                                        const int32_t* __restrict__ slots) {
+                                                        const int32_t* __restrict__ row_end, const int32_t* positions,
+                                                        const int32_t* slots) {
   __shared__ int bg_row;
   pdl_wait();
   pdl_launch_dependents();
@@ -993,9 +993,9 @@ __global__ void __launch_bounds__(128) embed_sum_kernel(const int32_t* __restric
 // in flight before the one reduction.
 constexpr int ON_MAX_TOP = 16;
 template <typename TX, int NT, int R>
-__global__ void __launch_bounds__(NT) out_norm_add_kernel(float* __restrict__ h, const float* __restrict__ a, const float* __restrict__ a_scale,
-                                                          const float* __restrict__ y, const float* __restrict__ weight,
-                                                          const int32_t* __restrict__ pair_slot, int top, const float* __restrict__ gain, float mult,
+__global__ void __launch_bounds__(NT) out_norm_add_kernel(float* h, const float* a, const float* a_scale,
+                                                          const float* y, const float* weight,
+                                                          const int32_t* pair_slot, int top, const float* __restrict__ gain, float mult,
                                                           int W, float eps, TX* __restrict__ x_next) {
   __shared__ float red[NT / 32];
   __shared__ float w_s[ON_MAX_TOP];
@@ -1067,9 +1067,9 @@ __global__ void __launch_bounds__(NT) out_norm_add_kernel(float* __restrict__ h,
 
 // the same for any width and any number of choices: the row staged in shared memory, one number at a time
 template <typename TX>
-__global__ void __launch_bounds__(256) out_norm_add_any_kernel(float* __restrict__ h, const float* __restrict__ a, const float* __restrict__ a_scale,
-                                                               const float* __restrict__ y, const float* __restrict__ weight,
-                                                               const int32_t* __restrict__ pair_slot, int top, const float* __restrict__ gain,
+__global__ void __launch_bounds__(256) out_norm_add_any_kernel(float* h, const float* a, const float* a_scale,
+                                                               const float* y, const float* weight,
+                                                               const int32_t* pair_slot, int top, const float* __restrict__ gain,
                                                                float mult, int W, float eps, TX* __restrict__ x_next) {
   extern __shared__ float lrow[];
   __shared__ float red[8];
