@@ -276,6 +276,7 @@ few_attn_kernel(const bf16* qkv, const bf16* __restrict__ qw, const bf16* __rest
   __shared__ __align__(16) bf16 kv_new[2][FA_HD];         // the new token's key and value
   __shared__ FaRecord rec[FA_WARPS], all[FA_CTAS];
   pdl_launch_dependents();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this CTA runs: see the first remote store
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
@@ -424,6 +425,9 @@ few_attn_kernel(const bf16* qkv, const bf16* __restrict__ qw, const bf16* __rest
     }
     return v;
   };
+  // every CTA of the cluster has started (its shared memory is live) before anyone stores into the first one's: a CTA without pages is here almost at once,
+  // and the dependency wait says nothing about the other CTAs
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
   const uint32_t mine = (uint32_t)__cvta_generic_to_shared(&all[rank]);
   uint32_t dst;
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(dst) : "r"(mine));
