@@ -126,6 +126,19 @@ extern "C" int b2k_linear_split3(const float* x, void* planes, const void* w, fl
   return launch_linear_split3(x, (bf16*)planes, (const bf16*)w, out, rows, N, K, wait, (cudaStream_t)stream, tile);
 }
 
+extern "C" int b2k_linear_split3_wide(const float* x, const float* w, void* planes, size_t plane_numbers, void* narrow, size_t narrow_numbers, float* out, int rows, int N,
+                                      int K, void* stream) {
+  B2_REQUIRE(x && w && planes && narrow && out, "b2k_linear_split3_wide: null pointer");
+  B2WaitLimit wait;
+  CAPI_TRY(hook_waits(&wait));
+  Split3Scratch t;
+  t.planes = (bf16*)planes;
+  t.narrow = (bf16*)narrow;
+  t.plane_numbers = plane_numbers;
+  t.narrow_numbers = narrow_numbers;
+  return launch_linear_split3_wide(x, w, out, rows, N, K, t, wait, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_heads_postmix(const float* q, const void* k_cache, const void* v_cache, int heads, int kv_heads, int dim, int vdim, float scale, float slope_exp,
                                  int window, int keep_first, const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, int ntiles, const float* talk,
                                  const float* gate, int gate_ld, void* out, void* stream) {

@@ -359,12 +359,7 @@ struct b2_engine {
   float* l_attn_scratch = nullptr;   // key splits of a decode step's latent attention
   bf16* l_xperm = nullptr;           // prompt-sized steps: the feed-forward input rows in expert (slot) order
   float* l_upf = nullptr;            // ... and the experts' up-projection sums before the activation
-  // fp32 mode of the layer-list families: bf16 copies of the weight matrices, which are bf16 numbers, and the planes of a product's input rows (gemm_sum.cu)
-  struct F32Copy { const char* base; size_t elems; bf16* copy; };
-  std::vector<F32Copy> f32_copies;
-  bf16* f32_planes = nullptr;
-  size_t f32_planes_elems = 0;       // numbers of x that they hold
-  bool f32_stale = false;            // a weight was loaded behind the copies
+  Split3Scratch f32_tc;              // fp32 mode of the layer-list families: scratch of the products on the tensor pipe (gemm_sum.cu)
   int32_t* h_offsets = nullptr;      // pinned: the experts' slot ranges of the step, read back for the per-expert launches
   size_t l_attn_scratch_floats = 0;
   float* dbg_hidden_f32 = nullptr;
@@ -994,25 +989,18 @@ bool list_use_tc() {
   return use_tc;
 }
 bool list_dense_tc(const b2_engine* e, int M, int N, int K) { return list_use_tc() && !e->f32 && (M > 64 || N >= 16384) && N >= 128 && K % 64 == 0; }
-// fp32 products on the tensor pipe (three exact bf16 products, gemm_sum.cu): where the weights' copy and the planes are there, the rows' planes fit, and the launch
-// is on the engine's own stream (the planes are one buffer; short steps run some products beside others on side streams).  From seventeen rows on, or from four
+// fp32 products on the tensor pipe (three exact bf16 products, gemm_sum.cu; every matrix of an fp32 engine is a widened bf16 one, see put_operand): where the launch
+// is on the engine's own stream (the scratch is one; short steps run some products beside others on side streams).  From seventeen rows on, or from four
 // where the weights are many; fewer take the kernel that streams the weights, whose time grows with the rows (their shared-memory reads bound it: 6 x 32000 x 1024
 // 89 us there, 30 here).  A Kedasun prompt of 100 tokens, two layers, width 1024: 1260 us on the register tiles, 600 here.
-const bf16* list_f32_copy(const b2_engine* e, const void* A, const void* Wt, int M, int N, int K, cudaStream_t ls) {
-  if (!e->f32 || e->f32_planes == nullptr || ls != e->stream || !linear_sum_shapes_ok(M, 1, N, K) || (size_t)M * K > e->f32_planes_elems) return nullptr;
-  if (!(M > 16 || (M >= 4 && N >= 16384)) || (reinterpret_cast<uintptr_t>(A) & 15) != 0) return nullptr;
-  for (const auto& c : e->f32_copies) {
-    const size_t at = (size_t)(reinterpret_cast<const char*>(Wt) - c.base) / 4;
-    if (c.copy != nullptr && reinterpret_cast<const char*>(Wt) >= c.base && at + (size_t)N * K <= c.elems && at % 8 == 0) return c.copy + at;
-  }
-  return nullptr;
+bool list_f32_tc(const b2_engine* e, const void* A, const void* Wt, int M, int N, int K, cudaStream_t ls) {
+  return e->f32 && ls == e->stream && (M > 16 || (M >= 4 && N >= 16384)) && linear_split3_wide_ok(e->f32_tc, A, Wt, M, N, K);
 }
 int list_dense(b2_engine* e, const void* A, const void* Wt, float* C, int M, int N, int K, float alpha, cudaStream_t stream = nullptr) {
   cudaStream_t ls = stream ? stream : e->stream;
   const int f = e->f32 ? 1 : 0;
-  if (alpha == 1.f) {
-    if (const bf16* wb = list_f32_copy(e, A, Wt, M, N, K, ls)) return launch_linear_split3((const float*)A, e->f32_planes, wb, C, M, N, K, e->wait_limit(), ls);
-  }
+  if (alpha == 1.f && list_f32_tc(e, A, Wt, M, N, K, ls))
+    return launch_linear_split3_wide((const float*)A, (const float*)Wt, C, M, N, K, e->f32_tc, e->wait_limit(), ls);
   static const bool few_head = [] { const char* v = getenv("B2_FEW_HEAD"); return !(v && *v == '0'); }();
   if (few_head && !f && N >= 16384 && few_head_ok(M, N, K)) return launch_few_head((const bf16*)Wt, (const bf16*)A, C, M, N, K, alpha, ls);
   if (alpha == 1.f && list_dense_tc(e, M, N, K)) {
@@ -1270,6 +1258,24 @@ void latent_rebuild_free(b2_engine* e) {
   };
   drop(e->lx_rows); drop(e->lx_kv); drop(e->lx_k); drop(e->lx_v); drop(e->lx_r); drop(e->d_xtiles); drop(e->d_xctx); drop(e->d_xtable);
   drop_host(e->h_xtiles); drop_host(e->h_xctx); drop_host(e->h_xtable);
+}
+
+// The scratch of an fp32 engine's products on the tensor pipe: 96 and 64 MB whatever the model (a step's rows in fewer where they are fewer), behind the cache.  One
+// matrix at a time is narrowed into it, 6 bytes of traffic per weight and product: copies of all matrices beside the fp32 ones would save that (two layers of
+// width 1024 and their head, a prompt of 1500 tokens: about 60 of 1100 us), and take half as much again as the weights from what the caller left for other engines.
+// Without room for it the products take the register tiles of gemm_any.cu.
+void list_f32_scratch(b2_engine* e) {
+  static const bool on = [] { const char* v = getenv("B2_F32_TC"); return !(v && *v == '0'); }();   // 0: the register tiles (cross-check)
+  if (!on) return;
+  Split3Scratch t;
+  t.plane_numbers = std::min((size_t)1 << 24, (size_t)e->cap_tokens << 14);
+  t.narrow_numbers = (size_t)1 << 25;
+  if (cudaMalloc(&t.planes, t.plane_numbers * 6) == cudaSuccess && cudaMalloc(&t.narrow, t.narrow_numbers * 2) == cudaSuccess) {
+    e->f32_tc = t;
+    return;
+  }
+  cudaGetLastError();
+  if (t.planes) cudaFree(t.planes);
 }
 
 // A Lerasun engine takes what the rebuilt form needs -- a layer's up-projections as one matrix (the key part a second time: 2 MB at 16 heads and a latent of
@@ -3291,7 +3297,6 @@ int heads_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&q, std::max<size_t>(elems, 1) * es));
     *p = q;
     e->weight_bytes += (int64_t)(elems * es);
-    if (e->f32) e->f32_copies.push_back({q, elems, nullptr});
     return 0;
   };
   auto falloc = [&](float** p, size_t n) -> int {
@@ -3411,7 +3416,6 @@ int state_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&q, std::max<size_t>(elems, 1) * es));
     *p = q;
     e->weight_bytes += (int64_t)(elems * es);
-    if (e->f32) e->f32_copies.push_back({q, elems, nullptr});
     return 0;
   };
   auto falloc = [&](float** p, size_t n) -> int {
@@ -3715,7 +3719,6 @@ int mixed_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&q, std::max<size_t>(elems, 1) * es));
     *p = q;
     e->weight_bytes += (int64_t)(elems * es);
-    if (e->f32) e->f32_copies.push_back({q, elems, nullptr});
     return 0;
   };
   auto falloc = [&](float** p, size_t n) -> int {
@@ -3984,7 +3987,6 @@ int outnorm_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&q, std::max<size_t>(elems, 1) * es));
     *p = q;
     e->weight_bytes += (int64_t)(elems * es);
-    if (e->f32) e->f32_copies.push_back({q, elems, nullptr});
     return 0;
   };
   auto falloc = [&](float** p, size_t n) -> int {
@@ -4258,7 +4260,6 @@ int streams_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&q, std::max<size_t>(elems, 1) * es));
     *p = q;
     e->weight_bytes += (int64_t)(elems * es);
-    if (e->f32) e->f32_copies.push_back({q, elems, nullptr});
     return 0;
   };
   auto falloc = [&](float** p, size_t m) -> int {
@@ -4545,7 +4546,6 @@ int list_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&q, std::max<size_t>(elems, 1) * es));
     *p = q;
     e->weight_bytes += (int64_t)(elems * es);
-    if (e->f32) e->f32_copies.push_back({q, elems, nullptr});
     return 0;
   };
   auto falloc = [&](float** p, size_t n) -> int {
@@ -4661,7 +4661,6 @@ int list_engine_alloc(b2_engine* e) {
 }
 
 int layer_tensor(b2_engine* e, const std::string& name, const void* host, size_t nbytes) {
-  if (e->finalized) e->f32_stale = true;   // (a tensor that is loaded again: its bf16 copy is made again before the next step)
   const b2_config& c = e->cfg;
   if (list_arch(c.arch)) return list_tensor(e, name, host, nbytes);
   const int H = c.hidden, I = c.intermediate;
@@ -5297,6 +5296,7 @@ extern "C" int b2_engine_create(const b2_config* cfg, const char* safetensors_pa
           e->regions.push_back({reinterpret_cast<char*>(e->kv_pool + (size_t)r * e->layer_kv_elems), blk_elems * 2});
       }
       if (c.arch == B2_ARCH_LERASUN) E_TRY(latent_rebuild_setup(e));
+      if (ls && e->f32) list_f32_scratch(e);
       e->free_blocks.reserve(nb);
       for (int64_t b = nb - 1; b >= 1; --b) e->free_blocks.push_back((int32_t)b);  // page 0 = null page
       e->blk_ref.assign(nb, 0);
@@ -5343,61 +5343,12 @@ extern "C" int b2_engine_load_safetensors(b2_engine* e, const char* path) {
   return load_safetensors(e, path);
 }
 
-// fp32 mode: bf16 copies of the weight matrices and the planes for a step's rows, as far as memory is there (512 MB stay free: the products without them take
-// the register tiles of gemm_any.cu).  A matrix that holds anything but bf16 numbers gets no copy.
-static int list_f32_prepare(b2_engine* e) {
-  static const bool on = [] { const char* v = getenv("B2_F32_TC"); return !(v && *v == '0'); }();   // 0: the register tiles (cross-check)
-  e->f32_stale = false;
-  if (!e->f32 || !on) return 0;
-  auto room = [](size_t bytes) {
-    size_t free_b = 0, total_b = 0;
-    return cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && free_b >= bytes + ((size_t)512 << 20);
-  };
-  size_t widest = (size_t)e->cfg.hidden;
-  for (const auto& L : e->ll)
-    widest = std::max({widest, (size_t)std::max(L.sp.ff_dim, 0), (size_t)std::max(L.sp.shared_ff, 0), (size_t)L.sp.heads * L.sp.vdim + (size_t)L.sp.s_heads * L.sp.s_vdim});
-  if (e->f32_planes == nullptr) {
-    const size_t elems = (size_t)e->cap_tokens * widest;
-    if (!room(elems * 6) || cudaMalloc(&e->f32_planes, elems * 6) != cudaSuccess) {
-      cudaGetLastError();
-      e->f32_planes = nullptr;
-      return 0;
-    }
-    e->f32_planes_elems = elems;
-  }
-  uint32_t* inexact = nullptr;
-  B2_CUDA_OK(cudaMalloc(&inexact, 4));
-  int rc = 0;
-  for (auto& c : e->f32_copies) {
-    if (c.elems < 4096 || (c.base == (const char*)e->l_embed && e->l_head != e->l_embed)) continue;   // (rows are looked up there)
-    if (c.copy == nullptr && (!room(c.elems * 2) || cudaMalloc(&c.copy, c.elems * 2) != cudaSuccess)) {
-      cudaGetLastError();
-      c.copy = nullptr;
-      continue;
-    }
-    uint32_t bad = 1;
-    if (cudaMemsetAsync(inexact, 0, 4, e->stream) != cudaSuccess || (rc = launch_bf16_copy((const float*)c.base, c.copy, c.elems, inexact, e->stream)) != 0 ||
-        cudaMemcpyAsync(&bad, inexact, 4, cudaMemcpyDeviceToHost, e->stream) != cudaSuccess || cudaStreamSynchronize(e->stream) != cudaSuccess) {
-      if (rc == 0) rc = -5;
-      break;
-    }
-    if (bad != 0) {
-      cudaFree(c.copy);
-      c.copy = nullptr;
-    }
-  }
-  cudaFree(inexact);
-  if (rc != 0) b2_set_error("fp32 weights: %s", cudaGetErrorString(cudaGetLastError()));
-  return rc;
-}
-
 extern "C" int b2_engine_finalize(b2_engine* e) {
   B2_REQUIRE(e, "b2_engine_finalize: null engine");
   const int arch = e->cfg.arch;
   if (arch == B2_ARCH_BUMALIX || arch == B2_ARCH_TINEVIK || arch == B2_ARCH_TOLANEX || arch == B2_ARCH_RESITAR) {
     B2_CUDA_OK(cudaSetDevice(e->device));
     B2_TRY(arch == B2_ARCH_RESITAR ? streams_finalize(e) : arch == B2_ARCH_BUMALIX ? state_finalize(e) : arch == B2_ARCH_TINEVIK ? mixed_finalize(e) : outnorm_finalize(e));
-    B2_TRY(list_f32_prepare(e));
     e->finalized = true;
     return 0;
   }
@@ -5409,8 +5360,6 @@ extern "C" int b2_engine_finalize(b2_engine* e) {
     for (size_t l = 0; l < e->ll.size(); ++l)   // the blend weight: needed by the layers that blend, harmless elsewhere
       B2_REQUIRE(e->ll[l].vmix_mode != 2 || e->loaded.count("l" + std::to_string(l) + ".mix.vmix"), "weights incomplete: l%zu.mix.vmix missing", l);
     B2_REQUIRE(have == want, "weights incomplete: %d of %d tensors loaded", have, want);
-    B2_CUDA_OK(cudaSetDevice(e->device));
-    B2_TRY(list_f32_prepare(e));
     e->finalized = true;
     return 0;
   }
@@ -5455,8 +5404,7 @@ extern "C" void b2_engine_free(b2_engine* e) {
   F(e->partial2); F(e->attn_scratch2); F(e->ssq);
   if (e->l_head == e->l_embed) e->l_head = nullptr;   // (a tied head is the embedding table)
   latent_rebuild_free(e);
-  for (auto& c : e->f32_copies) F(c.copy);
-  F(e->f32_planes);
+  F(e->f32_tc.planes); F(e->f32_tc.narrow);
   for (auto& t : e->rot_tables) F(t.table);
   F(e->l_shift); F(e->l_ao); F(e->l_rkvg); F(e->l_lr); F(e->l_cv);
   F(e->l_final_bias); F(e->l_bigram); F(e->l_pos); F(e->l_tok_ring); F(e->l_sg); F(e->l_rz);
@@ -5719,7 +5667,6 @@ int prefill_impl(b2_engine* e, const int32_t* ids, const int32_t* seq_offsets, i
                  int32_t nrows, float* out_logits, int32_t* out_tokens) {
   B2_REQUIRE(e && ids && seq_offsets && seq_ids && nseq >= 1, "b2_prefill: bad arguments");
   B2_REQUIRE(e->finalized, "b2_prefill: weights not finalized");
-  if (e->f32_stale) B2_TRY(list_f32_prepare(e));
   B2_REQUIRE(nseq <= e->cfg.max_seqs, "b2_prefill: %d sequences > max_seqs %d", nseq, e->cfg.max_seqs);
   B2_CUDA_OK(cudaSetDevice(e->device));
   const int T_in = seq_offsets[nseq] - seq_offsets[0];
@@ -5860,7 +5807,6 @@ namespace {
 // Prepares device state for a decode step over seq_ids; returns padded batch B.
 int prepare_decode(b2_engine* e, int n, const int32_t* seq_ids, const int32_t* in_tokens, int* B_out, int* split_out) {
   B2_REQUIRE(e->finalized, "decode: weights not finalized");
-  if (e->f32_stale) B2_TRY(list_f32_prepare(e));
   B2_REQUIRE(n >= 1 && n <= e->cfg.max_seqs, "decode: batch %d outside [1, max_seqs=%d]", n, e->cfg.max_seqs);
   int max_len = 0;
   for (int i = 0; i < n; ++i) {

@@ -95,7 +95,7 @@ struct GsWalk {
 template <int BN, int EPI, int SPLIT>   // SPLIT: planes of x (0: x as it is, its whole K in the accumulator)
 __global__ void __launch_bounds__(GS_THREADS, 1)
 linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const int32_t* offsets, int groups,
-                  int rows_total, void* out, int N, int K, const B2WaitLimit limit) {
+                  int rows_total, void* out, int N, int K, int ldo, const B2WaitLimit limit) {
   using C = GsCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::STAGES];
@@ -206,24 +206,24 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
     };
     auto store = [&](int c0, int col, const uint32_t (&r)[32]) {   // 32 rows of x from c0 of the tile on, this thread's weight row
       if (col >= N) return;
-      const size_t at = (size_t)(w.row0 + c0) * N + col;
+      const size_t at = (size_t)(w.row0 + c0) * ldo + col;
       const int have = w.rows - c0;   // rows of this block that are the group's
       if constexpr (EPI == SUM_EPI_F32) {
         float* d = reinterpret_cast<float*>(out) + at;
         if (have >= 32) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) d[(size_t)j * N] = __uint_as_float(r[j]);
+          for (int j = 0; j < 32; ++j) d[(size_t)j * ldo] = __uint_as_float(r[j]);
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j)
-            if (j < have) d[(size_t)j * N] = __uint_as_float(r[j]);
+            if (j < have) d[(size_t)j * ldo] = __uint_as_float(r[j]);
         }
       } else {
         bf16* d = reinterpret_cast<bf16*>(out) + at;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
           const float a = fmaxf(__uint_as_float(r[j]), 0.f);
-          if (j < have) d[(size_t)j * N] = __float2bfloat16_rn(a * a);
+          if (j < have) d[(size_t)j * ldo] = __float2bfloat16_rn(a * a);
         }
       }
     };
@@ -295,8 +295,9 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
 }
 
-// planes [3][n] bf16 whose sum is x: every plane the nearest bf16 to what is left (a value that rounds to infinity is cut instead; infinities and NaN stay in the first)
-__global__ void __launch_bounds__(256) split3_kernel(const float4* x, uint2* planes, size_t n4) {
+// planes [3][n] bf16 whose sum is x: every plane the nearest bf16 to what is left (a value that rounds to infinity is cut instead; infinities and NaN stay in the first).
+// w given: fp32 numbers that are bf16 numbers, written to narrow as such
+__global__ void __launch_bounds__(256) split3_kernel(const float4* x, uint2* planes, size_t n4, const uint4* __restrict__ w, uint2* narrow, size_t w4) {
   pdl_wait();
   pdl_launch_dependents();
   for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n4; i += (size_t)gridDim.x * 256) {
@@ -318,21 +319,15 @@ __global__ void __launch_bounds__(256) split3_kernel(const float4* x, uint2* pla
 #pragma unroll
     for (int p = 0; p < 3; ++p) planes[(size_t)p * n4 + i] = make_uint2(h[p][0] | h[p][1] << 16, h[p][2] | h[p][3] << 16);
   }
-}
-
-// bf16 copies of fp32 numbers; *inexact becomes 1 when one of them is not a bf16 number
-__global__ void __launch_bounds__(256) bf16_copy_kernel(const uint32_t* __restrict__ w, uint16_t* __restrict__ out, size_t n, uint32_t* inexact) {
-  bool bad = false;
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
-    const uint32_t b = w[i];
-    bad = bad || (b & 0xffffu) != 0;
-    out[i] = (uint16_t)(b >> 16);
+#pragma unroll 4
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < w4; i += (size_t)gridDim.x * 256) {
+    const uint4 v = w[i];
+    narrow[i] = make_uint2(__byte_perm(v.x, v.y, 0x7632), __byte_perm(v.z, v.w, 0x7632));   // (the upper halves)
   }
-  if (bad) *inexact = 1;
 }
 
 template <int BN, int EPI, int SPLIT = 0>
-int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, const B2WaitLimit& wait, cudaStream_t s) {
+int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int ldo = 0) {
   using C = GsCfg<BN>;
   static B2PerDeviceOnce attr_once;
   if (attr_once.need()) B2_CUDA_OK(cudaFuncSetAttribute(linear_sum_kernel<BN, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
@@ -357,7 +352,7 @@ int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = b2_pdl_enabled() ? 2 : 1;
-  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_sum_kernel<BN, EPI, SPLIT>, tw, tx, offsets, groups, rows, out, N, K, wait));
+  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_sum_kernel<BN, EPI, SPLIT>, tw, tx, offsets, groups, rows, out, N, K, ldo > 0 ? ldo : N, wait));
   return 0;
 }
 
@@ -396,27 +391,53 @@ int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int 
   return -22;
 }
 
+static int launch_split3(const float* x, bf16* planes, size_t nx, const float* w, bf16* narrow, size_t nw, cudaStream_t s) {
+  const size_t n4 = nx / 4, w4 = nw / 4;
+  B2_CUDA_OK(b2_launch(split3_kernel, dim3((unsigned)std::min<size_t>((std::max(n4, w4) + 255) / 256, (size_t)device_num_sms() * 16)), dim3(256), 0, s, (const float4*)x,
+                       (uint2*)planes, n4, (const uint4*)w, (uint2*)narrow, w4));
+  return 0;
+}
+static int launch_planes(const bf16* planes, const bf16* w, float* out, int rows, int N, int K, int ldo, const B2WaitLimit& wait, cudaStream_t s, int bn) {
+  if (bn == 0) bn = sum_pick_bn(rows, 1, N);
+  return bn == 128 ? launch_sum<128, SUM_EPI_F32, 3>(planes, w, nullptr, 1, rows, out, N, K, wait, s, ldo)
+                   : launch_sum<256, SUM_EPI_F32, 3>(planes, w, nullptr, 1, rows, out, N, K, wait, s, ldo);
+}
 int launch_linear_split3(const float* x, bf16* planes, const bf16* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int bn) {
   if (rows <= 0) return 0;
   B2_REQUIRE(linear_sum_shapes_ok(rows, 1, N, K) && (reinterpret_cast<uintptr_t>(x) & 15) == 0, "linear_split3: %d rows, N=%d K=%d not built", rows, N, K);
-  const size_t n4 = (size_t)rows * K / 4;
-  B2_CUDA_OK(b2_launch(split3_kernel, dim3((unsigned)std::min<size_t>((n4 + 255) / 256, (size_t)device_num_sms() * 16)), dim3(256), 0, s, (const float4*)x, (uint2*)planes, n4));
-  if (bn == 0) bn = sum_pick_bn(rows, 1, N);
-  return bn == 128 ? launch_sum<128, SUM_EPI_F32, 3>(planes, w, nullptr, 1, rows, out, N, K, wait, s)
-                   : launch_sum<256, SUM_EPI_F32, 3>(planes, w, nullptr, 1, rows, out, N, K, wait, s);
+  int rc = launch_split3(x, planes, (size_t)rows * K, nullptr, nullptr, 0, s);
+  return rc != 0 ? rc : launch_planes(planes, w, out, rows, N, K, 0, wait, s, bn);
+}
+
+// Rows of x and of w that the scratch takes at a time, in whole tiles where they are not all of them (0: none)
+static int split3_piece(int rows, int K, size_t numbers) {
+  const size_t most = numbers / (size_t)K;
+  return (size_t)rows <= most ? rows : (int)(most / 256 * 256);
+}
+bool linear_split3_wide_ok(const Split3Scratch& t, const void* x, const void* w, int rows, int N, int K) {
+  return t.planes != nullptr && t.narrow != nullptr && linear_sum_shapes_ok(rows, 1, N, K) && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0 &&
+         split3_piece(rows, K, t.plane_numbers) > 0 && split3_piece(N, K, t.narrow_numbers) >= std::min(N, 256);
+}
+int launch_linear_split3_wide(const float* x, const float* w, float* out, int rows, int N, int K, const Split3Scratch& t, const B2WaitLimit& wait, cudaStream_t s) {
+  if (rows <= 0) return 0;
+  B2_REQUIRE(linear_split3_wide_ok(t, x, w, rows, N, K), "linear_split3_wide: %d rows, N=%d K=%d not built", rows, N, K);
+  const int pr = split3_piece(rows, K, t.plane_numbers), pn = split3_piece(N, K, t.narrow_numbers);
+  for (int n0 = 0; n0 < N; n0 += pn) {
+    const int nn = std::min(pn, N - n0);
+    for (int r0 = 0; r0 < rows; r0 += pr) {
+      const int rr = std::min(pr, rows - r0);
+      int rc = launch_split3(x + (size_t)r0 * K, t.planes, (size_t)rr * K, r0 == 0 ? w + (size_t)n0 * K : nullptr, t.narrow, r0 == 0 ? (size_t)nn * K : 0, s);
+      if (rc == 0) rc = launch_planes(t.planes, t.narrow, out + (size_t)r0 * N + n0, rr, nn, K, N, wait, s, 0);
+      if (rc != 0) return rc;
+    }
+  }
+  return 0;
 }
 
 int launch_linear_sum_fine(const void* x, const void* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s) {
   if (rows <= 0) return 0;
   B2_REQUIRE(linear_sum_shapes_ok(rows, 1, N, K), "linear_sum_fine: %d rows, N=%d K=%d not built", rows, N, K);
   return launch_sum<128, SUM_EPI_F32, 1>(x, w, nullptr, 1, rows, out, N, K, wait, s);
-}
-
-int launch_bf16_copy(const float* w, bf16* out, size_t n, uint32_t* inexact, cudaStream_t s) {
-  if (n == 0) return 0;
-  bf16_copy_kernel<<<(unsigned)std::min<size_t>((n + 255) / 256, (size_t)device_num_sms() * 16), 256, 0, s>>>((const uint32_t*)w, (uint16_t*)out, n, inexact);
-  B2_CUDA_OK(cudaGetLastError());
-  return 0;
 }
 
 }  // namespace b2

@@ -121,10 +121,15 @@ int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int 
                       cudaStream_t s, int bn = 0);
 // the same for fp32 x [rows][K] and bf16 weights, fp32 precision: x goes to three bf16 planes ([3][rows][K], scratch) whose sum it is
 int launch_linear_split3(const float* x, bf16* planes, const bf16* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int bn = 0);
+// ... and for fp32 weights that are bf16 numbers, as a checkpoint's are: each product narrows its matrix into the scratch, which holds any shape in pieces
+struct Split3Scratch {
+  bf16 *planes = nullptr, *narrow = nullptr;
+  size_t plane_numbers = 0, narrow_numbers = 0;   // numbers of x (three planes each) and of w at a time
+};
+bool linear_split3_wide_ok(const Split3Scratch& t, const void* x, const void* w, int rows, int N, int K);
+int launch_linear_split3_wide(const float* x, const float* w, float* out, int rows, int N, int K, const Split3Scratch& t, const B2WaitLimit& wait, cudaStream_t s);
 // bf16 x with the same sums (128 of the K in the accumulator at a time, rounded to nearest between them): router logits
 int launch_linear_sum_fine(const void* x, const void* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s);
-// bf16 copy of n fp32 numbers; *inexact (device) becomes 1 when one of them is not a bf16 number
-int launch_bf16_copy(const float* w, bf16* out, size_t n, uint32_t* inexact, cudaStream_t s);
 // gemm_gateup.cu: the prefill-sized counterpart (two accumulators per tile, SwiGLU in the epilogue)
 bool gateup_prefill_shapes_ok(int T, int I, int K);
 int launch_gateup_swiglu_prefill(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* act, int T, int I, int K, int x_row0, cudaStream_t s);

@@ -437,6 +437,10 @@ int b2k_few_attn(const void* qkv, const void* qnorm_w, const void* knorm_w, cons
                  const int32_t* block_table, int bt_stride, const int32_t* seq_lens, void* out, int B, int nq, int nkv, float eps, float scale, void* stream);
 /* out[rows][N] = x[rows][K] . w[N][K]^T at fp32 precision for fp32 x and bf16 w, as three exact bf16 products; planes: bf16 scratch [3][rows][K]. */
 int b2k_linear_split3(const float* x, void* planes_bf16, const void* w_bf16, float* out, int rows, int N, int K, int tile, void* stream);
+/* ... for fp32 w of bf16 numbers, narrowed into scratch first; the scratch holds plane_numbers numbers of x (three bf16 each) and narrow_numbers of w, and the product
+ * goes in pieces of whole tiles where that is less than all of them (at least 256 rows of each). */
+int b2k_linear_split3_wide(const float* x, const float* w, void* planes_bf16, size_t plane_numbers, void* narrow_bf16, size_t narrow_numbers, float* out, int rows, int N,
+                           int K, void* stream);
 /* Prompt attention whose softmax weights are mixed over at most sixteen heads (csrc/attn_postmix.cu): out[t][a] = sigmoid(gate[t][a]) * sum_j (sum_b talk[a][b] P_b[t][j])
  * v_{kv(a)}[j], P_b = softmax(scale q_b k - slope_b distance), slope_b = 2^(-slope_exp (b + 1) / heads) (slope_exp 0: none).  q fp32 [T][heads * dim]; caches bf16
  * [pages][block_size][kv_heads * dim or vdim]; tiles: {first row, its position, rows <= 64, block-table row}; gate may be null; out bf16 [T][heads * vdim]. */

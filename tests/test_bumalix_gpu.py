@@ -155,6 +155,22 @@ def test_each_mechanism_alone(name):
             assert err(e.get_logits(1)[0], ref[p]) < F32_BAR, "decoded position %d" % p
 
 
+def test_fp32_joined_projection_of_megabytes():
+    """fp32: the fused projection is a new matrix once the low-rank rows have joined it; at two megabytes and more the old one had a mapping of its own.  Its prompt product
+    takes the three-plane form, decode steps the kernel that reads the fp32 matrix."""
+    cfg = model([(par(4, 2, 64, 64, 0.125, 40, 4, 64, 128, 8.0, rank=16), None), (delta(8, 8, 64, 64, 4, rank=24), None)], vocab=97, width=512)
+    w = random_weights(cfg, seed=74)
+    toks = tokens(cfg, 140, 75)
+    ref = ref_logits(cfg, w, toks)
+    with engine(cfg, w) as e:
+        sid = e.seq_create(160)
+        lg, _ = e.prefill_logits([sid], [toks[:130]], list(range(130)))
+        assert err(lg, ref[:130]) < F32_BAR
+        for p in range(130, 140):
+            e.decode_step([sid], in_tokens=[toks[p]], want_output=False)
+            assert err(e.get_logits(1)[0], ref[p]) < F32_BAR
+
+
 def test_router_weights_scale_the_input_not_the_output():
     """The restatement itself: with a gated expert, weighting the input differs from weighting the output, and the engine follows
     the first."""

@@ -609,7 +609,7 @@ def test_fp32_prompt_rows_take_nothing_from_what_they_do_not_see(mixer, bad, cle
 
 
 def test_fp32_products_follow_a_reloaded_weight():
-    """The fp32 products of prompt size read bf16 copies of the weights: a tensor that is loaded again behind the finalisation counts from the next step on."""
+    """The fp32 products of prompt size narrow the weights to bf16: a tensor that is loaded again behind the finalisation counts from the next step on."""
     import ctypes as C
     cfg = cfg_c()
     w = random_weights(cfg, seed=5)
@@ -622,3 +622,17 @@ def test_fp32_products_follow_a_reloaded_weight():
         assert e.lib.b2_engine_load_tensor(e.h, b"l0.mlp.down", C.c_void_p(t.data_ptr()), t.numel() * 2) == 0
         got, _ = e.prefill_logits([e.seq_create(256)], [toks], [199])
     assert err(got[0], ref_logits(cfg, new, toks)[199]) < F32_BAR
+
+
+def test_fp32_weights_are_held_once():
+    """The products on the tensor pipe work in a scratch of fixed size that the engine takes when it is made: loading and finalising take no device memory, so what the
+    caller left for others stays."""
+    cfg = model([(att(4, 2, 64, 64, 0.125, rot=64), ff(8192))], vocab=8000, width=512)
+    w = {k: v.to(torch.bfloat16) for k, v in random_weights(cfg, seed=8).items()}
+    P = pkg()
+    with P.Engine(P.EngineConfig.kedasun(cfg, compute_f32=True, max_model_len=256, num_blocks=20, max_seqs=2, max_batch_tokens=256)) as e:
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        e.load_state_dict(w)
+        assert e.info()["weight_bytes"] > 80 << 20
+        assert before - torch.cuda.mem_get_info()[0] < 6 << 20   # (copies of the matrices would be 42 MB)

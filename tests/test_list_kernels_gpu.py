@@ -218,6 +218,27 @@ def test_linear_split3(lib, tile, rows, N, K):
     assert torch.isfinite(planes[:, 0].float()).all() and ((got[0] - big).abs() <= 2.0 ** -15 * (odd[0].double().abs().cuda() @ dw.double().abs().T))[sure & torch.isfinite(got[0])].all()
 
 
+@pytest.mark.parametrize("rows,N,K,rows_at_a_time,cols_at_a_time", [(1, 64, 64, 1, 64), (255, 300, 128, 255, 256), (300, 600, 320, 256, 256), (1030, 257, 64, 300, 600),
+                                                                     (513, 1100, 192, 512, 511)])
+def test_linear_split3_wide(lib, rows, N, K, rows_at_a_time, cols_at_a_time):
+    """fp32 weights that are bf16 numbers, narrowed into the scratch: the bits of the product with bf16 weights, whole and in pieces of whole tiles, and nothing else written."""
+    g = torch.Generator().manual_seed(rows + N + K)
+    x = (torch.randn(rows, K, generator=g) * torch.exp2(torch.randint(-20, 20, (rows, K), generator=g).float())).cuda()
+    w = (torch.randn(N, K, generator=g) * K ** -0.5).to(torch.bfloat16).cuda()
+    w[0, 0], w[N - 1, K - 1] = float("inf"), -0.0
+    whole, planes = torch.empty(rows, N, device="cuda"), torch.empty(3, rows, K, dtype=torch.bfloat16, device="cuda")
+    chk(lib, lib.b2k_linear_split3(ptr(x), ptr(planes), ptr(w), ptr(whole), rows, N, K, 0, cuda_stream_ptr()))
+    nx, nw = rows_at_a_time * K, cols_at_a_time * K
+    planes, narrow = torch.full((3 * nx + 8,), 3.0, dtype=torch.bfloat16, device="cuda"), torch.full((nw + 8,), 3.0, dtype=torch.bfloat16, device="cuda")
+    out, wide = torch.full((rows + 3, N), 7.0, device="cuda"), w.float()
+    chk(lib, lib.b2k_linear_split3_wide(ptr(x), ptr(wide), ptr(planes), nx, ptr(narrow), nw, ptr(out), rows, N, K, cuda_stream_ptr()))
+    torch.cuda.synchronize()
+    assert torch.equal(out[:rows].view(torch.int32), whole.view(torch.int32)) and (out[rows:] == 7.0).all()
+    assert (planes[3 * nx:] == 3.0).all() and (narrow[nw:] == 3.0).all()
+    if rows > 256:   # no whole tile fits
+        assert lib.b2k_linear_split3_wide(ptr(x), ptr(wide), ptr(planes), 255 * K, ptr(narrow), nw, ptr(out), rows, N, K, cuda_stream_ptr()) != 0
+
+
 @pytest.mark.parametrize("heads,kv,dim,vdim,window,keep,bs", [(16, 8, 128, 128, 70, 9, 16), (16, 16, 64, 64, 0, 0, 32), (5, 1, 128, 64, 33, 0, 48), (8, 4, 64, 128, 16, 40, 16),
                                                               (1, 1, 128, 128, 1, 5, 16), (12, 4, 128, 128, 100, 16, 64)])
 def test_heads_postmix(lib, heads, kv, dim, vdim, window, keep, bs):

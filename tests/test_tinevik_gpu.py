@@ -189,6 +189,15 @@ def test_each_mechanism_alone(name):
         run_schedule(e, cfg, toks, ref, F32_BAR, [2, 31, 3, 16, 2], 54)         # portions, then 21 decode steps
 
 
+def test_fp32_joined_projection_of_megabytes():
+    """fp32: the fused projection is a new matrix once the low-rank rows have joined it; at two megabytes and more the old one had a mapping of its own."""
+    cfg = model([(gla(4, 64, 128, 8.0, rank=24), None)], vocab=97, width=512)
+    w = random_weights(cfg, seed=76)
+    toks = tokens(cfg, 140, 77)
+    with engine(cfg, w) as e:
+        run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), F32_BAR, [100, 30], 130)
+
+
 @pytest.mark.parametrize("make", [cfg_a, cfg_b, cfg_c])
 def test_bf16_close_to_the_restatement(make):
     cfg = make()
