@@ -316,7 +316,7 @@ struct b2_engine {
   int prefill_pairs = 1;  // B2_PREFILL_PAIRS: see prefill_tile_pairs()
   int prefill_mc = 1;  // B2_MC: prefill projections on pairs of CTAs (gemm_mc.cu)
   int gu_prefill_fused = 1;  // B2_GU_FUSED: prefill-sized gate/up projection with SwiGLU in its epilogue (gemm_gateup.cu)
-  bool step_long = false;   // the step's contexts are too long for those kernels (pick_attn_split)
+  bool step_long = false;   // the step's contexts are too long for gemm_few.cu's kernels (pick_attn_split)
   int use_few = 1;    // B2_FEW: 0 = at most eight sequences take the kernels of larger batches (cross-check)
   int use_pair = 1;   // B2_PAIR: bit 0 gate/up + SwiGLU, bit 1 QKV + QK-norm/RoPE/KV write as fused cluster-pair launches (gemm_pair.cu)
 
@@ -459,15 +459,6 @@ int bucket_batch(int B) {
   for (int v : bk)
     if (B <= v) return v;
   return ((B + 127) / 128) * 128;
-}
-
-int pick_attn_split(b2_engine* e, int B, int max_len) {
-  // The slot of the graph key tells the step variants apart: 1 arg-max only, 2 logits written too; + 2 where the contexts are too long for the kernels of few
-  // sequences (gemm_few.cu: a cluster per sequence and kv head, however long the sequence, against attn_decode.cu's even share of all pages per warp).
-  // 16 steps of 28 layers, ms, few / larger batches' kernels: 1 x 1500 tokens 10.4 / 22.6, 1 x 12000 25.6 / 31.9, 4 x 1500 12.7 / 22.4, 4 x 4000 17.7 / 24.3,
-  // 8 x 1500 17.9 / 20.7, 8 x 4000 28.1 / 27.1, 4 x 12000 34.4 / 32.9.
-  const bool long_contexts = B <= 8 && (long)B * max_len > 24576;
-  return ((e->debug_flags & 2) ? 2 : 1) + (long_contexts ? 2 : 0);
 }
 
 // ---- one Linear layer: picks SIMT GEMV or the tcgen05 kernel, bf16 or split-K partial output
@@ -785,6 +776,26 @@ int forward_opt(b2_engine* e, int T, int ntiles, int nlast) {
   return lm_head_and_argmax(e, nlast, xl, xb);
 }
 
+// The fused launches that a decode step of T rows takes
+struct DecodeForms { bool qkv_pair = false, gu_pair = false, resid = false, few = false; };
+DecodeForms decode_forms(const b2_engine* e, const LayerW& L, int T, bool beside_attention) {
+  const b2_config& c = e->cfg;
+  const int H = c.hidden, I = c.intermediate;
+  auto skipped = [&](int k) { return ((e->skip_mask >> k) & 1u) != 0; };
+  DecodeForms f;
+  const bool pair_ok = !beside_attention && e->force_gemm_impl != 0 && T > e->simt_max_tokens && pair_shapes_ok(T, H) && !(e->debug_flags & 1) && e->kv_l2_budget <= 0;
+  f.qkv_pair = pair_ok && (e->use_pair & 2) && c.arch == B2_ARCH_QWEN3 && e->native_geom && e->rotary_dim == 128 && L.qnorm != nullptr && !skipped(B2K_ROPE_KV);
+  f.gu_pair = pair_ok && (e->use_pair & 1) && I % 64 == 0 && !skipped(B2K_ACT);
+  // ... with both in place the O / down projections add into the residual stream themselves (gemm_resid.cu) and the
+  // pair kernels normalise h as they load it: no norm kernel inside the layer loop (skip-mask ablations take the old path)
+  f.resid = f.qkv_pair && f.gu_pair && (e->use_pair & 4) && e->ssq != nullptr && H / 16 <= 64 && resid_shapes_ok(T, H, e->q_size) && resid_shapes_ok(T, H, I) &&
+            !skipped(B2K_NORM) && !skipped(B2K_GEMM_O) && !skipped(B2K_GEMM_DOWN) && !skipped(B2K_GEMM_QKV) && !skipped(B2K_GEMM_GATEUP);
+  // ... and at most eight sequences take the kernels of gemm_few.cu, unless their contexts are too long (pick_attn_split)
+  f.few = f.resid && few_shapes_ok(T, H, e->q_size, I) && e->nq == 2 * e->nkv && e->hd == 128 && c.block_size == 16 && c.sliding_window <= 0 && e->use_few &&
+          e->skip_mask == 0 && !e->l2_weight_prefetch;
+  return f;
+}
+
 // The decoder layers and the final norm over the lane's rows [row0, row0 + T): everything between the embedding and
 // the lm_head.  Qwen3 / Phi-3 (HF:models/qwen3/modeling_qwen3.py:423-434).
 int forward_layers(b2_engine* e, const Lane& ln, int T, int ntiles) {
@@ -830,19 +841,10 @@ int forward_layers(b2_engine* e, const Lane& ln, int T, int ntiles) {
     bf16* vp = kp + e->layer_kv_elems;
     // decode-sized forwards: the fused cluster-pair launches of gemm_pair.cu take the place of (projection, element-wise
     // kernel) pairs where the model's shapes allow it
-    const bool pair_ok = ntiles == 0 && !ln.beside_attention && e->force_gemm_impl != 0 && T > e->simt_max_tokens && pair_shapes_ok(T, H) &&
-                         !(e->debug_flags & 1) && e->kv_l2_budget <= 0;
-    const bool qkv_pair = pair_ok && (e->use_pair & 2) && c.arch == B2_ARCH_QWEN3 && e->native_geom && e->rotary_dim == 128 && L.qnorm != nullptr &&
-                          !((e->skip_mask >> B2K_ROPE_KV) & 1u);
-    const bool gu_pair = pair_ok && (e->use_pair & 1) && I % 64 == 0 && !((e->skip_mask >> B2K_ACT) & 1u);
-    // ... and with both in place the O / down projections add into the residual stream themselves (gemm_resid.cu) and the
-    // pair kernels normalise h as they load it: no norm kernel inside the layer loop (skip-mask ablations take the old path)
-    const bool resid = qkv_pair && gu_pair && (e->use_pair & 4) && e->ssq != nullptr && H / 16 <= 64 && resid_shapes_ok(T, H, e->q_size) &&
-                       resid_shapes_ok(T, H, I) && !((e->skip_mask >> B2K_NORM) & 1u) && !((e->skip_mask >> B2K_GEMM_O) & 1u) &&
-                       !((e->skip_mask >> B2K_GEMM_DOWN) & 1u) && !((e->skip_mask >> B2K_GEMM_QKV) & 1u) && !((e->skip_mask >> B2K_GEMM_GATEUP) & 1u);
-    // ... and at most eight sequences take the kernels of gemm_few.cu: five launches a layer too, for a chain that is bound by latencies
-    if (resid && few_shapes_ok(T, H, e->q_size, I) && e->nq == 2 * e->nkv && e->hd == 128 && c.block_size == 16 && c.sliding_window <= 0 && e->use_few && !e->step_long && e->skip_mask == 0 &&
-        !e->l2_weight_prefetch) {
+    // (at most eight sequences: five launches a layer too, for a chain that is bound by latencies)
+    const DecodeForms forms = ntiles == 0 ? decode_forms(e, L, T, ln.beside_attention) : DecodeForms();
+    const bool qkv_pair = forms.qkv_pair, gu_pair = forms.gu_pair, resid = forms.resid;
+    if (forms.few && !e->step_long) {
       {
         KL k(e, B2K_GEMM_QKV);
         B2_TRY(launch_few_qkv(L.wqkv, h, L.ln1, c.rms_eps, qkvb, T, e->qkv_size, H, st));
@@ -2417,6 +2419,17 @@ int forward_streams_list(b2_engine* e, int T, int ntiles, int nlast) {
 bool two_lane_decode(const b2_engine* e, int T, int ntiles) {
   return ntiles == 0 && e->mb_min_batch > 0 && T >= e->mb_min_batch && T <= 128 && T % 2 == 0 && e->stream2 != nullptr &&
          !e->profiling && !(e->debug_flags & 1) && e->force_gemm_impl != 0 && (T / 2) > e->simt_max_tokens;
+}
+
+// The slot of the graph key tells the step variants apart: 1 arg-max only, 2 logits written too; + 2 where the step would take the kernels of few sequences
+// but its contexts hold too many tokens in all for them (gemm_few.cu: a cluster per sequence and kv head, however long the sequence, against attn_decode.cu's even
+// share of all pages per warp).
+// 16 steps of 28 layers, ms, few / larger batches' kernels: 1 x 1500 tokens 10.4 / 22.6, 1 x 12000 25.6 / 31.9, 4 x 1500 12.7 / 22.4, 4 x 4000 17.7 / 24.3,
+// 8 x 1500 17.9 / 20.7, 8 x 4000 28.1 / 27.1, 4 x 12000 34.4 / 32.9.
+constexpr long FEW_CONTEXT_TOKENS = 24576;
+int pick_attn_split(const b2_engine* e, int B, long context_tokens) {
+  const bool too_long = context_tokens > FEW_CONTEXT_TOKENS && !e->layers.empty() && !two_lane_decode(e, B, 0) && decode_forms(e, e->layers[0], B, false).few;
+  return ((e->debug_flags & 2) ? 2 : 1) + (too_long ? 2 : 0);
 }
 
 int forward(b2_engine* e, int T, int ntiles, int nlast, int attn_split) {
@@ -5808,14 +5821,14 @@ namespace {
 int prepare_decode(b2_engine* e, int n, const int32_t* seq_ids, const int32_t* in_tokens, int* B_out, int* split_out) {
   B2_REQUIRE(e->finalized, "decode: weights not finalized");
   B2_REQUIRE(n >= 1 && n <= e->cfg.max_seqs, "decode: batch %d outside [1, max_seqs=%d]", n, e->cfg.max_seqs);
-  int max_len = 0;
+  long context_tokens = 0;
   for (int i = 0; i < n; ++i) {
     B2_TRY(check_seq(e, seq_ids[i]));
     Seq& s = e->seqs[seq_ids[i]];
     B2_REQUIRE(s.len >= 1, "decode: sequence %d has no prefilled tokens", seq_ids[i]);
     B2_REQUIRE(s.len + 1 <= s.reserved, "decode: sequence %d would exceed its reservation (%d tokens)", seq_ids[i], s.reserved);
     s.chain_open = false;  // generated tokens are not registered in the prefix cache
-    max_len = std::max(max_len, s.len + 1);
+    context_tokens += s.len + 1;
   }
   const int B = e->cfg.use_cuda_graphs ? bucket_batch(n) : n;
   const bool same = (int)e->cur_batch.size() == n && e->cur_B == B && std::equal(seq_ids, seq_ids + n, e->cur_batch.begin());
@@ -5845,7 +5858,7 @@ int prepare_decode(b2_engine* e, int n, const int32_t* seq_ids, const int32_t* i
     B2_CUDA_OK(cudaEventRecord(e->ev_tok, e->stream));
   }
   *B_out = B;
-  *split_out = pick_attn_split(e, B, max_len);
+  *split_out = pick_attn_split(e, B, context_tokens);
   return 0;
 }
 }  // namespace
@@ -5939,9 +5952,9 @@ extern "C" int b2_decode_run(b2_engine* e, int32_t nseq, const int32_t* seq_ids,
   cudaEvent_t ev0 = e->ev_pool[e->ev_pool.size() - 2], ev1 = e->ev_pool[e->ev_pool.size() - 1];
   int done = 0;
   {
-    int max_len = 0;
-    for (int i = 0; i < nseq; ++i) max_len = std::max(max_len, e->seqs[seq_ids[i]].len + steps);
-    split = pick_attn_split(e, B, max_len);  // one graph for the whole run
+    long context_tokens = 0;
+    for (int i = 0; i < nseq; ++i) context_tokens += e->seqs[seq_ids[i]].len + steps;
+    split = pick_attn_split(e, B, context_tokens);  // one graph for the whole run
   }
   if (graphs_enabled(e)) B2_TRY(ensure_graph(e, B, split));
   B2_CUDA_OK(cudaEventRecord(ev0, e->stream));
