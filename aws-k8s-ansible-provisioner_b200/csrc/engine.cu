@@ -3614,7 +3614,6 @@ int state_engine_alloc(b2_engine* e) {
   B2_TRY(dalloc(&e->l_ntiles, (size_t)1));
   if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
     B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
-    B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
   }
   B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));
   B2_CUDA_OK(cudaMemset(e->l_pair_slot, 0, Tc * max_top * 4));
@@ -3920,7 +3919,6 @@ int mixed_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&e->l_ntiles, (size_t)1));
     if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
-      B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
     }
     B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));
     B2_CUDA_OK(cudaMemset(e->l_pair_slot, 0, Tc * max_top * 4));
@@ -4177,7 +4175,7 @@ int outnorm_engine_alloc(b2_engine* e) {
     B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));
     if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
-      B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
+      if (Tc * max_top >= (size_t)LIST_SILU_EXPERT_ROWS) B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));   // (list_gated_experts)
     }
   }
   for (int32_t** p : {&e->d_row_seq, &e->d_row_first, &e->d_row_end}) {
@@ -4483,7 +4481,7 @@ int streams_engine_alloc(b2_engine* e) {
     B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));
     if (!e->f32 && Tc * max_top >= (size_t)list_tc_expert_rows() && max_exp > 1) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
-      B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
+      if (Tc * max_top >= (size_t)LIST_SILU_EXPERT_ROWS) B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));   // (list_gated_experts)
     }
   }
   for (int32_t** p : {&e->d_row_seq, &e->d_row_first, &e->d_row_end}) {
@@ -4664,8 +4662,6 @@ int list_engine_alloc(b2_engine* e) {
     B2_TRY(dalloc(&e->l_attn_scratch, e->l_attn_scratch_floats));
     if (max_top > 0 && Tc * max_top >= (size_t)list_tc_expert_rows()) {   // prompt-sized expert products on the tcgen05 projection kernel
       B2_TRY(dalloc(&e->l_xperm, Tc * max_top * W));
-      B2_TRY(dalloc(&e->l_upf, Tc * max_top * max_ff));
-      B2_CUDA_OK(cudaMallocHost(&e->h_offsets, (size_t)(max_exp + 1) * sizeof(int32_t)));
     }
   }
   B2_CUDA_OK(cudaMemset(e->l_ntiles, 0, 4));

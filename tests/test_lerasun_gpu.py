@@ -550,3 +550,17 @@ def test_layers_with_and_without_the_rebuilt_form():
         y, _ = e.prefill_logits([s[1], s[0]], [p[1][20:], p[0][140:]], list(range(180)))
         for got, ref in ((x[:140], refs[0][:140]), (x[140:], refs[1][:20]), (y[:20], refs[1][20:]), (y[20:], refs[0][140:])):
             assert np.abs(got - ref).max() / scale < BF16_BAR
+
+
+def test_a_step_of_experts_takes_the_buffers_that_it_uses():
+    """The experts' activation (8192 tokens, four choices, 1024 wide: 67 MB), their output and the gathered rows; the sums in front of the activation stay in the product."""
+    P = pkg()
+    cfg = {"architecture": "Lerasun", "vocab": 211, "width": 128, "logit_scale": 0.5, "norm": {"eps": 1e-6},
+           "layers": [layer(mixer(2, 32, 16, 32, 64, 0.2), moe(1024, 8, 4, 1, 1))]}
+    engine(cfg, random_weights(cfg, seed=3), f32=False).close()   # (modules and the allocator's first pools)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    with P.Engine(P.EngineConfig.lerasun(cfg, max_model_len=1024, num_blocks=80, max_seqs=4, max_batch_tokens=8192)):
+        taken = before - torch.cuda.mem_get_info()[0]
+    act, out, rows = 8192 * 4 * 1024 * 2, 8192 * 4 * 128 * 4, 8192 * 4 * 128 * 2
+    assert taken < act + out + rows + (110 << 20), taken   # (the sums as fp32 would be 134 MB)
