@@ -63,7 +63,7 @@ struct AdPos {  // a position on the page line
 };
 
 #ifndef B2_ATTN_TRACE_BY_SMID
-#define B2_ATTN_TRACE_BY_SMID 1  // timing breadcrumbs indexed by SM id (tools/attn_timeline.py)
+#define B2_ATTN_TRACE_BY_SMID 1  // timing breadcrumbs indexed by SM id
 #endif
 template <int AD_WARPS, int AD_STAGES>
 __global__ void __launch_bounds__(AD_WARPS * 32, 1)
@@ -423,7 +423,7 @@ attn_decode_kernel(const bf16* q, const bf16* k_pages, const bf16* v_pages,
   }
   arrive_all(pending, npending);
   B2_STAMP_END_AUX(B2K_ATTN_DECODE, (unsigned)tag);  // warp 0's end: all warps of a CTA run the same number of pages
-  if (dbg_time) {  // timing breadcrumbs for tools/attn_timeline.py (unused words of the geometry header)
+  if (dbg_time) {  // timing breadcrumbs (unused words of the geometry header)
     unsigned long long t_end;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
     int* meta = reinterpret_cast<int*>(scratch);

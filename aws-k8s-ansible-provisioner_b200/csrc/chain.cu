@@ -41,7 +41,7 @@ struct ChainMaps {
   CUtensorMap x[4];  // attn, x, act, x                 box 64 x BN
 };
 
-// Optional trace (tools/chain_timeline.py): thread 0 of every CTA stamps %globaltimer when it enters
+// Optional trace: thread 0 of every CTA stamps %globaltimer when it enters
 // each step (slot = step), when its CTA has finished the step's work (16 + step) and when it leaves the
 // kernel: trace[blockIdx.x * 32 + slot].
 __device__ unsigned long long* g_chain_trace = nullptr;

@@ -168,12 +168,12 @@ inline cudaError_t b2_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 }
 
 // ---------------------------------------------------------------------------------------
-// Step timeline (tools/step_timeline.py): when a trace buffer is registered (b2k_debug_step_trace), thread 0 of
+// Step timeline: when a trace buffer is registered (b2k_debug_step_trace), thread 0 of
 // every CTA of every kernel on the decode path appends one record {class | blockIdx << 8 | smid << 32 | aux << 40, CTA start,
 // dependency wait returned, CTA end} (%globaltimer, ns).  buf[0] = record counter (atomic), buf[1] = capacity in
 // records, records start at buf[4].  Each .cu file holds its own copy of the pointer (no relocatable device code);
 // B2_STEP_TRACE_DEFINE(setter) defines it and its host-side setter.  Compiled in only with -DB2_STEP_TRACE
-// (tools/build_variant.sh trace -DB2_STEP_TRACE -> libb2engine_trace.so, which tools/step_timeline.py loads).
+// (a library built with -DB2_STEP_TRACE).
 // ---------------------------------------------------------------------------------------
 #ifdef B2_STEP_TRACE
 #define B2_STEP_TRACE_DEFINE(setter)                                              \
@@ -186,7 +186,7 @@ inline cudaError_t b2_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, si
 #define B2_STEP_TRACE_DEFINE(setter)                                                                              \
   int setter(unsigned long long* dev_buf) {                                                                       \
     if (dev_buf == nullptr) return 0;                                                                             \
-    b2_set_error("step trace: this library was built without -DB2_STEP_TRACE (tools/build_variant.sh trace ...)"); \
+    b2_set_error("step trace: this library was built without -DB2_STEP_TRACE"); \
     return -38;                                                                                                   \
   }
 #endif

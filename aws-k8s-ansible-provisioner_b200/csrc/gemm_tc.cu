@@ -26,7 +26,7 @@ namespace b2 {
 
 B2_STEP_TRACE_DEFINE(step_trace_set_gemm)
 
-// Optional phase trace (tools/gemm_timeline.py): when a buffer is registered, every CTA stamps
+// Optional phase trace: when a buffer is registered, every CTA stamps
 // %globaltimer at its phase boundaries into trace[blockIdx.x * 8 + slot].
 __device__ unsigned long long* g_tc_trace = nullptr;
 __device__ __forceinline__ void tc_stamp(int slot) {
@@ -68,7 +68,7 @@ __device__ __forceinline__ unsigned long long tc_argmax_pack(float v, int idx) {
 // warps put up to two on a scheduler, so it fits beside that CTA only if 2 x 32 x (200 + R) <= 16384, R <= 56.
 // XCP (decode shapes: one tile per CTA, its k-blocks all fit the stage ring): the X tiles do not come through the
 // tensor map but through cp.async issued by the four epilogue warps, which are idle until the accumulator is ready.
-// Measured in the captured step (tools/step_timeline.py): with TMA the first X tile lands 0.6-0.8 us after the
+// Measured in the captured step: with TMA the first X tile lands 0.6-0.8 us after the
 // dependency wait and every further one 0.35 us later (the tiled copy of a 64-row box is 64 requests of 128 bytes,
 // and dozens of CTAs ask for the same rows), so a CTA with 4-6 k-blocks issued its last MMA 1.8-2.4 us after the
 // wait; 128 threads x 16-byte LDGSTS have the whole slice in flight at once.

@@ -464,7 +464,7 @@ int b2k_qkv_rope_norm(const void* h_bf16, const void* w_qkv_bf16, const void* no
                       const int32_t* slots, void* q_out, void* k_pages, void* v_pages, int T, int nq, int nkv, int K, int block_size,
                       float eps, void* stream);
 
-/* Diagnostics (tools/step_timeline.py): register a device buffer of uint64 in which thread 0 of every CTA of every
+/* Diagnostics (a library built with -DB2_STEP_TRACE): register a device buffer of uint64 in which thread 0 of every CTA of every
  * kernel on the decode path appends one 4-word record {class | blockIdx << 8 | smid << 32 | aux << 40, CTA start,
  * dependency wait returned, CTA end} in %globaltimer ns.  The caller sets buf[0] = 0 (record counter) and
  * buf[1] = capacity in records; records start at buf[4].  NULL switches the trace off.  class 100 = a projection

@@ -47,7 +47,7 @@ def assert_bf16_close(got: torch.Tensor, ref: torch.Tensor, max_ulp: int, max_mi
 
 
 def rel_err(got: torch.Tensor, ref: torch.Tensor) -> float:
-    """max |got-ref| / max |ref|  -- the 'within 1e-2 relative' metric of BASELINE.json's north_star."""
+    """max |got-ref| / max |ref|  -- the 'within 1e-2 relative' metric."""
     g, r = got.float().cpu(), ref.float().cpu()
     return ((g - r).abs().max() / r.abs().max().clamp_min(1e-30)).item()
 
@@ -93,10 +93,9 @@ def kv_swizzle(pages: torch.Tensor) -> torch.Tensor:
 
 def record_parity(key: str, value) -> None:
     """Keeps the numbers a parity test printed (leading-match counts, gaps at the first mismatch, errors) in a JSON
-    file that outlives `pytest -q`: gpurun_out/parity.json on the GPU box (merged back by gpurun; copied to
-    profiles/ when committed as evidence)."""
+    file that outlives `pytest -q`: build/parity.json."""
     import json
-    d = os.path.join(ROOT, "gpurun_out")
+    d = os.path.join(ROOT, "build")
     try:
         os.makedirs(d, exist_ok=True)
         path = os.path.join(d, "parity.json")

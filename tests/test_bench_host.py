@@ -87,7 +87,7 @@ def test_single_rank_needs_no_process_group(monkeypatch):
 
 
 def test_timed_window_is_pinned_to_c2_whatever_the_step_count():
-    """VERDICT r1 #2: --steps must not shrink the workload.  Every (K, W) is timed around C2's mean context
+    """--steps must not shrink the workload.  Every (K, W) is timed around C2's mean context
     (512-token prompts, 256 new tokens -> 640.5) and both arms print the same config."""
     sys.path.insert(0, ROOT)
     import bench
@@ -97,7 +97,7 @@ def test_timed_window_is_pinned_to_c2_whatever_the_step_count():
         assert abs((lo + hi) / 2.0 - 640.5) <= 4.5, (K, W, lo, hi)
         cfg = bench.c2_config(1, K, W)
         assert cfg["new_tokens"] == 256 and cfg["timed_context"] == [lo, hi] and cfg["workload"] == "C2"
-        assert "5.9" in cfg["l2"]  # 5.90 GB +- the window's centre: SURVEY.md section 8d
+        assert "5.9" in cfg["l2"]  # 5.90 GB +- the window's centre
     # the reference arm prints exactly the GPU arm's config for the same flags
     import types
     got = []

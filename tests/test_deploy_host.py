@@ -1,4 +1,4 @@
-"""The launch boundary (SURVEY.md 8b "Launch"; /root/reference llm-d-deploy.yaml:147-151 copies the chart's slim base to
+"""The launch boundary (llm-d-deploy.yaml:147-151 copies the chart's slim base to
 custom-base.yaml, :176-184 hands it to llmd-installer.sh): deploy/values-b2serve.yaml must survive a deep merge into
 such a base file, and the argv the image's ENTRYPOINT + CMD plus the values file's extraArgs produce must be one that
 b2serve's own flag parser accepts.  helm/docker/yq are absent here: the merge is yq's `. * $i` (maps merge key by key,

@@ -1,6 +1,6 @@
 """Engine-level parity (GPU), through the C ABI: prefill + decode of the Qwen3 architecture against
 the oracle (HF transformers Qwen3 on CPU and its pinned restatement), on identical weights and
-inputs.  Tolerances are BASELINE.json's: greedy token ids identical (tie-aware: a mismatch is only
+inputs.  Tolerances: greedy token ids identical (tie-aware: a mismatch is only
 tolerated where the oracle's own top-1/top-2 logit gap is within bf16 noise), logits and per-layer
 hidden states within 1e-2 relative."""
 import importlib
@@ -17,7 +17,7 @@ from oracle.qwen3_oracle import (QWEN3_0_6B, QWEN3_TINY, KVState, Restated, atte
 
 pytestmark = pytest.mark.gpu
 GOLD = os.path.join(ROOT, "tests", "golden")
-REL_TOL = 1e-2  # "per-layer bf16 logits must agree within 1e-2 relative" (BASELINE.json north_star)
+REL_TOL = 1e-2  # "per-layer bf16 logits must agree within 1e-2 relative"
 
 
 @pytest.fixture(scope="module")
@@ -235,7 +235,7 @@ def test_errors_are_reported(P, tiny):
 
 
 # ---------------------------------------------------------------------------------------------
-# Full-size architecture, BASELINE.json config 1: batch 1, 128-token prompt -> 128 tokens
+# Full-size architecture: batch 1, 128-token prompt -> 128 tokens
 # ---------------------------------------------------------------------------------------------
 @pytest.fixture(scope="module")
 def full(P):
@@ -259,7 +259,7 @@ def test_full_c1_greedy_and_logits(P, full):
     with torch.no_grad():
         out = model(torch.tensor([full_ids]), output_hidden_states=True)
         # HF's own second attention implementation on the same weights: the bf16 noise floor of the
-        # oracle itself (SURVEY.md 7.2-1 measured sdpa vs eager at 1.5e-2 on the last layers)
+        # oracle itself (measured: sdpa vs eager at 1.5e-2 on the last layers)
         model.set_attn_implementation("eager")
         out_e = model(torch.tensor([full_ids]), output_hidden_states=True)
         model.set_attn_implementation("sdpa")
@@ -363,7 +363,7 @@ def test_full_alternative_decode_schedules(P, full, monkeypatch, chain):
 
 
 def test_full_batch64_properties(P):
-    """BASELINE.json config 2 shapes (batch 64, paged KV) through size-independent properties.
+    """The served shapes (batch 64, paged KV) through size-independent properties.
     64 copies of one prompt: the prefill (one CTA per sequence tile) must give 64 identical first tokens;
     decode must be deterministic run to run.  Decode attention balances pages over its warps, so where
     a sequence's pages are cut depends on its position in the batch: copies may legitimately separate at
@@ -485,7 +485,7 @@ def test_sharded_checkpoint_and_dtypes(P, tiny, tmp_path):
 
 
 def test_prefix_cache_reuses_prompt_pages(P, tiny):
-    """vLLM's --enable-prefix-caching in the engine (SURVEY.md 8f rank 2: the router's prefix affinity needs it): a second
+    """vLLM's --enable-prefix-caching in the engine (the router's prefix affinity needs it): a second
     prompt that shares a 448-token prefix with an earlier one prefills only its tail, gives the same greedy ids as the
     cold run, and pages are neither leaked nor rewritten while shared."""
     model, sd = tiny

@@ -1,9 +1,9 @@
-"""OPT variant of the hot path (SURVEY.md 8a row a13) through the C ABI on the GPU, against HF
+"""OPT variant of the hot path through the C ABI on the GPU, against HF
 OPTForCausalLM's own outputs (tests/golden/opt_tiny.npz) and the pinned restatement
 (oracle/opt_oracle.py).  Bars as for the other engine tests: hidden states and logits within 1e-2
 relative (or 1.5x / 2x the oracle's own bf16 noise floor where that is larger), greedy ids identical
 except after a step whose oracle top-2 gap is within bf16 noise.  OPT's 64-wide heads and one query
-head per kv head run zero-padded through the 128-wide kernels (DESIGN.md section 4)."""
+head per kv head run zero-padded through the 128-wide kernels."""
 import os
 
 import numpy as np

@@ -1,9 +1,9 @@
-"""Phi-3 variant of the hot path (SURVEY.md 8a row a14) through the C ABI on the GPU, against HF
+"""Phi-3 variant of the hot path through the C ABI on the GPU, against HF
 Phi3ForCausalLM's own outputs (tests/golden/phi3_tiny.npz) and against the pinned restatement
 (oracle/phi3_oracle.py).  Same bars as the Qwen3 engine tests: hidden states and logits within 1e-2
-relative (BASELINE.json), greedy ids identical except after a step whose oracle top-2 gap is within
+relative, greedy ids identical except after a step whose oracle top-2 gap is within
 bf16 noise.  The engine runs these models through its 128-wide, two-query-heads-per-kv-head kernels
-with zero padding placed in the weights (DESIGN.md section 4), so these tests are also the check that
+with zero padding placed in the weights, so these tests are also the check that
 the padding changes nothing."""
 import os
 

@@ -58,7 +58,7 @@ def test_restatement_is_bit_exact_vs_hf(tiny):
 
 
 def test_explicit_rounding_points_within_tolerance(tiny):
-    """attention_explicit (bf16 P, fp32 statistics) vs HF sdpa: the tolerance BASELINE.json states
+    """attention_explicit (bf16 P, fp32 statistics) vs HF sdpa: the stated tolerance
     for floating point is 1e-2 relative on logits."""
     model, sd, g = tiny
     ids = torch.from_numpy(g["prompt_ids"]).long()
@@ -82,7 +82,7 @@ def test_rope_table_inv_freq_is_fp32():
 
 
 def test_chat_template_fixture_matches_survey():
-    """SURVEY.md section 8c quotes four renderings of templates/opt-chat-template.yaml; the committed
+    """There are four quoted renderings of templates/opt-chat-template.yaml; the committed
     fixture must reproduce them (and the Phi variant with Human for User)."""
     fx = json.load(open(os.path.join(GOLD, "chat_templates.json")))
     opt = fx["opt-chat-template"]
@@ -98,7 +98,7 @@ def test_chat_template_fixture_matches_survey():
 
 
 def test_full_size_golden_is_reproducible():
-    """Config 1 of BASELINE.json on the real architecture: HF greedy ids (128 -> 128) must equal the
+    """A 128-token prompt on the real architecture: HF greedy ids (128 -> 128) must equal the
     committed fixture.  ~40 s of CPU; pins torch/transformers version drift."""
     fx = json.load(open(os.path.join(GOLD, "qwen3_0p6b_c1.json")))
     arch = QWEN3_0_6B
@@ -114,7 +114,7 @@ def test_full_size_golden_is_reproducible():
         1.0, abs(fx["weight_digests"]["model.embed_tokens.weight"]["sum"]))
 
 
-# ---- Phi-3 variant (SURVEY.md 8a row a14) ----------------------------------------------------
+# ---- Phi-3 variant ----------------------------------------------------
 @pytest.mark.parametrize("tag", ["full", "partial", "window"])
 def test_phi3_restatement_matches_golden(tag):
     """oracle/phi3_oracle.py against HF's own outputs (tests/golden/phi3_tiny.npz, written by
@@ -148,7 +148,7 @@ def test_phi3_restatement_matches_golden(tag):
                 assert gaps[b, int(d[0])] <= 0.0625
 
 
-# ---- OPT variant (SURVEY.md 8a row a13) -------------------------------------------------------
+# ---- OPT variant -------------------------------------------------------
 def test_opt_restatement_matches_golden():
     """oracle/opt_oracle.py against HF OPTForCausalLM's own outputs (tests/golden/opt_tiny.npz):
     teacher-forced logits bit for bit, greedy ids identical."""

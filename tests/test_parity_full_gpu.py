@@ -1,5 +1,5 @@
-"""Parity at the shapes that are benchmarked (GPU), against HF transformers itself, at the bars BASELINE.json's
-north_star states: greedy token ids identical over the first 128 generated tokens, logits within 1e-2 relative.
+"""Parity at the shapes that are benchmarked (GPU), against HF transformers itself, at these
+bars: greedy token ids identical over the first 128 generated tokens, logits within 1e-2 relative.
 
 "Identical" is asserted tie-aware, and the tie bar is tied to what is measured, not to a constant: where the engine's
 greedy token first differs from HF's, HF's own top-1/top-2 logit gap at that step must be within 2 bf16 ulp of the top
@@ -8,7 +8,7 @@ flip must be explained by the logit noise that was measured, nothing else.  Ever
 tokens, so the logits of ALL 128 steps are compared, also after such a flip.  The noise floor of the oracle itself is
 HF's second attention implementation (eager vs sdpa) on the same weights and tokens.
 
-The counts and gaps are written to gpurun_out/parity.json (tests/_util.record_parity), copied to profiles/qwen3_b_parity.json."""
+The counts and gaps are written to build/parity.json (tests/_util.record_parity)."""
 import os
 
 import numpy as np
@@ -74,7 +74,7 @@ def check_stream(tag, got_tok, got_logits, ref_tok, ref_logits, floor_logits):
 
 
 # ---------------------------------------------------------------------------------------------
-# BASELINE.json config 2's shape: batch 64, 512-token prompts, graph decode; 8 sequences x 128 tokens against HF
+# The served shape: batch 64, 512-token prompts, graph decode; 8 sequences x 128 tokens against HF
 # ---------------------------------------------------------------------------------------------
 C2_PICK = [0, 9, 18, 27, 36, 45, 54, 63]
 
@@ -139,7 +139,7 @@ def test_c2_shape_128_tokens_against_hf(P, c2_ref, two_lane):
 
 
 # ---------------------------------------------------------------------------------------------
-# the full 12-layer OPT-125m, batch 8, 128 -> 32 tokens against HF
+# The full 12-layer OPT-125m, batch 8, 128 -> 32 tokens against HF
 # ---------------------------------------------------------------------------------------------
 @pytest.mark.timeout(900)
 def test_c3_opt125m_full_depth_against_hf(P):
@@ -182,7 +182,7 @@ def test_c3_opt125m_full_depth_against_hf(P):
 
 
 # ---------------------------------------------------------------------------------------------
-# BASELINE.json config 4: Phi-3-mini-4k at full depth and width, one sequence, 64 teacher-forced positions past the
+# Phi-3-mini-4k at full depth and width, one sequence, 64 teacher-forced positions past the
 # 2047-token window, every layer's hidden state against HF
 # ---------------------------------------------------------------------------------------------
 @pytest.mark.timeout(2400)
@@ -290,7 +290,7 @@ def test_sampled_distribution_matches_softmax(P, temperature, top_k, top_p):
 
 
 def test_unseeded_sampling_never_emits_impossible_tokens(P):
-    """with top-k/top-p off, a uniform that could round to exactly 1.0 made a uniformly random
+    """With top-k/top-p off, a uniform that could round to exactly 1.0 made a uniformly random
     vocabulary id win with probability V x 2^-24 per draw -- 0.9 % at V = 151 936.  Full vocabulary, a sharp temperature
     (so that all but a handful of tokens are impossible), 4 000 draws without a seed: the old code fails this ~36 times."""
     arch = QWEN3_0_6B

@@ -1,5 +1,5 @@
 """b2route (csrc/router/router.cpp), the load- and prefix-aware front for several model-server replicas
-(SURVEY.md 8f rank 2), against fake replicas on localhost (CPU, no GPU): relaying of plain and streamed
+against fake replicas on localhost (CPU, no GPU): relaying of plain and streamed
 responses, prefix affinity, load shedding from the scraped vllm:* series, fail-over and its own /metrics."""
 import http.client
 import http.server

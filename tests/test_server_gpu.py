@@ -1,6 +1,6 @@
 """HTTP contract of the model-server binary (GPU): replays the two calls of the reference's smoke test
 (llm-d-test.yaml:32-43 GET /v1/models, :61-73 POST /v1/completions with {"model", "prompt"}) plus the
-chat, streaming, metrics and error surface of SURVEY.md section 8b, against b2serve on localhost with a
+chat, streaming, metrics and error surface, against b2serve on localhost with a
 scaled-down Qwen3 checkpoint; greedy completions are checked against the oracle."""
 import http.client
 import importlib
@@ -352,7 +352,7 @@ def test_starts_with_the_argv_the_image_and_the_values_file_give():
     """The launch boundary (llm-d-deploy.yaml:147-151,176-184): the pod runs deploy/Dockerfile's ENTRYPOINT + CMD with
     the chart's extraArgs (deploy/values-b2serve.yaml) appended.  Exactly that argv -- only the binary's path is the
     in-tree build instead of /opt/b2/bin -- must come up on port 8000, with no checkpoint at /models (random-init
-    weights of the served architecture, as BASELINE.json prescribes), and answer the reference's two requests."""
+    weights of the served architecture), and answer the reference's two requests."""
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
     import re

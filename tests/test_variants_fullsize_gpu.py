@@ -1,4 +1,4 @@
-"""BASELINE.json configs 3 and 4 at their full shapes (GPU), through size-independent properties.
+"""OPT-125m and Phi-3-mini at their full shapes (GPU), through size-independent properties.
 The CPU oracle cannot run these sizes in test time (config 4's prefill alone is ~500 TFLOP), so what is
 checked is what must hold for ANY correct engine at any size: identical prompts give identical first
 tokens, the same batch gives the same bits run after run, a sequence decodes the same stream inside a
@@ -141,7 +141,7 @@ def test_c4_phi3mini_batch32_prefill2048(P):
     prompt = make_prompts(1, PL, arch.vocab, seed=1)[0].tolist()
     toks, solo = properties(e, B, prompt, PL + 32, STEPS, chunk=4)
     # copies of one sequence sit in different rows, and decode attention cuts a row's pages by its place in the batch
-    # (DESIGN.md section 2): they may part at a step whose top two logits are within bf16 noise of each other, not elsewhere
+    # (sums in another order): they may part at a step whose top two logits are within bf16 noise of each other, not elsewhere
     if not (toks[0] == toks[0, 0]).all():
         assert properties.step0_gap_ulp <= 2.0, "first decode step differs across identical sequences away from a tie (gap %.1f ulp)" % properties.step0_gap_ulp
     together = (toks == toks[:, :1]).all(axis=0).mean()
