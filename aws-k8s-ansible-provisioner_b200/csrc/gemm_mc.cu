@@ -13,6 +13,7 @@
 //   * "accumulator empty" (the first CTA's): a lane of every epilogue warp of both CTAs
 // Everything else is gemm_tc.cu's plain bf16 path: swap-AB (weight rows on MMA-M, tokens on MMA-N), double-buffered TMEM
 // accumulator, four epilogue warps, same k order -> the same bits (tests/test_kernels_gpu.py::test_linear_multicast).
+#include "cta_pair.cuh"
 #include "kernels.h"
 
 namespace b2 {
@@ -30,44 +31,6 @@ constexpr int MC_SMEM_BYTES = MC_STAGES * MC_STAGE_BYTES + 2 * MC_OUT_BYTES + 10
 constexpr int MC_ROPE_GROUPS = 4;                             // ROPE variant: epilogue warp groups (four warps each)
 constexpr int MC_ROPE_ROWS = 16;                              // ... and tokens per staged block (4 KB; the groups' blocks fill the two 8 KB buffers)
 constexpr int MC_ROPE_THREADS = 64 + 128 * MC_ROPE_GROUPS;
-
-__device__ __forceinline__ uint32_t mc_cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t mc_first_cta(uint32_t addr) {   // the same place in the first CTA's shared memory
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
-  return r;
-}
-// into this CTA's shared memory; the bytes are counted on a barrier of either CTA of the pair
-__device__ __forceinline__ void mc_tma_load_2d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst_smem), "l"(tmap), "r"(bar),
-               "r"(c0), "r"(c1)
-               : "memory");
-}
-// D[256 x 256, 128 rows in each CTA's TMEM] (+)= A[256] * B[256]: each CTA's shared memory holds 128 rows of A and 128 of B
-__device__ __forceinline__ void mc_mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void mc_commit(uint32_t bar) {   // to the barrier of both CTAs
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
-}
-__device__ __forceinline__ void mc_arrive_cluster(uint32_t cluster_bar) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
-}
-__device__ __forceinline__ void mc_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // ROPE variant (QKV projection of a Qwen3-geometry prefill: one 128-wide head per weight-row tile): the staged 32-token block
 // is not stored as it is but finished as qknorm_rope_kv does -- per-head RMS norm of q and k, RoPE, then q through a TMA store
@@ -100,7 +63,7 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   __shared__ __align__(16) bf16 s_gain[ROPE ? 256 : 8];             // QK-norm gains, q then k
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = mc_cluster_rank();
+  const uint32_t rank = pair_rank();
   const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
   const int kb_total = K / MC_BK;
   const int total = m_pairs * n_tiles;
@@ -127,7 +90,7 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   const B2Waits wait{&gave_up, limit};
-  mc_cluster_sync();  // the peer's barriers exist before anything of mine can arrive on them, and its TMEM is taken
+  pair_cluster_sync();  // the peer's barriers exist before anything of mine can arrive on them, and its TMEM is taken
   pdl_wait();
   if (threadIdx.x == 0) pdl_launch_dependents();
   int sent = 0;   // (producer: stages filled)
@@ -140,11 +103,11 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
       for (int kb = 0; kb < kb_total; ++kb) {
         const int s = sent % MC_STAGES;
         if (!wait(empty_bar[s], ((sent / MC_STAGES) & 1) ^ 1)) return;  // the pair's MMAs are done with this stage
-        const uint32_t fb = mc_first_cta(smem_u32(&full_bar[s]));
+        const uint32_t fb = pair_first_cta(smem_u32(&full_bar[s]));
         if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * MC_STAGE_BYTES);
         const uint32_t ws = smem_base + s * MC_STAGE_BYTES;
-        mc_tma_load_2d(ws, &tmap_w, kb * MC_BK, m_tile * MC_BM, fb);
-        mc_tma_load_2d(ws + MC_W_BYTES, &tmap_x, kb * MC_BK, n_tile * MC_BN + (int)rank * (MC_BN / 2) + x_row0, fb);   // this CTA's half of the token rows
+        pair_tma_load_2d(ws, &tmap_w, kb * MC_BK, m_tile * MC_BM, fb);
+        pair_tma_load_2d(ws + MC_W_BYTES, &tmap_x, kb * MC_BK, n_tile * MC_BN + (int)rank * (MC_BN / 2) + x_row0, fb);   // this CTA's half of the token rows
         ++sent;
       }
     }
@@ -168,17 +131,17 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
         const uint64_t da = umma_desc_sw128(ws), db = umma_desc_sw128(ws + MC_W_BYTES);
 #pragma unroll
         for (int k = 0; k < MC_BK / 16; ++k)
-          mc_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
-        mc_commit(smem_u32(&empty_bar[s]));
+          pair_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (kb > 0 || k > 0) ? 1u : 0u);
+        pair_commit(smem_u32(&empty_bar[s]));
       }
-      mc_commit(smem_u32(&tmem_full_bar[as]));
+      pair_commit(smem_u32(&tmem_full_bar[as]));
     }
   };
   // a warp's share of the accumulator is in registers: back to the MMA thread, which waits for both CTAs' warps
   auto hand_back = [&](int as) {
     tc_fence_before();
     __syncwarp();
-    if (lane == 0) mc_arrive_cluster(mc_first_cta(smem_u32(&tmem_empty_bar[as])));
+    if (lane == 0) pair_arrive(pair_first_cta(smem_u32(&tmem_empty_bar[as])));
   };
   auto finish = [&]() {
     if constexpr (!ROPE) {
@@ -372,7 +335,7 @@ linear_mc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_consta
   }
   // no CTA leaves while its peer's loads may still be counted on its barriers, or the pair's MMAs read its shared memory
   __syncwarp();
-  mc_cluster_sync();
+  pair_cluster_sync();
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");

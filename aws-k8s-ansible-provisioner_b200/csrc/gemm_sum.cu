@@ -8,10 +8,12 @@
 //     the next group (or to nobody: zero-filled) and are not stored.
 //   * epilogue: fp32 sums straight from registers (a warp's 32 weight rows are 128 contiguous bytes of an output row), or, for squared-ReLU experts, their
 //     activation rounded to the bf16 operand of the second product.
-//   * SPLIT (3; 1: the same sums for bf16 x): x is fp32, given as three bf16 planes whose sum it is (split3_kernel: 8 + 8 + 8 bits of the 24), and the weights are bf16 numbers, so the three
+//   * SPLIT 3: x is fp32, given as three bf16 planes whose sum it is (split3_kernel: 8 + 8 + 8 bits of the 24), and the weights are bf16 numbers, so the three
 //     products are exact.  The tensor pipe's accumulator rounds every addition towards zero, so it holds only 128 of the K at a time, smallest plane first: the
-//     epilogue's warps keep the running sums of a tile in registers and add a chunk, rounded to nearest, while the next one is multiplied.
+//     epilogue's warps keep the running sums of a tile in registers and add a chunk, rounded to nearest, while the next one is multiplied.  SPLIT 1: the same
+//     sums for bf16 x.
 // Bound: tensor pipe under the power cap, and the last wave.
+#include "cta_pair.cuh"
 #include "kernels.h"
 
 namespace b2 {
@@ -30,41 +32,6 @@ struct GsCfg {
 };
 constexpr int GS_CHUNK_KB = 2;   // SPLIT: k-blocks per chunk
 constexpr int GS_EPI_WARPS = 8, GS_THREADS = 64 + 32 * GS_EPI_WARPS;
-
-__device__ __forceinline__ uint32_t gs_cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t gs_first_cta(uint32_t addr) {   // the same place in the first CTA's shared memory
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
-  return r;
-}
-// into this CTA's shared memory; the bytes are counted on a barrier of either CTA of the pair
-__device__ __forceinline__ void gs_tma_load_2d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, uint32_t bar) {
-  asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst_smem), "l"(tmap), "r"(bar),
-               "r"(c0), "r"(c1)
-               : "memory");
-}
-// D[256 x BN, 128 rows in each CTA's TMEM] (+)= A[256] * B[BN]: each CTA's shared memory holds 128 rows of A and half of B
-__device__ __forceinline__ void gs_mma_bf16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
-      "}\n" ::"r"(tmem_d),
-      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void gs_commit(uint32_t bar) {   // to the barrier of both CTAs
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
-}
-__device__ __forceinline__ void gs_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // The tiles of all groups, in order: group by group, tile of rows by tile of rows, weight-row pair fastest.  A walker moves forward only.
 template <int BN>
@@ -108,7 +75,7 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   __shared__ int s_off[GS_MAX_GROUPS + 1];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = gs_cluster_rank();
+  const uint32_t rank = pair_rank();
   const int cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
   constexpr int PLANES = SPLIT > 0 ? SPLIT : 1;
   const int kb_total = K / GS_BK, chunk_kb = SPLIT > 0 ? GS_CHUNK_KB : kb_total, m_pairs = (N + 2 * GS_BM - 1) / (2 * GS_BM);
@@ -142,7 +109,7 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   tc_fence_after();
   const uint32_t tmem_base = tmem_slot;
   const B2Waits wait{&gave_up, limit};
-  gs_cluster_sync();  // the peer's barriers exist before anything of mine can arrive on them, and its TMEM is taken
+  pair_cluster_sync();  // the peer's barriers exist before anything of mine can arrive on them, and its TMEM is taken
   int sent = 0;       // (producer: stages filled)
 
   auto produce = [&]() {   // (one thread)
@@ -157,11 +124,11 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           for (int kb = c0; kb < min(kb_total, c0 + chunk_kb); ++kb) {
             const int s = sent % C::STAGES;
             if (!wait(empty_bar[s], ((sent / C::STAGES) & 1) ^ 1)) return;  // the pair's MMAs are done with this stage
-            const uint32_t fb = gs_first_cta(smem_u32(&full_bar[s]));
+            const uint32_t fb = pair_first_cta(smem_u32(&full_bar[s]));
             if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full_bar[s]), 2 * C::STAGE_BYTES);
             const uint32_t ws = smem_base + s * C::STAGE_BYTES;
-            gs_tma_load_2d(ws, &tmap_w, kb * GS_BK, wrow, fb);
-            gs_tma_load_2d(ws + GS_W_BYTES, &tmap_x, kb * GS_BK, plane * rows_total + xrow, fb);   // (rows behind a plane's end: the next plane's, not stored)
+            pair_tma_load_2d(ws, &tmap_w, kb * GS_BK, wrow, fb);
+            pair_tma_load_2d(ws + GS_W_BYTES, &tmap_x, kb * GS_BK, plane * rows_total + xrow, fb);   // (rows behind a plane's end: the next plane's, not stored)
             ++sent;
           }
     }
@@ -187,10 +154,10 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
           const uint64_t da = umma_desc_sw128(ws), db = umma_desc_sw128(ws + GS_W_BYTES);
 #pragma unroll
           for (int k = 0; k < GS_BK / 16; ++k)
-            gs_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
-          gs_commit(smem_u32(&empty_bar[s]));
+            pair_mma_bf16(tmem_d, da + (uint64_t)(2 * k), db + (uint64_t)(2 * k), idesc, (i > 0 || k > 0) ? 1u : 0u);
+          pair_commit(smem_u32(&empty_bar[s]));
         }
-        gs_commit(smem_u32(&tmem_full_bar[as]));
+        pair_commit(smem_u32(&tmem_full_bar[as]));
       }
   };
   auto finish = [&]() {
@@ -202,7 +169,7 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       tc_fence_before();
       __syncwarp();
       if (lane == 0)
-        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(gs_first_cta(smem_u32(&tmem_empty_bar[as]))) : "memory");
+        pair_arrive(pair_first_cta(smem_u32(&tmem_empty_bar[as])));
     };
     auto store = [&](int c0, int col, const uint32_t (&r)[32]) {   // 32 rows of x from c0 of the tile on, this thread's weight row
       if (col >= N) return;
@@ -288,7 +255,7 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   }
   // no CTA leaves while its peer's loads may still be counted on its barriers, or the pair's MMAs read its shared memory
   __syncwarp();
-  gs_cluster_sync();
+  pair_cluster_sync();
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::TMEM_COLS) : "memory");
