@@ -1597,7 +1597,7 @@ __global__ void __launch_bounds__(PX_THREADS, 1) heads_attention_premix_mma_kern
   for (int idx = tid; idx < H * PX_ROWS * (D / 4); idx += PX_THREADS) {
     const int c = idx % (D / 4), r = (idx / (D / 4)) % PX_ROWS, h = idx / ((D / 4) * PX_ROWS);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < ntok) v = reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h) * D)[c];
+    if (r < ntok) v = ld_written(reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h) * D) + c);
     __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
     uint2 pk;
     pk.x = *reinterpret_cast<unsigned*>(&lo);
@@ -1946,7 +1946,7 @@ __global__ void __launch_bounds__(PX_THREADS, NC == 8 ? 2 : 1) heads_attention_p
   for (int idx = tid; idx < HC * PX_ROWS * (D / 4); idx += PX_THREADS) {
     const int c = idx % (D / 4), r = (idx / (D / 4)) % PX_ROWS, h = idx / ((D / 4) * PX_ROWS);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < ntok) v = reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h0 + h) * D)[c];
+    if (r < ntok) v = ld_written(reinterpret_cast<const float4*>(a.q + ((size_t)(q_row0 + r) * H + h0 + h) * D) + c);
     uint2 hi, lo;
     hi.x = pack_bf16x2(v.x, v.y);
     hi.y = pack_bf16x2(v.z, v.w);

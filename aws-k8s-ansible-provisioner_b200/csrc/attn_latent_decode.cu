@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(LD_THREADS, 2) latent_decode_kernel(LatentDeco
     const int r4 = R >> 2;
 #pragma unroll 9
     for (int c = tid & 7; c < (D >> 2); c += 8) {
-      const float4 v = c < r4 ? qa[c] : qr[c - r4];
+      const float4 v = ld_written(c < r4 ? qa + c : qr + (c - r4));
       uint2 pk;
       pk.x = r < nh ? pack_bf16x2(v.x, v.y) : 0u;
       pk.y = r < nh ? pack_bf16x2(v.z, v.w) : 0u;

@@ -73,10 +73,21 @@ __device__ __forceinline__ uint4 ld_stream(const void* p) {
   return r;
 }
 
-// the same for what a kernel of the step wrote (cache rows)
+// The same for what a kernel of the step wrote (cache rows); ld_written: through L1.  Volatile statements keep their order, so these stay behind the dependency wait;
+// they are not tied to the stores around them, as a load through a pointer out of an argument struct is (its space is unknown: it may be shared memory).
 __device__ __forceinline__ uint4 ld_stream_written(const void* p) {
   uint4 r;
-  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p) : "memory");
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ uint4 ld_written(const uint4* p) {
+  uint4 r;
+  asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ float4 ld_written(const float4* p) {
+  float4 r;
+  asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
   return r;
 }
 

@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(32 * NW) gemm_any_rows_mma_kernel(AnyGemm g) {
         const bool in = k + c * 8 < K;
 #pragma unroll
         for (int t = 0; t < NT; ++t)
-          tv[u][t] = (in && tok[t] != nullptr) ? *reinterpret_cast<const uint4*>(tok[t] + k) : make_uint4(0, 0, 0, 0);
+          tv[u][t] = (in && tok[t] != nullptr) ? ld_written(reinterpret_cast<const uint4*>(tok[t] + k)) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)

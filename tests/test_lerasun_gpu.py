@@ -552,6 +552,22 @@ def test_layers_with_and_without_the_rebuilt_form():
             assert np.abs(got - ref).max() / scale < BF16_BAR
 
 
+@pytest.mark.parametrize("width,rank", [(2048, 1024), (2052, 1001)])
+def test_rows_at_the_edge_of_the_registers(width, rank):
+    """The norm in front of a layer holds rows of up to 2048 in registers (wider ones are read twice), the latent's norm up to 1024, the widest there is."""
+    cfg = {"architecture": "Lerasun", "vocab": 61, "width": width, "logit_scale": 0.5, "norm": {"eps": 1e-6}, "layers": [layer(mixer(2, 8, 4, 8, rank, 0.2), moe(16, 3, 2, 1, 1))]}
+    w = random_weights(cfg, seed=81)
+    toks = tokens(cfg, 40, 82)
+    ref = Oracle(cfg, w).forward(toks).numpy()
+    with engine(cfg, w) as e:
+        sid = e.seq_create(48)
+        lg, _ = e.prefill_logits([sid], [toks[:36]], list(range(36)))
+        assert err(lg, ref[:36]) < F32_BAR
+        for p in range(36, 40):
+            e.decode_step([sid], in_tokens=[toks[p]], want_output=False)
+            assert err(e.get_logits(1)[0], ref[p]) < F32_BAR
+
+
 def test_a_step_of_experts_takes_the_buffers_that_it_uses():
     """The experts' activation (8192 tokens, four choices, 1024 wide: 67 MB), their output and the gathered rows; the sums in front of the activation stay in the product."""
     P = pkg()
