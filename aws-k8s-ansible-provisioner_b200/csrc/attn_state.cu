@@ -23,10 +23,14 @@
 // reads.  The convolution keeps its last inputs in a ring of `taps` rows per slot indexed by position mod taps, for the
 // same reason.
 //
-// The scan is sequential in time and parallel over (sequence, head, value column): a CTA owns up to 128 columns of one
-// head's state for one portion, eight lanes share four neighbouring columns and split the key channels (channel i * 8 + j
-// belongs to lane j; the packed form, which all usual sizes take: see state_scan_packed_kernel), each lane keeps its channels of its columns in registers for the whole portion.  Tokens are staged through shared memory by asynchronous copies, a chunk ahead.  The arithmetic of a token does
-// not depend on where the portion was cut, so prefill, chunked prefill and token-by-token decoding give the same bits.
+// The scan is sequential in time and parallel over (sequence, head, value column).  A CTA owns some columns of one head's state for one
+// portion, and a group of lanes shares a few neighbouring columns and splits the key channels; each lane keeps its channels of its columns in
+// registers for the whole portion.
+//   state_scan_packed   (all usual sizes) sixteen lanes, two or four columns, pairs of neighbouring channels
+//   state_scan          (any sizes) eight lanes, four columns, channel i * 8 + j in lane j
+// Tokens are staged through shared memory by asynchronous copies, a chunk ahead.  The arithmetic of a token does not depend on where the portion
+// was cut: prefill, chunked prefill and token-by-token decoding give the same bits, except under the two rules with one decay per head in packed
+// form, where a decay multiplies a factor that enters the state at the end of a portion (a rounding apart).
 //
 // Kernels:
 //   lowrank_act        y = act(W2 . lr + bias) for the low-rank second stages (decays, output gates), fp32; lowrank_act_tile: prompt-sized steps

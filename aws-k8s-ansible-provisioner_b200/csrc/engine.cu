@@ -984,8 +984,9 @@ constexpr int LIST_SILU_EXPERT_ROWS = 2048;   // (token, choice) pairs of a step
 int list_tc_expert_rows() { return any_gemm_ragged_rows_limit() + 1; }
 
 // C (fp32 [M][N]) = alpha * A (operand type [M][K]) . Wt^T for the layer-list families.  Prompt-sized bf16 products whose K the tcgen05
-// projection kernel can tile (gemm_tc.cu: TMA needs 16-byte rows, its k-block is 64) take that kernel, fp32 sums written directly;
-// everything else -- decode steps, fp32 mode, odd shapes -- takes gemm_any.cu.
+// projection kernel can tile (gemm_tc.cu: TMA needs 16-byte rows, its k-block is 64) take that kernel, or CTA pairs where they are many (gemm_sum.cu), fp32 sums written
+// directly; few rows against many weight rows take gemm_few.cu's head kernel, larger fp32 products the tensor pipe (list_f32_tc);
+// everything else -- decode steps, short fp32 products, odd shapes -- takes gemm_any.cu.
 bool list_use_tc() {
   static const bool use_tc = [] { const char* v = getenv("B2_LIST_TC"); return !(v && *v == '0'); }();
   return use_tc;
@@ -993,8 +994,9 @@ bool list_use_tc() {
 bool list_dense_tc(const b2_engine* e, int M, int N, int K) { return list_use_tc() && !e->f32 && (M > 64 || N >= 16384) && N >= 128 && K % 64 == 0; }
 // fp32 products on the tensor pipe (three exact bf16 products, gemm_sum.cu; every matrix of an fp32 engine is a widened bf16 one, see put_operand): where the launch
 // is on the engine's own stream (the scratch is one; short steps run some products beside others on side streams).  From seventeen rows on, or from four
-// where the weights are many; fewer take the kernel that streams the weights, whose time grows with the rows (their shared-memory reads bound it: 6 x 32000 x 1024
-// 89 us there, 30 here).  A Kedasun prompt of 100 tokens, two layers, width 1024: 1260 us on the register tiles, 600 here.
+// where the weights are many; fewer take the kernel that streams the weights, whose time grows with the rows (their shared-memory reads bound it).  Two layers of
+// Kedasun, us, register tiles / here: a prompt of 17 tokens 602 / 567 (width 1024) and 1335 / 965 (2048), of 100 tokens 1257 / 623 and 2644 / 1035; a decode step of 4
+// sequences, whose head alone takes this form, 394 / 392 and 728 / 698, of 16 530 / 495 and 1446 / 1216.
 bool list_f32_tc(const b2_engine* e, const void* A, const void* Wt, int M, int N, int K, cudaStream_t ls) {
   return e->f32 && ls == e->stream && (M > 16 || (M >= 4 && N >= 16384)) && linear_split3_wide_ok(e->f32_tc, A, Wt, M, N, K);
 }
@@ -1003,6 +1005,8 @@ int list_dense(b2_engine* e, const void* A, const void* Wt, float* C, int M, int
   const int f = e->f32 ? 1 : 0;
   if (alpha == 1.f && list_f32_tc(e, A, Wt, M, N, K, ls))
     return launch_linear_split3_wide((const float*)A, (const float*)Wt, C, M, N, K, e->f32_tc, e->wait_limit(), ls);
+  // Few rows against many weight rows, heads and wide up-projections: the kernel that streams the weights through registers (us, tcgen05 tiles / here: 8 x 16384 x 4096
+  // 26.4 / 24.6, 8 x 22016 x 4096 46.1 / 32.1, 1 x 16384 x 1024 9.8 / 7.0, 16 x 16512 x 2048 15.1 / 14.2, 16 x 32000 x 2048 26.2 / 26.3).
   static const bool few_head = [] { const char* v = getenv("B2_FEW_HEAD"); return !(v && *v == '0'); }();
   if (few_head && !f && N >= 16384 && few_head_ok(M, N, K)) return launch_few_head((const bf16*)Wt, (const bf16*)A, C, M, N, K, alpha, ls);
   if (alpha == 1.f && list_dense_tc(e, M, N, K)) {
@@ -1264,7 +1268,7 @@ void latent_rebuild_free(b2_engine* e) {
 
 // The scratch of an fp32 engine's products on the tensor pipe: 96 and 64 MB whatever the model (a step's rows in fewer where they are fewer), behind the cache.  One
 // matrix at a time is narrowed into it, 6 bytes of traffic per weight and product: copies of all matrices beside the fp32 ones would save that (two layers of
-// width 1024 and their head, a prompt of 1500 tokens: about 60 of 1100 us), and take half as much again as the weights from what the caller left for other engines.
+// width 1024 and their head, three prompts of up to 500 tokens: 1038 us with copies, 1082 so), and take half as much again as the weights from what the caller left for other engines.
 // Without room for it the products take the register tiles of gemm_any.cu.
 void list_f32_scratch(b2_engine* e) {
   static const bool on = [] { const char* v = getenv("B2_F32_TC"); return !(v && *v == '0'); }();   // 0: the register tiles (cross-check)
@@ -2425,7 +2429,8 @@ bool two_lane_decode(const b2_engine* e, int T, int ntiles) {
 // but its contexts hold too many tokens in all for them (gemm_few.cu: a cluster per sequence and kv head, however long the sequence, against attn_decode.cu's even
 // share of all pages per warp).
 // 16 steps of 28 layers, ms, few / larger batches' kernels: 1 x 1500 tokens 10.4 / 22.6, 1 x 12000 25.6 / 31.9, 4 x 1500 12.7 / 22.4, 4 x 4000 17.7 / 24.3,
-// 8 x 1500 17.9 / 20.7, 8 x 4000 28.1 / 27.1, 4 x 12000 34.4 / 32.9.
+// 8 x 1500 17.9 / 20.7, 8 x 4000 28.1 / 27.1, 4 x 12000 34.4 / 32.9.  Unequal ones: 3100 + 4 x 50 12.9 / 36.9, 10000 + 7 x 60 22.2 / 32.8, 12000 + 7 x 1500 25.3 / 27.9,
+// 16000 + 7 x 600 30.5 / 31.7, 16000 + 8000 30.3 / 30.4.
 constexpr long FEW_CONTEXT_TOKENS = 24576;
 int pick_attn_split(const b2_engine* e, int B, long context_tokens) {
   const bool too_long = context_tokens > FEW_CONTEXT_TOKENS && !e->layers.empty() && !two_lane_decode(e, B, 0) && decode_forms(e, e->layers[0], B, false).few;
@@ -2959,10 +2964,10 @@ int list_tensor(b2_engine* e, const std::string& name, const void* host, size_t 
     } else if (sp.ff == B2_FF_SCALED_GATED_EXPERTS) {
       const size_t sf = sp.shared_ff;
       if (rest == "mlp.router") {
-      B2_TRY(want((size_t)sp.experts * W));
-      if (L.router_op) B2_TRY(put_operand(e, L.router_op, 0, src, (size_t)sp.experts * W));
-      return done(put_f32(L.router, src, (size_t)sp.experts * W, 0.0f));
-    }
+        B2_TRY(want((size_t)sp.experts * W));
+        if (L.router_op) B2_TRY(put_operand(e, L.router_op, 0, src, (size_t)sp.experts * W));
+        return done(put_f32(L.router, src, (size_t)sp.experts * W, 0.0f));
+      }
       if (sf > 0 && rest == "mlp.shared.gate") { B2_TRY(want(sf * W)); return done(put_operand(e, L.sh_up, 0, src, sf * W)); }
       if (sf > 0 && rest == "mlp.shared.up") { B2_TRY(want(sf * W)); return done(put_operand(e, L.sh_up, sf * W, src, sf * W)); }
       if (sf > 0 && rest == "mlp.shared.down") { B2_TRY(want(W * sf)); return done(put_operand(e, L.sh_down, 0, src, W * sf)); }
