@@ -256,6 +256,16 @@ def test_bf16_head_mixed_attention_on_clusters(heads, kv, dim, vdim, T):
         run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), BF16_BAR, [T - 21, 18], T - 3)
 
 
+def test_bf16_wide_up_projection_of_few_rows():
+    """bf16: an up-projection of 16384 rows takes the heads' kernel in short portions and decode steps, and the tcgen05 product in longer ones."""
+    cfg = model([(gla(2, 32, 64, 16.0, rank=16), dense(16384))], vocab=300, width=128)
+    w = random_weights(cfg, seed=78)
+    toks = tokens(cfg, 70, 79)
+    ref = ref_logits(cfg, w, toks)
+    with engine(cfg, w, f32=False) as e:
+        run_schedule(e, cfg, toks, ref, BF16_BAR, [40, 9, 1, 16], 66)
+
+
 def test_bf16_long_step_runs_the_experts_one_by_one():
     """A step with at least 2048 (token, choice) pairs takes the per-expert tensor-core products; short portions of the same prompt take
     the ragged ones: both agree with the restatement."""
