@@ -1353,6 +1353,69 @@ __global__ void __launch_bounds__(512) heads_finish_halves_kernel(const float* p
   }
 }
 
+// The same for prompt steps whose attention is attn_premix_tc.cu's: heads of 128 + 128 with two query heads per key/value head, a bf16 cache.  A CTA takes one token, a warp a head at a
+// time, a lane four neighbouring channels (16 bytes); the partner of a rotation pair is another lane's.  Queries leave as bf16 value and remainder, [key/value head][token][head of
+// two][value, remainder][128], which is how the products read them; the values' cosines and sines of every token are kept for the turn back (turn [T][64 | 64]).
+// Bound by memory and, a token at a time, by the angles.  4096 tokens of 32 heads: what it adds to the step 149 us (heads_finish_halves_kernel, a channel at a time) -> 72.
+__global__ void __launch_bounds__(256) heads_finish_planes_kernel(const float* proj, int ld, HeadsGeom g, const float* __restrict__ q_gain, const float* __restrict__ k_gain,
+                                                                  const int32_t* positions, const int32_t* slots, int T, bf16* q_planes, float* turn, bf16* __restrict__ k_cache,
+                                                                  bf16* __restrict__ v_cache) {
+  __shared__ __align__(16) float cs[256];   // q and k: cos [half] | sin [half] at 0, at most 64 each; values: cos | sin at 128
+  pdl_wait();
+  pdl_launch_dependents();
+  const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int pos = positions[t], slot = slots[t], half = g.rot_dims / 2;
+  if (tid < half) {
+    const double inv_factor = g.rot_factor > 0.f ? 1.0 / (double)g.rot_factor : 1.0;
+    const double f = exp2(-2.0 * (double)tid / (double)g.rot_dims * log2((double)g.rot_base)) * inv_factor;
+    double sd, cd;
+    sincos((double)pos * f, &sd, &cd);
+    cs[tid] = (float)cd;
+    cs[half + tid] = (float)sd;
+  } else if (tid >= 128 && tid < 192 && g.rot_values) {
+    pair_cos_sin(pos, tid - 128, 128, g.rot_base, &cs[tid], &cs[tid + 64]);
+  }
+  const float4* row = reinterpret_cast<const float4*>(proj + (size_t)t * ld) + lane;
+  const int H = g.heads, nqk = H + g.kv_heads, units = nqk + g.kv_heads;   // units are 128 numbers each, one behind the other in the row
+  __syncthreads();
+  auto turned = [&](float4 y, const float* c, int dims) {   // pairs (d, d + dims / 2) of the first `dims`: four channels of one lane go with four of the lane dims / 8 away
+    const int hl = dims / 8;   // lanes of a half
+    const int other = lane < hl ? lane + hl : lane < 2 * hl ? lane - hl : lane;
+    const float4 z = make_float4(__shfl_sync(0xffffffffu, y.x, other), __shfl_sync(0xffffffffu, y.y, other), __shfl_sync(0xffffffffu, y.z, other), __shfl_sync(0xffffffffu, y.w, other));
+    if (lane >= 2 * hl) return y;
+    const int i = 4 * (lane < hl ? lane : lane - hl);
+    const float4 co = *reinterpret_cast<const float4*>(c + i), si = *reinterpret_cast<const float4*>(c + dims / 2 + i);
+    if (lane < hl) return make_float4(y.x * co.x - z.x * si.x, y.y * co.y - z.y * si.y, y.z * co.z - z.z * si.z, y.w * co.w - z.w * si.w);
+    return make_float4(y.x * co.x + z.x * si.x, y.y * co.y + z.y * si.y, y.z * co.z + z.z * si.z, y.w * co.w + z.w * si.w);
+  };
+  auto packed = [](float4 y) { return make_uint2(pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w)); };
+#pragma unroll 4
+  for (int u = warp; u < units; u += 8) {
+    float4 y = row[32 * u];
+    if (u < nqk) {
+      const float* gain = u < H ? q_gain : k_gain;
+      if (gain != nullptr) {
+        const float r = 1.0f / sqrtf(warp_sum(fmaf(y.x, y.x, fmaf(y.y, y.y, fmaf(y.z, y.z, y.w * y.w)))) / 128.f + g.eps);
+        const float4 w = *(reinterpret_cast<const float4*>(gain) + lane);
+        y = make_float4(y.x * r * w.x, y.y * r * w.y, y.z * r * w.z, y.w * r * w.w);
+      }
+      if (half > 0) y = turned(y, cs, g.rot_dims);
+      if (u < H) {
+        const uint2 hi = packed(y), lo = packed(make_float4(y.x - bf16lo(hi.x), y.y - bf16hi(hi.x), y.z - bf16lo(hi.y), y.w - bf16hi(hi.y)));
+        uint2* d = reinterpret_cast<uint2*>(q_planes + (((size_t)(u >> 1) * T + t) * 4 + 2 * (u & 1)) * 128) + lane;
+        d[0] = hi;
+        d[32] = lo;
+      } else if (slot >= 0) {
+        *(reinterpret_cast<uint2*>(k_cache + ((size_t)slot * g.kv_heads + u - H) * 128) + lane) = packed(y);
+      }
+    } else {
+      if (g.rot_values) y = turned(y, cs + 128, 128);
+      if (slot >= 0) *(reinterpret_cast<uint2*>(v_cache + ((size_t)slot * g.kv_heads + u - nqk) * 128) + lane) = packed(y);
+    }
+  }
+  if (g.rot_values && warp == 7) *(reinterpret_cast<float4*>(turn + (size_t)t * 128) + lane) = *reinterpret_cast<const float4*>(cs + 128 + 4 * lane);
+}
+
 // All heads of `qt` query tokens of one sequence per CTA (eight warps), because a mixed score of one head needs the scores of every head
 // for the same (query, key) pair.  Keys go by in tiles of 32, upwards from the first visible one.  Per tile: for every key/value head its
 // K rows are staged and the group's query heads score them (lane j scores key j; scale, cap); then every (token, head) mixes its row of
@@ -1875,7 +1938,8 @@ bool premix_mma_fits(const HeadsGeom& g) {
 // others have read it -- is an arrival behind the reads and a wait a whole K copy later.
 // The plain kernel kept queries and weights in fp32, so both enter the tensor-core products here as two bf16 numbers (value, and what its rounding left:
 // 16 bits of mantissa against bf16 K and V rows that are exact): the distance from the 64-bit result stays what it was.  The 4 x 1024 tokens: 1.93 ms.  No
-// pipe is near its limit (42 % of the issue slots, the LSU at 43 %): copies, the scores of other CTAs and the barriers are waited for.
+// pipe is near its limit (42 % of the issue slots, the LSU at 43 %): copies, the scores of other CTAs and the barriers are waited for.  Heads of 128 + 128 in groups of two take
+// attn_premix_tc.cu instead.
 // Every row sees all keys up to its own, and the scores are always mixed: no layer asks for a window or for unmixed scores at these sizes.
 struct PremixClusterLayout {
   int HC, GC, QP, KP, OP;
@@ -2477,6 +2541,16 @@ int launch_heads_finish_halves(const float* proj, int ld, const HeadsGeom& g, co
   else
     B2_CUDA_OK(b2_launch(heads_finish_halves_kernel<bf16>, dim3(T), block, smem, s, proj, ld, g, q_gain, k_gain, positions, slots, q_out,
                          (bf16*)k_cache, (bf16*)v_cache));
+  return 0;
+}
+
+int launch_heads_finish_planes(const float* proj, int ld, const HeadsGeom& g, const float* q_gain, const float* k_gain, const int32_t* positions, const int32_t* slots, bf16* q_planes,
+                               float* turn, bf16* k_cache, bf16* v_cache, int T, cudaStream_t s) {
+  if (T <= 0) return 0;
+  B2_REQUIRE(g.dim == 128 && g.vdim == 128 && g.heads == 2 * g.kv_heads && g.rot_dims >= 0 && g.rot_dims <= 128 && g.rot_dims % 8 == 0 && ld % 4 == 0,
+             "heads_finish_planes: %d heads of %d + %d numbers (%d rotated, rows of %d) have no such form", g.heads, g.dim, g.vdim, g.rot_dims, ld);
+  B2_REQUIRE(turn != nullptr || !g.rot_values, "heads_finish_planes: rotated values need room for their cosines and sines");
+  B2_CUDA_OK(b2_launch(heads_finish_planes_kernel, dim3(T), dim3(256), 0, s, proj, ld, g, q_gain, k_gain, positions, slots, T, q_planes, turn, k_cache, v_cache));
   return 0;
 }
 

@@ -150,6 +150,18 @@ extern "C" int b2k_heads_postmix(const float* q, const void* k_cache, const void
                               (bf16*)out, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_heads_premix(const void* q_planes, const void* k_cache, const void* v_cache, int64_t cache_rows, int heads, float scale, float softcap, const float* talk_host,
+                                const float* turn, const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, const int32_t* tiles_host, int ntiles, void* out,
+                                int T, float* scratch, size_t scratch_floats, void* stream) {
+  B2_REQUIRE(q_planes && k_cache && v_cache && block_table && tiles && tiles_host && talk_host && out && scratch, "b2k_heads_premix: null pointer");
+  B2WaitLimit wait;
+  CAPI_TRY(hook_waits(&wait));
+  HeadsGeom g{};
+  g.heads = heads; g.kv_heads = heads / 2; g.dim = g.vdim = 128; g.scale = scale; g.softcap = softcap; g.rot_values = turn != nullptr;
+  return launch_heads_premix_tc((const bf16*)q_planes, (const bf16*)k_cache, (const bf16*)v_cache, cache_rows, g, talk_host, turn, block_table, bt_stride, block_size,
+                                (const PrefillTile*)tiles, (const PrefillTile*)tiles_host, ntiles, (bf16*)out, T, scratch, scratch_floats, wait, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
                               const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
                               const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,

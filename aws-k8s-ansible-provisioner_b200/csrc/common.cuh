@@ -322,6 +322,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const CUtensorMap
       "l"(tmap), "r"(bar), "r"(c0), "r"(c1)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d(uint32_t dst_smem, const CUtensorMap* tmap, int c0, int c1, int c2, int c3, uint32_t bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::"r"(dst_smem),
+      "l"(tmap), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+      : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
@@ -409,6 +415,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   d |= (uint64_t)2 << 61;
   return d;
 }
+// The same with the 8-row groups `group_bytes` apart (a multiple of 1024).
+__device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr, uint32_t group_bytes) {
+  return umma_desc_sw128(smem_addr) + ((uint64_t)((group_bytes - 1024) >> 4) << 32);
+}
 // Instruction descriptor: D fp32, A/B bf16, both K-major, M x N tile.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24);
@@ -423,3 +433,5 @@ int b2_make_tmap_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_
 // General form: box = box_cols x box_rows elements; swizzle128 = 0 copies rows as they are (for data that is stored swizzled).
 int b2_make_tmap_bf16_ex(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, uint32_t box_cols, uint32_t box_rows,
                          int swizzle128);
+// The same for any rank (dims and box innermost first, stride_bytes of the dims behind the innermost), 128-byte swizzle.
+int b2_make_tmap_bf16_swizzled(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* stride_bytes, const uint32_t* box);

@@ -107,6 +107,7 @@ struct ListLayer {
         *out_gain_r = nullptr, *poly = nullptr;
   size_t a2_floats = 0, g2_floats = 0;
   std::vector<uint16_t> a1_host, g1_host;
+  std::vector<float> talk_host;   // `talk` for kernels that take it as a parameter
   // Layer norms with gain and bias around every sublayer (Tinevik): gain1 / gain1b / gain2 / gain2b hold the gains, these the biases.  Its
   // state mixer projects q | k | v | g (| a1) in `wqd` (off_s*), its softmax mixer q | k | v with one gain per head entry for q and for k
   // (`qk_gain` = [dim] | [dim]) and the score-mixing matrix `talk`, its latent mixer dq | dkv | g in `wqd` (off_sq / off_sk / off_sg), the
@@ -362,6 +363,8 @@ struct b2_engine {
   Split3Scratch f32_tc;              // fp32 mode of the layer-list families: scratch of the products on the tensor pipe (gemm_sum.cu)
   int32_t* h_offsets = nullptr;      // pinned: the experts' slot ranges of the step, read back for the per-expert launches
   size_t l_attn_scratch_floats = 0;
+  float *l_premix = nullptr, *l_turn = nullptr;   // Tinevik prompts: mixed scores on their way, cosines and sines of the tokens' values (attn_premix_tc.cu)
+  size_t l_premix_floats = 0;
   float* dbg_hidden_f32 = nullptr;
   int dbg_slots = 0;                 // residual-stream captures per forward: embeddings + one per layer run
   // matrix-state mixers and the layer loop (Bumalix)
@@ -1896,15 +1899,27 @@ int forward_mixed_list(b2_engine* e, int T, int ntiles, int nlast) {
       g.softcap = sp.softcap;
       char* kc = e->regions[R.k_region].base;
       char* vc = e->regions[R.v_region].base;
+      const bool tc = tiles != nullptr && sp.score_mix && !L.talk_host.empty() && e->l_premix != nullptr && heads_premix_tc_ok(g, c.block_size) && heads_premix_tc_scratch_floats(g, 0, c.max_model_len) > 0;
       {
         KL k(e, B2K_ROPE_KV);
-        if (!k.skip()) B2_TRY(launch_heads_finish_halves(e->l_qd, L.nqd, g, L.qk_gain, L.qk_gain + sp.dim, e->d_positions, e->d_slots, e->l_q, kc, vc, f, T, st));
+        if (k.skip()) {
+        } else if (tc) {
+          B2_TRY(launch_heads_finish_planes(e->l_qd, L.nqd, g, L.qk_gain, L.qk_gain + sp.dim, e->d_positions, e->d_slots, (bf16*)e->l_q, e->l_turn, (bf16*)kc, (bf16*)vc, T, st));
+        } else {
+          B2_TRY(launch_heads_finish_halves(e->l_qd, L.nqd, g, L.qk_gain, L.qk_gain + sp.dim, e->d_positions, e->d_slots, e->l_q, kc, vc, f, T, st));
+        }
       }
       {
         KL k(e, ntiles > 0 ? B2K_MISC : B2K_ATTN_DECODE);
-        if (!k.skip()) B2_TRY(launch_heads_attention_premix(e->l_q, kc, vc, f, g, sp.score_mix ? L.talk : nullptr, e->d_block_table, e->bt_stride, c.block_size,
-                                                            tiles, ntiles, e->d_positions, e->d_seq_lens, e->l_av, f, T, st, e->l_attn_scratch,
-                                                            e->l_attn_scratch_floats, c.max_model_len));
+        if (k.skip()) {
+        } else if (tc) {
+          B2_TRY(launch_heads_premix_tc((const bf16*)e->l_q, (const bf16*)kc, (const bf16*)vc, (int64_t)e->num_blocks * c.block_size, g, L.talk_host.data(), sp.rot_values ? e->l_turn : nullptr,
+                                        e->d_block_table, e->bt_stride, c.block_size, tiles, e->h_tiles, ntiles, (bf16*)e->l_av, T, e->l_premix, e->l_premix_floats,
+                                        e->wait_limit(), st));
+        } else {
+          B2_TRY(launch_heads_attention_premix(e->l_q, kc, vc, f, g, sp.score_mix ? L.talk : nullptr, e->d_block_table, e->bt_stride, c.block_size, tiles, ntiles, e->d_positions,
+                                               e->d_seq_lens, e->l_av, f, T, st, e->l_attn_scratch, e->l_attn_scratch_floats, c.max_model_len));
+        }
       }
     } else {   // B2_MIXER_GATED_LATENT
       const LatentGeom g{sp.heads, sp.dim, 0, sp.vdim, sp.kv_rank, 0, 0.f, sp.scale, c.rms_eps, sp.window};
@@ -3031,7 +3046,15 @@ int list_tensor(b2_engine* e, const std::string& name, const void* host, size_t 
       if (rest == "mix.v") { B2_TRY(want(nv * W)); return done(put_operand(e, L.wqd, (nq + nk) * W, src, nv * W)); }
       if (rest == "mix.q.norm") { B2_TRY(want(dn)); return done(put_f32(L.qk_gain, src, dn, 0.0f)); }
       if (rest == "mix.k.norm") { B2_TRY(want(dn)); return done(put_f32(L.qk_gain + dn, src, dn, 0.0f)); }
-      if (rest == "mix.talk") { B2_TRY(want(H * H)); return done(put_f32(L.talk, src, H * H, 0.0f)); }
+      if (rest == "mix.talk") {
+        B2_TRY(want(H * H));
+        L.talk_host.resize(H * H);
+        for (size_t i = 0; i < (size_t)H * H; ++i) {
+          const uint32_t u = (uint32_t)src[i] << 16;
+          memcpy(&L.talk_host[i], &u, 4);
+        }
+        return done(put_f32(L.talk, src, H * H, 0.0f));
+      }
     } else {
       const size_t qr = sp.q_rank;
       if (rest == "mix.dq") { B2_TRY(want(qr * W)); return done(put_operand(e, L.wqd, (size_t)L.off_sq * W, src, qr * W)); }
@@ -3897,7 +3920,17 @@ int mixed_engine_alloc(b2_engine* e) {
   B2_TRY(aalloc(&e->l_xl, (size_t)e->l_rows_cap * W));
   size_t scratch = 0;   // the key splits of a decode step's attention (one buffer: the layers run one after the other)
   for (const ListLayer& L : e->ll)
-    if (L.sp.mixer == B2_MIXER_MIXED_SCORE_ATTENTION) scratch = std::max(scratch, heads_attention_premix_scratch_floats(bucket_batch(c.max_seqs), L.sp.heads, L.sp.vdim));
+    if (L.sp.mixer == B2_MIXER_MIXED_SCORE_ATTENTION) {
+      scratch = std::max(scratch, heads_attention_premix_scratch_floats(bucket_batch(c.max_seqs), L.sp.heads, L.sp.vdim));
+      HeadsGeom g{L.sp.heads, L.sp.kv_heads, L.sp.dim, L.sp.vdim};
+      g.rot_dims = L.sp.rot_dims;
+      g.window = L.sp.window;
+      if (!e->f32 && L.sp.score_mix && heads_premix_tc_ok(g, c.block_size)) e->l_premix_floats = std::max(e->l_premix_floats, heads_premix_tc_scratch_floats(g, (int)Tc, c.max_model_len));
+    }
+  if (e->l_premix_floats > 0) {
+    B2_TRY(dalloc(&e->l_premix, e->l_premix_floats));
+    B2_TRY(dalloc(&e->l_turn, Tc * 128));
+  }
   if (any_latent) {
     B2_TRY(aalloc(&e->l_x2, Tc * max_qr));
     B2_TRY(aalloc(&e->l_qnope, Tc * max_hd));
@@ -5426,7 +5459,7 @@ extern "C" void b2_engine_free(b2_engine* e) {
   F(e->l_xperm); F(e->l_upf); if (e->h_offsets) cudaFreeHost(e->h_offsets);
   F(e->l_q); F(e->l_vfirst); F(e->l_cross); F(e->l_qb); F(e->d_row_seq); F(e->d_row_first); F(e->d_row_end);
   F(e->l_mix); F(e->l_y); F(e->l_rw); F(e->l_logits); F(e->l_x1); F(e->l_x2); F(e->l_qnope); F(e->l_olat); F(e->l_av); F(e->l_act); F(e->l_xl);
-  F(e->l_attn_scratch); F(e->l_idx); F(e->l_offsets); F(e->l_slot_token); F(e->l_pair_slot); F(e->l_tile_group); F(e->l_tile_row0); F(e->l_ntiles); F(e->dbg_hidden_f32);
+  F(e->l_attn_scratch); F(e->l_premix); F(e->l_turn); F(e->l_idx); F(e->l_offsets); F(e->l_slot_token); F(e->l_pair_slot); F(e->l_tile_group); F(e->l_tile_row0); F(e->l_ntiles); F(e->dbg_hidden_f32);
   for (auto& L : e->ll) {
     if (!L.uv_in_ukv) F(L.uv);
     F(L.wqd); F(L.ukT); F(L.wo); F(L.up); F(L.down); F(L.gain1); F(L.gain2); F(L.lat_gain); F(L.sink); F(L.router); F(L.corr);

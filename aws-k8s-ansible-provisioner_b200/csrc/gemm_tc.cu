@@ -539,6 +539,24 @@ int b2_make_tmap_bf16_ex(CUtensorMap* out, const void* base, uint64_t rows, uint
   return 0;
 }
 
+int b2_make_tmap_bf16_swizzled(CUtensorMap* out, const void* base, int rank, const uint64_t* dims, const uint64_t* stride_bytes, const uint32_t* box) {
+  auto fn = b2::get_encode_fn();
+  B2_REQUIRE(fn != nullptr, "cuTensorMapEncodeTiled driver entry point not available");
+  B2_REQUIRE(rank >= 2 && rank <= 5 && ((uintptr_t)base & 15) == 0, "tensor map: rank %d, base must be 16-byte aligned", rank);
+  cuuint64_t d[5], st[5];
+  cuuint32_t b[5], estr[5] = {1, 1, 1, 1, 1};
+  for (int i = 0; i < rank; ++i) {
+    d[i] = dims[i];
+    b[i] = box[i];
+    if (i > 0) st[i - 1] = stride_bytes[i - 1];
+    B2_REQUIRE(i == 0 || stride_bytes[i - 1] % 16 == 0, "tensor map: strides must be multiples of 16 bytes");
+  }
+  const CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, st, b, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  B2_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeTiled failed with CUresult %d (rank %d)", (int)r, rank);
+  return 0;
+}
+
 namespace b2 {
 
 int tc_set_trace(unsigned long long* dev_buf) {

@@ -453,6 +453,15 @@ int launch_heads_attention_premix(const float* q, const void* k_cache, const voi
 // scratch: device floats for the key splits of a decode step (heads_attention_premix_scratch_floats); without it a decode step runs unsplit,
 // a CTA per sequence.  max_context: the longest sequence the engine holds (bounds the number of splits).
 size_t heads_attention_premix_scratch_floats(int max_rows, int heads, int vdim);
+// attn_premix_tc.cu: the same for prompt portions, 8, 16 or 32 heads of 128 + 128, two per key/value head, over a bf16 cache (cache_rows: rows of the region), scores through `scratch`;
+// queries and the values' cosines and sines (turn [T][128], null without g.rot_values) as launch_heads_finish_planes leaves them, the mixing matrix in host memory, the tile list in both.
+bool heads_premix_tc_ok(const HeadsGeom& g, int block_size);
+size_t heads_premix_tc_scratch_floats(const HeadsGeom& g, int max_tokens, int max_context);
+int launch_heads_finish_planes(const float* proj, int ld, const HeadsGeom& g, const float* q_gain, const float* k_gain, const int32_t* positions, const int32_t* slots, bf16* q_planes,
+                               float* turn, bf16* k_cache, bf16* v_cache, int T, cudaStream_t s);
+int launch_heads_premix_tc(const bf16* q_planes, const bf16* k_cache, const bf16* v_cache, int64_t cache_rows, const HeadsGeom& g, const float* talk_host, const float* turn,
+                           const int32_t* block_table, int bt_stride, int block_size, const PrefillTile* tiles, const PrefillTile* tiles_host, int ntiles, bf16* out, int T,
+                           float* scratch, size_t scratch_floats, const B2WaitLimit& wait, cudaStream_t s);
 int launch_talk_gate(const float* cross, const float* talk, const float* gate, int gate_ld, void* out, int out_f32, int heads, int kv_heads,
                      int vdim, int T, cudaStream_t s);
 // attn_postmix.cu: both in one for prompt portions over a bf16 cache, the weights mixed instead of the outputs; out bf16 [T][heads * vdim]

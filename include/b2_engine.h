@@ -447,6 +447,13 @@ int b2k_linear_split3_wide(const float* x, const float* w, void* planes_bf16, si
 int b2k_heads_postmix(const float* q, const void* k_cache, const void* v_cache, int heads, int kv_heads, int dim, int vdim, float scale, float slope_exp, int window,
                       int keep_first, const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, int ntiles, const float* talk, const float* gate,
                       int gate_ld, void* out, void* stream);
+/* Prompt attention whose scores are mixed over the heads before the softmax (csrc/attn_premix_tc.cu): 8, 16 or 32 heads of 128 + 128, two per key/value head.
+ * out[t][a] = softmax_j(sum_b talk[a][b] c(q_b . k_j)) v_j, c(x) = softcap tanh(scale x / softcap) (softcap 0: scale x); with turn [T][128] = cos | sin the pairs (d, d + 64) of the
+ * sum are turned by minus the angle.  q_planes bf16 [kv head][T][head of two][value, remainder][128]; caches bf16 [cache_rows][kv_heads * 128]; tiles as above, in device and in host
+ * memory, talk in host memory; out bf16 [T][heads * 128]; the scratch holds 128 numbers for every (head, query, 128 keys) of the tiles under way, and the call goes in pieces of whole tiles. */
+int b2k_heads_premix(const void* q_planes, const void* k_cache, const void* v_cache, int64_t cache_rows, int heads, float scale, float softcap, const float* talk_host, const float* turn,
+                     const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, const int32_t* tiles_host, int ntiles, void* out, int T, float* scratch,
+                     size_t scratch_floats, void* stream);
 /* The recurrence of the matrix-state mixers over `portions` portions (portion i ends at row last_rows[i]; last_rows null: every row is one of one token); rule as
  * StateRule in csrc/kernels.h; all tensors fp32: q / k rows of kv_heads * dim, v rows of heads * vdim, decay [T][heads * dim] or [T][heads] by the rule, beta
  * [T][heads], skip [heads], bonus [heads][dim] (null where the rule has none), state [slots][2][heads][dim][vdim], out [T][heads * vdim]. */

@@ -239,6 +239,60 @@ def test_linear_split3_wide(lib, rows, N, K, rows_at_a_time, cols_at_a_time):
         assert lib.b2k_linear_split3_wide(ptr(x), ptr(wide), ptr(planes), 255 * K, ptr(narrow), nw, ptr(out), rows, N, K, cuda_stream_ptr()) != 0
 
 
+@pytest.mark.parametrize("heads,softcap,turned,bs,pieces", [(32, 20.0, True, 16, False), (32, 0.0, False, 64, True), (16, 50.0, True, 32, True), (8, 3.0, False, 16, False)])
+def test_heads_premix(lib, heads, softcap, turned, bs, pieces):
+    """Portions around the tiles of 64, the units of 8 or 16 tokens and the blocks of 128 keys, some behind earlier tokens; `pieces`: a scratch that holds two tiles' units at most.
+    Against 64 bits over the same queries (value + remainder), keys and values: scores and weights carry sixteen bits, so what is left is fp32 sums and the bf16 result, as in the
+    test below."""
+    g = torch.Generator().manual_seed(heads * 10 + bs)
+    portions = [(0, 1), (0, 17), (100, 64), (3, 33), (200, 130), (0, 256), (121, 7), (127, 2)]            # (earlier tokens, tokens)
+    kv, T, width = heads // 2, sum(n for _, n in portions), max((p + n + bs - 1) // bs for p, n in portions)
+    pages = len(portions) * width + 2
+    bt = torch.randperm(pages, generator=g)[:len(portions) * width].view(-1, width).to(torch.int32)
+    q = torch.randn(T, heads, 128, generator=g)
+    hi = q.to(torch.bfloat16)
+    lo = (q - hi.float()).to(torch.bfloat16)
+    planes = torch.stack([hi, lo], 2).view(T, kv, 2, 2, 128).permute(1, 0, 2, 3, 4).contiguous()
+    kc, vc = (torch.randn(pages, bs, kv * 128, generator=g).to(torch.bfloat16) for _ in range(2))
+    talk = torch.eye(heads) + 0.2 * torch.randn(heads, heads, generator=g)
+    ang = torch.rand(T, 64, generator=g) * 6.0
+    turn = torch.cat([torch.cos(ang), torch.sin(ang)], 1).contiguous()
+    tiles, at = [], 0
+    for b, (p, n) in enumerate(portions):
+        tiles += [(at + i, p + i, min(64, n - i), b) for i in range(0, n, 64)]
+        at += n
+    host = torch.tensor(tiles, dtype=torch.int32)
+    unit = heads * (8 if heads == 32 else 16) * 128
+    units = [(r + 7 if heads == 32 else r + 15) // (8 if heads == 32 else 16) * ((p + r - 1) // 128 + 1) for _, p, r, _ in tiles]
+    room = (2 * max(units) if pieces else sum(units)) * unit
+    dev = [t.cuda() for t in (planes, kc, vc, bt, host, talk, turn)]
+    scratch = torch.full((room,), float("nan"), device="cuda")
+    out = torch.full((T + 1, heads * 128), float("nan"), dtype=torch.bfloat16, device="cuda")
+    scale = 128 ** -0.5
+    call = lambda room: lib.b2k_heads_premix(ptr(dev[0]), ptr(dev[1]), ptr(dev[2]), pages * bs, heads, scale, softcap, ptr(talk), ptr(dev[6]) if turned else None, ptr(dev[3]), width, bs,
+                                             ptr(dev[4]), ptr(host), len(tiles), ptr(out), T, ptr(scratch), room, cuda_stream_ptr())
+    chk(lib, call(room))
+    torch.cuda.synchronize()
+    assert torch.isnan(out[T]).all() and call(unit) != 0   # (a tile that does not fit is refused)
+    at = 0
+    for b, (p, n) in enumerate(portions):
+        idx, S = bt[b].long(), p + n
+        k, v = (c[idx].reshape(-1, kv, 128)[:S].double().repeat_interleave(2, 1) for c in (kc, vc))
+        s = torch.einsum("ihd,jhd->hij", (hi.double() + lo.double())[at:at + n], k) * scale
+        if softcap:
+            s = softcap * torch.tanh(s / softcap)
+        s = torch.einsum("ab,bij->aij", talk.double(), s)
+        pr = torch.softmax(s.masked_fill(torch.arange(S)[None, :] > torch.arange(p, S)[:, None], float("-inf")), -1)
+        ref, mag = (torch.einsum("hij,jhd->ihd", pr, x) for x in (v, v.abs()))
+        if turned:
+            c, sn = (x[at:at + n, None, :].double() for x in (turn[:, :64], turn[:, 64:]))
+            ref = torch.cat([ref[..., :64] * c + ref[..., 64:] * sn, ref[..., 64:] * c - ref[..., :64] * sn], -1)
+            mag = mag + mag.roll(64, -1)
+        got = out[at:at + n].cpu().double().view(n, heads, 128)
+        assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -14 * mag + 1e-6).all(), (b, (got - ref).abs().max())
+        at += n
+
+
 @pytest.mark.parametrize("heads,kv,dim,vdim,window,keep,bs", [(16, 8, 128, 128, 70, 9, 16), (16, 16, 64, 64, 0, 0, 32), (5, 1, 128, 64, 33, 0, 48), (8, 4, 64, 128, 16, 40, 16),
                                                               (1, 1, 128, 128, 1, 5, 16), (12, 4, 128, 128, 100, 16, 64)])
 def test_heads_postmix(lib, heads, kv, dim, vdim, window, keep, bs):
