@@ -97,6 +97,21 @@ extern "C" int b2k_linear_sum(const void* x, const void* w, const int32_t* offse
   return launch_linear_sum(x, w, offsets, groups, rows, out, N, K, epilogue, wait, (cudaStream_t)stream, tile);
 }
 
+extern "C" int b2k_linear_xielu(const void* x, const void* w, const float* pq, void* act, int rows, int N, int K, int tile, void* stream) {
+  B2_REQUIRE(x && w && pq && act, "b2k_linear_xielu: null pointer");
+  B2WaitLimit wait;
+  CAPI_TRY(hook_waits(&wait));
+  return launch_linear_sum(x, w, nullptr, 1, rows, act, N, K, SUM_EPI_XIELU, wait, (cudaStream_t)stream, tile, pq);
+}
+
+extern "C" int b2k_gateup_clamped(const void* x, const void* w_gu, void* act, int T, int I, int K, float limit, float sharp, void* stream) {
+  B2_REQUIRE(x && w_gu && act, "b2k_gateup_clamped: null pointer");
+  CUtensorMap tw, tx;
+  CAPI_TRY(b2_make_tmap_bf16(&tw, w_gu, (uint64_t)2 * I, (uint64_t)K, (uint64_t)K, 128));
+  CAPI_TRY(b2_make_tmap_bf16(&tx, x, (uint64_t)T, (uint64_t)K, (uint64_t)K, 128));
+  return launch_gateup_clamped_prefill(tw, tx, (bf16*)act, T, I, K, limit, sharp, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_few_linear(const void* w, const void* x, const void* gain, float eps, void* out, int T, int N, int K, int mode, void* stream) {
   B2_REQUIRE(w && x && out && (mode == 1 || gain) && mode >= 0 && mode <= 2, "b2k_few_linear: bad arguments");
   B2_REQUIRE(few_shapes_ok(T, K, K, K), "b2k_few_linear: T=%d N=%d K=%d not built", T, N, K);

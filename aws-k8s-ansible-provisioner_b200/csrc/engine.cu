@@ -1556,11 +1556,17 @@ int forward_heads_list(b2_engine* e, int T, int ntiles, int nlast) {
         KL k(e, B2K_NORM);
         if (!k.skip()) B2_TRY(launch_group_norm(e->l_h, L.gain2, e->l_x1, f, T, W, groups, c.rms_eps, nullptr, st));
       }
-      {
-        KL k(e, B2K_GEMM_GATEUP);  // gate | up: one projection
-        if (!k.skip()) B2_TRY(list_dense(e, e->l_x1, L.up, e->l_y, T, 2 * sp.ff_dim, W, 1.f));
-      }
-      {
+      if (!f && list_gate_up_fused(T, sp.ff_dim, W) && e->skip_mask == 0) {   // prompt-sized: the activation in the product's epilogue
+        KL k(e, B2K_GEMM_GATEUP);
+        CUtensorMap tw, tx;
+        B2_TRY(b2_make_tmap_bf16(&tw, L.up, (uint64_t)2 * sp.ff_dim, (uint64_t)W, (uint64_t)W, 128));
+        B2_TRY(b2_make_tmap_bf16(&tx, e->l_x1, (uint64_t)T, (uint64_t)W, (uint64_t)W, 128));
+        B2_TRY(launch_gateup_clamped_prefill(tw, tx, (bf16*)e->l_act, T, sp.ff_dim, W, sp.ff_limit, KEDASUN_GATE_SHARP, st));
+      } else {
+        {
+          KL k(e, B2K_GEMM_GATEUP);  // gate | up: one projection
+          if (!k.skip()) B2_TRY(list_dense(e, e->l_x1, L.up, e->l_y, T, 2 * sp.ff_dim, W, 1.f));
+        }
         KL k(e, B2K_ACT);
         if (!k.skip()) B2_TRY(launch_clamped_gate(e->l_y, e->l_act, f, T, sp.ff_dim, sp.ff_limit, KEDASUN_GATE_SHARP, st));
       }
@@ -1980,11 +1986,16 @@ int forward_mixed_list(b2_engine* e, int T, int ntiles, int nlast) {
       const float* wn = fuse_next ? NL->gain1 : nullptr;
       const float* bn = fuse_next ? NL->bias1 : nullptr;
       if (sp.ff == B2_FF_XIELU) {
-        {
+        // (prompt-sized: the activation in the product's epilogue instead of an fp32 [T][ff] between two kernels)
+        const bool act_fused = !f && T > 128 && list_dense_tc(e, T, sp.ff_dim, W) && linear_sum_pays(T, sp.ff_dim) && e->skip_mask == 0;
+        if (act_fused) {
           KL k(e, B2K_GEMM_GATEUP);
-          if (!k.skip()) B2_TRY(dense(e->l_x1, L.up, e->l_upf, T, sp.ff_dim, W));
-        }
-        {
+          B2_TRY(launch_linear_sum(e->l_x1, L.up, nullptr, 1, T, e->l_act, sp.ff_dim, W, SUM_EPI_XIELU, e->wait_limit(), st, 0, L.poly));
+        } else {
+          {
+            KL k(e, B2K_GEMM_GATEUP);
+            if (!k.skip()) B2_TRY(dense(e->l_x1, L.up, e->l_upf, T, sp.ff_dim, W));
+          }
           KL k(e, B2K_ACT);
           if (!k.skip()) B2_TRY(launch_xielu(e->l_upf, L.poly, e->l_act, f, (size_t)T * sp.ff_dim, st));
         }

@@ -6,8 +6,9 @@
 //   * groups: the experts' first rows are read from the device's own table when the kernel starts, so the host neither waits for it nor launches per expert.  A
 //     cluster walks the list of all experts' tiles with stride `clusters`, weight-row pair fastest; the rows that a group's last tile reads past its end belong to
 //     the next group (or to nobody: zero-filled) and are not stored.
-//   * epilogue: fp32 sums straight from registers (a warp's 32 weight rows are 128 contiguous bytes of an output row), or, for squared-ReLU experts, their
-//     activation rounded to the bf16 operand of the second product.
+//   * epilogue: fp32 sums straight from registers (a warp's 32 weight rows are 128 contiguous bytes of an output row), or, for squared-ReLU experts and Tinevik's dense
+//     feed-forward (4096 x 16384 at K 4096: 268 MB of sums written and read again otherwise, 2364 -> 2228 us of a whole call), the activation rounded to the bf16
+//     operand of the second product.
 //   * SPLIT 3: x is fp32, given as three bf16 planes whose sum it is (split3_kernel: 8 + 8 + 8 bits of the 24), and the weights are bf16 numbers, so the three
 //     products are exact.  The tensor pipe's accumulator rounds every addition towards zero, so it holds only 128 of the K at a time, smallest plane first: the
 //     epilogue's warps keep the running sums of a tile in registers and add a chunk, rounded to nearest, while the next one is multiplied.  SPLIT 1: the same
@@ -62,7 +63,7 @@ struct GsWalk {
 template <int BN, int EPI, int SPLIT>   // SPLIT: planes of x (0: x as it is, its whole K in the accumulator)
 __global__ void __launch_bounds__(GS_THREADS, 1)
 linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const int32_t* offsets, int groups,
-                  int rows_total, void* out, int N, int K, int ldo, const B2WaitLimit limit) {
+                  int rows_total, void* out, int N, int K, int ldo, const B2WaitLimit limit, const float* pq) {
   using C = GsCfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[C::STAGES];
@@ -171,6 +172,8 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
       if (lane == 0)
         pair_arrive(pair_first_cta(smem_u32(&tmem_empty_bar[as])));
     };
+    XieluCoef xc{};
+    if constexpr (EPI == SUM_EPI_XIELU) xc = xielu_coef(pq);
     auto store = [&](int c0, int col, const uint32_t (&r)[32]) {   // 32 rows of x from c0 of the tile on, this thread's weight row
       if (col >= N) return;
       const size_t at = (size_t)(w.row0 + c0) * ldo + col;
@@ -189,8 +192,8 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
         bf16* d = reinterpret_cast<bf16*>(out) + at;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
-          const float a = fmaxf(__uint_as_float(r[j]), 0.f);
-          if (j < have) d[(size_t)j * ldo] = __float2bfloat16_rn(a * a);
+          const float z = __uint_as_float(r[j]), a = fmaxf(z, 0.f);
+          if (j < have) d[(size_t)j * ldo] = __float2bfloat16_rn(EPI == SUM_EPI_XIELU ? xielu(xc, z) : a * a);
         }
       }
     };
@@ -294,7 +297,7 @@ __global__ void __launch_bounds__(256) split3_kernel(const float4* x, uint2* pla
 }
 
 template <int BN, int EPI, int SPLIT = 0>
-int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int ldo = 0) {
+int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int ldo = 0, const float* pq = nullptr) {
   using C = GsCfg<BN>;
   static B2PerDeviceOnce attr_once;
   if (attr_once.need()) B2_CUDA_OK(cudaFuncSetAttribute(linear_sum_kernel<BN, EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
@@ -319,7 +322,7 @@ int launch_sum(const void* x, const void* w, const int32_t* offsets, int groups,
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = b2_pdl_enabled() ? 2 : 1;
-  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_sum_kernel<BN, EPI, SPLIT>, tw, tx, offsets, groups, rows, out, N, K, ldo > 0 ? ldo : N, wait));
+  B2_CUDA_OK(cudaLaunchKernelEx(&cfg, linear_sum_kernel<BN, EPI, SPLIT>, tw, tx, offsets, groups, rows, out, N, K, ldo > 0 ? ldo : N, wait, pq));
   return 0;
 }
 
@@ -344,15 +347,18 @@ bool linear_sum_pays(int rows, int N) { return ((long)rows + 255) / 256 * ((N + 
 bool linear_sum_shapes_ok(int rows, int groups, int N, int K) { return rows >= 1 && groups >= 1 && groups <= GS_MAX_GROUPS && N >= 64 && K >= 64 && K % GS_BK == 0; }
 
 int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, const B2WaitLimit& wait,
-                      cudaStream_t s, int bn) {
+                      cudaStream_t s, int bn, const float* pq) {
   if (rows <= 0) return 0;
+  B2_REQUIRE(epilogue != SUM_EPI_XIELU || pq != nullptr, "linear_sum: the activation needs its numbers");
   B2_REQUIRE(linear_sum_shapes_ok(rows, groups, N, K) && (offsets != nullptr || groups == 1), "linear_sum: %d rows in %d groups, N=%d K=%d not built", rows, groups, N, K);
   if (bn == 0) bn = sum_pick_bn(rows, groups, N);
-#define B2_SUM_CASE(B, E) if (bn == B && epilogue == E) return launch_sum<B, E>(x, w, offsets, groups, rows, out, N, K, wait, s)
+#define B2_SUM_CASE(B, E) if (bn == B && epilogue == E) return launch_sum<B, E>(x, w, offsets, groups, rows, out, N, K, wait, s, 0, pq)
   B2_SUM_CASE(256, SUM_EPI_F32);
   B2_SUM_CASE(128, SUM_EPI_F32);
   B2_SUM_CASE(256, SUM_EPI_RELU2);
   B2_SUM_CASE(128, SUM_EPI_RELU2);
+  B2_SUM_CASE(256, SUM_EPI_XIELU);
+  B2_SUM_CASE(128, SUM_EPI_XIELU);
 #undef B2_SUM_CASE
   b2_set_error("linear_sum: tile %d, epilogue %d not built", bn, epilogue);
   return -22;

@@ -114,11 +114,11 @@ int launch_few_attn(const bf16* qkv, const bf16* qw, const bf16* kw, const bf16*
                     const int32_t* block_table, int bt_stride, const int32_t* seq_lens, bf16* out, int B, int nq, int nkv, float eps, float scale, cudaStream_t s);
 // gemm_sum.cu: prompt-sized products with fp32 sums out (or a squared-ReLU expert's bf16 activation), rows of one block or of the ragged blocks of
 // `groups` experts (offsets: [groups + 1] first rows, device memory; null: one block); w [groups * N][K]; bn: 0 = by the sizes
-enum { SUM_EPI_F32 = 0, SUM_EPI_RELU2 = 1 };
+enum { SUM_EPI_F32 = 0, SUM_EPI_RELU2 = 1, SUM_EPI_XIELU = 2 };   // the last two leave the bf16 activation: max(z, 0)^2; launch_xielu's, with its two numbers
 bool linear_sum_shapes_ok(int rows, int groups, int N, int K);
 bool linear_sum_pays(int rows, int N);   // one block of rows: faster than launch_linear_tc
 int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, const B2WaitLimit& wait,
-                      cudaStream_t s, int bn = 0);
+                      cudaStream_t s, int bn = 0, const float* pq = nullptr);
 // the same for fp32 x [rows][K] and bf16 weights, fp32 precision: x goes to three bf16 planes ([3][rows][K], scratch) whose sum it is
 int launch_linear_split3(const float* x, bf16* planes, const bf16* w, float* out, int rows, int N, int K, const B2WaitLimit& wait, cudaStream_t s, int bn = 0);
 // ... and for fp32 weights that are bf16 numbers, as a checkpoint's are: each product narrows its matrix into the scratch, which holds any shape in pieces
@@ -133,6 +133,8 @@ int launch_linear_sum_fine(const void* x, const void* w, float* out, int rows, i
 // gemm_gateup.cu: the prefill-sized counterpart (two accumulators per tile, SwiGLU in the epilogue)
 bool gateup_prefill_shapes_ok(int T, int I, int K);
 int launch_gateup_swiglu_prefill(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* act, int T, int I, int K, int x_row0, cudaStream_t s);
+// ... with Kedasun's activation, fp32 up to the rounding: g / (1 + e^(-sharp g)) * (u + 1), g = min(gate, limit), u = up within +-limit
+int launch_gateup_clamped_prefill(const CUtensorMap& tm_w, const CUtensorMap& tm_x128, bf16* act, int T, int I, int K, float limit, float sharp, cudaStream_t s);
 // Normalise-on-load (see gemm_pair.cu): x is the residual stream, ssq [pieces][ld] the per-16-feature sums of squares of
 // its rows (gemm_resid.cu writes them), gain the RMSNorm weight.  Default: x is used as given.
 struct PairNorm {
@@ -377,6 +379,13 @@ int launch_streams_sum(const float* h, int n, float* out, int T, int W, cudaStre
 int launch_token_shift(const void* x, int x_f32, const float* mu, void* ring, void* out, int T, int W, const int32_t* row_seq, const int32_t* row_first,
                        const int32_t* row_end, const int32_t* positions, const int32_t* slots, cudaStream_t s);
 // act[i] = softplus(p) z^2 + z / 2 for z > 0, (1/2 + softplus(q)) (exp(z) - 1 - z) + z / 2 otherwise; pq (device) = p, q
+// a(z) = softplus(p) z^2 + z / 2 for z > 0 and (1/2 + softplus(q)) (exp(z) - 1 - z) + z / 2 otherwise
+struct XieluCoef { float ap, an; };
+__device__ __forceinline__ XieluCoef xielu_coef(const float* pq) {
+  auto softplus = [](float x) { return x > 20.f ? x : log1pf(expf(x)); };
+  return XieluCoef{softplus(pq[0]), 0.5f + softplus(pq[1])};
+}
+__device__ __forceinline__ float xielu(const XieluCoef& c, float v) { return v > 0.f ? fmaf(c.ap * v, v, 0.5f * v) : fmaf(c.an, expm1f(v) - v, 0.5f * v); }
 int launch_xielu(const float* z, const float* pq, void* act, int act_f32, size_t n, cudaStream_t s);
 // out[t * out_ld + i] = scale * a[t][i] * sigmoid(gate[t * gate_ld + i]), a fp32 (or bf16: a_bf16) [T][N], out fp32 or bf16 (out_ld 0 = N)
 int launch_sigmoid_gate(const void* a, const float* gate, int gate_ld, void* out, int out_f32, int T, int N, cudaStream_t s, int a_bf16 = 0,

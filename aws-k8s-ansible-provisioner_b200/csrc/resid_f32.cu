@@ -638,18 +638,13 @@ __global__ void __launch_bounds__(128) layer_norm_add_kernel(float* h, const flo
   for (int i = threadIdx.x; i < W; i += 128) x_next[(size_t)t * W + i] = (TX)((lrow[i] - mean2) * r2 * w_next[i] + b_next[i]);
 }
 
-__device__ __forceinline__ float softplus_f(float x) { return x > 20.f ? x : log1pf(expf(x)); }
-
-// act = a(z), a(z) = softplus(p) z^2 + z / 2 for z > 0 and (1/2 + softplus(q)) (exp(z) - 1 - z) + z / 2 otherwise; pq (device) = p, q
+// act = a(z), pq (device) = p, q
 template <typename TX>
 __global__ void __launch_bounds__(256) xielu_kernel(const float* z, const float* __restrict__ pq, TX* __restrict__ act, size_t n) {
   pdl_wait();
   pdl_launch_dependents();
-  const float ap = softplus_f(pq[0]), an = 0.5f + softplus_f(pq[1]);
-  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
-    const float v = z[i];
-    act[i] = (TX)(v > 0.f ? fmaf(ap * v, v, 0.5f * v) : fmaf(an, expm1f(v) - v, 0.5f * v));
-  }
+  const XieluCoef c = xielu_coef(pq);
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) act[i] = (TX)xielu(c, z[i]);
 }
 
 // out[t * out_ld + i] = scale * a[t][i] * sigmoid(gate[t * gate_ld + i]); VEC: four numbers at a time (rows and bases on 16-byte boundaries)

@@ -426,6 +426,10 @@ int b2k_linear_multicast(const void* x_bf16, const void* w_bf16, void* out_bf16,
  * rows the kernel reads from device memory (offsets [groups + 1], the last one = rows): out[row][N] = x[row][K] . w_g[N][K]^T as fp32 (epilogue 0) or
  * bf16(max(sum, 0)^2) (1), or, for one block, fp32 with the sums rounded to nearest every 128 of K (2).  K % 64 == 0; tile: 0 (by the sizes), 128 or 256 rows of x. */
 int b2k_linear_sum(const void* x_bf16, const void* w_bf16, const int32_t* offsets, int groups, int rows, void* out, int N, int K, int epilogue, int tile, void* stream);
+/* The same product with Tinevik's activation on it, a(z) = softplus(p) z^2 + z / 2 for z > 0 and (1/2 + softplus(q)) (e^z - 1 - z) + z / 2 otherwise, pq = p, q; act bf16 [rows][N]. */
+int b2k_linear_xielu(const void* x_bf16, const void* w_bf16, const float* pq, void* act_bf16, int rows, int N, int K, int tile, void* stream);
+/* act [T][I] bf16 = g / (1 + e^(-sharp g)) (u + 1), g = min(gate, limit), u = up within +-limit, gate | up = x . Wgu^T in fp32 (T >= 256, I in steps of 128, K of 64 from 256). */
+int b2k_gateup_clamped(const void* x_bf16, const void* w_gu_bf16, void* act_bf16, int T, int I, int K, float limit, float sharp, void* stream);
 /* A decode step's products for at most eight sequences (csrc/gemm_few.cu), K % 32 == 0, all bf16: mode 0: out[T][N] = RMSNorm(x) . w^T; 1: out += x . w^T (gain unused);
  * 2: out[T][N] = silu(g) * u with g | u = RMSNorm(x) . w^T, w [2N][K] (gate rows, then up rows). */
 int b2k_few_linear(const void* w, const void* x, const void* gain, float eps, void* out, int T, int N, int K, int mode, void* stream);

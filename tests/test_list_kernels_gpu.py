@@ -239,6 +239,40 @@ def test_linear_split3_wide(lib, rows, N, K, rows_at_a_time, cols_at_a_time):
         assert lib.b2k_linear_split3_wide(ptr(x), ptr(wide), ptr(planes), 255 * K, ptr(narrow), nw, ptr(out), rows, N, K, cuda_stream_ptr()) != 0
 
 
+@pytest.mark.parametrize("rows,N,K,tile", [(129, 256, 64, 128), (300, 320, 192, 256), (700, 1024, 1024, 0)])
+def test_linear_xielu(lib, rows, N, K, tile):
+    """Against 64 bits: the activation's slope is at most 2 softplus(p) |z| + 1/2 and 1.2 below zero, its argument is an fp32 sum, the result one rounding to bf16."""
+    g = torch.Generator().manual_seed(rows)
+    x, w = torch.randn(rows, K, generator=g).to(torch.bfloat16), (torch.randn(N, K, generator=g) * K ** -0.5).to(torch.bfloat16)
+    pq = torch.tensor([0.3, -0.2])
+    act = torch.full((rows + 1, N), float("nan"), dtype=torch.bfloat16, device="cuda")
+    dx, dw, dp = x.cuda(), w.cuda(), pq.cuda()
+    chk(lib, lib.b2k_linear_xielu(ptr(dx), ptr(dw), ptr(dp), ptr(act), rows, N, K, tile, cuda_stream_ptr()))
+    z = x.double() @ w.double().t()
+    ap, an = torch.nn.functional.softplus(pq.double())
+    ref = torch.where(z > 0, ap * z * z + z / 2, (0.5 + an) * (torch.expm1(z) - z) + z / 2)
+    assert torch.isnan(act[rows]).all()
+    err = (act[:rows].cpu().double() - ref).abs()
+    assert (err <= 2.0 ** -8 * ref.abs() + (2 * z.abs() + 1) * 2.0 ** -17).all(), err.max()
+
+
+@pytest.mark.parametrize("T,I,K", [(256, 128, 256), (300, 384, 512), (513, 1024, 1024)])
+def test_gateup_clamped(lib, T, I, K):
+    """Against 64 bits: gate and up are fp32 sums (2^-17 of a few units), both factors are at most limit and limit + 1 wide, the result is one rounding to bf16."""
+    g = torch.Generator().manual_seed(T)
+    x, w = torch.randn(T, K, generator=g).to(torch.bfloat16), (torch.randn(2 * I, K, generator=g) * 3 * K ** -0.5).to(torch.bfloat16)
+    act = torch.full((T + 1, I), float("nan"), dtype=torch.bfloat16, device="cuda")
+    dx, dw = x.cuda(), w.cuda()
+    limit, sharp = 5.0, 1.7
+    chk(lib, lib.b2k_gateup_clamped(ptr(dx), ptr(dw), ptr(act), T, I, K, limit, sharp, cuda_stream_ptr()))
+    z = x.double() @ w.double().t()
+    gate, up = z[:, :I].clamp(max=limit), z[:, I:].clamp(-limit, limit)
+    ref = gate * torch.sigmoid(sharp * gate) * (up + 1)
+    assert torch.isnan(act[T]).all()
+    err = (act[:T].cpu().double() - ref).abs()
+    assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -14).all(), err.max()
+
+
 @pytest.mark.parametrize("heads,softcap,turned,bs,pieces", [(32, 20.0, True, 16, False), (32, 0.0, False, 64, True), (16, 50.0, True, 32, True), (8, 3.0, False, 16, False)])
 def test_heads_premix(lib, heads, softcap, turned, bs, pieces):
     """Portions around the tiles of 64, the units of 8 or 16 tokens and the blocks of 128 keys, some behind earlier tokens; `pieces`: a scratch that holds two tiles' units at most.
