@@ -779,9 +779,11 @@ int forward_opt(b2_engine* e, int T, int ntiles, int nlast) {
   return lm_head_and_argmax(e, nlast, xl, xb);
 }
 
-// The fused launches that a decode step of T rows takes
+// The fused launches that a decode step of T rows, or a short prompt's, takes.  Prompts, us a call of 28 layers of the served model, stand-alone kernels / these: 17 tokens
+// 1083 / 950, 24 tokens 1074 / 939, 48 tokens 1205 / 1090, 64 tokens 1177 / 1115.  With two token tiles from 65 tokens on they would run in two waves (100 tokens 1398 / 1597;
+// the QKV projection's alone 1385 / 1369).
 struct DecodeForms { bool qkv_pair = false, gu_pair = false, resid = false, few = false; };
-DecodeForms decode_forms(const b2_engine* e, const LayerW& L, int T, bool beside_attention) {
+DecodeForms decode_forms(const b2_engine* e, const LayerW& L, int T, bool beside_attention, bool prompt = false) {
   const b2_config& c = e->cfg;
   const int H = c.hidden, I = c.intermediate;
   auto skipped = [&](int k) { return ((e->skip_mask >> k) & 1u) != 0; };
@@ -794,7 +796,7 @@ DecodeForms decode_forms(const b2_engine* e, const LayerW& L, int T, bool beside
   f.resid = f.qkv_pair && f.gu_pair && (e->use_pair & 4) && e->ssq != nullptr && H / 16 <= 64 && resid_shapes_ok(T, H, e->q_size) && resid_shapes_ok(T, H, I) &&
             !skipped(B2K_NORM) && !skipped(B2K_GEMM_O) && !skipped(B2K_GEMM_DOWN) && !skipped(B2K_GEMM_QKV) && !skipped(B2K_GEMM_GATEUP);
   // ... and at most eight sequences take the kernels of gemm_few.cu, unless their contexts are too long (pick_attn_split)
-  f.few = f.resid && few_shapes_ok(T, H, e->q_size, I) && e->nq == 2 * e->nkv && e->hd == 128 && c.block_size == 16 && c.sliding_window <= 0 && e->use_few &&
+  f.few = f.resid && !prompt && few_shapes_ok(T, H, e->q_size, I) && e->nq == 2 * e->nkv && e->hd == 128 && c.block_size == 16 && c.sliding_window <= 0 && e->use_few &&
           e->skip_mask == 0 && !e->l2_weight_prefetch;
   return f;
 }
@@ -842,10 +844,10 @@ int forward_layers(b2_engine* e, const Lane& ln, int T, int ntiles) {
     LayerW& L = e->layers[l];
     bf16* kp = e->kv_pool + (size_t)(2 * l) * e->layer_kv_elems;
     bf16* vp = kp + e->layer_kv_elems;
-    // decode-sized forwards: the fused cluster-pair launches of gemm_pair.cu take the place of (projection, element-wise
+    // decode-sized forwards and short prompts: the fused cluster-pair launches of gemm_pair.cu take the place of (projection, element-wise
     // kernel) pairs where the model's shapes allow it
     // (at most eight sequences: five launches a layer too, for a chain that is bound by latencies)
-    const DecodeForms forms = ntiles == 0 ? decode_forms(e, L, T, ln.beside_attention) : DecodeForms();
+    const DecodeForms forms = decode_forms(e, L, T, ln.beside_attention, ntiles > 0);
     const bool qkv_pair = forms.qkv_pair, gu_pair = forms.gu_pair, resid = forms.resid;
     if (forms.few && !e->step_long) {
       {
