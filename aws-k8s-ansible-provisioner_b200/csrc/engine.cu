@@ -2584,16 +2584,15 @@ struct Uploads {
   }
 };
 __global__ void __launch_bounds__(256) upload_kernel(const Uploads l) {
-  for (int k = 0; k < l.n; ++k) {
-    const Upload u = l.u[k];
-    for (int i = blockIdx.x * 256 + threadIdx.x; i < u.ints; i += gridDim.x * 256) u.dst[i] = *(const volatile int32_t*)(u.src + i);
-  }
+  const Upload u = l.u[blockIdx.y];   // (a row of CTAs per list: one list after the other would be a trip to the host each, 14 - 24 us instead of 5 - 10)
+#pragma unroll 4
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < u.ints; i += gridDim.x * 256) u.dst[i] = u.src[i];
 }
 int launch_uploads(const Uploads& l, cudaStream_t s, bool then_kernels) {
   int most = 0;
   for (int k = 0; k < l.n; ++k) most = std::max(most, l.u[k].ints);
   if (most == 0) return 0;
-  upload_kernel<<<std::min(148, (most + 255) / 256), 256, 0, s>>>(l);
+  upload_kernel<<<dim3(std::min(32, (most + 255) / 256), l.n), 256, 0, s>>>(l);
   B2_CUDA_OK(cudaGetLastError());
   if (then_kernels) b2_pdl_skip_next();   // the step's kernels read these lists in front of their dependency wait: the first of them starts when all of this is done
   return 0;
