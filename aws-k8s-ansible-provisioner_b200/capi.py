@@ -78,6 +78,8 @@ SIGNATURES = {
     "b2_prefill": (_I, [_P, _I32P, _I32P, C.c_int32, _I32P, _I32P]),
     "b2_decode_step": (_I, [_P, C.c_int32, _I32P, _I32P, _I32P]),
     "b2_decode_run": (_I, [_P, C.c_int32, _I32P, C.c_int32, _I32P, C.POINTER(C.c_float)]),
+    "b2_host_alloc": (_I, [C.c_size_t, C.POINTER(_P)]),
+    "b2_host_free": (None, [_P]),
     "b2_get_logits": (_I, [_P, C.c_int32, C.POINTER(C.c_float)]),
     "b2_config_from_dir": (_I, [C.c_char_p, C.POINTER(b2_config), C.POINTER(b2_layer_spec), C.c_int32]),
     "b2_prefill_logits": (_I, [_P, _I32P, _I32P, C.c_int32, _I32P, _I32P, C.c_int32, C.POINTER(C.c_float), _I32P]),

@@ -6228,6 +6228,15 @@ extern "C" int b2_get_logits(b2_engine* e, int32_t nseq, float* out_logits) {
   return read_bf16_rows(e, out_logits, e->logits, n);
 }
 
+extern "C" int b2_host_alloc(size_t bytes, void** out) {
+  B2_REQUIRE(bytes > 0 && out, "b2_host_alloc: bad arguments");
+  B2_CUDA_OK(cudaHostAlloc(out, bytes, cudaHostAllocPortable));
+  return 0;
+}
+extern "C" void b2_host_free(void* p) {
+  if (p) cudaFreeHost(p);
+}
+
 extern "C" int b2_set_next_tokens(b2_engine* e, int32_t nseq, const int32_t* seq_ids, const int32_t* tokens) {
   B2_REQUIRE(e && seq_ids && tokens, "b2_set_next_tokens: null argument");
   B2_REQUIRE((int)e->cur_batch.size() == nseq && std::equal(seq_ids, seq_ids + nseq, e->cur_batch.begin()),

@@ -308,6 +308,9 @@ int  b2_prefill_logits(b2_engine* e, const int32_t* ids, const int32_t* seq_offs
 
 /* Logits of the last forward's last positions, [nseq][vocab] fp32 on the host. */
 int  b2_get_logits(b2_engine* e, int32_t nseq, float* out_logits);
+/* Page-locked host memory (usable with every device): results that are read back land in it by one copy, without fresh pages to fill. */
+int  b2_host_alloc(size_t bytes, void** out);
+void b2_host_free(void* p);
 /* Residual stream after layer `layer` (0-based; -1 = embeddings, num_layers = final norm
  * output) for the tokens of the last forward, [ntokens][hidden] as bf16 bits on the host.
  * Only filled when debug capture was enabled with b2_set_debug(e, 1). */
