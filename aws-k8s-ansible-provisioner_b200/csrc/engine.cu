@@ -1017,7 +1017,7 @@ int list_dense(b2_engine* e, const void* A, const void* Wt, float* C, int M, int
   if (alpha == 1.f && list_dense_tc(e, M, N, K)) {
     if (M > 128 && linear_sum_pays(M, N)) return launch_linear_sum(A, Wt, nullptr, 1, M, C, N, K, SUM_EPI_F32, e->wait_limit(), ls);
     TcGemmArgs a;
-    a.bn = tc_pick_bn(M);
+    a.bn = tc_pick_bn_wave(M, N, e->num_sms);
     B2_TRY(b2_make_tmap_bf16(&a.tmap_w, Wt, (uint64_t)N, (uint64_t)K, (uint64_t)K, 128));
     B2_TRY(b2_make_tmap_bf16(&a.tmap_x, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)a.bn));
     a.T = M; a.N = N; a.K = K;
@@ -1181,7 +1181,7 @@ constexpr int LATENT_REBUILD_ROWS = 128;    // portions of at least this many to
 // C (bf16 [M][N]) = A (bf16 [M][K]) . Wt^T on the tcgen05 projection kernel (K a multiple of 64, N at least 128)
 int list_dense_bf16(b2_engine* e, const bf16* A, const bf16* Wt, bf16* C, int M, int N, int K, cudaStream_t s) {
   TcGemmArgs a;
-  a.bn = tc_pick_bn(M);
+  a.bn = tc_pick_bn_wave(M, N, e->num_sms);
   B2_TRY(b2_make_tmap_bf16(&a.tmap_w, Wt, (uint64_t)N, (uint64_t)K, (uint64_t)K, 128));
   B2_TRY(b2_make_tmap_bf16(&a.tmap_x, A, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)a.bn));
   a.T = M; a.N = N; a.K = K;

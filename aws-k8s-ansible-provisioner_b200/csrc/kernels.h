@@ -90,6 +90,7 @@ int tc_pick_bn(int T);
 int tc_set_trace(unsigned long long* dev_buf);  // diagnostics: per-CTA phase timestamps (null = off)
 // choose a split-K factor so that tiles * splits fills the SMs (each split gets >= 1 k-block)
 int tc_pick_nsplit(int T, int N, int K, int num_sms);
+int tc_pick_bn_wave(int T, int N, int num_sms);
 
 // ---- gemm_pair.cu: a projection and the element-wise kernel behind it in one launch (clusters of two CTAs split K and
 //      exchange accumulator halves through distributed shared memory); at most 64 tokens, K <= 1024 ----
