@@ -2324,7 +2324,8 @@ int forward_streams_list(b2_engine* e, int T, int ntiles, int nlast) {
         KL k(e, B2K_GEMM_QKV);   // r, k, v and the gate, each from its own blend
         if (!k.skip()) {
           if (list_dense_tc(e, T, HR, W)) {
-            for (int m = 0; m < 4; ++m) B2_TRY(dense(blend(m), (const char*)L.wshift + (size_t)m * HR * W * es, e->l_rkvg + m * TH, T, HR, W, sB));
+            // (blends, weights and outputs lie one behind the other: four groups of one launch; 1011 tokens 32 us instead of 57 one by one)
+            B2_TRY(launch_linear_sum(blend(0), L.wshift, nullptr, 4, 4 * T, e->l_rkvg, HR, W, SUM_EPI_F32, e->wait_limit(), sB));
           } else {
             AnyGemm a;
             a.A = e->l_shift; a.W = L.wshift; a.C = e->l_rkvg; a.M = T; a.N = HR; a.K = W; a.lda = W; a.ldw = W; a.ldc = HR;

@@ -59,7 +59,7 @@ struct GsWalk {
   }
 };
 
-// offsets: [groups + 1] first rows of the groups in device memory, or null: one group of `rows_total` rows
+// offsets: [groups + 1] first rows of the groups in device memory, or null: groups of rows_total / groups rows
 template <int BN, int EPI, int SPLIT>   // SPLIT: planes of x (0: x as it is, its whole K in the accumulator)
 __global__ void __launch_bounds__(GS_THREADS, 1)
 linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const int32_t* offsets, int groups,
@@ -102,8 +102,8 @@ linear_sum_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_const
   if (threadIdx.x == 0) pdl_launch_dependents();
   if (offsets != nullptr) {
     for (int i = threadIdx.x; i <= groups; i += GS_THREADS) s_off[i] = min(max(offsets[i], 0), rows_total);
-  } else if (threadIdx.x < 2) {
-    s_off[threadIdx.x] = threadIdx.x * rows_total;
+  } else {   // groups of the same size
+    for (int i = threadIdx.x; i <= groups; i += GS_THREADS) s_off[i] = rows_total / groups * i;
   }
   tc_fence_before();
   __syncthreads();
@@ -350,7 +350,7 @@ int launch_linear_sum(const void* x, const void* w, const int32_t* offsets, int 
                       cudaStream_t s, int bn, const float* pq) {
   if (rows <= 0) return 0;
   B2_REQUIRE(epilogue != SUM_EPI_XIELU || pq != nullptr, "linear_sum: the activation needs its numbers");
-  B2_REQUIRE(linear_sum_shapes_ok(rows, groups, N, K) && (offsets != nullptr || groups == 1), "linear_sum: %d rows in %d groups, N=%d K=%d not built", rows, groups, N, K);
+  B2_REQUIRE(linear_sum_shapes_ok(rows, groups, N, K) && (offsets != nullptr || rows % groups == 0), "linear_sum: %d rows in %d groups, N=%d K=%d not built", rows, groups, N, K);
   if (bn == 0) bn = sum_pick_bn(rows, groups, N);
 #define B2_SUM_CASE(B, E) if (bn == B && epilogue == E) return launch_sum<B, E>(x, w, offsets, groups, rows, out, N, K, wait, s, 0, pq)
   B2_SUM_CASE(256, SUM_EPI_F32);

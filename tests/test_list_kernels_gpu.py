@@ -239,6 +239,20 @@ def test_linear_split3_wide(lib, rows, N, K, rows_at_a_time, cols_at_a_time):
         assert lib.b2k_linear_split3_wide(ptr(x), ptr(wide), ptr(planes), 255 * K, ptr(narrow), nw, ptr(out), rows, N, K, cuda_stream_ptr()) != 0
 
 
+@pytest.mark.parametrize("rows,groups,N,K", [(1, 4, 64, 64), (65, 4, 320, 128), (300, 4, 2048, 192), (257, 3, 256, 64)])
+def test_linear_sum_equal_groups(lib, rows, groups, N, K):
+    """Groups of the same size without a table: the same bits as a launch for each."""
+    g = torch.Generator().manual_seed(rows)
+    x, w = (torch.randn(groups, n, K, generator=g).to(torch.bfloat16).cuda() for n in (rows, N))
+    for tile in (128, 256):
+        out, one = torch.full((groups * rows + 1, N), float("nan"), device="cuda"), torch.empty(groups, rows, N, device="cuda")
+        chk(lib, lib.b2k_linear_sum(ptr(x), ptr(w), None, groups, groups * rows, ptr(out), N, K, 0, tile, cuda_stream_ptr()))
+        for i in range(groups):
+            chk(lib, lib.b2k_linear_sum(ptr(x[i]), ptr(w[i]), None, 1, rows, ptr(one[i]), N, K, 0, tile, cuda_stream_ptr()))
+        assert torch.equal(out[:-1].view_as(one), one) and torch.isnan(out[-1]).all()
+    assert lib.b2k_linear_sum(ptr(x), ptr(w), None, groups, groups * rows + 1, ptr(out), N, K, 0, 128, cuda_stream_ptr()) != 0
+
+
 @pytest.mark.parametrize("rows,N,K,tile", [(129, 256, 64, 128), (300, 320, 192, 256), (700, 1024, 1024, 0)])
 def test_linear_xielu(lib, rows, N, K, tile):
     """Against 64 bits: the activation's slope is at most 2 softplus(p) |z| + 1/2 and 1.2 below zero, its argument is an fp32 sum, the result one rounding to bf16."""
