@@ -132,10 +132,38 @@ def _p32(a: np.ndarray):
     return a.ctypes.data_as(C.POINTER(C.c_int32))
 
 
+class _PageLocked:
+    """Page-locked blocks that no engine uses, for the next one: at most `LIMIT` bytes once `trim` has run, which making and closing an engine do.  (Never freed where an
+    array goes: that would make the driver wait inside somebody's call.)"""
+
+    LIMIT = 64 << 20
+
+    def __init__(self):
+        self.lock, self.idle = threading.Lock(), collections.deque()   # (bytes, address, library); threads and finalizers append
+
+    def take(self, lib, size: int):
+        with self.lock:
+            for b in list(self.idle):
+                if size <= b[0] <= 2 * size and b[2] is lib:
+                    self.idle.remove(b)
+                    return b
+        p = C.c_void_p()
+        return (size, p.value, lib) if lib.b2_host_alloc(size, C.byref(p)) == 0 else None
+
+    def trim(self, limit: int | None = None) -> None:
+        with self.lock:
+            while sum(b[0] for b in list(self.idle)) > (self.LIMIT if limit is None else limit):
+                size, p, lib = self.idle.popleft()
+                lib.b2_host_free(p)
+
+
+_page_locked = _PageLocked()
+
+
 class _Results:
     """fp32 result arrays in memory that is used again once nobody holds the array that lay in it, nor a view of that: fresh pages cost more than the copy.
 
-    Two page-locked blocks of `first` bytes, where that is little (2 - 3 ms each, 20 - 50 for 39 MB), take the copy directly: a call that returned 2 MB of logits 1189 -> 909 us.
+    Two page-locked blocks of `first` bytes, where that is little (2 - 3 ms each when new, 20 - 50 for 39 MB), take the copy directly: a call that returned 2 MB of logits 1189 -> 909 us.
     Results that do not fit them lie in ordinary memory (39 MB of bf16 rows widened on the host: 3.1 -> 1.8 ms), of which at most `LIMIT` bytes in `BLOCKS` blocks are kept;
     a caller that holds more results than that gets new arrays."""
 
@@ -143,13 +171,14 @@ class _Results:
 
     def __init__(self, lib, first: int):
         self.lib, self.lock = lib, threading.Lock()
-        self.free, self.back = [], collections.deque()   # (bytes, address, its owner or None: page-locked); `back`: what arrays left behind (finalizers only append)
+        self.free, self.back = [], collections.deque()   # (bytes, address, its owner: an array, or the library that made it page-locked); `back`: what arrays left behind
         self.blocks = self.bytes = 0
         self.open = True
         for _ in range(2):
-            p = C.c_void_p()
-            if 0 < first <= self.PINNED and lib.b2_host_alloc(first, C.byref(p)) == 0:
-                self.free.append((first, p.value, None))
+            block = _page_locked.take(lib, first) if 0 < first <= self.PINNED else None
+            if block is not None:
+                self.free.append(block)
+        _page_locked.trim()
 
     def array(self, rows: int, cols: int) -> np.ndarray:
         need, got = rows * cols * 4, None
@@ -182,14 +211,15 @@ class _Results:
                     block = blocks.pop()
                 except IndexError:   # (another thread took the last one)
                     break
-                if block[2] is None:
-                    self.lib.b2_host_free(block[1])
+                if not isinstance(block[2], np.ndarray):
+                    _page_locked.idle.append(block)
 
     def close(self) -> None:
-        """What is held now is freed when its last array goes."""
+        """What is held now is given back when its last array goes."""
         with self.lock:
             self.open = False
             self._drop()
+        _page_locked.trim()
 
 
 class Engine:

@@ -59,11 +59,18 @@ def test_blocks_are_bounded_and_given_back(first):
     gc.collect()
     again = [r.array(3, 70000) for _ in range(2)]
     assert {addr(a) for a in again} == kept
+    small = r.array(1, 1)
     r.close()
-    assert not lib.held and (again[0].sum(), again[1].sum()) == (210000.0, 210000.0)
+    assert (again[0].sum(), again[1].sum()) == (210000.0, 210000.0)
     again.clear()
+    del small
     gc.collect()
     assert not r.free and not r.back and r.array(1, 1).shape == (1, 1)
+    next_one = engine._Results(lib, first)   # (the closed engine's page-locked blocks serve the next one)
+    assert len(lib.held) == (2 if first == 1 << 16 else 0)
+    next_one.close()
+    engine._page_locked.trim(0)
+    assert not lib.held
 
 
 def test_threads():
