@@ -572,7 +572,7 @@ int tc_pick_bn(int T) {
   return 256;
 }
 
-// The narrowest tile of tokens, from 32 on, whose tiles still run in one wave: a product that fills half of the SMs with 256-token tiles takes half the time with twice as many.
+// The narrowest tile of tokens, from 32 on, whose tiles still run in one wave: a product that fills half of the SMs with 256-token tiles gains from twice as many.
 // 1011 rows of x, us in the step: 2048 x 2048 (64 tiles of 256, 128 of 128) 17.2 / 13.9, 2048 x 6144 36.5 / 32.5, 128 x 2048 (4, 32 of 32) 15 / 12.5.  The sums are the same,
 // bit for bit.  (Split-K products of the GQA families stay with tc_pick_bn: 129 tokens 1561 us a call, with tiles of 128 and half the splits 1648.)
 int tc_pick_bn_wave(int T, int N, int num_sms) {

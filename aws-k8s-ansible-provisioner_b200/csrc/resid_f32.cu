@@ -337,9 +337,10 @@ __device__ __forceinline__ void st4(float* p, const float (&v)[4]) { *reinterpre
 __device__ __forceinline__ void st4(bf16* p, const float (&v)[4]) { *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3])); }
 
 // The same with the row held in registers (NV runs of 1024 numbers) and 16-byte accesses: the row is read once.  Bound by memory.
-// 16384 rows of 9216, bf16 out: 215 -> 175 us (906 MB: 5.2 TB/s).
+// 16384 rows of 9216, bf16 out: 215 -> 175 us (906 MB: 5.2 TB/s) with two rows on an SM at a time; behind its product, where that one's last lines are still on their way
+// out, 219 -> 180 with four.
 template <typename TX, int NV>
-__global__ void __launch_bounds__(256) poly_norm_vec_kernel(const float* z, const float* __restrict__ coef, TX* __restrict__ act, int F,
+__global__ void __launch_bounds__(256, NV <= 9 ? 4 : NV <= 12 ? 3 : 2) poly_norm_vec_kernel(const float* z, const float* __restrict__ coef, TX* __restrict__ act, int F,
                                                             float eps) {
   __shared__ float red[3][8];
   pdl_wait();
@@ -1236,9 +1237,13 @@ int launch_poly_norm(const float* z, const float* coef, void* act, int act_f32, 
     if (act_f32) B2_CUDA_OK(b2_launch(poly_norm_vec_kernel<float, NV>, dim3(T), dim3(256), 0, s, z, coef, (float*)act, F, eps));            \
     else B2_CUDA_OK(b2_launch(poly_norm_vec_kernel<bf16, NV>, dim3(T), dim3(256), 0, s, z, coef, (bf16*)act, F, eps));                      \
   } while (0)
-    if (F <= 4096) PN_LAUNCH(4);
-    else if (F <= 8192) PN_LAUNCH(8);
-    else if (F <= 12288) PN_LAUNCH(12);
+    // (as few registers as the row takes: rows on their way are what hides the memory's latency)
+    const int nv = (F + 1023) / 1024;
+    if (nv <= 3) PN_LAUNCH(3);
+    else if (nv <= 5) PN_LAUNCH(5);
+    else if (nv <= 7) PN_LAUNCH(7);
+    else if (nv <= 9) PN_LAUNCH(9);
+    else if (nv <= 12) PN_LAUNCH(12);
     else PN_LAUNCH(16);
 #undef PN_LAUNCH
     return 0;
