@@ -10,9 +10,9 @@
 //   premix_values  64 query tokens of one key/value head's two heads per CTA: the scratch rows as they are (fp32), causal mask, online softmax, P . V on warp-level MMAs with the
 //                  weights as bf16 value + remainder, the turn back by the query's position, one rounding.
 // Units of whole tiles are cut into launches that fit the scratch.
-// Measured, 4 x 1024 tokens of 32 heads: the cluster kernel of attn_heads.cu 1860 us, here 300 + 195 (16 heads: 495 -> 90 + 127).  premix_scores takes 187 us without the mix and the
+// Measured, 4 x 1024 tokens of 32 heads: the cluster kernel of attn_heads.cu 1860 us, here 212 + 180 (16 heads: 495 -> 86 + 126).  premix_scores takes 187 us without the mix and the
 // cap (K and Q on their way, 640 bytes a pair from L2, in 2 KB copies 226) and the mix's multiply-adds 70 at the FMA pipe's rate; sixteen warps with the matrix in shared memory took 314,
-// eight 330.  premix_values is bound by the warp-level MMAs (40 % busy) and the latencies between them.
+// eight 330, the matrix in constant memory with running places 299.  premix_values is bound by the warp-level MMAs (40 % busy) and the latencies between them.
 #include "kernels.h"
 
 #include <algorithm>
@@ -218,8 +218,8 @@ premix_scores_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
       for (int i = 0; i < H / 2; ++i)
 #pragma unroll
         for (int t = 0; t < QT; ++t) acc[i][t] = 0ull;
-#pragma unroll 1
-      for (int g2 = 0; g2 < G / 2; ++g2, ++it) {   // (two key/value heads at a time: a warp's way from the barrier to its scores is longer than its sums for one)
+#pragma unroll
+      for (int g2 = 0; g2 < G / 2; ++g2, ++it) {   // (unrolled: the matrix's entries have fixed places in constant memory then, and are operands of the sums; loads of them 299 -> 212 us.  Two key/value heads at a time: a warp's way from the barrier to its scores is longer than its sums for one)
         const int sl = it % C::SLOTS;
         if (!wait.warp(slot_full[sl], (it / C::SLOTS) & 1)) return;
         tc_fence_after();
