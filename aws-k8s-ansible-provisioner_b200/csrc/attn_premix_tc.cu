@@ -541,8 +541,8 @@ bool heads_premix_tc_ok(const HeadsGeom& g, int block_size) {
   return (g.heads == 8 || g.heads == 16 || g.heads == 32) && g.kv_heads * 2 == g.heads && g.dim == 128 && g.vdim == 128 && g.window <= 0 && g.rot_dims % 8 == 0 && block_size > 0 && block_size % 16 == 0;
 }
 
-// Room for the units of a whole call, at most 512 MB (4 096 units of 32 heads); 0 where one tile of the longest context would not fit that.  4 x 1024 tokens of 32 heads, 2 304 units: 453 us
-// with room for all, 521 with 192 MB (two launches of each kernel, and their last waves).
+// Room for the units of a whole call, at most 512 MB (4 096 units of 32 heads); 0 where one tile of the longest context would not fit that.  4 x 1024 tokens of 32 heads, 2 304 units: in
+// 192 MB 68 us more than with room for all (two launches of each kernel, and their last waves).
 size_t heads_premix_tc_scratch_floats(const HeadsGeom& g, int max_tokens, int max_context) {
   const int qb = g.heads == 32 ? 8 : 16;
   const size_t unit = (size_t)g.heads * qb * PT_KEYS, blocks = ((size_t)max_context + PT_KEYS - 1) / PT_KEYS + 1;
