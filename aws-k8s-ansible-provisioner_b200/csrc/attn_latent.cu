@@ -63,6 +63,9 @@ __device__ __forceinline__ void pair_cos_sin(int pos, int i, int dims, float bas
   *s = (float)sd;
 }
 
+// A pair turned by its angle, with the products that go unrounded into the sums named: left to the compiler, they differ from kernel to kernel.
+__device__ __forceinline__ float2 turned_pair(float u, float v, float c, float s) { return make_float2(__fmaf_rn(u, c, -__fmul_rn(v, s)), __fmaf_rn(u, s, __fmul_rn(v, c))); }
+
 constexpr int LF_REG = 8;   // numbers of a latent in a thread: kv_rank <= 1024, as everywhere
 template <typename TX, typename TC>
 __global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int ld, LatentGeom g, int has_kv,
@@ -97,8 +100,9 @@ __global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int
     const bool has_v = 2 * p + 1 < g.rot_dim;
     const float u = src[0], v = has_v ? src[1] : 0.f;
     if (p < half && has_v) {
-      dst[0] = u * cs[p] - v * cs[half + p];
-      dst[1] = v * cs[p] + u * cs[half + p];
+      const float2 y = turned_pair(u, v, cs[p], cs[half + p]);
+      dst[0] = y.x;
+      dst[1] = y.y;
     } else {
       dst[0] = u;
       if (has_v) dst[1] = v;
@@ -125,8 +129,9 @@ __global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int
     const float u = kr[2 * p], v = has_v ? kr[2 * p + 1] : 0.f;
     TC* dst = crow + g.kv_rank + 2 * p;
     if (p < half && has_v) {
-      stf(dst, u * cs[p] - v * cs[half + p]);
-      stf(dst + 1, v * cs[p] + u * cs[half + p]);
+      const float2 y = turned_pair(u, v, cs[p], cs[half + p]);
+      stf(dst, y.x);
+      stf(dst + 1, y.y);
     } else {
       stf(dst, u);
       if (has_v) stf(dst + 1, v);
@@ -135,11 +140,12 @@ __global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int
 }
 
 // The same four numbers at a time, a warp a head: head widths, the latent's width and the rows in multiples of four, bases on 16-byte boundaries, a bf16 cache.  Bound by memory; the form
-// above divides to find each number's head and moves four bytes at a time.  24 decode steps of four sequences and their prompts, two layers: 3134 -> 3040 us.
+// above divides to find each number's head and moves four bytes at a time.  24 decode steps of four sequences and their prompts, two layers: 3134 -> 3040 us.  Sums and
+// turns are that form's, in its order: both give the same bits.
 __global__ void __launch_bounds__(256) latent_finish4_kernel(const float* qd, int ld, LatentGeom g, int has_kv, const float* __restrict__ latent_gain, const int32_t* positions,
                                                              const int32_t* slots, bf16* __restrict__ q_nope, float* __restrict__ q_rot, bf16* __restrict__ cache) {
   extern __shared__ __align__(16) float cs[];   // [rot_dims / 2] cos | sin
-  __shared__ float red[8];
+  __shared__ __align__(16) float lat_s[1024];
   pdl_wait();
   pdl_launch_dependents();
   const int t = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -148,25 +154,24 @@ __global__ void __launch_bounds__(256) latent_finish4_kernel(const float* qd, in
   const float4* lat = reinterpret_cast<const float4*>(row + g.heads * hw);
   float4 lv = make_float4(0.f, 0.f, 0.f, 0.f);   // (kv_rank <= 1024)
   if (slot >= 0 && tid < g.kv_rank / 4) lv = lat[tid];
+  reinterpret_cast<float4*>(lat_s)[tid] = lv;
   if (tid < half) pair_cos_sin(pos, tid, g.rot_dims, g.rot_base, &cs[tid], &cs[half + tid]);
   auto packed = [](const float4& y) { return make_uint2(pack_bf16x2(y.x, y.y), pack_bf16x2(y.z, y.w)); };
 #pragma unroll 4
   for (int a = warp; a < g.heads; a += 8)
     for (int c = lane; c < g.dim / 4; c += 32)
       reinterpret_cast<uint2*>(q_nope + ((size_t)t * g.heads + a) * g.dim)[c] = packed(reinterpret_cast<const float4*>(row + a * hw)[c]);
-  const float ss = warp_sum(fmaf(lv.x, lv.x, fmaf(lv.y, lv.y, fmaf(lv.z, lv.z, lv.w * lv.w))));
-  if (lane == 0) red[warp] = ss;
   __syncthreads();
   auto turned = [&](float4 y, int c) {   // pairs 2 c and 2 c + 1 of a rotated piece: those below rot_dims turn, the rest passes
     if (2 * c < half) {
-      const float co = cs[2 * c], si = cs[half + 2 * c], u = y.x;
-      y.x = u * co - y.y * si;
-      y.y = y.y * co + u * si;
+      const float2 z = turned_pair(y.x, y.y, cs[2 * c], cs[half + 2 * c]);
+      y.x = z.x;
+      y.y = z.y;
     }
     if (2 * c + 1 < half) {
-      const float co = cs[2 * c + 1], si = cs[half + 2 * c + 1], u = y.z;
-      y.z = u * co - y.w * si;
-      y.w = y.w * co + u * si;
+      const float2 z = turned_pair(y.z, y.w, cs[2 * c + 1], cs[half + 2 * c + 1]);
+      y.z = z.x;
+      y.w = z.y;
     }
     return y;
   };
@@ -176,8 +181,16 @@ __global__ void __launch_bounds__(256) latent_finish4_kernel(const float* qd, in
     reinterpret_cast<float4*>(q_rot + (size_t)t * g.heads * g.rot_dim)[i] = turned(reinterpret_cast<const float4*>(row + a * hw + g.dim)[c], c);
   }
   if (slot < 0) return;
-  const float sum = ((red[0] + red[1]) + (red[2] + red[3])) + ((red[4] + red[5]) + (red[6] + red[7]));
-  const float r = 1.0f / sqrtf(sum / (float)g.kv_rank + g.eps);
+  float ss[4] = {0.f, 0.f, 0.f, 0.f};   // the form above has 128 threads: what its thread 32 q + lane sums, every warp here for itself (zeros behind the latent)
+  for (int k = 0; 128 * k < g.kv_rank; ++k)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float v = lat_s[128 * k + 32 * q + lane];
+      ss[q] = fmaf(v, v, ss[q]);
+    }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) ss[q] = warp_sum(ss[q]);
+  const float r = 1.0f / sqrtf((ss[0] + ss[1] + ss[2] + ss[3]) / (float)g.kv_rank + g.eps);
   bf16* crow = cache + (size_t)slot * (g.kv_rank + g.rot_dim);
   if (tid < g.kv_rank / 4) {
     const float4 w = reinterpret_cast<const float4*>(latent_gain)[tid];

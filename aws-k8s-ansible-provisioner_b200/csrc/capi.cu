@@ -177,6 +177,14 @@ extern "C" int b2k_heads_premix(const void* q_planes, const void* k_cache, const
                                 (const PrefillTile*)tiles, (const PrefillTile*)tiles_host, ntiles, (bf16*)out, T, scratch, scratch_floats, wait, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_latent_finish(const float* qd, int ld, int heads, int dim, int rot_dim, int kv_rank, int rot_dims, float rot_base, float eps, int has_kv, const float* latent_gain,
+                                 const int32_t* positions, const int32_t* slots, void* q_nope, float* q_rot, void* cache, int T, void* stream) {
+  B2_REQUIRE(qd && positions && q_nope && (q_rot || rot_dim == 0) && (!has_kv || (latent_gain && slots && cache)), "b2k_latent_finish: null pointer");
+  LatentGeom g{};
+  g.heads = heads; g.dim = dim; g.rot_dim = rot_dim; g.kv_rank = kv_rank; g.rot_dims = rot_dims; g.rot_base = rot_base; g.eps = eps;
+  return launch_latent_finish(qd, ld, g, has_kv, latent_gain, positions, slots, q_nope, 0, q_rot, cache, 0, T, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_state_scan(const float* q, int ldq, const float* k, int ldk, const float* v, int ldv, const float* decay, const float* beta, const float* skip,
                               const float* bonus, int heads, int kv_heads, int dim, int vdim, int rule, float qscale, float* state, int portions,
                               const int32_t* last_rows, const int32_t* row_seq, const int32_t* row_first, const int32_t* row_end, const int32_t* positions,

@@ -461,6 +461,11 @@ int b2k_heads_postmix(const float* q, const void* k_cache, const void* v_cache, 
 int b2k_heads_premix(const void* q_planes, const void* k_cache, const void* v_cache, int64_t cache_rows, int heads, float scale, float softcap, const float* talk_host, const float* turn,
                      const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, const int32_t* tiles_host, int ntiles, void* out, int T, float* scratch,
                      size_t scratch_floats, void* stream);
+/* What follows the joint query | latent projection of a bf16 layer (csrc/attn_latent.cu): qd [T][ld] fp32 = per head [dim | rot_dim], then (has_kv) the latent of kv_rank numbers and the
+ * key's rotated piece.  q_nope bf16 [T][heads * dim]; q_rot fp32 [T][heads * rot_dim], the first rot_dims of each turned by the position; with has_kv the token's cache row slots[t]
+ * (bf16 [kv_rank + rot_dim], none for a slot below 0): the latent over its root mean square times its gain, and the turned key piece. */
+int b2k_latent_finish(const float* qd, int ld, int heads, int dim, int rot_dim, int kv_rank, int rot_dims, float rot_base, float eps, int has_kv, const float* latent_gain,
+                      const int32_t* positions, const int32_t* slots, void* q_nope, float* q_rot, void* cache, int T, void* stream);
 /* The recurrence of the matrix-state mixers over `portions` portions (portion i ends at row last_rows[i]; last_rows null: every row is one of one token); rule as
  * StateRule in csrc/kernels.h; all tensors fp32: q / k rows of kv_heads * dim, v rows of heads * vdim, decay [T][heads * dim] or [T][heads] by the rule, beta
  * [T][heads], skip [heads], bonus [heads][dim] (null where the rule has none), state [slots][2][heads][dim][vdim], out [T][heads * vdim]. */

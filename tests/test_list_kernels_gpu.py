@@ -287,6 +287,36 @@ def test_gateup_clamped(lib, T, I, K):
     assert (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -14).all(), err.max()
 
 
+@pytest.mark.parametrize("heads,dim,rot,rank,rot_dims", [(16, 128, 64, 512, 64), (16, 128, 0, 512, 0), (5, 12, 8, 1024, 6), (3, 132, 12, 36, 2), (1, 4, 4, 260, 4), (9, 64, 24, 132, 24)])
+def test_latent_finish_forms_agree(lib, heads, dim, rot, rank, rot_dims):
+    """The form that moves four numbers at a time against the general one (which rows off a 16-byte boundary take), bit for bit, and both against 64 bits."""
+    g = torch.Generator().manual_seed(rank + heads)
+    T, kv0 = 300, heads * (dim + rot)
+    ld = kv0 + rank + rot + 4
+    qd = torch.randn(T, ld, generator=g) * torch.exp(torch.randn(T, 1, generator=g))
+    gain, pos = 1.0 + 0.1 * torch.randn(rank, generator=g), torch.randint(0, 5000, (T,), generator=g, dtype=torch.int32)
+    slots = torch.randperm(T + 9, generator=g)[:T].to(torch.int32)
+    slots[::7] = -1
+    got = []
+    for off in (0, 1):
+        buf = torch.zeros(T * ld + 4, device="cuda")
+        x = buf[off:off + T * ld]
+        x.copy_(qd.view(-1))
+        dg, dp, ds = gain.cuda(), pos.cuda(), slots.cuda()
+        nope, qr = torch.full((T, heads * dim), float("nan"), dtype=torch.bfloat16, device="cuda"), torch.full((T, max(heads * rot, 1)), float("nan"), device="cuda")
+        cache = torch.full((T + 9, rank + rot), 7.0, dtype=torch.bfloat16, device="cuda")
+        chk(lib, lib.b2k_latent_finish(ptr(x), ld, heads, dim, rot, rank, rot_dims, 10000.0, 1e-6, 1, ptr(dg), ptr(dp), ptr(ds), ptr(nope), ptr(qr), ptr(cache), T, cuda_stream_ptr()))
+        torch.cuda.synchronize()
+        got.append((nope.cpu(), qr.cpu()[:, :heads * rot], cache.cpu()))
+    for a, b in zip(*got):
+        assert torch.equal(a, b), (a.float() - b.float()).abs().max()
+    lat = qd[:, kv0:kv0 + rank].double()
+    ref = lat / torch.sqrt((lat * lat).mean(1, keepdim=True) + 1e-6) * gain.double()
+    seen = slots >= 0
+    rows = got[0][2][slots[seen].long(), :rank].double()
+    assert ((rows - ref[seen]).abs() <= 2.0 ** -8 * ref[seen].abs() + 1e-6).all()
+
+
 @pytest.mark.parametrize("heads,softcap,turned,bs,pieces", [(32, 20.0, True, 16, False), (32, 0.0, False, 64, True), (16, 50.0, True, 32, True), (8, 3.0, False, 16, False)])
 def test_heads_premix(lib, heads, softcap, turned, bs, pieces):
     """Portions around the tiles of 64, the units of 8 or 16 tokens and the blocks of 128 keys, some behind earlier tokens; `pieces`: a scratch that holds two tiles' units at most.
