@@ -2712,8 +2712,7 @@ int launch_heads_finish_table(const float* proj, int ld, const HeadsGeom& g, con
 
 int launch_rot_table(const double* freqs, int half, double mul, float* table, int npos, cudaStream_t s) {
   if (half <= 0 || npos <= 0) return 0;
-  rot_table_kernel<<<npos, 128, 0, s>>>(freqs, half, mul, table);
-  B2_CUDA_OK(cudaGetLastError());
+  B2_CUDA_OK(b2_launch_plain(rot_table_kernel, dim3(npos), dim3(128), 0, s, freqs, half, mul, table));
   return 0;
 }
 

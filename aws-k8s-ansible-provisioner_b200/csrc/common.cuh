@@ -163,6 +163,17 @@ inline void b2_prefer_max_smem(void (*kernel)(KArgs...), B2PerDeviceOnce& once) 
       cudaGetLastError();  // a preference only
   }
 }
+// An ordinary launch.  Its own result is what says whether it went out: cudaGetLastError() would hand over what an earlier call of this thread left behind, an allocation that failed and
+// was done without, say.
+template <typename... KArgs, typename... Args>
+inline cudaError_t b2_launch_plain(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
 template <typename... KArgs, typename... Args>
 inline cudaError_t b2_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

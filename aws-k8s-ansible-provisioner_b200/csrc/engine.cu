@@ -2593,8 +2593,7 @@ int launch_uploads(const Uploads& l, cudaStream_t s, bool then_kernels) {
   int most = 0;
   for (int k = 0; k < l.n; ++k) most = std::max(most, l.u[k].ints);
   if (most == 0) return 0;
-  upload_kernel<<<dim3(std::min(32, (most + 255) / 256), l.n), 256, 0, s>>>(l);
-  B2_CUDA_OK(cudaGetLastError());
+  B2_CUDA_OK(b2_launch_plain(upload_kernel, dim3(std::min(32, (most + 255) / 256), l.n), dim3(256), 0, s, l));
   if (then_kernels) b2_pdl_skip_next();   // the step's kernels read these lists in front of their dependency wait: the first of them starts when all of this is done
   return 0;
 }

@@ -159,8 +159,7 @@ int launch_sample_rows(const bf16* logits, const SampleRow* rows_host, SampleRow
   static_assert(sizeof(SampleRow) == sizeof(SampleRowDev), "host and device row records must match");
   B2_REQUIRE(V % 8 == 0, "sampling: vocabulary %d must be a multiple of 8", V);
   B2_CUDA_OK(cudaMemcpyAsync(stage_dev, rows_host, sizeof(SampleRow) * (size_t)nrows, cudaMemcpyHostToDevice, s));
-  sample_rows_kernel<<<nrows, 1024, 0, s>>>(logits, reinterpret_cast<const SampleRowDev*>(stage_dev), out, V, step);
-  B2_CUDA_OK(cudaGetLastError());
+  B2_CUDA_OK(b2_launch_plain(sample_rows_kernel, dim3(nrows), dim3(1024), 0, s, logits, reinterpret_cast<const SampleRowDev*>(stage_dev), out, V, step));
   return 0;
 }
 

@@ -234,6 +234,37 @@ def test_errors_are_reported(P, tiny):
     e.close()
 
 
+def test_a_refused_engine_leaves_the_others_alone(P, tiny):
+    """An engine that does not fit into memory is an error of its own call: prompts, sampling, new decode batches and new engines behind it work as before."""
+    _, sd = tiny
+    sizes = dict(max_model_len=64, num_blocks=16, max_seqs=2, max_batch_tokens=64)
+    e = make_engine(P, QWEN3_TINY, sd, **sizes)
+    e.set_debug(logits=True)
+    prompt = [[3 + i for i in range(20)]]
+
+    def refuse():
+        with pytest.raises(P.B2Error, match="cudaMalloc"):
+            make_engine(P, QWEN3_TINY, sd, **dict(sizes, num_blocks=1 << 28))   # terabytes
+
+    a = e.seq_create(40)
+    want = [e.prefill([a], prompt), e.decode_step([a]), e.sample(1, temperature=1.0, top_p=0.5, seed=7)]
+    e.seq_free(a)
+    refuse()
+    b = e.seq_create(40)
+    got = [e.prefill([b], prompt)]
+    refuse()
+    got.append(e.decode_step([b]))
+    refuse()
+    got.append(e.sample(1, temperature=1.0, top_p=0.5, seed=7))
+    for x, y in zip(got, want):
+        assert (x == y).all()
+    refuse()
+    other = make_engine(P, QWEN3_TINY, sd, **sizes)
+    assert (other.prefill([other.seq_create(40)], prompt) == want[0]).all()
+    other.close()
+    e.close()
+
+
 # ---------------------------------------------------------------------------------------------
 # Full-size architecture: batch 1, 128-token prompt -> 128 tokens
 # ---------------------------------------------------------------------------------------------
