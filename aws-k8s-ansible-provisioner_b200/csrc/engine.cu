@@ -1328,6 +1328,35 @@ int latent_rebuild_setup(b2_engine* e) {
   return 0;
 }
 
+// What attn_premix_tc.cu's form of the mixed scores needs (up to 512 MB of scratch, the cosines and sines of a step's tokens), taken in the same way: behind the cache, where it leaves
+// 512 MB free.  Without it the prompts of such layers take the kernels of attn_heads.cu.
+int mixed_scores_setup(b2_engine* e) {
+  const b2_config& c = e->cfg;
+  size_t floats = 0;
+  for (const ListLayer& L : e->ll) {
+    if (L.sp.mixer != B2_MIXER_MIXED_SCORE_ATTENTION || !L.sp.score_mix || e->f32) continue;
+    HeadsGeom g{L.sp.heads, L.sp.kv_heads, L.sp.dim, L.sp.vdim};
+    g.rot_dims = L.sp.rot_dims;
+    g.window = L.sp.window;
+    if (heads_premix_tc_ok(g, c.block_size)) floats = std::max(floats, heads_premix_tc_scratch_floats(g, e->cap_tokens, c.max_model_len));
+  }
+  if (floats == 0) return 0;
+  const size_t turns = (size_t)e->cap_tokens * 128;
+  size_t free_b = 0, total_b = 0;
+  B2_CUDA_OK(cudaMemGetInfo(&free_b, &total_b));
+  if ((floats + turns) * sizeof(float) + ((size_t)512 << 20) > free_b) return 0;
+  float *scores = nullptr, *turn = nullptr;
+  if (dalloc(&scores, floats) != 0 || dalloc(&turn, turns) != 0) {   // (another process was quicker)
+    cudaGetLastError();
+    if (scores) cudaFree(scores);
+    return 0;
+  }
+  e->l_premix = scores;
+  e->l_premix_floats = floats;
+  e->l_turn = turn;
+  return 0;
+}
+
 int forward_list(b2_engine* e, int T, int ntiles, int nlast) {
   const b2_config& c = e->cfg;
   const int W = c.hidden, f = e->f32 ? 1 : 0;
@@ -3965,17 +3994,7 @@ int mixed_engine_alloc(b2_engine* e) {
   B2_TRY(aalloc(&e->l_xl, (size_t)e->l_rows_cap * W));
   size_t scratch = 0;   // the key splits of a decode step's attention (one buffer: the layers run one after the other)
   for (const ListLayer& L : e->ll)
-    if (L.sp.mixer == B2_MIXER_MIXED_SCORE_ATTENTION) {
-      scratch = std::max(scratch, heads_attention_premix_scratch_floats(bucket_batch(c.max_seqs), L.sp.heads, L.sp.vdim));
-      HeadsGeom g{L.sp.heads, L.sp.kv_heads, L.sp.dim, L.sp.vdim};
-      g.rot_dims = L.sp.rot_dims;
-      g.window = L.sp.window;
-      if (!e->f32 && L.sp.score_mix && heads_premix_tc_ok(g, c.block_size)) e->l_premix_floats = std::max(e->l_premix_floats, heads_premix_tc_scratch_floats(g, (int)Tc, c.max_model_len));
-    }
-  if (e->l_premix_floats > 0) {
-    B2_TRY(dalloc(&e->l_premix, e->l_premix_floats));
-    B2_TRY(dalloc(&e->l_turn, Tc * 128));
-  }
+    if (L.sp.mixer == B2_MIXER_MIXED_SCORE_ATTENTION) scratch = std::max(scratch, heads_attention_premix_scratch_floats(bucket_batch(c.max_seqs), L.sp.heads, L.sp.vdim));
   if (any_latent) {
     B2_TRY(aalloc(&e->l_x2, Tc * max_qr));
     B2_TRY(aalloc(&e->l_qnope, Tc * max_hd));
@@ -5388,6 +5407,7 @@ extern "C" int b2_engine_create(const b2_config* cfg, const char* safetensors_pa
           e->regions.push_back({reinterpret_cast<char*>(e->kv_pool + (size_t)r * e->layer_kv_elems), blk_elems * 2});
       }
       if (c.arch == B2_ARCH_LERASUN) E_TRY(latent_rebuild_setup(e));
+      if (mixed_arch) E_TRY(mixed_scores_setup(e));
       if (ls && e->f32) list_f32_scratch(e);
       e->free_blocks.reserve(nb);
       for (int64_t b = nb - 1; b >= 1; --b) e->free_blocks.push_back((int32_t)b);  // page 0 = null page

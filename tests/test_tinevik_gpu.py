@@ -256,6 +256,33 @@ def test_bf16_head_mixed_attention_on_clusters(heads, kv, dim, vdim, T):
         run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), BF16_BAR, [T - 21, 18], T - 3)
 
 
+def test_too_little_memory_for_the_mixed_scores():
+    """An engine that fits without the mixed scores' scratch (514 MB here) is not refused: its prompts take the clusters' kernel."""
+    cfg = model([(att(32, 16, 128, 128, 128 ** -0.5, rot=(3000.0, 64, 2.0), cap=25.0), None)], vocab=211, width=96)
+    w = random_weights(cfg, seed=61)
+    toks = tokens(cfg, 95, 62)
+    ref = ref_logits(cfg, w, toks)
+    sizes = {"max_model_len": 4096, "num_blocks": 40, "max_batch_tokens": 4096}
+
+    def free():
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    with engine(cfg, w, f32=False, **sizes) as e:   # (what a process loads once is loaded here)
+        run_schedule(e, cfg, toks, ref, BF16_BAR, [60, 30], 90)
+    before = free()
+    with engine(cfg, w, f32=False, **sizes) as e:
+        takes = before - free()
+        run_schedule(e, cfg, toks, ref, BF16_BAR, [60, 30], 90)
+    held = torch.empty(free() - (takes - (256 << 20)), dtype=torch.uint8, device="cuda")
+    try:
+        with engine(cfg, w, f32=False, **sizes) as e:
+            run_schedule(e, cfg, toks, ref, BF16_BAR, [60, 30], 90)
+    finally:
+        del held
+        torch.cuda.empty_cache()
+
+
 def test_bf16_wide_up_projection_of_few_rows():
     """bf16: an up-projection of 16384 rows takes the heads' kernel in short portions and decode steps, and the tcgen05 product in longer ones."""
     cfg = model([(gla(2, 32, 64, 16.0, rank=16), dense(16384))], vocab=300, width=128)
