@@ -16,6 +16,7 @@
 #include "kernels.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace b2 {
 
@@ -354,7 +355,8 @@ __global__ void __launch_bounds__(256, 2) premix_values_kernel(const PtArgs a, c
   const int hd = warp >> 2, row0 = (warp & 3) * 16;   // this warp's head of the two, its first token of the tile
   const uint32_t vs = smem_u32(smem_raw), ss = vs + 2 * PV_V_BYTES + warp * (2 * PV_S_BYTES);
   const int32_t* bt = a.block_table + (size_t)tl.bt_row * a.bt_stride;
-  const int steps = pos_hi / PV_KEYS + 1, mine = row0 < tl.nrows ? (tl.q_pos0 + min(row0 + 15, tl.nrows - 1)) / PV_KEYS + 1 : 0;   // steps with keys that this warp sees
+  const int last_key = tl.q_pos0 + min(row0 + 15, tl.nrows - 1);   // of this warp's queries
+  const int steps = pos_hi / PV_KEYS + 1, mine = row0 < tl.nrows ? last_key / PV_KEYS + 1 : 0;   // steps with keys that this warp sees
 
   // scratch rows of this lane: 2 i + (lane >> 4) of the warp's sixteen; eight (QB 8) or all of them lie in one unit, the others nkb units on
   const int r1 = lane >> 4, c16 = lane & 15;
@@ -442,8 +444,9 @@ __global__ void __launch_bounds__(256, 2) premix_values_kernel(const PtArgs a, c
         }
       }
       const int k = lane & 15, key = k < 8 ? 4 * (k >> 1) + (k & 1) : 4 * ((k - 8) >> 1) + 2 + (k & 1);
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
+      // A weight of 0 times an infinity is a NaN: what lies behind the last key that the warp's sixteen queries see stays out of their products.
+      const int last_seen = last_key - k0;   // (>= 0)
+      auto product = [&](int kk, auto at_end) {   // keys 16 kk .. of the step; at_end: those behind `last_seen` count as zeros
         uint32_t hi[4], lo[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {   // rows fg, fg + 8 of keys 4 ft, 4 ft + 1, then of 4 ft + 2, 4 ft + 3
@@ -451,17 +454,34 @@ __global__ void __launch_bounds__(256, 2) premix_values_kernel(const PtArgs a, c
           hi[i] = pack_bf16x2(x, y);
           lo[i] = pack_bf16x2(x - bf16lo(hi[i]), y - bf16hi(hi[i]));
         }
+        uint32_t keep[2];   // of the pairs of keys 4 ft, 4 ft + 1 and 4 ft + 2, 4 ft + 3
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int left = last_seen - (16 * kk + 4 * ft + 2 * i);
+          keep[i] = left >= 1 ? 0xffffffffu : left == 0 ? 0xffffu : 0u;
+        }
         const uint32_t vrow = vd + (16 * kk + key) * 256, sw = pv_swizzle(key);   // (16 kk does not move the swizzle)
 #pragma unroll
         for (int nb = 0; nb < 8; nb += 2) {   // (four sums at a time: a product waits for the one before it on the same sum)
           uint32_t vb[2][4];
 #pragma unroll
-          for (int i = 0; i < 2; ++i) pv_ldmatrix_trans(vb[i], vrow + (((uint32_t)(2 * (nb + i) + (lane >> 4)) ^ sw) << 4));
+          for (int i = 0; i < 2; ++i) {
+            pv_ldmatrix_trans(vb[i], vrow + (((uint32_t)(2 * (nb + i) + (lane >> 4)) ^ sw) << 4));
+            if constexpr (decltype(at_end)::value) {
+#pragma unroll
+              for (int r = 0; r < 4; ++r) vb[i][r] &= keep[r & 1];
+            }
+          }
 #pragma unroll
           for (int i = 0; i < 4; ++i) pv_mma(o[2 * nb + i], lo, vb[i >> 1][2 * (i & 1)], vb[i >> 1][2 * (i & 1) + 1]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) pv_mma(o[2 * nb + i], hi, vb[i >> 1][2 * (i & 1)], vb[i >> 1][2 * (i & 1) + 1]);
         }
+      };
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk) {
+        if (16 * kk + 15 <= last_seen) product(kk, std::false_type{});
+        else if (16 * kk <= last_seen) product(kk, std::true_type{});
       }
     }
     __syncthreads();   // this step's buffers are read: the load of the step after the next may write them

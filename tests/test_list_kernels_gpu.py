@@ -371,6 +371,46 @@ def test_heads_premix(lib, heads, softcap, turned, bs, pieces):
         at += n
 
 
+@pytest.mark.parametrize("heads", [32, 16, 8])
+@pytest.mark.parametrize("before,n", [(0, 64), (0, 130), (37, 64), (101, 50), (64, 16)])
+def test_heads_premix_reach_of_a_value(lib, heads, before, n):
+    """A value that is not finite reaches the rows that see it and, of those that do not, only the ones in front of it among the same sixteen queries of a tile (0 times it is a NaN):
+    the other rows have the bits that they have without it."""
+    g = torch.Generator().manual_seed(heads + n)
+    kv, S, bs = heads // 2, before + n, 16
+    width = (S + bs - 1) // bs
+    bt = torch.randperm(width + 1, generator=g)[:width].view(1, -1).to(torch.int32).cuda()
+    planes = torch.randn(kv, n, 2, 2, 128, generator=g).to(torch.bfloat16)
+    planes[:, :, :, 1] *= 2.0 ** -9
+    planes = planes.cuda()
+    kc, vc = (torch.randn((width + 1) * bs, kv, 128, generator=g).to(torch.bfloat16).cuda() for _ in range(2))
+    talk = torch.eye(heads) + 0.2 * torch.randn(heads, heads, generator=g)
+    host = torch.tensor([(i, before + i, min(64, n - i), 0) for i in range(0, n, 64)], dtype=torch.int32)
+    tiles = host.cuda()
+    room = len(host) * 64 * heads * 128 * ((S - 1) // 128 + 1)
+    scratch = torch.empty(room, device="cuda")
+
+    def call():
+        out = torch.zeros(n, heads * 128, dtype=torch.bfloat16, device="cuda")
+        chk(lib, lib.b2k_heads_premix(ptr(planes), ptr(kc), ptr(vc), (width + 1) * bs, heads, 128 ** -0.5, 0.0, ptr(talk), None, ptr(bt), width, bs, ptr(tiles), ptr(host), len(host), ptr(out),
+                                      n, ptr(scratch), room, cuda_stream_ptr()))
+        torch.cuda.synchronize()
+        return out.cpu()
+
+    clean = call()
+    assert torch.isfinite(clean.float()).all()
+    for i in sorted({0, 1, 15, 16, 33, n // 2, n - 2, n - 1} & set(range(n))):   # the token that is not finite
+        p = before + i
+        row = int(bt[0, p // bs]) * bs + p % bs
+        kept = vc[row].clone()
+        vc[row] = float("inf") if i % 2 else float("nan")
+        got = call()
+        vc[row] = kept
+        free = i // 64 * 64 + i % 64 // 16 * 16   # rows in front of the sixteen that hold it
+        assert torch.equal(got[:free], clean[:free]), (i, free)
+        assert not torch.isfinite(got[i:].float()).any()
+
+
 @pytest.mark.parametrize("heads,kv,dim,vdim,window,keep,bs", [(16, 8, 128, 128, 70, 9, 16), (16, 16, 64, 64, 0, 0, 32), (5, 1, 128, 64, 33, 0, 48), (8, 4, 64, 128, 16, 40, 16),
                                                               (1, 1, 128, 128, 1, 5, 16), (12, 4, 128, 128, 100, 16, 64)])
 def test_heads_postmix(lib, heads, kv, dim, vdim, window, keep, bs):
