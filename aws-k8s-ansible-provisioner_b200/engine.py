@@ -132,53 +132,20 @@ def _p32(a: np.ndarray):
     return a.ctypes.data_as(C.POINTER(C.c_int32))
 
 
-class _PageLocked:
-    """Page-locked blocks that no engine uses, for the next one: at most `LIMIT` bytes once `trim` has run, which making and closing an engine do.  (Never freed where an
-    array goes: that would make the driver wait inside somebody's call.)"""
-
-    LIMIT = 64 << 20
-
-    def __init__(self):
-        self.lock, self.idle = threading.Lock(), collections.deque()   # (bytes, address, library); threads and finalizers append
-
-    def take(self, lib, size: int):
-        with self.lock:
-            for b in list(self.idle):
-                if size <= b[0] <= 2 * size and b[2] is lib:
-                    self.idle.remove(b)
-                    return b
-        p = C.c_void_p()
-        return (size, p.value, lib) if lib.b2_host_alloc(size, C.byref(p)) == 0 else None
-
-    def trim(self, limit: int | None = None) -> None:
-        with self.lock:
-            while sum(b[0] for b in list(self.idle)) > (self.LIMIT if limit is None else limit):
-                size, p, lib = self.idle.popleft()
-                lib.b2_host_free(p)
-
-
-_page_locked = _PageLocked()
-
-
 class _Results:
     """fp32 result arrays in memory that is used again once nobody holds the array that lay in it, nor a view of that: fresh pages cost more than the copy.
 
-    Two page-locked blocks of `first` bytes, where that is little (2 - 3 ms each when new, 20 - 50 for 39 MB), take the copy directly: a call that returned 2 MB of logits 1189 -> 909 us.
-    Results that do not fit them lie in ordinary memory (39 MB of bf16 rows widened on the host: 3.1 -> 1.8 ms), of which at most `LIMIT` bytes in `BLOCKS` blocks are kept;
-    a caller that holds more results than that gets new arrays."""
+    At most `BLOCKS` blocks of `LIMIT` bytes in all are kept; a caller that holds more results than that gets new arrays.  The memory is ordinary: a copy to a device that a caller starts
+    from a result without waiting for it has left the array when the call returns, which one from page-locked memory would not have.  us a call, fresh / kept / page-locked: 2 MB of logits
+    1191 / 1003 / 898, 0.8 MB 992 / 883 / 843; 39 MB of bf16 rows widened on the host 3.1 / 1.8 ms.  Arrays go wherever the collector runs, inside this class too: what they leave behind
+    is put down without a lock."""
 
-    PINNED, BLOCKS, LIMIT = 8 << 20, 2, 128 << 20
+    BLOCKS, LIMIT = 4, 128 << 20
 
-    def __init__(self, lib, first: int):
-        self.lib, self.lock = lib, threading.Lock()
-        self.free, self.back = [], collections.deque()   # (bytes, address, its owner: an array, or the library that made it page-locked); `back`: what arrays left behind
-        self.blocks = self.bytes = 0
-        self.open = True
-        for _ in range(2):
-            block = _page_locked.take(lib, first) if 0 < first <= self.PINNED else None
-            if block is not None:
-                self.free.append(block)
-        _page_locked.trim()
+    def __init__(self):
+        self.lock, self.open = threading.Lock(), True
+        self.free, self.back = [], collections.deque()   # byte arrays; `back`: what arrays left behind
+        self.blocks = self.bytes = 0                     # kept, lent ones among them
 
     def array(self, rows: int, cols: int) -> np.ndarray:
         need, got = rows * cols * 4, None
@@ -186,40 +153,27 @@ class _Results:
             while self.back:
                 self.free.append(self.back.popleft())
             if self.open and need > 0:
-                got = min((b for b in self.free if b[0] >= need), key=lambda b: b[0], default=None)
+                got = min((b for b in self.free if b.nbytes >= need), key=lambda b: b.nbytes, default=None)
                 if got is not None:
                     self.free = [b for b in self.free if b is not got]
                 elif self.blocks < self.BLOCKS and self.bytes + need <= self.LIMIT:
-                    own = np.empty(need, dtype=np.uint8)
-                    got = (need, own.ctypes.data, own)
+                    got = np.empty(need, dtype=np.uint8)
                     self.blocks, self.bytes = self.blocks + 1, self.bytes + need
         if got is None:
             return np.zeros((rows, cols), dtype=np.float32)
-        owner = (C.c_char * got[0]).from_address(got[1])   # (every view of the array keeps it alive)
+        owner = (C.c_char * got.nbytes).from_address(got.ctypes.data)   # (every view of the array keeps it alive)
         weakref.finalize(owner, _Results._give_back, self, got).atexit = False
         return np.frombuffer(owner, dtype=np.float32, count=rows * cols).reshape(rows, cols)
 
     def _give_back(self, block) -> None:
-        self.back.append(block)
-        if not self.open:
-            self._drop()
-
-    def _drop(self) -> None:
-        for blocks in (self.back, self.free):
-            while blocks:
-                try:
-                    block = blocks.pop()
-                except IndexError:   # (another thread took the last one)
-                    break
-                if not isinstance(block[2], np.ndarray):
-                    _page_locked.idle.append(block)
+        if self.open:
+            self.back.append(block)
 
     def close(self) -> None:
-        """What is held now is given back when its last array goes."""
-        with self.lock:
-            self.open = False
-            self._drop()
-        _page_locked.trim()
+        """What is lent now is freed when its last array goes."""
+        self.open = False
+        self.back.clear()
+        self.free = []
 
 
 class Engine:
@@ -270,7 +224,7 @@ class Engine:
         check(self.lib.b2_engine_create(C.byref(c), path, device, C.byref(h)), self.lib)
         self.h = h
         self.device = device
-        self._results = _Results(self.lib, 2 * int(cfg.max_seqs) * int(cfg.vocab) * 4)   # (two rows of logits a sequence)
+        self._results = _Results()
 
     @classmethod
     def from_model_dir(cls, model_dir: str, device: int = 0, dtype: str = "bfloat16", **runtime) -> "Engine":

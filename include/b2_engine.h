@@ -308,7 +308,8 @@ int  b2_prefill_logits(b2_engine* e, const int32_t* ids, const int32_t* seq_offs
 
 /* Logits of the last forward's last positions, [nseq][vocab] fp32 on the host. */
 int  b2_get_logits(b2_engine* e, int32_t nseq, float* out_logits);
-/* Page-locked host memory (usable with every device): results that are read back land in it by one copy, without fresh pages to fill. */
+/* Page-locked host memory (usable with every device): a call's results land in it by one copy (2 MB of logits: 105 us less a call than in ordinary memory that is used again).  Copies
+ * that the caller starts from it run on when the starting call has returned: it may be given to a call of this library again when they are done. */
 int  b2_host_alloc(size_t bytes, void** out);
 void b2_host_free(void* p);
 /* Residual stream after layer `layer` (0-based; -1 = embeddings, num_layers = final norm

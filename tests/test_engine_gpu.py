@@ -597,6 +597,36 @@ def test_logits_of_few_and_many_rows(P, nseq):
     eng.close()
 
 
+def test_a_copy_that_was_started_from_a_result_is_not_overtaken(P):
+    """Logits on their way to a device while the array is dropped and the next ones are read: the copy has the values that it was started with."""
+    cfg = P.EngineConfig(num_layers=1, hidden=256, num_q_heads=2, num_kv_heads=1, head_dim=128, intermediate=256, vocab=131 * 1001, max_model_len=32, num_blocks=16, max_seqs=2,
+                         max_batch_tokens=64)
+    eng = P.Engine(cfg)
+    g = torch.Generator().manual_seed(3)
+    eng.load_state_dict({k: (torch.randn(s, generator=g) * 0.05).to(torch.bfloat16) for k, s in importlib.import_module(P.__name__ + ".weights").tensor_shapes(cfg).items()})
+    eng.set_debug(logits=True)
+    sid = eng.seq_create(16)
+    eng.prefill([sid], [[7, 9, 11]])
+    side = torch.cuda.Stream()
+    on_device = [torch.empty(1, cfg.vocab, device="cuda") for _ in range(5)]
+    for cycles in (0, 400_000_000):   # (the first pass loads and captures what the second would wait for)
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(cycles)   # what the copies wait behind
+        want = []
+        for d in on_device:
+            logits = eng.get_logits(1)
+            want.append(logits.copy())
+            with torch.cuda.stream(side):
+                d.copy_(torch.from_numpy(logits), non_blocking=True)
+            del logits
+            eng.decode_step([sid])
+        torch.cuda.synchronize()
+        for i, (d, w) in enumerate(zip(on_device, want)):
+            assert (d.cpu().numpy() == w).all() and not (w == want[i - 1]).all(), i
+    eng.close()
+
+
 @pytest.mark.parametrize("n", [199, 700])
 def test_prefill_reports_a_wait_that_ran_out(P, tiny, monkeypatch, n):
     """A prompt kernel whose waits run out (here: are given no time) makes the call an error; the caller's other engines are not touched by it.  Long prompts have their
