@@ -51,6 +51,33 @@ def test_blocks_are_bounded_and_given_back(rows):
     assert not r.free and not r.back and r.array(1, 1).shape == (1, 1)
 
 
+def test_later_sizes_take_the_place_of_idle_ones():
+    r = engine._Results()
+    large = r.BLOCKS * 1000
+    held = [r.array(1, 500) for _ in range(r.BLOCKS)]
+    addrs = {addr(a) for a in held}
+    fresh = r.array(1, large)   # (every block is lent)
+    assert r.blocks == r.BLOCKS and r.bytes == r.BLOCKS * 2000
+    del held
+    gc.collect()
+    a = r.array(1, large)
+    at = addr(a)
+    assert r.blocks == r.BLOCKS and r.bytes == (r.BLOCKS - 1) * 2000 + large * 4 and len(r.free) == r.BLOCKS - 1
+    del a
+    gc.collect()
+    few = r.array(1, 500)   # a small result does not take the large block
+    assert addr(few) in addrs
+    b = r.array(1, large)
+    assert addr(b) == at
+    del b
+    gc.collect()
+    most = r.array(1, (r.LIMIT - 2000) // 4)   # makes room for itself as far as idle blocks go
+    assert r.bytes == r.LIMIT and r.blocks == 2 and not r.free
+    beyond = r.array(1, r.LIMIT // 4 + 1)
+    assert beyond.shape == (1, r.LIMIT // 4 + 1) and r.bytes == r.LIMIT
+    del fresh, few, most
+
+
 def test_threads():
     r = engine._Results()
 
