@@ -1,4 +1,5 @@
 """The engine's result arrays: memory is used again only when neither an array nor a view of it is left, is bounded, is ordinary memory, and is given back."""
+import concurrent.futures
 import gc
 import importlib
 import threading
@@ -78,19 +79,47 @@ def test_later_sizes_take_the_place_of_idle_ones():
     del fresh, few, most
 
 
-def test_threads():
-    r = engine._Results()
+def hold_and_compare(r, threads=6, turns=200):
+    """Every thread makes a result, fills it and holds it until all of them have one: the addresses of those that are held together, turn by turn; raises what a thread raises."""
+    meet, held = threading.Barrier(threads, timeout=60), [[None] * threads for _ in range(turns)]
 
     def work(k):
-        for i in range(200):
-            a = r.array(1, 64)
-            a[:] = k * 1000 + i
-            assert (a == k * 1000 + i).all()
+        try:
+            for i in range(turns):
+                a = r.array(1, 64)
+                a[:] = k * 1000 + i
+                held[i][k] = addr(a)
+                meet.wait()
+                assert (a == k * 1000 + i).all()
+                meet.wait()   # (nobody makes the next one before all have looked)
+                del a
+        except BaseException:
+            meet.abort()
+            raise
 
-    ts = [threading.Thread(target=work, args=(k,)) for k in range(6)]
-    [t.start() for t in ts]
-    [t.join() for t in ts]
-    assert r.blocks <= r.BLOCKS
+    with concurrent.futures.ThreadPoolExecutor(threads) as pool:
+        for done in [pool.submit(work, k) for k in range(threads)]:
+            done.result()
+    return held
+
+
+def test_threads():
+    r = engine._Results()
+    assert all(len(set(addrs)) == len(addrs) for addrs in hold_and_compare(r))
+    assert r.blocks <= r.BLOCKS and len(r.free) + len(r.back) == r.blocks
+
+
+def test_threads_see_memory_that_is_lent_twice():
+    """The check above on a pool that gives everybody the same memory."""
+
+    class Wrong(engine._Results):
+        one = np.zeros((1, 64), dtype=np.float32)
+
+        def array(self, rows, cols):
+            return self.one
+
+    with pytest.raises((AssertionError, threading.BrokenBarrierError)):
+        hold_and_compare(Wrong())
 
 
 class Lib:
