@@ -230,7 +230,6 @@ premix_scores_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_co
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
             if constexpr (CT == 8) pt_tmem_ld8(from + (uint32_t)(sl * 2 * C::NCOL + i * C::NCOL), r[i]);
-            else if constexpr (CT == 32) tmem_ld32(from + (uint32_t)(sl * 2 * C::NCOL + i * C::NCOL), r[i]);
             else tmem_ld16(from + (uint32_t)(sl * 2 * C::NCOL + i * C::NCOL), r[i]);
           }
           tmem_ld_wait();

@@ -177,6 +177,14 @@ extern "C" int b2k_heads_premix(const void* q_planes, const void* k_cache, const
                                 (const PrefillTile*)tiles, (const PrefillTile*)tiles_host, ntiles, (bf16*)out, T, scratch, scratch_floats, wait, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_heads_finish_planes(const float* proj, int ld, int heads, int rot_dims, float rot_base, float rot_factor, int rot_values, float eps, const float* q_gain,
+                                       const float* k_gain, const int32_t* positions, const int32_t* slots, void* q_planes, float* turn, void* k_cache, void* v_cache, int T, void* stream) {
+  B2_REQUIRE(proj && positions && slots && q_planes && k_cache && v_cache, "b2k_heads_finish_planes: null pointer");
+  HeadsGeom g{};
+  g.heads = heads; g.kv_heads = heads / 2; g.dim = g.vdim = 128; g.rot_dims = rot_dims; g.rot_base = rot_base; g.rot_factor = rot_factor; g.rot_values = rot_values; g.eps = eps;
+  return launch_heads_finish_planes(proj, ld, g, q_gain, k_gain, positions, slots, (bf16*)q_planes, turn, (bf16*)k_cache, (bf16*)v_cache, T, (cudaStream_t)stream);
+}
+
 extern "C" int b2k_latent_finish(const float* qd, int ld, int heads, int dim, int rot_dim, int kv_rank, int rot_dims, float rot_base, float eps, int has_kv, const float* latent_gain,
                                  const int32_t* positions, const int32_t* slots, void* q_nope, float* q_rot, void* cache, int T, void* stream) {
   B2_REQUIRE(qd && positions && q_nope && (q_rot || rot_dim == 0) && (!has_kv || (latent_gain && slots && cache)), "b2k_latent_finish: null pointer");

@@ -462,6 +462,11 @@ int b2k_heads_postmix(const float* q, const void* k_cache, const void* v_cache, 
 int b2k_heads_premix(const void* q_planes, const void* k_cache, const void* v_cache, int64_t cache_rows, int heads, float scale, float softcap, const float* talk_host, const float* turn,
                      const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, const int32_t* tiles_host, int ntiles, void* out, int T, float* scratch,
                      size_t scratch_floats, void* stream);
+/* What stands in front of it: proj [T][ld] fp32 = queries | keys | values, heads of 128, two query heads per key/value head.  Queries and keys over their root mean square times the gain
+ * (null: as they are), pairs (m, m + rot_dims / 2) of the first rot_dims turned by position * rot_base^(-2 m / rot_dims) / rot_factor; with rot_values the values' pairs (m, m + 64) by
+ * position * rot_base^(-2 m / 128), cosines and sines in turn.  Keys and values go to the cache rows slots[t] (none below 0). */
+int b2k_heads_finish_planes(const float* proj, int ld, int heads, int rot_dims, float rot_base, float rot_factor, int rot_values, float eps, const float* q_gain, const float* k_gain,
+                            const int32_t* positions, const int32_t* slots, void* q_planes, float* turn, void* k_cache, void* v_cache, int T, void* stream);
 /* What follows the joint query | latent projection of a bf16 layer (csrc/attn_latent.cu): qd [T][ld] fp32 = per head [dim | rot_dim], then (has_kv) the latent of kv_rank numbers and the
  * key's rotated piece.  q_nope bf16 [T][heads * dim]; q_rot fp32 [T][heads * rot_dim], the first rot_dims of each turned by the position; with has_kv the token's cache row slots[t]
  * (bf16 [kv_rank + rot_dim], none for a slot below 0): the latent over its root mean square times its gain, and the turned key piece. */

@@ -371,6 +371,60 @@ def test_heads_premix(lib, heads, softcap, turned, bs, pieces):
         at += n
 
 
+@pytest.mark.parametrize("heads,rot,factor,values,gains", [(32, 64, 4.0, True, True), (32, 0, 1.0, False, True), (16, 128, 1.0, True, True), (8, 128, 2.0, False, False), (8, 8, 0.0, True, True),
+                                                           (16, 72, 3.0, False, True), (2, 64, 1.0, True, False)])
+def test_heads_finish_planes(lib, heads, rot, factor, values, gains):
+    """Against 64 bits: cosines and sines are rounded once (2^-24 of 1), a query is fp32 sums of a few roundings held in sixteen bits (value + remainder, 2^-17), keys and values are one
+    rounding to bf16."""
+    g = torch.Generator().manual_seed(heads + rot)
+    T, kv = 131, heads // 2
+    width = (heads + 2 * kv) * 128
+    proj = torch.randn(T, width + 8, generator=g) * torch.exp(torch.randn(T, 1, generator=g))
+    qg, kg = 1.0 + 0.2 * torch.randn(2, 128, generator=g)
+    pos = torch.randint(0, 5000, (T,), generator=g, dtype=torch.int32)
+    pos[:3] = torch.tensor([0, 1, 4999], dtype=torch.int32)
+    slots = torch.randperm(T + 5, generator=g)[:T].to(torch.int32)
+    slots[::6] = -1
+    dev = [t.cuda() for t in (proj, qg, kg, pos, slots)]
+    planes = torch.full((kv * T * 512 + 8,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    turn = torch.full((T + 1, 128), float("nan"), device="cuda")
+    kc, vc = (torch.full((T + 5, kv * 128), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    base, eps = 3000.0, 1e-5
+    chk(lib, lib.b2k_heads_finish_planes(ptr(dev[0]), width + 8, heads, rot, base, factor, int(values), eps, ptr(dev[1]) if gains else None, ptr(dev[2]) if gains else None, ptr(dev[3]),
+                                         ptr(dev[4]), ptr(planes), ptr(turn) if values else None, ptr(kc), ptr(vc), T, cuda_stream_ptr()))
+    torch.cuda.synchronize()
+
+    def turned(x, dims, f):   # [T][heads][128]; pairs (m, m + dims / 2)
+        m = torch.arange(dims // 2, dtype=torch.float64)
+        ang = pos.double()[:, None] * base ** (-2.0 * m / dims) * f
+        c, s = torch.cos(ang)[:, None], torch.sin(ang)[:, None]
+        a, b = x[..., :dims // 2], x[..., dims // 2:dims]
+        return torch.cat([a * c - b * s, b * c + a * s, x[..., dims:]], -1), torch.cat([torch.cos(ang), torch.sin(ang)], 1)
+
+    x = proj[:, :width].double().view(T, -1, 128)
+    q, k, v = x[:, :heads], x[:, heads:heads + kv], x[:, heads + kv:]
+    norm = lambda y, w: y / torch.sqrt((y * y).mean(-1, keepdim=True) + eps) * w.double() if gains else y
+    q, k = norm(q, qg), norm(k, kg)
+    inv = 1.0 / factor if factor > 0 else 1.0
+    if rot:
+        q, k = turned(q, rot, inv)[0], turned(k, rot, inv)[0]
+    near = lambda got, ref, bits: ((got - ref).abs() <= 2.0 ** -bits * ref.abs() + 2.0 ** -21 * ref.abs().amax(-1, keepdim=True)).all()
+    assert torch.isnan(planes[-8:]).all()
+    hi, lo = planes[:-8].view(kv, T, 2, 2, 128).cpu().double().unbind(3)
+    assert near((hi + lo).permute(1, 0, 2, 3).reshape(T, heads, 128), q, 16) and (hi.permute(1, 0, 2, 3).reshape(T, heads, 128) - q).abs().max() > 0
+    if values:
+        v, cs = turned(v, 128, 1.0)
+        assert (turn[:T].cpu().double() - cs).abs().max() <= 2.0 ** -23
+    assert torch.isnan(turn[T if values else 0:]).all()
+    seen = slots >= 0
+    rows = slots[seen].long()
+    for cache, ref in ((kc.cpu(), k), (vc.cpu(), v)):
+        assert near(cache[rows].double().view(-1, kv, 128), ref[seen], 8)
+        rest = torch.ones(T + 5, dtype=torch.bool)
+        rest[rows] = False
+        assert (cache[rest] == 7.0).all()
+
+
 @pytest.mark.parametrize("heads", [32, 16, 8])
 @pytest.mark.parametrize("before,n", [(0, 64), (0, 130), (37, 64), (101, 50), (64, 16)])
 def test_heads_premix_reach_of_a_value(lib, heads, before, n):

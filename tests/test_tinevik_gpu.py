@@ -243,7 +243,7 @@ def test_bf16_head_mixed_attention_on_tensor_cores(heads, kv, dim, vdim):
             assert at == decode_from and np.median(rel) < BF16_BAR / 3 and max(rel) < 3 * BF16_BAR, (cuts, np.median(rel), max(rel))
 
 
-@pytest.mark.parametrize("heads,kv,dim,vdim", [(32, 16, 128, 128), (24, 8, 48, 96), (20, 4, 64, 128), (16, 8, 16, 256), (12, 4, 32, 192)])
+@pytest.mark.parametrize("heads,kv,dim,vdim", [(32, 16, 128, 128), (32, 8, 128, 128), (24, 8, 48, 96), (20, 4, 64, 128), (16, 8, 16, 256), (12, 4, 32, 192)])
 @pytest.mark.parametrize("T", [33, 95])
 def test_bf16_head_mixed_attention_on_clusters(heads, kv, dim, vdim, T):
     """Sizes whose heads do not fit one CTA: clusters of eight and of four, CTAs with fewer heads than they have room for, odd blocks of sixteen dims, output
@@ -254,6 +254,48 @@ def test_bf16_head_mixed_attention_on_clusters(heads, kv, dim, vdim, T):
     toks = tokens(cfg, T, 59)
     with engine(cfg, w, f32=False) as e:
         run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), BF16_BAR, [T - 21, 18], T - 3)
+
+
+@pytest.mark.parametrize("heads", [8, 16, 32])
+@pytest.mark.parametrize("cap,rot,factor", [(25.0, (3000.0, 64, 2.0), 1.0), (None, None, 1.0), (2.0, (3000.0, 128, None), 6.0), (1e8, (3000.0, 8, 2.0), 3.0)])
+def test_bf16_mixed_scores_of_wide_heads(heads, cap, rot, factor):
+    """Heads of 128 + 128 in groups of two (attn_premix_tc.cu in prompts): rotations of no, some and all dims, low, high and no caps; a prompt in portions that start inside a unit and
+    cross a block of 128 keys, then decode steps over the rows that they left."""
+    cfg = model([(att(heads, heads // 2, 128, 128, 128 ** -0.5, rot=rot, cap=cap), None)], vocab=211, width=96)
+    w = sharpen(cfg, random_weights(cfg, seed=64), factor=factor)
+    w["l0.mix.talk"] = (torch.randn(heads, heads, generator=torch.Generator().manual_seed(65)) * heads ** -0.5).to(torch.bfloat16).float()
+    toks = tokens(cfg, 170, 66)
+    with engine(cfg, w, f32=False) as e:
+        run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), BF16_BAR, [71, 2, 66, 27], 166)
+
+
+def test_bf16_mixed_scores_in_pieces():
+    """Five prompts whose mixed scores (5 x 1024 units of 8 tokens x 128 keys) are more than the scratch holds (4096): in one call, cut between them, as each alone."""
+    cfg = model([(att(32, 16, 128, 128, 128 ** -0.5, rot=(3000.0, 64, 2.0), cap=25.0), None)], vocab=211, width=96)
+    w = random_weights(cfg, seed=67)
+    prompts = [tokens(cfg, 1024, 68 + i) for i in range(5)]
+    at = [0, 63, 500, 1023]
+    with engine(cfg, w, f32=False, max_model_len=1040, num_blocks=340, max_seqs=5, max_batch_tokens=5120) as e:
+        sids = [e.seq_create(1024) for _ in prompts]
+        all_of, _ = e.prefill_logits(sids, prompts, [1024 * i + r for i in range(5) for r in at])
+        for s in sids:
+            e.seq_free(s)
+        for i, p in enumerate(prompts):
+            s = e.seq_create(1024)
+            one, _ = e.prefill_logits([s], [p], at)
+            e.seq_free(s)
+            assert (one == all_of[4 * i:4 * i + 4]).all(), (i, np.abs(one - all_of[4 * i:4 * i + 4]).max())
+    ref = ref_logits(cfg, w, prompts[0][:64])
+    assert err(all_of[:2], ref[[0, 63]]) < BF16_BAR
+
+
+def test_bf16_mixed_scores_of_an_engine_for_long_contexts():
+    """Where a tile of the longest context does not fit the scratch, prompts take the clusters' kernel."""
+    cfg = model([(att(32, 16, 128, 128, 128 ** -0.5, rot=(3000.0, 64, 2.0), cap=25.0), None)], vocab=211, width=96)
+    w = random_weights(cfg, seed=69)
+    toks = tokens(cfg, 95, 70)
+    with engine(cfg, w, f32=False, max_model_len=65536) as e:
+        run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), BF16_BAR, [60, 30], 90)
 
 
 def test_too_little_memory_for_the_mixed_scores():
