@@ -110,6 +110,7 @@ SIGNATURES = {
     "b2k_linear_split3": (_I, [_P, _P, _P, _P, _I, _I, _I, _I, _P]),
     "b2k_linear_split3_wide": (_I, [_P, _P, _P, C.c_size_t, _P, C.c_size_t, _P, _I, _I, _I, _P]),
     "b2k_heads_premix": (_I, [_P, _P, _P, C.c_int64, _I, C.c_float, C.c_float, _P, _P, _P, _I, _I, _P, _P, _I, _P, _I, _P, C.c_size_t, _P]),
+    "b2k_heads_premix_pays": (_I, [_I, _P, _I, C.c_size_t]),
     "b2k_heads_finish_planes": (_I, [_P, _I, _I, _I, C.c_float, C.c_float, _I, C.c_float, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P]),
     "b2k_heads_postmix": (_I, [_P, _P, _P, _I, _I, _I, _I, C.c_float, C.c_float, _I, _I, _P, _I, _I, _P, _I, _P, _P, _I, _P, _P]),
     "b2k_latent_finish": (_I, [_P, _I, _I, _I, _I, _I, _I, C.c_float, C.c_float, _I, _P, _P, _P, _P, _P, _P, _I, _P]),

@@ -560,14 +560,49 @@ bool heads_premix_tc_ok(const HeadsGeom& g, int block_size) {
   return (g.heads == 8 || g.heads == 16 || g.heads == 32) && g.kv_heads * 2 == g.heads && g.dim == 128 && g.vdim == 128 && g.window <= 0 && g.rot_dims % 8 == 0 && block_size > 0 && block_size % 16 == 0;
 }
 
-// Room for the units of a whole call, at most 512 MB (4 096 units of 32 heads); 0 where one tile of the longest context would not fit that.  4 x 1024 tokens of 32 heads, 2 304 units: in
-// 192 MB 68 us more than with room for all (two launches of each kernel, and their last waves).
+// Room for the units of a whole call, at most 512 MB (4 096 units of 32 heads).  4 x 1024 tokens of 32 heads, 2 304 units: in 192 MB 68 us more than with room for all (two launches of each
+// kernel, and their last waves).
 size_t heads_premix_tc_scratch_floats(const HeadsGeom& g, int max_tokens, int max_context) {
   const int qb = g.heads == 32 ? 8 : 16;
   const size_t unit = (size_t)g.heads * qb * PT_KEYS, blocks = ((size_t)max_context + PT_KEYS - 1) / PT_KEYS + 1;
   const size_t most = (size_t)128 * 1024 * 1024 / unit, tile = 64 / qb * blocks;
-  if (tile > most) return 0;
   return std::min(most, std::max(tile, ((size_t)max_tokens / qb + 64) * blocks)) * unit;
+}
+
+// A call takes this form where all of its tiles fit the scratch and where it is the faster one.  Behind long contexts the scratch holds few tiles' scores: a launch of premix_values then is a
+// CTA per tile and key/value head, 68 ns a key of its longest context whatever else the chip could do, and the next launch waits for it.  The kernels of attn_heads.cu walk a context with
+// a CTA (a cluster) per sixteen queries, slower but all of them at the same time.  ms a call of one layer, theirs / this: 32 heads, 64 tokens behind 60 000: 16.8 / 5.1, 384: 26.7 / 27.1,
+// 3000: 158 / 215; 3000 behind 16 000: 45.0 / 24.7; 16 heads, 512 behind 60 000: 18.4 / 17.2, 3000: 37.2 / 105, 3000 behind 16 000: 10.8 / 10.5; 8 heads, 768 behind 32 000: 5.4 / 4.8, 1024:
+// 5.5 / 7.1.  The estimates pick the faster form, to 3 %, at all of 270 points (64 - 4096 tokens behind 1000 - 60 000).
+bool heads_premix_tc_pays(const HeadsGeom& g, const PrefillTile* tiles_host, int ntiles, size_t scratch_floats) {
+  const int qb = g.heads == 32 ? 8 : 16;
+  const long cap = (long)(scratch_floats / ((size_t)g.heads * qb * PT_KEYS));
+  const double unit_ns = g.heads == 32 ? 92 : g.heads == 16 ? 75 : 30;        // of premix_scores, the chip full
+  const double chain_ns = g.heads == 32 ? 420 : g.heads == 16 ? 306 : 162;   // a key, of a walk over a context there
+  const long walks = g.heads == 32 ? 32 : 148;                                // at the same time
+  double here = 0, keys_sum = 0;
+  long units = 0, longest = 0, launch_longest = 0, groups = 0;
+  int n = 0;
+  for (int t = 0; t < ntiles; ++t) {
+    const PrefillTile& tl = tiles_host[t];
+    const long u = pt_units(tl, qb), keys = (long)tl.q_pos0 + tl.nrows, k16 = (tl.nrows + 15) / 16;
+    if (u > cap) return false;
+    if (tl.nrows <= 0) continue;
+    if (units + u > cap || n == PT_MAX_TILES) {   // (the launches of launch_premix_tc)
+      here += 68.0 * launch_longest + unit_ns * units;
+      units = launch_longest = n = 0;
+    }
+    units += u;
+    ++n;
+    launch_longest = std::max(launch_longest, keys);
+    longest = std::max(longest, keys);
+    groups += k16;
+    keys_sum += (double)k16 * keys;
+  }
+  if (groups == 0) return true;
+  here += 68.0 * launch_longest + unit_ns * units;
+  const double there = chain_ns * std::max((double)longest, keys_sum / groups * ((groups + walks - 1) / walks));
+  return here <= there;
 }
 
 int launch_heads_premix_tc(const bf16* q_planes, const bf16* k_cache, const bf16* v_cache, int64_t cache_rows, const HeadsGeom& g, const float* talk_host, const float* turn,

@@ -177,6 +177,13 @@ extern "C" int b2k_heads_premix(const void* q_planes, const void* k_cache, const
                                 (const PrefillTile*)tiles, (const PrefillTile*)tiles_host, ntiles, (bf16*)out, T, scratch, scratch_floats, wait, (cudaStream_t)stream);
 }
 
+extern "C" int b2k_heads_premix_pays(int heads, const int32_t* tiles_host, int ntiles, size_t scratch_floats) {
+  B2_REQUIRE(tiles_host && ntiles > 0 && (heads == 8 || heads == 16 || heads == 32), "b2k_heads_premix_pays: bad arguments");
+  HeadsGeom g{};
+  g.heads = heads; g.kv_heads = heads / 2; g.dim = g.vdim = 128;
+  return heads_premix_tc_pays(g, (const PrefillTile*)tiles_host, ntiles, scratch_floats) ? 1 : 0;
+}
+
 extern "C" int b2k_heads_finish_planes(const float* proj, int ld, int heads, int rot_dims, float rot_base, float rot_factor, int rot_values, float eps, const float* q_gain,
                                        const float* k_gain, const int32_t* positions, const int32_t* slots, void* q_planes, float* turn, void* k_cache, void* v_cache, int T, void* stream) {
   B2_REQUIRE(proj && positions && slots && q_planes && k_cache && v_cache, "b2k_heads_finish_planes: null pointer");

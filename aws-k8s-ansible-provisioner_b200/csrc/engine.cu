@@ -1936,7 +1936,8 @@ int forward_mixed_list(b2_engine* e, int T, int ntiles, int nlast) {
       g.softcap = sp.softcap;
       char* kc = e->regions[R.k_region].base;
       char* vc = e->regions[R.v_region].base;
-      const bool tc = tiles != nullptr && sp.score_mix && !L.talk_host.empty() && e->l_premix != nullptr && heads_premix_tc_ok(g, c.block_size) && heads_premix_tc_scratch_floats(g, 0, c.max_model_len) > 0;
+      const bool tc = tiles != nullptr && sp.score_mix && !L.talk_host.empty() && e->l_premix != nullptr && heads_premix_tc_ok(g, c.block_size) &&
+                      heads_premix_tc_pays(g, e->h_tiles, ntiles, e->l_premix_floats);
       {
         KL k(e, B2K_ROPE_KV);
         if (k.skip()) {

@@ -467,6 +467,7 @@ size_t heads_attention_premix_scratch_floats(int max_rows, int heads, int vdim);
 // queries and the values' cosines and sines (turn [T][128], null without g.rot_values) as launch_heads_finish_planes leaves them, the mixing matrix in host memory, the tile list in both.
 bool heads_premix_tc_ok(const HeadsGeom& g, int block_size);
 size_t heads_premix_tc_scratch_floats(const HeadsGeom& g, int max_tokens, int max_context);
+bool heads_premix_tc_pays(const HeadsGeom& g, const PrefillTile* tiles_host, int ntiles, size_t scratch_floats);   // this call; false too where a tile does not fit the scratch
 int launch_heads_finish_planes(const float* proj, int ld, const HeadsGeom& g, const float* q_gain, const float* k_gain, const int32_t* positions, const int32_t* slots, bf16* q_planes,
                                float* turn, bf16* k_cache, bf16* v_cache, int T, cudaStream_t s);
 int launch_heads_premix_tc(const bf16* q_planes, const bf16* k_cache, const bf16* v_cache, int64_t cache_rows, const HeadsGeom& g, const float* talk_host, const float* turn,

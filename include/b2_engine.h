@@ -462,6 +462,8 @@ int b2k_heads_postmix(const float* q, const void* k_cache, const void* v_cache, 
 int b2k_heads_premix(const void* q_planes, const void* k_cache, const void* v_cache, int64_t cache_rows, int heads, float scale, float softcap, const float* talk_host, const float* turn,
                      const int32_t* block_table, int bt_stride, int block_size, const int32_t* tiles, const int32_t* tiles_host, int ntiles, void* out, int T, float* scratch,
                      size_t scratch_floats, void* stream);
+/* 1: a call with these tiles (host memory) takes it, given a scratch of that size; 0: the kernels of csrc/attn_heads.cu. */
+int b2k_heads_premix_pays(int heads, const int32_t* tiles_host, int ntiles, size_t scratch_floats);
 /* What stands in front of it: proj [T][ld] fp32 = queries | keys | values, heads of 128, two query heads per key/value head.  Queries and keys over their root mean square times the gain
  * (null: as they are), pairs (m, m + rot_dims / 2) of the first rot_dims turned by position * rot_base^(-2 m / rot_dims) / rot_factor; with rot_values the values' pairs (m, m + 64) by
  * position * rot_base^(-2 m / 128), cosines and sines in turn.  Keys and values go to the cache rows slots[t] (none below 0). */

@@ -289,13 +289,30 @@ def test_bf16_mixed_scores_in_pieces():
     assert err(all_of[:2], ref[[0, 63]]) < BF16_BAR
 
 
-def test_bf16_mixed_scores_of_an_engine_for_long_contexts():
-    """Where a tile of the longest context does not fit the scratch, prompts take the clusters' kernel."""
+def test_bf16_mixed_scores_behind_a_long_context():
+    """An engine for contexts whose tiles do not fit the scratch: short prompts as in an engine for short ones, bit for bit; a call of many tokens behind 40 000, which the clusters'
+    kernel takes, against the same tokens in portions of 128, which go through the scratch."""
     cfg = model([(att(32, 16, 128, 128, 128 ** -0.5, rot=(3000.0, 64, 2.0), cap=25.0), None)], vocab=211, width=96)
     w = random_weights(cfg, seed=69)
-    toks = tokens(cfg, 95, 70)
-    with engine(cfg, w, f32=False, max_model_len=65536) as e:
-        run_schedule(e, cfg, toks, ref_logits(cfg, w, toks), BF16_BAR, [60, 30], 90)
+    toks = tokens(cfg, 40000 + 1664, 70)
+    rows = [0, 127, 128, 1000, 1663]
+    with engine(cfg, w, f32=False) as e:
+        short, _ = e.prefill_logits([e.seq_create(95)], [toks[:95]], list(range(95)))
+    with engine(cfg, w, f32=False, max_model_len=100000, num_blocks=2700, max_batch_tokens=4096) as e:
+        s = e.seq_create(95)
+        got, _ = e.prefill_logits([s], [toks[:95]], list(range(95)))
+        e.seq_free(s)
+        assert (got == short).all()
+        s = e.seq_create(len(toks))
+        for at in range(0, 40000, 4000):
+            e.prefill([s], [toks[at:at + 4000]])
+        whole, _ = e.prefill_logits([s], [toks[40000:]], rows)
+        e.seq_truncate(s, 40000)
+        for at in range(0, 1664, 128):
+            inside = [r - at for r in rows if at <= r < at + 128]
+            part, _ = e.prefill_logits([s], [toks[40000 + at:40000 + at + 128]], inside)
+            for r, x in zip(inside, part):
+                assert err(x, whole[rows.index(at + r)]) < BF16_BAR / 3, at + r
 
 
 def test_too_little_memory_for_the_mixed_scores():

@@ -5,6 +5,8 @@ import ctypes as C
 import json
 import math
 
+import numpy as np
+import pytest
 import torch
 
 from oracle import tinevik_oracle as O
@@ -207,3 +209,28 @@ def test_whole_model_shapes_and_borrowed_tensors():
     short, _ = O.forward(cfg, w, toks[:6])
     assert torch.allclose(short, logits[:6], atol=1e-5)          # causal throughout
     assert O.greedy(cfg, w, toks[:4], 3)[0] == int(torch.argmax(O.forward(cfg, w, toks[:4])[0][-1]))
+
+
+@pytest.mark.parametrize("heads,before,tokens,this_form", [
+    (32, 0, 1, True), (8, 0, 40, True), (16, 0, 4096, True), (32, 8000, 4096, True), (32, 16000, 3000, True), (32, 32000, 1024, True), (32, 32000, 2048, False), (32, 60000, 64, True),
+    (32, 60000, 256, True), (32, 60000, 768, False), (32, 60000, 3000, False), (16, 16000, 1024, True), (16, 16000, 2048, False), (16, 32000, 512, True), (16, 32000, 1024, False),
+    (16, 60000, 256, True), (16, 60000, 768, False), (8, 16000, 1536, True), (8, 16000, 2048, False), (8, 32000, 768, True), (8, 32000, 1024, False), (8, 60000, 512, True),
+    (8, 60000, 3000, False)])
+def test_mixed_scores_take_the_faster_form(lib, heads, before, tokens, this_form):
+    """Measured points (one layer, us a call in both forms) on both sides of the line; an empty tile and a batch of short prompts change nothing."""
+    tiles = [(i, before + i, min(64, tokens - i), 0) for i in range(0, tokens, 64)]
+    room = 128 << 20
+    call = lambda tiles, room=room: lib.b2k_heads_premix_pays(heads, np.array(tiles, dtype=np.int32).ctypes.data_as(C.c_void_p), len(tiles), room)
+    assert call(tiles) == int(this_form)
+    assert call([(0, 0, 0, 0)] + tiles + [(0, before + tokens, 0, 0)]) == int(this_form)
+    short = [(0, 0, 64, i) for i in range(200)]
+    assert call(short) == 1
+    largest = max(-(-n // (8 if heads == 32 else 16)) * ((p + n - 1) // 128 + 1) for _, p, n, _ in tiles) * heads * (8 if heads == 32 else 16) * 128
+    assert call(tiles, largest - 1) == 0 and call([(0, 0, 64, 0)], 0) == 0     # a tile that does not fit
+
+
+def test_mixed_scores_of_tiles_beyond_the_scratch(lib):
+    """A scratch holds 4 096 units of 32 heads: a tile of 64 queries up to position 65 535, and none behind it."""
+    room = 128 << 20
+    call = lambda first: lib.b2k_heads_premix_pays(32, np.array([(0, first, 64, 0)], dtype=np.int32).ctypes.data_as(C.c_void_p), 1, room)
+    assert call(65535 - 63) == 1 and call(65536 - 63) == 0
