@@ -6251,7 +6251,14 @@ extern "C" int b2_get_logits(b2_engine* e, int32_t nseq, float* out_logits) {
 
 extern "C" int b2_host_alloc(size_t bytes, void** out) {
   B2_REQUIRE(bytes > 0 && out, "b2_host_alloc: bad arguments");
-  B2_CUDA_OK(cudaHostAlloc(out, bytes, cudaHostAllocPortable));
+  *out = nullptr;
+  const cudaError_t rc = cudaHostAlloc(out, bytes, cudaHostAllocPortable);
+  if (rc != cudaSuccess) {   // (the caller may go on without: nothing of it is left for who asks for the thread's last error)
+    cudaGetLastError();
+    *out = nullptr;
+    b2_set_error("b2_host_alloc: %zu bytes: %s", bytes, cudaGetErrorString(rc));
+    return -12;
+  }
   return 0;
 }
 extern "C" void b2_host_free(void* p) {

@@ -3,6 +3,7 @@ the oracle (HF transformers Qwen3 on CPU and its pinned restatement), on identic
 inputs.  Tolerances: greedy token ids identical (tie-aware: a mismatch is only
 tolerated where the oracle's own top-1/top-2 logit gap is within bf16 noise), logits and per-layer
 hidden states within 1e-2 relative."""
+import ctypes as C
 import importlib
 import json
 import os
@@ -595,6 +596,23 @@ def test_logits_of_few_and_many_rows(P, nseq):
     assert (one[0] == full[0]).all()
     assert (eng.get_logits(nseq) == full).all()
     eng.close()
+
+
+def test_page_locked_memory(P, tiny):
+    """b2_host_alloc: too much is refused and leaves nothing behind; logits that are read into such a block are those of get_logits."""
+    _, sd = tiny
+    e = make_engine(P, QWEN3_TINY, sd, max_model_len=64, num_blocks=16, max_seqs=2, max_batch_tokens=64)
+    e.set_debug(logits=True)
+    p = C.c_void_p(1)
+    assert e.lib.b2_host_alloc(1 << 55, C.byref(p)) == -12 and p.value is None and e.lib.b2_host_alloc(0, C.byref(p)) != 0
+    e.prefill([e.seq_create(40)], [[3 + i for i in range(20)]])
+    n = QWEN3_TINY.vocab
+    assert e.lib.b2_host_alloc(4 * n, C.byref(p)) == 0
+    assert e.lib.b2_get_logits(e.h, 1, C.cast(p, C.POINTER(C.c_float))) == 0
+    assert (np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_float)), (n,)) == e.get_logits(1)[0]).all()
+    e.lib.b2_host_free(p)
+    e.lib.b2_host_free(None)
+    e.close()
 
 
 def test_a_copy_that_was_started_from_a_result_is_not_overtaken(P):
