@@ -63,9 +63,6 @@ __device__ __forceinline__ void pair_cos_sin(int pos, int i, int dims, float bas
   *s = (float)sd;
 }
 
-// A pair turned by its angle, with the products that go unrounded into the sums named: left to the compiler, they differ from kernel to kernel.
-__device__ __forceinline__ float2 turned_pair(float u, float v, float c, float s) { return make_float2(__fmaf_rn(u, c, -__fmul_rn(v, s)), __fmaf_rn(u, s, __fmul_rn(v, c))); }
-
 constexpr int LF_REG = 8;   // numbers of a latent in a thread: kv_rank <= 1024, as everywhere
 template <typename TX, typename TC>
 __global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int ld, LatentGeom g, int has_kv,
@@ -100,9 +97,8 @@ __global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int
     const bool has_v = 2 * p + 1 < g.rot_dim;
     const float u = src[0], v = has_v ? src[1] : 0.f;
     if (p < half && has_v) {
-      const float2 y = turned_pair(u, v, cs[p], cs[half + p]);
-      dst[0] = y.x;
-      dst[1] = y.y;
+      dst[0] = u * cs[p] - v * cs[half + p];
+      dst[1] = v * cs[p] + u * cs[half + p];
     } else {
       dst[0] = u;
       if (has_v) dst[1] = v;
@@ -129,15 +125,18 @@ __global__ void __launch_bounds__(128) latent_finish_kernel(const float* qd, int
     const float u = kr[2 * p], v = has_v ? kr[2 * p + 1] : 0.f;
     TC* dst = crow + g.kv_rank + 2 * p;
     if (p < half && has_v) {
-      const float2 y = turned_pair(u, v, cs[p], cs[half + p]);
-      stf(dst, y.x);
-      stf(dst + 1, y.y);
+      stf(dst, u * cs[p] - v * cs[half + p]);
+      stf(dst + 1, v * cs[p] + u * cs[half + p]);
     } else {
       stf(dst, u);
       if (has_v) stf(dst + 1, v);
     }
   }
 }
+
+// A pair turned by its angle as the kernel above turns it: the compiler lets one product of each sum go unrounded into it, the second number's another one for a query than for a key.
+__device__ __forceinline__ float2 turned_query(float u, float v, float c, float s) { return make_float2(__fmaf_rn(u, c, -__fmul_rn(v, s)), __fmaf_rn(u, s, __fmul_rn(v, c))); }
+__device__ __forceinline__ float2 turned_key(float u, float v, float c, float s) { return make_float2(__fmaf_rn(u, c, -__fmul_rn(v, s)), __fmaf_rn(v, c, __fmul_rn(u, s))); }
 
 // The same four numbers at a time, a warp a head: head widths, the latent's width and the rows in multiples of four, bases on 16-byte boundaries, a bf16 cache.  Bound by memory; the form
 // above divides to find each number's head and moves four bytes at a time.  24 decode steps of four sequences and their prompts, two layers: 3134 -> 3040 us.  Sums and
@@ -162,14 +161,14 @@ __global__ void __launch_bounds__(256) latent_finish4_kernel(const float* qd, in
     for (int c = lane; c < g.dim / 4; c += 32)
       reinterpret_cast<uint2*>(q_nope + ((size_t)t * g.heads + a) * g.dim)[c] = packed(reinterpret_cast<const float4*>(row + a * hw)[c]);
   __syncthreads();
-  auto turned = [&](float4 y, int c) {   // pairs 2 c and 2 c + 1 of a rotated piece: those below rot_dims turn, the rest passes
+  auto turned = [&](float4 y, int c, auto pair) {   // pairs 2 c and 2 c + 1 of a rotated piece: those below rot_dims turn, the rest passes
     if (2 * c < half) {
-      const float2 z = turned_pair(y.x, y.y, cs[2 * c], cs[half + 2 * c]);
+      const float2 z = pair(y.x, y.y, cs[2 * c], cs[half + 2 * c]);
       y.x = z.x;
       y.y = z.y;
     }
     if (2 * c + 1 < half) {
-      const float2 z = turned_pair(y.z, y.w, cs[2 * c + 1], cs[half + 2 * c + 1]);
+      const float2 z = pair(y.z, y.w, cs[2 * c + 1], cs[half + 2 * c + 1]);
       y.z = z.x;
       y.w = z.y;
     }
@@ -178,7 +177,7 @@ __global__ void __launch_bounds__(256) latent_finish4_kernel(const float* qd, in
   const int rq = g.rot_dim / 4;
   for (int i = tid; i < g.heads * rq; i += 256) {
     const int a = i / rq, c = i - a * rq;
-    reinterpret_cast<float4*>(q_rot + (size_t)t * g.heads * g.rot_dim)[i] = turned(reinterpret_cast<const float4*>(row + a * hw + g.dim)[c], c);
+    reinterpret_cast<float4*>(q_rot + (size_t)t * g.heads * g.rot_dim)[i] = turned(reinterpret_cast<const float4*>(row + a * hw + g.dim)[c], c, turned_query);
   }
   if (slot < 0) return;
   float ss[4] = {0.f, 0.f, 0.f, 0.f};   // the form above has 128 threads: what its thread 32 q + lane sums, every warp here for itself (zeros behind the latent)
@@ -196,7 +195,7 @@ __global__ void __launch_bounds__(256) latent_finish4_kernel(const float* qd, in
     const float4 w = reinterpret_cast<const float4*>(latent_gain)[tid];
     reinterpret_cast<uint2*>(crow)[tid] = packed(make_float4(lv.x * r * w.x, lv.y * r * w.y, lv.z * r * w.z, lv.w * r * w.w));
   }
-  for (int c = tid; c < rq; c += 256) reinterpret_cast<uint2*>(crow + g.kv_rank)[c] = packed(turned(lat[g.kv_rank / 4 + c], c));
+  for (int c = tid; c < rq; c += 256) reinterpret_cast<uint2*>(crow + g.kv_rank)[c] = packed(turned(lat[g.kv_rank / 4 + c], c, turned_key));
 }
 
 // What follows a fused projection whose output holds a query latent and a key/value latent (proj [T][ld] fp32, the query latent of
