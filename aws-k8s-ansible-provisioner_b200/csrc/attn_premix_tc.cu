@@ -556,6 +556,9 @@ int launch_premix_tc(const bf16* q_planes, const bf16* k_cache, const bf16* v_ca
 
 }  // namespace
 
+// Sizes: a mix thread holds heads x QB / 4 running sums (64 registers' worth at 16 and 32 heads, beside the scores of two key/value heads) and the matrix's entries as operands at fixed
+// places, so a head count is a kernel of its own; heads are swept in fours; a score's columns are laid out for two heads of a key/value head, its operand rows for 128 dims, and the values'
+// turn back pairs d with d + 64.  Others keep attn_heads.cu.  Sixteen rows of a page are one copy of K: pages in multiples of that.
 bool heads_premix_tc_ok(const HeadsGeom& g, int block_size) {
   return (g.heads == 8 || g.heads == 16 || g.heads == 32) && g.kv_heads * 2 == g.heads && g.dim == 128 && g.vdim == 128 && g.window <= 0 && g.rot_dims % 8 == 0 && block_size > 0 && block_size % 16 == 0;
 }

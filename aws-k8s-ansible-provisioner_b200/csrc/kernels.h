@@ -379,7 +379,6 @@ int launch_streams_sum(const float* h, int n, float* out, int T, int W, cudaStre
 // portion's last row.
 int launch_token_shift(const void* x, int x_f32, const float* mu, void* ring, void* out, int T, int W, const int32_t* row_seq, const int32_t* row_first,
                        const int32_t* row_end, const int32_t* positions, const int32_t* slots, cudaStream_t s);
-// act[i] = softplus(p) z^2 + z / 2 for z > 0, (1/2 + softplus(q)) (exp(z) - 1 - z) + z / 2 otherwise; pq (device) = p, q
 // a(z) = softplus(p) z^2 + z / 2 for z > 0 and (1/2 + softplus(q)) (exp(z) - 1 - z) + z / 2 otherwise
 struct XieluCoef { float ap, an; };
 __device__ __forceinline__ XieluCoef xielu_coef(const float* pq) {
@@ -387,6 +386,7 @@ __device__ __forceinline__ XieluCoef xielu_coef(const float* pq) {
   return XieluCoef{softplus(pq[0]), 0.5f + softplus(pq[1])};
 }
 __device__ __forceinline__ float xielu(const XieluCoef& c, float v) { return v > 0.f ? fmaf(c.ap * v, v, 0.5f * v) : fmaf(c.an, expm1f(v) - v, 0.5f * v); }
+// act[i] = a(z[i]); pq (device) = p, q
 int launch_xielu(const float* z, const float* pq, void* act, int act_f32, size_t n, cudaStream_t s);
 // out[t * out_ld + i] = scale * a[t][i] * sigmoid(gate[t * gate_ld + i]), a fp32 (or bf16: a_bf16) [T][N], out fp32 or bf16 (out_ld 0 = N)
 int launch_sigmoid_gate(const void* a, const float* gate, int gate_ld, void* out, int out_f32, int T, int N, cudaStream_t s, int a_bf16 = 0,
